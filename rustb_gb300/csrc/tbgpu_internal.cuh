@@ -278,6 +278,10 @@ int fourier_mixed_packed(ModelDev& m, cudaStream_t st, bool* packed);
 size_t eig_workspace_bytes(int N, int64_t batch, int precision);
 int eig_batched(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, void* work,
                 size_t work_bytes, int* status_d);
+// The FP64 solver behind it (eig64.cu): A destroyed, U may be null, nothing
+// allocated; timed = false launches the kernels without event records.
+bool eig64_fits(int N);
+int eig64(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* status_d, bool timed = true);
 
 // Spin-current dressing J = 1/2 {S, V} (in place through scratch).
 int spin_dress(cudaStream_t st, int N, int64_t norb, int64_t batch, int spin, zc* V, int64_t ldV,
