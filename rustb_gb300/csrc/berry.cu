@@ -110,6 +110,45 @@ __global__ void __launch_bounds__(256) zgemm_small_kernel(int N, int64_t batch, 
     }
 }
 
+// B_c = U^H (V_c U) written over V_c for both components, one CTA per matrix
+// with U, V_c and V_c U in shared memory, one output element per thread at a
+// time.  The FP64 pipe is the bound (two warp FMAs hold it longer than the two
+// shared loads they need), so nothing is gained by register tiles and the only
+// loss is the last round of threads (fit_threads): 16 N^3 FMA run without
+// padding, where 64 x 64 tiles did 7.4 times the work at 26 bands (8.18 -> 1.15
+// ms per 2304 matrices) and 4.5 times at 33 (7.68 -> 1.73 ms per 1681).
+constexpr int kRotSmemMaxN = 64;  // 3 N^2 elements fit one SM
+__global__ void __launch_bounds__(256) rotate_smem_kernel(int N, int64_t batch, const zc* __restrict__ U,
+                                                          zc* __restrict__ V, int64_t ldV, int64_t sComp) {
+    extern __shared__ __align__(16) unsigned char rot_smem[];
+    const int NN = N * N;
+    zc* X = reinterpret_cast<zc*>(rot_smem);
+    zc* A = X + NN;
+    zc* W = A + NN;
+    for (int64_t b = blockIdx.x; b < batch; b += gridDim.x) {
+        for (int e = threadIdx.x; e < NN; e += blockDim.x) X[e] = U[b * NN + e];
+        for (int c = 0; c < 2; ++c) {
+            zc* Vc = V + b * ldV + c * sComp;
+            for (int e = threadIdx.x; e < NN; e += blockDim.x) A[e] = Vc[e];
+            __syncthreads();
+            for (int e = threadIdx.x; e < NN; e += blockDim.x) {
+                const int i = e / N, j = e - i * N;
+                zc acc = mk(0.0, 0.0);
+                for (int l = 0; l < N; ++l) fma_cx(acc, A[i * N + l], X[l * N + j]);
+                W[e] = acc;
+            }
+            __syncthreads();
+            for (int e = threadIdx.x; e < NN; e += blockDim.x) {
+                const int i = e / N, j = e - i * N;
+                zc acc = mk(0.0, 0.0);
+                for (int l = 0; l < N; ++l) fma_cjx(acc, X[l * N + i], W[l * N + j]);
+                Vc[e] = acc;
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // Omega_n = sum_{m != n} -2 Im(Bx[n,m] By[m,n]) / ((E_n - E_m)^2 + eta^2), one warp per row n.
 // With MET, also the quantum metric g_n = sum_{m != n} Re(Bx[n,m] By[m,n]) / ((E_n - E_m)^2 + eta^2)
 // (src/quantum_geometry.rs:160-187: the real part of the same tensor).
@@ -340,6 +379,13 @@ static int launch_berry(cudaStream_t st, int N, int64_t batch, const zc* Bx, con
     return TBG_OK;
 }
 
+// Threads (a multiple of 32, at most 256) whose rounds over n items leave the
+// fewest idle.
+int fit_threads(int n) {
+    const int rounds = (n + 255) / 256;
+    return ((n + rounds - 1) / rounds + 31) & ~31;
+}
+
 // Bx = U^H (Vx U), By = U^H (Vy U) written over Vx / Vy, then Omega (and the metric when Met is given).
 int berry_rotate(cudaStream_t st, int N, int64_t batch, const zc* U, const zc* Vx, const zc* Vy, int64_t ldV,
                  const double* E, double eta, double* Omega, zc* scratch, double* Met) {
@@ -347,6 +393,19 @@ int berry_rotate(cudaStream_t st, int N, int64_t batch, const zc* U, const zc* V
     zc* Vxm = const_cast<zc*>(Vx);
     zc* Vym = const_cast<zc*>(Vy);
     int rc;
+    if (N > kSmallMaxN && N <= kRotSmemMaxN) {
+        const size_t smem = 3 * sizeof(zc) * NN;
+        cudaError_t e = cudaFuncSetAttribute(rotate_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(3 * sizeof(zc) * kRotSmemMaxN * kRotSmemMaxN));
+        if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(rotate_smem_kernel)");
+        {
+            KTimer kt(st, "zgemm_batched_kernel", 32.0 * (double)N * N * N * batch);
+            rotate_smem_kernel<<<(unsigned)std::min<int64_t>(batch, 152LL * 64), fit_threads((int)NN), smem, st>>>(
+                N, batch, U, Vxm, ldV, Vy - Vx);
+            TBG_LAUNCHED("rotate_smem_kernel");
+        }
+        return launch_berry(st, N, batch, Vx, Vy, ldV, E, eta, Omega, Met);
+    }
     rc = zgemm_batched(st, N, batch, false, Vx, ldV, U, NN, scratch, NN);
     if (rc) return rc;
     rc = zgemm_batched(st, N, batch, true, U, NN, scratch, NN, Vxm, ldV);

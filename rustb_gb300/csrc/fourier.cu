@@ -445,6 +445,50 @@ __global__ void __launch_bounds__(256) commutator_kernel(int N, const zc* __rest
     }
 }
 
+// The same for up to kCommSmemMaxN bands, one CTA per k-point with H and A in
+// shared memory and one element of the result per thread at a time (FP64-pipe
+// bound, as rotate_smem_kernel); the Atom-gauge phases and the zeroed diagonal
+// of A (velocity.rs:646-656) are applied while it is loaded.  33 bands: the
+// term with its Fourier sums 9.2 -> 4.5 ms per 1681 k-points and two
+// projections, against 16 x 16 tiles padded to 48.
+constexpr int kCommSmemMaxN = 80;  // 2 N^2 elements within the opt-in limit
+__global__ void __launch_bounds__(256) commutator_smem_kernel(int N, int64_t nk, const zc* __restrict__ H,
+                                                              const zc* __restrict__ Alat,
+                                                              const zc* __restrict__ orbph, int gauge,
+                                                              zc* __restrict__ V, int64_t ldV) {
+    extern __shared__ __align__(16) unsigned char comm_smem[];
+    const int NN = N * N;
+    zc* sH = reinterpret_cast<zc*>(comm_smem);
+    zc* sA = sH + NN;
+    for (int64_t kk = blockIdx.x; kk < nk; kk += gridDim.x) {
+        const zc* ph = orbph + kk * N;
+        for (int e = threadIdx.x; e < NN; e += blockDim.x) {
+            sH[e] = H[kk * NN + e];
+            zc a = Alat[kk * NN + e];
+            if (gauge == TBG_GAUGE_ATOM) {
+                const int m = e / N, n = e - m * N;
+                a = (m == n) ? mk(0.0, 0.0) : a * cmul(ph[m], ph[n]);
+            }
+            sA[e] = a;
+        }
+        __syncthreads();
+        zc* Vk = V + kk * ldV;
+        for (int e = threadIdx.x; e < NN; e += blockDim.x) {
+            const int i = e / N, j = e - i * N;
+            zc ha = mk(0.0, 0.0), ah = mk(0.0, 0.0);
+            for (int l = 0; l < N; ++l) {
+                fma_cx(ha, sH[i * N + l], sA[l * N + j]);
+                fma_cx(ah, sA[i * N + l], sH[l * N + j]);
+            }
+            zc v = Vk[e];
+            v.re -= ha.im - ah.im;  // + i (HA - AH)
+            v.im += ha.re - ah.re;
+            Vk[e] = v;
+        }
+        __syncthreads();
+    }
+}
+
 // combined rmatrix table for projection p: rm_p[r][e] = sum_d w_pd rmatrix[r][d][e]
 __global__ void rmat_combine_kernel(int64_t n_rmat, int dim, int N, const double* __restrict__ w,
                                     const zc* __restrict__ rm, zc* __restrict__ out) {
@@ -1105,6 +1149,21 @@ int rmatrix_term(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k
         rc = dispatch_gemm(st, 0, nk, (int)m.n_rmat, nR, N, ph, tab, nullptr, orbph, nullptr,
                            TBG_GAUGE_LATTICE, A, NN, nullptr, 0);
         if (rc != TBG_OK) break;
+        if (N <= kCommSmemMaxN) {
+            const size_t smem = 2 * sizeof(zc) * NN;
+            cudaError_t e = cudaFuncSetAttribute(commutator_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)(2 * sizeof(zc) * kCommSmemMaxN * kCommSmemMaxN));
+            if (e != cudaSuccess) {
+                rc = cuda_error(e, "cudaFuncSetAttribute(commutator_smem_kernel)");
+                break;
+            }
+            commutator_smem_kernel<<<(unsigned)std::min<int64_t>(nk, 152LL * 64), fit_threads((int)NN), smem, st>>>(
+                N, nk, H, A, orbph, gauge, V + (int64_t)p * NN, (int64_t)nproj * NN);
+            count_launch();
+            e = cudaGetLastError();
+            if (e != cudaSuccess) rc = cuda_error(e, "commutator_smem_kernel");
+            continue;
+        }
         if (gauge == TBG_GAUGE_ATOM) {
             const int64_t t2 = nk * NN;
             rmat_gauge_kernel<<<(unsigned)std::min<int64_t>((t2 + 255) / 256, 65535 * 8), 256, 0, st>>>(

@@ -287,6 +287,9 @@ int eig64(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* s
 int spin_dress(cudaStream_t st, int N, int64_t norb, int64_t batch, int spin, zc* V, int64_t ldV,
                zc* scratch);
 
+// Threads of a CTA (a multiple of 32, at most 256) for n equal items.
+int fit_threads(int n);
+
 // Rotation into the eigenbasis + band-resolved Berry curvature:
 // Omega (batch, N) from U (batch, N, N), Vx/Vy (batch strided), E; the
 // quantum metric (batch, N) too when Met is not null.
