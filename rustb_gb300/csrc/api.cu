@@ -44,7 +44,7 @@ int cuda_error(cudaError_t e, const char* where) {
 void count_launch(int n) { g_launches += n; }
 
 int zgemm_batched(cudaStream_t st, int N, int64_t batch, bool conj_a, const zc* A, int64_t sA, const zc* B,
-                  int64_t sB, zc* C, int64_t sC);
+                  int64_t sB, zc* C, int64_t sC, int* status_d);
 int berry_from_bands(cudaStream_t st, int N, int64_t batch, const zc* Bx, const zc* By, int64_t ldB,
                      const double* E, double eta, double* Omega);
 
@@ -244,11 +244,7 @@ int check_spin(const tbg_model* m, int spin) {
     return TBG_OK;
 }
 
-int check_status(int* status_d, cudaStream_t st) {
-    int h = 0;
-    cudaError_t e = cudaMemcpyAsync(&h, status_d, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return cuda_error(e, "status readback");
+int status_error(int h) {
     // a time-out first: the kernels after it read what the aborted one left
     if (h & 2) return set_error(TBG_E_TIMEOUT, "a bounded device wait ran out in a tensor-core kernel");
     if (h & 1) return set_error(TBG_E_NOCONV, "eigensolver input contains NaN or Inf");
@@ -256,6 +252,14 @@ int check_status(int* status_d, cudaStream_t st) {
         return set_error(TBG_E_NOCONV,
                          "Wilson loop: an overlap matrix is singular (the occupied bands touch others on the loop)");
     return TBG_OK;
+}
+
+int check_status(int* status_d, cudaStream_t st) {
+    int h = 0;
+    cudaError_t e = cudaMemcpyAsync(&h, status_d, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return cuda_error(e, "status readback");
+    return status_error(h);
 }
 
 double lattice_det(const std::vector<double>& lat, int dim) {
@@ -371,7 +375,7 @@ int run_berry_chunk(Ctx& ctx, BerryJob& J, int64_t nkc, int64_t* clusters_d) {
             rc = fourier_mixed(m, ctx.st, nkc, J.k_d, J.dirs_d, J.H, J.V, P, J.fwork, J.fwork_bytes);
             if (rc) return rc;
             if (m.n_rmat > 0) {
-                rc = rmatrix_term(m, ctx.st, nkc, J.k_d, TBG_GAUGE_ATOM, 2, J.dirs_d, J.H, J.V, J.scratch);
+                rc = rmatrix_term(m, ctx.st, nkc, J.k_d, TBG_GAUGE_ATOM, 2, J.dirs_d, J.H, J.V, J.status_d);
                 if (rc) return rc;
             }
             // V is (nkc, 2, N, N); the pairs hold the components as separate blocks
@@ -381,10 +385,10 @@ int run_berry_chunk(Ctx& ctx, BerryJob& J, int64_t nkc, int64_t* clusters_d) {
         }
         return berry_tail(ctx, J, nkc, clusters_d);
     }
-    rc = fourier_direct(m, ctx.st, nkc, J.k_d, TBG_GAUGE_ATOM, 2, J.dirs_d, J.H, J.V, NN, 2 * NN);
+    rc = fourier_direct(m, ctx.st, nkc, J.k_d, TBG_GAUGE_ATOM, 2, J.dirs_d, J.H, J.V, NN, 2 * NN, J.status_d);
     if (rc) return rc;
     if (m.n_rmat > 0) {
-        rc = rmatrix_term(m, ctx.st, nkc, J.k_d, TBG_GAUGE_ATOM, 2, J.dirs_d, J.H, J.V, J.scratch);
+        rc = rmatrix_term(m, ctx.st, nkc, J.k_d, TBG_GAUGE_ATOM, 2, J.dirs_d, J.H, J.V, J.status_d);
         if (rc) return rc;
     }
     return berry_tail(ctx, J, nkc, clusters_d);
@@ -422,7 +426,8 @@ int berry_tail(Ctx& ctx, BerryJob& J, int64_t nkc, int64_t* clusters_d) {
     }
     rc = eig_batched(ctx.st, N, nkc, J.H, J.E, J.U, nullptr, 0, J.status_d);
     if (rc) return rc;
-    return berry_rotate(ctx.st, N, nkc, J.U, J.V, J.V + NN, 2 * NN, J.E, J.eta, J.Om, J.scratch, J.Met);
+    return berry_rotate(ctx.st, N, nkc, J.U, J.V, J.V + NN, 2 * NN, J.E, J.eta, J.Om, J.scratch, J.Met,
+                        J.status_d);
 }
 
 // FP64 band energies (ascending) on chunks of the uniform mesh, gen_kmesh
@@ -470,7 +475,7 @@ struct MeshEnergies {
         const int64_t n0 = kmesh[0], n1 = M->dim > 1 ? kmesh[1] : 1, n2 = M->dim > 2 ? kmesh[2] : 1;
         kmesh_kernel<<<blocks_for(nkc), 256, 0, ctx.st>>>(c0, nkc, M->dim, n0, n1, n2, k_d);
         TBG_LAUNCHED("kmesh_kernel");
-        int rc = fourier_direct(*M, ctx.st, nkc, k_d, TBG_GAUGE_ATOM, 0, nullptr, H, nullptr, NN, 0);
+        int rc = fourier_direct(*M, ctx.st, nkc, k_d, TBG_GAUGE_ATOM, 0, nullptr, H, nullptr, NN, 0, status_d);
         if (rc) return rc;
         return eig_batched(ctx.st, N, nkc, H, E, nullptr, nullptr, 0, status_d);
     }
@@ -620,6 +625,8 @@ int tbg_model_destroy(tbg_model* m) {
     cudaFree(M.hop_EB);
     cudaFree(M.hop_pair_d);
     cudaFree(M.pair_T);
+    cudaFree(M.oz_img);
+    cudaFree(M.oz_EB);
     M.ham = nullptr;
     delete m;
     return TBG_OK;
@@ -652,15 +659,19 @@ int tbg_gen_v_projected(const tbg_model* m, int64_t nk, const double* k, int gau
     zc* H = ctx.alloc<zc>(chunk * NN);
     zc* V = n_proj ? ctx.alloc<zc>(chunk * n_proj * NN) : nullptr;
     double* dirs_d = n_proj ? ctx.alloc<double>(n_proj * M.dim) : nullptr;
+    int* status_d = ctx.alloc<int>(1);
     if (ctx.rc) return ctx.rc;
+    TBG_CUDA(cudaMemsetAsync(status_d, 0, sizeof(int), ctx.st));
+    int status_h = 0;
     if (n_proj) TBG_CUDA(cudaMemcpyAsync(dirs_d, dirs, sizeof(double) * n_proj * M.dim, cudaMemcpyHostToDevice, ctx.st));
     for (int64_t c0 = 0; c0 < nk; c0 += chunk) {
         const int64_t nkc = std::min(chunk, nk - c0);
         TBG_CUDA(cudaMemcpyAsync(k_d, k + c0 * M.dim, sizeof(double) * nkc * M.dim, cudaMemcpyHostToDevice, ctx.st));
-        rc = fourier_direct(M, ctx.st, nkc, k_d, gauge, (int)n_proj, dirs_d, H, V, NN, n_proj * NN);
+        rc = fourier_direct(M, ctx.st, nkc, k_d, gauge, (int)n_proj, dirs_d, H, V, NN, n_proj * NN,
+                            status_d);
         if (rc) return rc;
         if (M.n_rmat > 0 && n_proj > 0) {
-            rc = rmatrix_term(M, ctx.st, nkc, k_d, gauge, (int)n_proj, dirs_d, H, V, nullptr);
+            rc = rmatrix_term(M, ctx.st, nkc, k_d, gauge, (int)n_proj, dirs_d, H, V, status_d);
             if (rc) return rc;
         }
         if (H_out)
@@ -668,9 +679,11 @@ int tbg_gen_v_projected(const tbg_model* m, int64_t nk, const double* k, int gau
         if (n_proj)
             TBG_CUDA(cudaMemcpyAsync(V_out + c0 * n_proj * NN * 2, V, sizeof(zc) * nkc * n_proj * NN,
                                      cudaMemcpyDeviceToHost, ctx.st));
+        if (c0 + nkc >= nk)
+            TBG_CUDA(cudaMemcpyAsync(&status_h, status_d, sizeof(int), cudaMemcpyDeviceToHost, ctx.st));
         if (ctx.sync("tbg_gen_v_projected")) return ctx.rc;
     }
-    return ctx.sync("tbg_gen_v_projected");
+    return status_error(status_h);
 }
 
 int tbg_gen_ham(const tbg_model* m, int64_t nk, const double* k, int gauge, double* H_out) {
@@ -709,7 +722,7 @@ static int solve_impl(const tbg_model* m, int64_t nk, const double* k, double* E
     for (int64_t c0 = 0; c0 < nk; c0 += chunk) {
         const int64_t nkc = std::min(chunk, nk - c0);
         TBG_CUDA(cudaMemcpyAsync(k_d, k + c0 * M.dim, sizeof(double) * nkc * M.dim, cudaMemcpyHostToDevice, ctx.st));
-        rc = fourier_direct(M, ctx.st, nkc, k_d, TBG_GAUGE_ATOM, 0, nullptr, H, nullptr, NN, 0);
+        rc = fourier_direct(M, ctx.st, nkc, k_d, TBG_GAUGE_ATOM, 0, nullptr, H, nullptr, NN, 0, status_d);
         if (rc) return rc;
         rc = eig_batched(ctx.st, N, nkc, H, E, U, nullptr, 0, status_d);
         if (rc) return rc;
@@ -769,7 +782,7 @@ static int solve_band_mixed(const tbg_model* m, int64_t nk, const double* k, dou
         if (tcf) {
             rc = fourier_mixed_pairs(const_cast<ModelDev&>(M), ctx.st, nkc, k_d, dirs_d, P, fwork, fwb);
         } else {
-            rc = fourier_direct(M, ctx.st, nkc, k_d, TBG_GAUGE_ATOM, 0, nullptr, H, nullptr, NN, 0);
+            rc = fourier_direct(M, ctx.st, nkc, k_d, TBG_GAUGE_ATOM, 0, nullptr, H, nullptr, NN, 0, status_d);
             if (!rc) rc = z_to_pairs(ctx.st, nkc, NN, H, NN, P);
         }
         if (rc) return rc;
@@ -1001,7 +1014,7 @@ int tbg_berry_curvature_multi(int64_t n_models, const tbg_model* const* models, 
                      ? fourier_mixed_pairs(Mi, ctx.st, g.n, kd, dirs_d, Ptmp, J.fwork, J.fwork_bytes,
                                            J.pairs + g.at * NN, nkc * NN)
                      : fourier_direct(Mi, ctx.st, g.n, kd, TBG_GAUGE_ATOM, 2, dirs_d, J.H + g.at * NN,
-                                      J.V + g.at * 2 * NN, NN, 2 * NN);
+                                      J.V + g.at * 2 * NN, NN, 2 * NN, J.status_d);
             if (rc) return rc;
         }
         // the rest once for the whole chunk
@@ -1313,7 +1326,8 @@ int tbg_wilson_loops(const tbg_model* m, int64_t n_loops, int64_t n_k, const dou
             TBG_CUDA(cudaMemcpy2DAsync(kp_d, sizeof(double) * T * dim, kv_d, sizeof(double) * n_k * dim,
                                        sizeof(double) * T * dim, nl, cudaMemcpyDeviceToDevice, ctx.st));
             const int64_t np = nl * T;
-            if ((rc = fourier_direct(M, ctx.st, np, kp_d, TBG_GAUGE_ATOM, 0, nullptr, H, nullptr, NN, 0))) return rc;
+            if ((rc = fourier_direct(M, ctx.st, np, kp_d, TBG_GAUGE_ATOM, 0, nullptr, H, nullptr, NN, 0, status_d)))
+                return rc;
             if (mixed) {
                 if ((rc = z_to_pairs(ctx.st, np, NN, H, NN, Hp))) return rc;
                 if ((rc = mixed_berry(ctx.st, N, np, Hp, nullptr, nullptr, 0.0, E, nullptr, mwork, mwb, status_d,
@@ -1399,7 +1413,7 @@ int tbg_hall_energy_cut(const tbg_model* m, const int64_t* kmesh, const double* 
         for (int64_t a0 = 0; a0 + sd < nk; a0 += J.chunk) {
             const int64_t na = std::min(J.chunk, nk - sd - a0);
             if ((rc = zgemm_batched(ctx.st, N, na, true, U_all + a0 * NN, NN, U_all + (a0 + sd) * NN, NN, J.scratch,
-                                    NN)))
+                                    NN, J.status_d)))
                 return rc;
             if ((rc = ec_abs2(ctx.st, na * NN, J.scratch, Rd))) return rc;
             TBG_CUDA(cudaMemcpy2DAsync(R_h.data() + ((size_t)a0 * dim + d) * NN, sizeof(double) * dim * NN, Rd,

@@ -16,75 +16,6 @@ namespace tbg {
 
 namespace {
 
-// C[b] = op(A[b]) * B[b] for square N x N row-major complex matrices,
-// op = identity or conjugate transpose.  64x64 output tile per CTA,
-// 4x4 outputs per thread, K staged 8 at a time.  FP64 (plain path).
-template <bool CONJ_A>
-__global__ void __launch_bounds__(256) zgemm_batched_kernel(int N, const zc* __restrict__ A, int64_t sA,
-                                                            const zc* __restrict__ B, int64_t sB,
-                                                            zc* __restrict__ C, int64_t sC) {
-    constexpr int BT = 64, KT = 8;
-    __shared__ zc tA[BT][KT + 1];
-    __shared__ zc tB[KT][BT];
-    const int64_t b = blockIdx.z;
-    const zc* Ab = A + b * sA;
-    const zc* Bb = B + b * sB;
-    zc* Cb = C + b * sC;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int row0 = blockIdx.y * BT, col0 = blockIdx.x * BT;
-    zc acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = mk(0.0, 0.0);
-    for (int l0 = 0; l0 < N; l0 += KT) {
-        for (int idx = threadIdx.x; idx < BT * KT; idx += 256) {
-            int r, l;
-            zc a = mk(0.0, 0.0);
-            if (CONJ_A) {
-                r = idx % BT;
-                l = idx / BT;
-                if (row0 + r < N && l0 + l < N) a = conj(Ab[(int64_t)(l0 + l) * N + row0 + r]);
-            } else {
-                l = idx % KT;
-                r = idx / KT;
-                if (row0 + r < N && l0 + l < N) a = Ab[(int64_t)(row0 + r) * N + l0 + l];
-            }
-            tA[r][l] = a;
-        }
-        for (int idx = threadIdx.x; idx < BT * KT; idx += 256) {
-            const int c = idx % BT, l = idx / BT;
-            zc v = mk(0.0, 0.0);
-            if (col0 + c < N && l0 + l < N) v = Bb[(int64_t)(l0 + l) * N + col0 + c];
-            tB[l][c] = v;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int l = 0; l < KT; ++l) {
-            zc a[4], bv[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = tA[ty + 16 * i][l];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) bv[j] = tB[l][tx + 16 * j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) fma_cx(acc[i][j], a[i], bv[j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = row0 + ty + 16 * i;
-        if (r >= N) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = col0 + tx + 16 * j;
-            if (c < N) Cb[(int64_t)r * N + c] = acc[i][j];
-        }
-    }
-}
-
 // Small matrices (N <= 16): one thread per output element, 256 / N^2 matrices
 // per block, operands read through L1.  C[b] = op(A[b]) B[b].
 template <bool CONJ_A>
@@ -114,10 +45,10 @@ __global__ void __launch_bounds__(256) zgemm_small_kernel(int N, int64_t batch, 
 // with U, V_c and V_c U in shared memory, one output element per thread at a
 // time.  The FP64 pipe is the bound (two warp FMAs hold it longer than the two
 // shared loads they need), so nothing is gained by register tiles and the only
-// loss is the last round of threads (fit_threads): 16 N^3 FMA run without
-// padding, where 64 x 64 tiles did 7.4 times the work at 26 bands (8.18 -> 1.15
-// ms per 2304 matrices) and 4.5 times at 33 (7.68 -> 1.73 ms per 1681).
-constexpr int kRotSmemMaxN = 64;  // 3 N^2 elements fit one SM
+// loss is the last round of threads (fit_threads): 16 N^3 FMA run without padding.
+// Above kRotSmemMaxN bands the tensor-core form is faster: 2304 matrices of 26
+// bands @R26@ against 1.15 ms, 1681 of 33 bands @R33@ against 1.73.
+constexpr int kRotSmemMaxN = 25;
 __global__ void __launch_bounds__(256) rotate_smem_kernel(int N, int64_t batch, const zc* __restrict__ U,
                                                           zc* __restrict__ V, int64_t ldV, int64_t sComp) {
     extern __shared__ __align__(16) unsigned char rot_smem[];
@@ -313,10 +244,11 @@ inline unsigned grid_for(int64_t total, int threads) {
 
 }  // namespace
 
+// C[b] = op(A[b]) B[b], op = identity or conjugate transpose, square row-major matrices.
 int zgemm_batched(cudaStream_t st, int N, int64_t batch, bool conj_a, const zc* A, int64_t sA, const zc* B,
-                  int64_t sB, zc* C, int64_t sC) {
-    KTimer kt(st, "zgemm_batched_kernel", 8.0 * (double)N * N * N * batch);
+                  int64_t sB, zc* C, int64_t sC, int* status_d) {
     if (N <= 16) {
+        KTimer kt(st, "zgemm_batched_kernel", 8.0 * (double)N * N * N * batch);
         const int per = 256 / (N * N);
         const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((batch + per - 1) / per, 152LL * 64));
         if (conj_a)
@@ -326,16 +258,14 @@ int zgemm_batched(cudaStream_t st, int N, int64_t batch, bool conj_a, const zc* 
         TBG_LAUNCHED("zgemm_small_kernel");
         return TBG_OK;
     }
-    for (int64_t b0 = 0; b0 < batch; b0 += 65535) {
-        const int64_t nb = std::min<int64_t>(65535, batch - b0);
-        dim3 grid((N + 63) / 64, (N + 63) / 64, (unsigned)nb);
-        if (conj_a)
-            zgemm_batched_kernel<true><<<grid, 256, 0, st>>>(N, A + b0 * sA, sA, B + b0 * sB, sB, C + b0 * sC, sC);
-        else
-            zgemm_batched_kernel<false><<<grid, 256, 0, st>>>(N, A + b0 * sA, sA, B + b0 * sB, sB, C + b0 * sC, sC);
-        TBG_LAUNCHED("zgemm_batched_kernel");
-    }
-    return TBG_OK;
+    int* ex = nullptr;
+    TBG_CUDA(cudaMallocAsync(&ex, sizeof(int) * 2 * batch * N, st));
+    int rc = conj_a ? oz64_col_exps(st, batch, N, N, A, N, sA, ex) : oz64_row_exps(st, batch, N, N, A, N, sA, ex);
+    if (!rc) rc = oz64_col_exps(st, batch, N, N, B, N, sB, ex + batch * N);
+    const Oz64Operand a = conj_a ? Oz64Operand{A, 1, N, sA, 1, ex} : Oz64Operand{A, N, 1, sA, 0, ex};
+    if (!rc) rc = oz64_gemm(st, batch, N, N, N, a, {B, 1, N, sB, 0, ex + batch * N}, C, N, sC, 0, status_d);
+    cudaFreeAsync(ex, st);
+    return rc;
 }
 
 int spin_dress(cudaStream_t st, int N, int64_t norb, int64_t batch, int spin, zc* V, int64_t ldV, zc* scratch) {
@@ -386,34 +316,48 @@ int fit_threads(int n) {
     return ((n + rounds - 1) / rounds + 31) & ~31;
 }
 
+// B_c = U^H (V_c U) over both components as products of exact digits on the
+// tensor cores (oz64.cu); ex holds 3 batch N line exponents.
+static int rotate_oz64(cudaStream_t st, int N, int64_t batch, const zc* U, zc* Vx, zc* Vy, int64_t ldV, zc* W, int* ex,
+                       int* status_d) {
+    const int64_t NN = (int64_t)N * N;
+    int *eu = ex, *ev = ex + batch * N, *ew = ev + batch * N;
+    int rc = oz64_col_exps(st, batch, N, N, U, N, NN, eu);
+    for (int c = 0; c < 2 && !rc; ++c) {
+        zc* V = c ? Vy : Vx;
+        if ((rc = oz64_row_exps(st, batch, N, N, V, N, ldV, ev))) break;
+        if ((rc = oz64_gemm(st, batch, N, N, N, {V, N, 1, ldV, 0, ev}, {U, 1, N, NN, 0, eu}, W, N, NN, 0, status_d)))
+            break;
+        if ((rc = oz64_col_exps(st, batch, N, N, W, N, NN, ew))) break;
+        rc = oz64_gemm(st, batch, N, N, N, {U, 1, N, NN, 1, eu}, {W, 1, N, NN, 0, ew}, V, N, ldV, 0, status_d);
+    }
+    return rc;
+}
+
 // Bx = U^H (Vx U), By = U^H (Vy U) written over Vx / Vy, then Omega (and the metric when Met is given).
 int berry_rotate(cudaStream_t st, int N, int64_t batch, const zc* U, const zc* Vx, const zc* Vy, int64_t ldV,
-                 const double* E, double eta, double* Omega, zc* scratch, double* Met) {
+                 const double* E, double eta, double* Omega, zc* scratch, double* Met, int* status_d) {
     const int64_t NN = (int64_t)N * N;
     zc* Vxm = const_cast<zc*>(Vx);
     zc* Vym = const_cast<zc*>(Vy);
-    int rc;
-    if (N > kSmallMaxN && N <= kRotSmemMaxN) {
-        const size_t smem = 3 * sizeof(zc) * NN;
-        cudaError_t e = cudaFuncSetAttribute(rotate_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)(3 * sizeof(zc) * kRotSmemMaxN * kRotSmemMaxN));
-        if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(rotate_smem_kernel)");
-        {
-            KTimer kt(st, "zgemm_batched_kernel", 32.0 * (double)N * N * N * batch);
-            rotate_smem_kernel<<<(unsigned)std::min<int64_t>(batch, 152LL * 64), fit_threads((int)NN), smem, st>>>(
-                N, batch, U, Vxm, ldV, Vy - Vx);
-            TBG_LAUNCHED("rotate_smem_kernel");
+    int rc = TBG_OK;
+    if (N <= kSmallMaxN) {
+        for (zc* V : {Vxm, Vym}) {
+            if ((rc = zgemm_batched(st, N, batch, false, V, ldV, U, NN, scratch, NN, status_d))) return rc;
+            if ((rc = zgemm_batched(st, N, batch, true, U, NN, scratch, NN, V, ldV, status_d))) return rc;
         }
-        return launch_berry(st, N, batch, Vx, Vy, ldV, E, eta, Omega, Met);
+    } else if (N <= kRotSmemMaxN) {
+        KTimer kt(st, "rotate_smem_kernel", 32.0 * (double)N * N * N * batch);
+        rotate_smem_kernel<<<(unsigned)std::min<int64_t>(batch, 152LL * 64), fit_threads((int)NN), 3 * sizeof(zc) * NN,
+                             st>>>(N, batch, U, Vxm, ldV, Vy - Vx);
+        TBG_LAUNCHED("rotate_smem_kernel");
+    } else {
+        int* ex = nullptr;
+        TBG_CUDA(cudaMallocAsync(&ex, sizeof(int) * 3 * batch * N, st));
+        rc = rotate_oz64(st, N, batch, U, Vxm, Vym, ldV, scratch, ex, status_d);
+        cudaFreeAsync(ex, st);
+        if (rc) return rc;
     }
-    rc = zgemm_batched(st, N, batch, false, Vx, ldV, U, NN, scratch, NN);
-    if (rc) return rc;
-    rc = zgemm_batched(st, N, batch, true, U, NN, scratch, NN, Vxm, ldV);
-    if (rc) return rc;
-    rc = zgemm_batched(st, N, batch, false, Vy, ldV, U, NN, scratch, NN);
-    if (rc) return rc;
-    rc = zgemm_batched(st, N, batch, true, U, NN, scratch, NN, Vym, ldV);
-    if (rc) return rc;
     return launch_berry(st, N, batch, Vx, Vy, ldV, E, eta, Omega, Met);
 }
 

@@ -65,16 +65,12 @@ constexpr int TK = 32;   // k-points per tile
 constexpr int TE = 64;   // matrix elements per tile
 constexpr int RC = 8;    // R rows per shared-memory stage
 
-// NP velocity projections (0..3).  coef: (NP, nR) = w_p . R_cart.
-// taup: (NP, N) = w_p . tau_cart (Atom gauge only).
-template <int NP>
-__global__ void __launch_bounds__(256) fourier_gemm_kernel(
-    int64_t nk, int nR, int ldph, int N, const zc* __restrict__ ph, const zc* __restrict__ hop,
-    const double* __restrict__ coef, const zc* __restrict__ orbph, const double* __restrict__ taup,
-    int gauge, zc* __restrict__ H, int64_t ldH, zc* __restrict__ V, int64_t ldV) {
+// A (nk, N^2) = sum_R ph(k, R) hop(R): the position-matrix sums of few k-points.
+__global__ void __launch_bounds__(256) fourier_gemm_kernel(int64_t nk, int nR, int ldph, int N,
+                                                           const zc* __restrict__ ph, const zc* __restrict__ hop,
+                                                           zc* __restrict__ H) {
     __shared__ zc s_hop[RC][TE];
     __shared__ zc s_ph[RC][TK];
-    __shared__ double s_coef[NP > 0 ? NP : 1][RC];
     const int tid = threadIdx.x;
     const int te = tid & 15;  // element lane: e = te + 16 j
     const int tk = tid >> 4;  // k lane: k = tk + 16 i
@@ -82,16 +78,11 @@ __global__ void __launch_bounds__(256) fourier_gemm_kernel(
     const int64_t e0 = (int64_t)blockIdx.x * TE;
     const int64_t k0 = (int64_t)blockIdx.y * TK;
 
-    zc accH[2][4];
-    zc accV[NP > 0 ? NP : 1][2][4];
+    zc acc[2][4];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            accH[i][j] = mk(0.0, 0.0);
-#pragma unroll
-            for (int p = 0; p < NP; ++p) accV[p][i][j] = mk(0.0, 0.0);
-        }
+        for (int j = 0; j < 4; ++j) acc[i][j] = mk(0.0, 0.0);
 
     for (int r0 = 0; r0 < nR; r0 += RC) {
         for (int idx = tid; idx < RC * TE; idx += 256) {
@@ -106,38 +97,25 @@ __global__ void __launch_bounds__(256) fourier_gemm_kernel(
             if (r0 + r < nR && k0 + kk < nk) u = ph[(k0 + kk) * ldph + r0 + r];
             s_ph[r][kk] = u;
         }
-        if (NP > 0 && tid < NP * RC) {
-            const int p = tid / RC, r = tid % RC;
-            s_coef[p][r] = (r0 + r < nR) ? coef[(int64_t)p * nR + r0 + r] : 0.0;
-        }
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < RC; ++r) {
             zc h[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) h[j] = s_hop[r][te + 16 * j];
-            double c[NP > 0 ? NP : 1];
-#pragma unroll
-            for (int p = 0; p < NP; ++p) c[p] = s_coef[p][r];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const zc u = s_ph[r][tk + 16 * i];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const zc t = u * h[j];
-                    accH[i][j].re += t.re;
-                    accH[i][j].im += t.im;
-#pragma unroll
-                    for (int p = 0; p < NP; ++p) {
-                        accV[p][i][j].re = fma(c[p], t.re, accV[p][i][j].re);
-                        accV[p][i][j].im = fma(c[p], t.im, accV[p][i][j].im);
-                    }
+                    acc[i][j].re += t.re;
+                    acc[i][j].im += t.im;
                 }
             }
         }
         __syncthreads();
     }
-
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const int64_t kk = k0 + tk + 16 * i;
@@ -145,24 +123,7 @@ __global__ void __launch_bounds__(256) fourier_gemm_kernel(
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int64_t e = e0 + te + 16 * j;
-            if (e >= NN) continue;
-            const int mrow = (int)(e / N), ncol = (int)(e % N);
-            const zc hl = accH[i][j];
-            zc g = mk(1.0, 0.0);
-            if (gauge == TBG_GAUGE_ATOM) g = cmul(orbph[kk * N + mrow], orbph[kk * N + ncol]);
-            if (H) H[kk * ldH + e] = hl * g;
-#pragma unroll
-            for (int p = 0; p < NP; ++p) {
-                // i * acc
-                zc v = mk(-accV[p][i][j].im, accV[p][i][j].re);
-                if (gauge == TBG_GAUGE_ATOM) {
-                    const double diff = taup[p * N + ncol] - taup[p * N + mrow];
-                    v.re -= diff * hl.im;
-                    v.im += diff * hl.re;
-                    v = v * g;
-                }
-                V[kk * ldV + p * NN + e] = v;
-            }
+            if (e < NN) H[kk * NN + e] = acc[i][j];
         }
     }
 }
@@ -191,33 +152,16 @@ __global__ void proj_coef_kernel(int nproj, int dim, const double* __restrict__ 
     }
 }
 
-template <int NP>
-int launch_gemm(cudaStream_t st, int64_t nk, int nR, int ldph, int N, const zc* ph, const zc* hop,
-                const double* coef, const zc* orbph, const double* taup, int gauge, zc* H, int64_t ldH,
-                zc* V, int64_t ldV) {
+int launch_gemm(cudaStream_t st, int64_t nk, int nR, int ldph, int N, const zc* ph, const zc* hop, zc* H) {
     const int64_t NN = (int64_t)N * N;
-    KTimer kt(st, "fourier_gemm_kernel", 8.0 * nR * (double)NN * nk * ((H ? 1 : 0) + NP));
+    KTimer kt(st, "fourier_gemm_kernel", 8.0 * nR * (double)NN * nk);
     for (int64_t kb = 0; kb < nk; kb += (int64_t)TK * 65535) {
         const int64_t nkb = std::min<int64_t>(nk - kb, (int64_t)TK * 65535);
         dim3 grid((unsigned)((NN + TE - 1) / TE), (unsigned)((nkb + TK - 1) / TK));
-        fourier_gemm_kernel<NP><<<grid, 256, 0, st>>>(nkb, nR, ldph, N, ph + kb * ldph, hop, coef,
-                                                        orbph + kb * N, taup, gauge,
-                                                        H ? H + kb * ldH : nullptr, ldH,
-                                                        V ? V + kb * ldV : nullptr, ldV);
+        fourier_gemm_kernel<<<grid, 256, 0, st>>>(nkb, nR, ldph, N, ph + kb * ldph, hop, H + kb * NN);
         TBG_LAUNCHED("fourier_gemm_kernel");
     }
     return TBG_OK;
-}
-
-int dispatch_gemm(cudaStream_t st, int np, int64_t nk, int nR, int ldph, int N, const zc* ph, const zc* hop,
-                  const double* coef, const zc* orbph, const double* taup, int gauge, zc* H, int64_t ldH,
-                  zc* V, int64_t ldV) {
-    switch (np) {
-        case 0: return launch_gemm<0>(st, nk, nR, ldph, N, ph, hop, coef, orbph, taup, gauge, H, ldH, V, ldV);
-        case 1: return launch_gemm<1>(st, nk, nR, ldph, N, ph, hop, coef, orbph, taup, gauge, H, ldH, V, ldV);
-        case 2: return launch_gemm<2>(st, nk, nR, ldph, N, ph, hop, coef, orbph, taup, gauge, H, ldH, V, ldV);
-        default: return launch_gemm<3>(st, nk, nR, ldph, N, ph, hop, coef, orbph, taup, gauge, H, ldH, V, ldV);
-    }
 }
 
 // Fourier sums from the +-R paired table (FP64; rows 2q, 2q + 1 of T are A_q,
@@ -225,8 +169,7 @@ int dispatch_gemm(cudaStream_t st, int np, int64_t nk, int nR, int ldph, int N, 
 // 2 pi k . R_q,
 //   H += c A_q + s B_q,   V_p += c_p(R_q) (c B_q - s A_q)   (c_p(R_0) = 0),
 // 8 + 2 NP FMAs per pair and element for two R (10 + 2 NP per R unpaired).
-// Same tiling and epilogue as fourier_gemm_kernel; the velocity accumulators
-// already hold V_p (no factor i).
+// The velocity accumulators already hold V_p (no factor i).
 template <int NP>
 __global__ void __launch_bounds__(256) fourier_pair_kernel(
     int64_t nk, int Kc, int N, const zc* __restrict__ cs, const zc* __restrict__ T, const int* __restrict__ pair,
@@ -391,67 +334,28 @@ int dispatch_pair(cudaStream_t st, int np, int64_t nk, int Kc, int N, const zc* 
     }
 }
 
-// Gauge transform + zeroed diagonal of the rmatrix Fourier sum (Atom gauge),
-// velocity.rs:646-656.
-__global__ void rmat_gauge_kernel(int64_t nk, int N, const zc* __restrict__ orbph, zc* __restrict__ A) {
+// i A of the rmatrix Fourier sum, with the gauge transform and the zeroed
+// diagonal of the Atom gauge (velocity.rs:646-656), in place.
+__global__ void rmat_gauge_kernel(int64_t nk, int N, int gauge, const zc* __restrict__ orbph, zc* __restrict__ A) {
     const int64_t NN = (int64_t)N * N;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < nk * NN;
          idx += (int64_t)gridDim.x * blockDim.x) {
         const int64_t kk = idx / NN;
         const int e = (int)(idx % NN), m = e / N, n = e % N;
         zc a = A[idx];
-        if (m == n) {
-            a = mk(0.0, 0.0);
-        } else {
-            a = a * cmul(orbph[kk * N + m], orbph[kk * N + n]);
-        }
-        A[idx] = a;
+        if (gauge == TBG_GAUGE_ATOM)
+            a = (m == n) ? mk(0.0, 0.0) : a * cmul(orbph[kk * N + m], orbph[kk * N + n]);
+        A[idx] = mk(-a.im, a.re);
     }
 }
 
-// V[k] += i (H A - A H) for one k per block row tile; simple tiled FP64 GEMM.
-__global__ void __launch_bounds__(256) commutator_kernel(int N, const zc* __restrict__ H, int64_t ldH,
-                                                         const zc* __restrict__ A, zc* __restrict__ V,
-                                                         int64_t ldV) {
-    const int64_t kk = blockIdx.z;
-    const zc* Hk = H + kk * ldH;
-    const zc* Ak = A + kk * (int64_t)N * N;
-    zc* Vk = V + kk * ldV;
-    __shared__ zc sH[16][17], sA[16][17], sA2[16][17], sH2[16][17];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int row = blockIdx.y * 16 + ty, col = blockIdx.x * 16 + tx;
-    zc acc = mk(0.0, 0.0);
-    for (int t0 = 0; t0 < N; t0 += 16) {
-        // (H A)[row][col] = sum_l H[row][l] A[l][col];  (A H)[row][col] = sum_l A[row][l] H[l][col]
-        sH[ty][tx] = (row < N && t0 + tx < N) ? Hk[(int64_t)row * N + t0 + tx] : mk(0.0, 0.0);
-        sA2[ty][tx] = (row < N && t0 + tx < N) ? Ak[(int64_t)row * N + t0 + tx] : mk(0.0, 0.0);
-        sA[ty][tx] = (t0 + ty < N && col < N) ? Ak[(int64_t)(t0 + ty) * N + col] : mk(0.0, 0.0);
-        sH2[ty][tx] = (t0 + ty < N && col < N) ? Hk[(int64_t)(t0 + ty) * N + col] : mk(0.0, 0.0);
-        __syncthreads();
-#pragma unroll
-        for (int l = 0; l < 16; ++l) {
-            fma_cx(acc, sH[ty][l], sA[l][tx]);
-            const zc t = sA2[ty][l] * sH2[l][tx];
-            acc.re -= t.re;
-            acc.im -= t.im;
-        }
-        __syncthreads();
-    }
-    if (row < N && col < N) {
-        zc v = Vk[(int64_t)row * N + col];
-        v.re -= acc.im;
-        v.im += acc.re;
-        Vk[(int64_t)row * N + col] = v;
-    }
-}
-
-// The same for up to kCommSmemMaxN bands, one CTA per k-point with H and A in
-// shared memory and one element of the result per thread at a time (FP64-pipe
-// bound, as rotate_smem_kernel); the Atom-gauge phases and the zeroed diagonal
-// of A (velocity.rs:646-656) are applied while it is loaded.  33 bands: the
-// term with its Fourier sums 9.2 -> 4.5 ms per 1681 k-points and two
-// projections, against 16 x 16 tiles padded to 48.
-constexpr int kCommSmemMaxN = 80;  // 2 N^2 elements within the opt-in limit
+// V[k] += i (H A - A H) for up to kCommSmemMaxN bands, one CTA per k-point with
+// H and A in shared memory and one element of the result per thread at a time
+// (FP64-pipe bound, as rotate_smem_kernel); the Atom-gauge phases and the zeroed
+// diagonal of A (velocity.rs:646-656) are applied while it is loaded.  Above, the
+// two products run on the tensor cores (oz64.cu): 33 bands, 1681 k-points, two
+// projections @COM@ ms against @COMS@ here.
+constexpr int kCommSmemMaxN = 25;
 __global__ void __launch_bounds__(256) commutator_smem_kernel(int N, int64_t nk, const zc* __restrict__ H,
                                                               const zc* __restrict__ Alat,
                                                               const zc* __restrict__ orbph, int gauge,
@@ -489,9 +393,11 @@ __global__ void __launch_bounds__(256) commutator_smem_kernel(int N, int64_t nk,
     }
 }
 
-// combined rmatrix table for projection p: rm_p[r][e] = sum_d w_pd rmatrix[r][d][e]
+// combined rmatrix table for projection p: rm_p[r][e] = sum_d w_pd rmatrix[r][d][e];
+// step 2 leaves room for i rm_p in the odd rows and fills it (the real-coefficient
+// form (cos + i sin) t = cos t + sin (i t))
 __global__ void rmat_combine_kernel(int64_t n_rmat, int dim, int N, const double* __restrict__ w,
-                                    const zc* __restrict__ rm, zc* __restrict__ out) {
+                                    const zc* __restrict__ rm, int step, zc* __restrict__ out) {
     const int64_t NN = (int64_t)N * N;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n_rmat * NN;
          idx += (int64_t)gridDim.x * blockDim.x) {
@@ -502,7 +408,8 @@ __global__ void rmat_combine_kernel(int64_t n_rmat, int dim, int N, const double
             s.re += w[d] * a.re;
             s.im += w[d] * a.im;
         }
-        out[idx] = s;
+        out[r * step * NN + e] = s;
+        if (step == 2) out[(r * 2 + 1) * NN + e] = mk(-s.im, s.re);
     }
 }
 
@@ -766,11 +673,11 @@ __global__ void pair_table_kernel(int np, const int* __restrict__ pi, const int*
 }
 
 // Real coefficients of the paired table, as complex numbers whose real and
-// imaginary parts are consecutive rows (Phi (3, nk, Kc), Kc = 1 + np): H row
-// (1, 0 | cos, sin ...), V_p rows (0, 0 | -c_p(R) sin, c_p(R) cos ...), from
+// imaginary parts are consecutive rows (Phi (1 + nproj, nk, Kc), Kc = 1 + np): H
+// row (1, 0 | cos, sin ...), V_p rows (0, 0 | -c_p(R) sin, c_p(R) cos ...), from
 //   i c_p(R) (t(R) e^{i theta} - t(-R) e^{-i theta}) = c_p(R) (B cos - A sin).
 __global__ void phases_real_kernel(int64_t nk, int dim, const double* __restrict__ k, int np,
-                                   const int* __restrict__ pair, const int* __restrict__ hamR, int nR,
+                                   const int* __restrict__ pair, const int* __restrict__ hamR, int nR, int nproj,
                                    const double* __restrict__ coef, zc* __restrict__ Phi) {
     const int Kc = np + 1;
     const int64_t total = nk * (int64_t)Kc;
@@ -778,25 +685,25 @@ __global__ void phases_real_kernel(int64_t nk, int dim, const double* __restrict
          idx += (int64_t)gridDim.x * blockDim.x) {
         const int64_t kk = idx / Kc;
         const int c = (int)(idx % Kc);
-        zc h = mk(1.0, 0.0), vx = mk(0.0, 0.0), vy = mk(0.0, 0.0);
-        if (c > 0) {
-            const int j = pair[c - 1];
-            const int* r = hamR + 3 * j;
-            const double* kv = k + kk * dim;
-            // same operation order as the reference: r0*k0 + r1*k1 + r2*k2
-            double s = (double)r[0] * kv[0];
-            if (dim > 1) s += (double)r[1] * kv[1];
-            if (dim > 2) s += (double)r[2] * kv[2];
-            double sn, cs;
-            sincos(kTwoPi * s, &sn, &cs);
-            const double c0 = coef[j], c1 = coef[nR + j];
-            h = mk(cs, sn);
-            vx = mk(-c0 * sn, c0 * cs);
-            vy = mk(-c1 * sn, c1 * cs);
+        if (c == 0) {
+            Phi[idx] = mk(1.0, 0.0);
+            for (int p = 0; p < nproj; ++p) Phi[(1 + p) * total + idx] = mk(0.0, 0.0);
+            continue;
         }
-        Phi[idx] = h;
-        Phi[total + idx] = vx;
-        Phi[2 * total + idx] = vy;
+        const int j = pair[c - 1];
+        const int* r = hamR + 3 * j;
+        const double* kv = k + kk * dim;
+        // same operation order as the reference: r0*k0 + r1*k1 + r2*k2
+        double s = (double)r[0] * kv[0];
+        if (dim > 1) s += (double)r[1] * kv[1];
+        if (dim > 2) s += (double)r[2] * kv[2];
+        double sn, cs;
+        sincos(kTwoPi * s, &sn, &cs);
+        Phi[idx] = mk(cs, sn);
+        for (int p = 0; p < nproj; ++p) {
+            const double cp = coef[(int64_t)p * nR + j];
+            Phi[(1 + p) * total + idx] = mk(-cp * sn, cp * cs);
+        }
     }
 }
 
@@ -956,7 +863,7 @@ int fourier_mixed_gemm(ModelDev& m, cudaStream_t st, int64_t nk, const double* k
                 nk, m.dim, k_d, 0, m.hamR_d, N, m.tau_d, ph3, orbph);
             const int64_t t2 = nk * (int64_t)m.hop_K;
             phases_real_kernel<<<(unsigned)std::min<int64_t>((t2 + 255) / 256, 65535 * 8), 256, 0, st>>>(
-                nk, m.dim, k_d, m.hop_np, m.hop_pair_d, m.hamR_d, nR, coef, ph3);
+                nk, m.dim, k_d, m.hop_np, m.hop_pair_d, m.hamR_d, nR, 2, coef, ph3);
         } else {
             const int64_t t1 = nk * (int64_t)(nR + N);
             phases_kernel<<<(unsigned)std::min<int64_t>((t1 + 255) / 256, 65535 * 8), 256, 0, st>>>(
@@ -1056,16 +963,156 @@ int fourier_mixed_pairs(ModelDev& m, cudaStream_t st, int64_t nk, const double* 
     return TBG_OK;
 }
 
+namespace {
+
+// Lattice-gauge sums G (1 + nproj blocks of nk N^2: H, V_p) -> H, V with the
+// orbital-position term and the gauge phases, as the epilogue of fourier_pair_kernel.
+__global__ void __launch_bounds__(256) gauge64_kernel(int64_t nk, int N, int nproj, const zc* __restrict__ G,
+                                                      const zc* __restrict__ orbph, const double* __restrict__ taup,
+                                                      int gauge, zc* __restrict__ H, int64_t ldH, zc* __restrict__ V,
+                                                      int64_t ldV) {
+    const int64_t NN = (int64_t)N * N;
+    for (int64_t kk = blockIdx.y; kk < nk; kk += gridDim.y) {
+        for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < (int)NN; e += gridDim.x * blockDim.x) {
+            const int mrow = e / N, ncol = e - mrow * N;
+            const zc hl = G[kk * NN + e];
+            zc g = mk(1.0, 0.0);
+            if (gauge == TBG_GAUGE_ATOM) g = cmul(orbph[kk * N + mrow], orbph[kk * N + ncol]);
+            if (H) H[kk * ldH + e] = gauge == TBG_GAUGE_ATOM ? hl * g : hl;
+            for (int p = 0; p < nproj; ++p) {
+                zc v = G[((1 + p) * nk + kk) * NN + e];
+                if (gauge == TBG_GAUGE_ATOM) {
+                    const double diff = taup[p * N + ncol] - taup[p * N + mrow];
+                    v.re -= diff * hl.im;
+                    v.im += diff * hl.re;
+                    v = v * g;
+                }
+                V[kk * ldV + p * NN + e] = v;
+            }
+        }
+    }
+}
+
+// The digit image of the paired table for the tensor-core form, built once per
+// model; the caller holds g_hop_mu.  Without memory for it m.oz_img stays null.
+int ensure_table_image(ModelDev& m, cudaStream_t st) {
+    if (m.oz_img || m.nonfinite) return TBG_OK;
+    const int64_t NN = (int64_t)m.nsta * m.nsta;
+    void* img = nullptr;
+    int* eb = nullptr;
+    if (cudaMalloc(&img, oz64_table_image_bytes(m.hop_K, NN)) != cudaSuccess ||
+        cudaMalloc(&eb, sizeof(int) * NN) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(img);
+        return TBG_OK;
+    }
+    int rc = oz64_table_image(st, m.hop_K, NN, m.pair_T, eb, img);
+    if (!rc) {
+        cudaError_t e = cudaStreamSynchronize(st);  // other streams use the image next
+        if (e != cudaSuccess) rc = cuda_error(e, "table image");
+    }
+    if (rc) {
+        cudaFree(img);
+        cudaFree(eb);
+        return rc;
+    }
+    m.oz_img = img;
+    m.oz_EB = eb;
+    return TBG_OK;
+}
+
+// FP64 instructions per lane of the direct sum above which the tensor-core form
+// is taken (@THR@)
+constexpr double kOzFourierWork = 2e7;
+constexpr int64_t kOzFourierBytes = 512LL << 20;  // sums held at a time
+
+// H and nproj projections on the tensor cores at FP64 accuracy (oz64.cu): the
+// real coefficients of every output (rows: H, V_0, V_1, ... per k-point) times
+// the paired table.
+int fourier_oz64(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k_d, int gauge, int nproj,
+                 const double* dirs_d, zc* H, zc* V, int64_t ldH, int64_t ldV, int* status_d) {
+    const int N = (int)m.nsta, nR = (int)m.nR, Kc = m.hop_K;
+    const int64_t NN = (int64_t)N * N;
+    int64_t sub = std::max<int64_t>(1, kOzFourierBytes / (int64_t)(sizeof(zc) * NN * (1 + nproj)));
+    sub = sub >= 128 ? sub / 128 * 128 : std::min<int64_t>(128, nk);
+    sub = std::min(sub, nk);
+    const int64_t M = sub * (1 + nproj);
+    const int npc = std::max(nproj, 1);
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off += (bytes + 255) & ~size_t(255);
+        return o;
+    };
+    const size_t o_phi = take(sizeof(zc) * M * Kc), o_orb = take(sizeof(zc) * sub * N);
+    const size_t o_coef = take(sizeof(double) * npc * nR), o_tau = take(sizeof(double) * npc * N);
+    const size_t o_ea = take(sizeof(int) * M), o_img = take(oz64_row_image_bytes(M, Kc));
+    const size_t o_g = take(sizeof(zc) * M * NN);
+    unsigned char* buf = nullptr;
+    TBG_CUDA(cudaMallocAsync(&buf, off, st));
+    zc* phi = reinterpret_cast<zc*>(buf + o_phi);
+    zc* orbph = reinterpret_cast<zc*>(buf + o_orb);
+    double* coef = reinterpret_cast<double*>(buf + o_coef);
+    double* taup = reinterpret_cast<double*>(buf + o_tau);
+    int* EA = reinterpret_cast<int*>(buf + o_ea);
+    zc* G = reinterpret_cast<zc*>(buf + o_g);
+    int rc = TBG_OK;
+    auto launched = [&](const char* what) {
+        count_launch();
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess && !rc) rc = cuda_error(e, what);
+    };
+    if (nproj > 0) {
+        const int total = nproj * (nR + N);
+        proj_coef_kernel<<<(total + 255) / 256, 256, 0, st>>>(nproj, m.dim, dirs_d, nR, m.Rcart_d, N, m.taucart_d, coef,
+                                                              taup);
+        launched("proj_coef_kernel");
+    }
+    for (int64_t k0 = 0; k0 < nk && !rc; k0 += sub) {
+        const int64_t nks = std::min(sub, nk - k0);
+        {
+            KTimer kt(st, "phases_kernel");
+            const int64_t t1 = nks * (int64_t)N, t2 = nks * (int64_t)Kc;
+            if (gauge == TBG_GAUGE_ATOM) {
+                phases_kernel<<<(unsigned)std::min<int64_t>((t1 + 255) / 256, 65535 * 8), 256, 0, st>>>(
+                    nks, m.dim, k_d + k0 * m.dim, 0, m.hamR_d, N, m.tau_d, phi, orbph);
+                launched("phases_kernel");
+            }
+            phases_real_kernel<<<(unsigned)std::min<int64_t>((t2 + 255) / 256, 65535 * 8), 256, 0, st>>>(
+                nks, m.dim, k_d + k0 * m.dim, m.hop_np, m.hop_pair_d, m.hamR_d, nR, nproj, coef, phi);
+            launched("phases_real_kernel");
+        }
+        if (!rc)
+            rc = oz64_table_product(st, nks * (1 + nproj), NN, Kc, phi, Kc, m.oz_EB, m.oz_img, G, EA, buf + o_img,
+                                    status_d);
+        if (rc) break;
+        KTimer kt(st, "gauge64_kernel");
+        const dim3 grid((unsigned)std::min<int64_t>((NN + 255) / 256, 1024), (unsigned)std::min<int64_t>(nks, 65535));
+        gauge64_kernel<<<grid, 256, 0, st>>>(nks, N, nproj, G, orbph, taup, gauge, H ? H + k0 * ldH : nullptr, ldH,
+                                             V ? V + k0 * ldV : nullptr, ldV);
+        launched("gauge64_kernel");
+    }
+    cudaFreeAsync(buf, st);
+    return rc;
+}
+
+}  // namespace
+
 int fourier_direct(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k_d, int gauge, int nproj,
-                   const double* dirs_d, zc* H, zc* V, int64_t ldH, int64_t ldV) {
+                   const double* dirs_d, zc* H, zc* V, int64_t ldH, int64_t ldV, int* status_d) {
     if (nk <= 0) return TBG_OK;
     const int N = (int)m.nsta, nR = (int)m.nR;
+    bool oz = false;
     {
         // the +-R paired table, built once per model (a cache: logically const)
         std::lock_guard<std::mutex> lk(g_hop_mu);
         int rc = ensure_pair_table(const_cast<ModelDev&>(m), st);
         if (rc) return rc;
+        oz = status_d && (double)nk * N * N * m.hop_K * (nproj > 0 ? 8 + 2 * nproj : 4) >= kOzFourierWork;
+        if (oz && (rc = ensure_table_image(const_cast<ModelDev&>(m), st))) return rc;
+        oz = oz && m.oz_img;
     }
+    if (oz) return fourier_oz64(m, st, nk, k_d, gauge, nproj, dirs_d, H, V, ldH, ldV, status_d);
     const int Kc = m.hop_K;
     zc *cs = nullptr, *orbph = nullptr;
     double *coef = nullptr, *taup = nullptr;
@@ -1112,75 +1159,78 @@ int fourier_direct(const ModelDev& m, cudaStream_t st, int64_t nk, const double*
 }
 
 int rmatrix_term(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k_d, int gauge, int nproj,
-                 const double* dirs_d, const zc* H, zc* V, zc* /*scratch*/) {
+                 const double* dirs_d, const zc* H, zc* V, int* status_d) {
     if (m.n_rmat <= 0 || nk <= 0 || nproj <= 0) return TBG_OK;
     KTimer kt(st, "rmatrix_term");
-    const int N = (int)m.nsta, nR = (int)m.nR;
+    const int N = (int)m.nsta, nR = (int)m.nR, nr = (int)m.n_rmat;
     const int64_t NN = (int64_t)N * N;
-    zc *ph = nullptr, *orbph = nullptr, *tab = nullptr, *A = nullptr;
-    TBG_CUDA(cudaMallocAsync(&ph, sizeof(zc) * nk * nR, st));
-    TBG_CUDA(cudaMallocAsync(&orbph, sizeof(zc) * nk * N, st));
-    TBG_CUDA(cudaMallocAsync(&tab, sizeof(zc) * m.n_rmat * NN, st));
-    TBG_CUDA(cudaMallocAsync(&A, sizeof(zc) * nk * NN, st));
+    // the same forms as fourier_direct's for the sums, as the rotation's for the products
+    const bool oz = (double)nk * NN * nr * 4.0 >= kOzFourierWork, tc = N > kCommSmemMaxN;
+    const int step = oz ? 2 : 1;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off += (bytes + 255) & ~size_t(255);
+        return o;
+    };
+    const size_t o_ph = take(sizeof(zc) * nk * nR), o_orb = take(sizeof(zc) * nk * N);
+    const size_t o_tab = take(sizeof(zc) * step * nr * NN), o_A = take(sizeof(zc) * nk * NN);
+    const size_t o_eb = take(oz ? sizeof(int) * NN : 0), o_ea = take(oz ? sizeof(int) * nk : 0);
+    const size_t o_tim = take(oz ? oz64_table_image_bytes(nr, NN) : 0), o_aim = take(oz ? oz64_row_image_bytes(nk, nr) : 0);
+    const size_t o_ex = take(tc ? sizeof(int) * 4 * nk * N : 0);
+    unsigned char* buf = nullptr;
+    TBG_CUDA(cudaMallocAsync(&buf, off, st));
+    zc* ph = reinterpret_cast<zc*>(buf + o_ph);
+    zc* orbph = reinterpret_cast<zc*>(buf + o_orb);
+    zc* tab = reinterpret_cast<zc*>(buf + o_tab);
+    zc* A = reinterpret_cast<zc*>(buf + o_A);
+    int *EB = reinterpret_cast<int*>(buf + o_eb), *EA = reinterpret_cast<int*>(buf + o_ea);
+    int *hr = reinterpret_cast<int*>(buf + o_ex), *hc = hr + nk * N, *ar = hc + nk * N, *ac = ar + nk * N;
     int rc = TBG_OK;
-    {
-        const int64_t total = nk * (int64_t)(nR + N);
-        const unsigned blocks = (unsigned)std::min<int64_t>((total + 255) / 256, 65535 * 8);
-        phases_kernel<<<blocks, 256, 0, st>>>(nk, m.dim, k_d, nR, m.hamR_d, N, m.tau_d, ph, orbph);
+    auto launched = [&](const char* what) {
         count_launch();
-    }
-    std::vector<double> dirs_h((size_t)nproj * m.dim);
-    if (cudaMemcpyAsync(dirs_h.data(), dirs_d, sizeof(double) * dirs_h.size(), cudaMemcpyDeviceToHost, st) !=
-            cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-        rc = cuda_error(cudaGetLastError(), "rmatrix_term: copy directions");
-    double* w_d = nullptr;
-    if (rc == TBG_OK) {
-        TBG_CUDA(cudaMallocAsync(&w_d, sizeof(double) * m.dim, st));
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess && !rc) rc = cuda_error(e, what);
+        return rc;
+    };
+    const unsigned wide = 65535 * 8;
+    phases_kernel<<<(unsigned)std::min<int64_t>((nk * (int64_t)(nR + N) + 255) / 256, wide), 256, 0, st>>>(
+        nk, m.dim, k_d, nR, m.hamR_d, N, m.tau_d, ph, orbph);
+    launched("phases_kernel");
+    if (tc && !rc) {
+        rc = oz64_row_exps(st, nk, N, N, H, N, NN, hr);
+        if (!rc) rc = oz64_col_exps(st, nk, N, N, H, N, NN, hc);
     }
     for (int p = 0; rc == TBG_OK && p < nproj; ++p) {
-        TBG_CUDA(cudaMemcpyAsync(w_d, dirs_d + (int64_t)p * m.dim, sizeof(double) * m.dim,
-                                 cudaMemcpyDeviceToDevice, st));
-        const int64_t tot = m.n_rmat * NN;
-        rmat_combine_kernel<<<(unsigned)std::min<int64_t>((tot + 255) / 256, 65535 * 8), 256, 0, st>>>(
-            m.n_rmat, m.dim, N, w_d, m.rmatrix, tab);
-        count_launch();
-        // A = sum_{r < n_rmat} u(k,r) rm_p[r]   (H-only contraction, lattice gauge)
-        rc = dispatch_gemm(st, 0, nk, (int)m.n_rmat, nR, N, ph, tab, nullptr, orbph, nullptr,
-                           TBG_GAUGE_LATTICE, A, NN, nullptr, 0);
-        if (rc != TBG_OK) break;
-        if (N <= kCommSmemMaxN) {
+        rmat_combine_kernel<<<(unsigned)std::min<int64_t>((nr * NN + 255) / 256, wide), 256, 0, st>>>(
+            nr, m.dim, N, dirs_d + (int64_t)p * m.dim, m.rmatrix, step, tab);
+        if (launched("rmat_combine_kernel")) break;
+        // A = sum_{r < n_rmat} u(k,r) rm_p[r]   (lattice gauge)
+        if (oz) {
+            rc = oz64_table_image(st, nr, NN, tab, EB, buf + o_tim);
+            if (!rc) rc = oz64_table_product(st, nk, NN, nr, ph, nR, EB, buf + o_tim, A, EA, buf + o_aim, status_d);
+        } else {
+            rc = launch_gemm(st, nk, nr, nR, N, ph, tab, A);
+        }
+        if (rc) break;
+        zc* Vp = V + (int64_t)p * NN;
+        const int64_t ldV = (int64_t)nproj * NN;
+        if (!tc) {
             const size_t smem = 2 * sizeof(zc) * NN;
-            cudaError_t e = cudaFuncSetAttribute(commutator_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)(2 * sizeof(zc) * kCommSmemMaxN * kCommSmemMaxN));
-            if (e != cudaSuccess) {
-                rc = cuda_error(e, "cudaFuncSetAttribute(commutator_smem_kernel)");
-                break;
-            }
             commutator_smem_kernel<<<(unsigned)std::min<int64_t>(nk, 152LL * 64), fit_threads((int)NN), smem, st>>>(
-                N, nk, H, A, orbph, gauge, V + (int64_t)p * NN, (int64_t)nproj * NN);
-            count_launch();
-            e = cudaGetLastError();
-            if (e != cudaSuccess) rc = cuda_error(e, "commutator_smem_kernel");
+                N, nk, H, A, orbph, gauge, Vp, ldV);
+            launched("commutator_smem_kernel");
             continue;
         }
-        if (gauge == TBG_GAUGE_ATOM) {
-            const int64_t t2 = nk * NN;
-            rmat_gauge_kernel<<<(unsigned)std::min<int64_t>((t2 + 255) / 256, 65535 * 8), 256, 0, st>>>(
-                nk, N, orbph, A);
-            count_launch();
-        }
-        dim3 grid((N + 15) / 16, (N + 15) / 16, (unsigned)nk);
-        commutator_kernel<<<grid, 256, 0, st>>>(N, H, NN, A, V + (int64_t)p * NN, (int64_t)nproj * NN);
-        count_launch();
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = cuda_error(e, "rmatrix_term kernels");
+        rmat_gauge_kernel<<<(unsigned)std::min<int64_t>((nk * NN + 255) / 256, wide), 256, 0, st>>>(nk, N, gauge, orbph,
+                                                                                                   A);
+        if (launched("rmat_gauge_kernel")) break;
+        // V += H (iA) - (iA) H
+        if ((rc = oz64_row_exps(st, nk, N, N, A, N, NN, ar)) || (rc = oz64_col_exps(st, nk, N, N, A, N, NN, ac))) break;
+        rc = oz64_gemm(st, nk, N, N, N, {H, N, 1, NN, 0, hr}, {A, 1, N, NN, 0, ac}, Vp, N, ldV, 1, status_d);
+        if (!rc) rc = oz64_gemm(st, nk, N, N, N, {A, N, 1, NN, 0, ar}, {H, 1, N, NN, 0, hc}, Vp, N, ldV, -1, status_d);
     }
-    if (w_d) cudaFreeAsync(w_d, st);
-    cudaFreeAsync(ph, st);
-    cudaFreeAsync(orbph, st);
-    cudaFreeAsync(tab, st);
-    cudaFreeAsync(A, st);
+    cudaFreeAsync(buf, st);
     return rc;
 }
 

@@ -194,6 +194,8 @@ struct ModelDev {
     int* hop_pair_d = nullptr;
     zc* pair_T = nullptr;          // the paired table (2 hop_K rows, nsta^2 columns)
     bool nonfinite = false;        // the table holds NaN or Inf (found when it is paired)
+    void* oz_img = nullptr;        // digit image of pair_T for the FP64-accurate products
+    int* oz_EB = nullptr;          // its column exponents (nsta^2)
 };
 
 // ------------------------------------------------------------------ errors --
@@ -230,13 +232,15 @@ void timing_flush();  // resolve recorded event pairs (after a stream sync)
 // ---------------------------------------------------------- kernel drivers --
 // Fourier sum, direct form: for nk k-points (device k, (nk, dim)), outputs
 // H (nk, N, N) (may be null) and V (nk, nproj, N, N) (may be null when
-// nproj == 0); dirs (nproj, dim) device (Cartesian weights).
+// nproj == 0); dirs (nproj, dim) device (Cartesian weights).  Large sums run on
+// the tensor cores (oz64.cu) when the caller gives a status word for their
+// bounded waits.
 int fourier_direct(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k_d, int gauge,
-                   int nproj, const double* dirs_d, zc* H, zc* V, int64_t ldH, int64_t ldV);
+                   int nproj, const double* dirs_d, zc* H, zc* V, int64_t ldH, int64_t ldV, int* status_d = nullptr);
 
 // Position-matrix commutator term added to V (HasRMatrix models).
 int rmatrix_term(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k_d, int gauge,
-                 int nproj, const double* dirs_d, const zc* H, zc* V, zc* scratch);
+                 int nproj, const double* dirs_d, const zc* H, zc* V, int* status_d);
 
 // Separable transform on a uniform mesh: k-points with flat indices
 // [k0, k0 + nk) of the mesh kmesh[dim].
@@ -294,7 +298,8 @@ int fit_threads(int n);
 // Omega (batch, N) from U (batch, N, N), Vx/Vy (batch strided), E; the
 // quantum metric (batch, N) too when Met is not null.
 int berry_rotate(cudaStream_t st, int N, int64_t batch, const zc* U, const zc* Vx, const zc* Vy,
-                 int64_t ldV, const double* E, double eta, double* Omega, zc* scratch, double* Met = nullptr);
+                 int64_t ldV, const double* E, double eta, double* Omega, zc* scratch, double* Met,
+                 int* status_d);
 
 // Occupation-weighted sums: per k and per mu -> S (batch, nmu).
 int occupation_sums(cudaStream_t st, int N, int64_t batch, const double* Omega, const double* E,
@@ -342,6 +347,26 @@ int ozaki_zgemm_tc(cudaStream_t st, bool conj_a, int fmt_a, int fmt_b, int64_t b
                    const void* A, int64_t lda, int64_t sA, const void* B, int64_t ldb, int64_t sB, float4* C,
                    int64_t ldc, int64_t sC, int* EA, int* EB, int* err, bool exps_ready = false,
                    int* Ecol = nullptr, bool mid = false);
+
+// FP64-accurate complex products on the tensor cores (oz64.cu).  An operand:
+// element (line, k) of op(A), or (k, line) of op(B), at p + b batch + i line + k
+// k_stride, conjugated when conj; exps: its line exponents (batch, lines).
+struct Oz64Operand {
+    const zc* p;
+    int64_t line, k, batch;
+    int conj;
+    const int* exps;
+};
+int oz64_row_exps(cudaStream_t st, int64_t batch, int M, int K, const zc* A, int64_t ld, int64_t sA, int* out);
+int oz64_col_exps(cudaStream_t st, int64_t batch, int K, int64_t Nc, const zc* B, int64_t ld, int64_t sB, int* out);
+// C (M x Nc) = (mode 0), += (1), -= (-1) op(A) op(B); a wait that runs out sets bit 1 of *err.
+int oz64_gemm(cudaStream_t st, int64_t batch, int M, int Nc, int K, const Oz64Operand& A, const Oz64Operand& B, zc* C,
+              int64_t ldc, int64_t sC, int mode, int* err);
+size_t oz64_table_image_bytes(int Kc, int64_t Nc);
+size_t oz64_row_image_bytes(int64_t M, int Kc);
+int oz64_table_image(cudaStream_t st, int Kc, int64_t Nc, const zc* T, int* EB, void* img);
+int oz64_table_product(cudaStream_t st, int64_t M, int64_t Nc, int Kc, const zc* coef, int64_t ld, const int* EB,
+                       const void* img, zc* C, int* EA, void* aimg, int* err);
 
 // Gaussian-smeared DOS: add the terms of count band energies ev (device) to
 // the compensated per-bin totals acc (2 E_n: sum, compensation).  part holds
