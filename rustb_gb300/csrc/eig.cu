@@ -35,6 +35,7 @@
 #include <cstdlib>
 #include <vector>
 
+#include "eig64.cuh"
 #include "tbgpu_internal.cuh"
 
 namespace tbg {
@@ -1293,7 +1294,7 @@ int eig_batched(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, 
     if (batch <= 0) return TBG_OK;
     if (N <= kSmallMaxN) return eig_small(st, N, batch, A, E, U, status_d);  // one thread per matrix
     if (N <= jacobi_max_n()) return eig_jacobi(st, N, batch, A, E, U, status_d);  // one warp per matrix
-    if (eig64_fits(N)) return eig64(st, N, batch, A, E, U, status_d);
+    if (N <= kBigMaxN) return eig64(st, N, batch, A, E, U, status_d);
     int G, PB;
     choose_g_pb<double>(N, false, 16, 16, G, PB);
     return launch_heev<double, false>(st, N, batch, A, E, U, work, work_bytes, status_d, "heev_kernel<double>", G,
@@ -1438,7 +1439,7 @@ extern "C" int tbg_internal_eig_f64(int n, int64_t nk, const double* H, double* 
             else if (n <= kSmallMaxN)
                 rc = eig_small(0, n, nk, static_cast<zc*>(dA), static_cast<double*>(dE), static_cast<zc*>(dU),
                                static_cast<int*>(dS));
-            else if (eig64_fits(n))
+            else if (n <= kBigMaxN)
                 rc = eig64(0, n, nk, static_cast<zc*>(dA), static_cast<double*>(dE), static_cast<zc*>(dU),
                            static_cast<int*>(dS));
             else {

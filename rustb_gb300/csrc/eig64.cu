@@ -44,6 +44,7 @@
 #include <cfloat>
 #include <cmath>
 
+#include "eig64.cuh"
 #include "tbgpu_internal.cuh"
 
 namespace tbg {
@@ -57,28 +58,6 @@ __device__ __forceinline__ double wsum(double v) {
     return v;
 }
 
-// 1 / x and 1 / sqrt(x) from the hardware's approximations (about 20 bits) and
-// one third-order step of the Newton family on the residual e = 1 - x y
-// (e = 1 - x y^2): y (1 + e + e^2), y (1 + e / 2 + 3 e^2 / 8).  For arguments
-// well inside the normal range.
-__device__ __forceinline__ double fast_rcp(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-__device__ __forceinline__ double fast_rsqrt(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x * y, y, 1.0);
-    return fma(y, e * fma(0.375, e, 0.5), y);
-}
-// sign flips and magnitude tests on the high word (integer pipe)
-__device__ __forceinline__ double flip_if(double x, bool f) {
-    return __hiloint2double(__double2hiint(x) ^ (f ? 0x80000000 : 0), __double2loint(x));
-}
-__device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
-
 __host__ __device__ __forceinline__ int pk_off(int N, int i) { return i * N - (i * (i - 1)) / 2; }
 
 // Reflector of step j by one warp: x = conj(row) (row = A(j, j + 1 ..), length
@@ -89,33 +68,8 @@ __device__ __forceinline__ void reflector64(const zc* row, int m, int lane, zc* 
     for (int i = lane; i < m; i += 32)
         if (i > 0) part += abs2(row[i]);
     const double xn = wsum(part);
-    const zc alpha = conj(row[0]);
     zc scal;
-    if (xn == 0.0 && alpha.im == 0.0) {
-        tau = mk(0.0, 0.0);
-        scal = mk(0.0, 0.0);
-        beta = alpha.re;
-    } else {
-        const double n2 = fma(alpha.re, alpha.re, fma(alpha.im, alpha.im, xn));
-        if (n2 > 1e-280 && n2 < 1e280) {
-            const double y = fast_rsqrt(n2);
-            double nrm = n2 * y;
-            nrm = fma(fma(-nrm, nrm, n2), 0.5 * y, nrm);
-            const bool neg = __double2hiint(alpha.re) >= 0;  // beta opposite in sign to Re(alpha)
-            beta = flip_if(nrm, neg);
-            const double ib = flip_if(y, neg);
-            const double dr = alpha.re - beta;
-            tau = mk(-dr * ib, -alpha.im * ib);
-            const double r = fast_rcp(fma(dr, dr, alpha.im * alpha.im));
-            scal = mk(dr * r, -alpha.im * r);
-        } else {
-            const double nrm = sqrt(n2);
-            beta = (alpha.re >= 0.0) ? -nrm : nrm;
-            tau = mk((beta - alpha.re) / beta, -alpha.im / beta);
-            const double dr = alpha.re - beta, dd = dr * dr + alpha.im * alpha.im;
-            scal = mk(dr / dd, -alpha.im / dd);
-        }
-    }
+    reflector_scalars64(conj(row[0]), xn, tau, scal, beta);
     for (int i = lane; i < m; i += 32) {
         const zc vi = (i == 0) ? mk(1.0, 0.0) : conj(row[i]) * scal;
         sv[i] = vi;
@@ -397,19 +351,31 @@ __device__ __forceinline__ void vector_side(zc* u, int r, int dir, int n, int N,
     }
 }
 
-// MPC matrices per CTA (1 when N > 64), one thread per eigenvalue.  Scratch:
-// VEC: the ratios of the twisted factorisation go to U(k, i).re, where the
-// vector then goes.  Values only: A (after d and e are read) holds the FP32 pivots.
+// Values only: the FP32 pivots of row k (N floats) go to A beside the diagonal.
+__device__ __forceinline__ float* pivot_row(zc* A, int N, int k) {
+    return reinterpret_cast<float*>(A + (size_t)k * N + (k < N / 2 ? N / 2 : 0));
+}
+
+// MPC matrices per CTA (1 when N > 64), one thread per eigenvalue; with few
+// matrices each is shared by `parts` CTAs of `len` eigenvalues (MPC = 1; E is then
+// put in order by tri64_order_kernel, the marks are cleared by the caller).
+// Scratch: VEC: the ratios of the twisted factorisation go to U(k, i).re, where
+// the vector then goes; values only: pivot_row.
 template <bool VEC>
-__global__ void __launch_bounds__(512) tri64_kernel(int N, int64_t batch, int MPC, zc* __restrict__ Ain,
+__global__ void __launch_bounds__(512) tri64_kernel(int N, int64_t batch, int MPC, int parts, int len,
+                                                    zc* __restrict__ Ain,
                                                     double* __restrict__ Eout, zc* __restrict__ Uout,
                                                     int* __restrict__ status) {
     extern __shared__ __align__(16) unsigned char smem64[];
     const size_t stride = (tri_smem_bytes(N) + 15) & ~size_t(15);
     const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nthr >> 5;
     const int W = (N + 31) / 32;
-    for (int64_t b0 = (int64_t)blockIdx.x * MPC; b0 < batch; b0 += (int64_t)gridDim.x * MPC) {
+    for (int64_t unit = blockIdx.x; unit < (batch + MPC - 1) / MPC * parts; unit += gridDim.x) {
+        const int64_t b0 = unit / parts * MPC;
         const int nm = (int)min((int64_t)MPC, batch - b0);
+        // this CTA's eigenvalues [i0, i0 + ni) of each matrix, [h0, h0 + nh) with their neighbours
+        const int i0 = (int)(unit % parts) * len, ni = min(len, N - i0);
+        const int h0 = max(i0 - 1, 0), nh = min(i0 + ni + 1, N) - h0;
         for (int t = tid; t < nm * N; t += nthr) {
             const int mt = t / N, k = t - mt * N;
             const TriShared s = tri_carve(smem64 + mt * stride, N);
@@ -471,8 +437,8 @@ __global__ void __launch_bounds__(512) tri64_kernel(int N, int64_t batch, int MP
         }
         __syncthreads();
         // FP32 bisection on the FP32 copy of T
-        for (int t = tid; t < nm * N; t += nthr) {
-            const int mt = t / N, i = t - mt * N;
+        for (int t = tid; t < nm * nh; t += nthr) {
+            const int mt = t / nh, i = h0 + t - mt * nh;
             const TriShared s = tri_carve(smem64 + mt * stride, N);
             float a = (float)*s.lo - 1e-6f, c = (float)*s.hi + 1e-6f;
             for (int it = 0; it < 26 && c - a > 1.5e-7f; ++it) {
@@ -493,8 +459,8 @@ __global__ void __launch_bounds__(512) tri64_kernel(int N, int64_t batch, int MP
             s.x0[i] = 0.5f * (a + c);
         }
         __syncthreads();
-        for (int t = tid; t < nm * N; t += nthr) {
-            const int mt = t / N, i = t - mt * N;
+        for (int t = tid; t < nm * ni; t += nthr) {
+            const int mt = t / ni, i = i0 + t - mt * ni;
             const int64_t b = b0 + mt;
             const TriShared s = tri_carve(smem64 + mt * stride, N);
             const float x0 = s.x0[i];
@@ -507,16 +473,16 @@ __global__ void __launch_bounds__(512) tri64_kernel(int N, int64_t batch, int MP
             double lam = 0.0;
             if (gl > kSame && gr > kSame) {
                 // twist index from the FP32 factorisation
-                float* fs = VEC ? reinterpret_cast<float*>(Uout + b * N * N + i)
-                                : reinterpret_cast<float*>(Ain + b * N * N) + i;
-                const size_t fstep = VEC ? 4 * (size_t)N : (size_t)N;
+                float* uf = VEC ? reinterpret_cast<float*>(Uout + b * N * N + i) : nullptr;
+                zc* Ab = Ain + b * N * N;
+                auto fs = [&](int k) -> float& { return VEC ? uf[4 * (size_t)N * k] : pivot_row(Ab, N, k)[i]; };
                 float q = s.fd[0] - x0;
                 if (fabsf(q) < 1e-7f) q = -1e-7f;
-                fs[0] = q;
+                fs(0) = q;
                 for (int k = 1; k < N; ++k) {
                     q = (s.fd[k] - x0) - __fdividef(s.fe2[k - 1], q);
                     if (fabsf(q) < 1e-7f) q = -1e-7f;
-                    fs[k * fstep] = q;
+                    fs(k) = q;
                 }
                 int r = N - 1;
                 float best = fabsf(q);
@@ -526,7 +492,7 @@ __global__ void __launch_bounds__(512) tri64_kernel(int N, int64_t batch, int MP
                     const float dk = s.fd[k] - x0;
                     q = dk - __fdividef(s.fe2[k], q);
                     if (fabsf(q) < 1e-7f) q = -1e-7f;
-                    const float g = fabsf(fs[k * fstep] + q - dk);
+                    const float g = fabsf(fs(k) + q - dk);
                     if (g < best) {
                         best = g;
                         r = k;
@@ -615,7 +581,7 @@ __global__ void __launch_bounds__(512) tri64_kernel(int N, int64_t batch, int MP
         __syncthreads();
         // eigenvalues bisected from their own brackets may differ in the last bits in
         // either order: each run of neighbours nearer than kSame is put in order
-        for (int t = tid; t < nm * N; t += nthr) {
+        if (parts == 1) for (int t = tid; t < nm * N; t += nthr) {
             const int mt = t / N, i = t - mt * N;
             const TriShared s = tri_carve(smem64 + mt * stride, N);
             if ((i > 0 && s.x0[i] - s.x0[i - 1] <= kSame) || i == N - 1 || s.x0[i + 1] - s.x0[i] > kSame) continue;
@@ -627,13 +593,41 @@ __global__ void __launch_bounds__(512) tri64_kernel(int N, int64_t batch, int MP
             }
         }
         __syncthreads();
-        for (int t = tid; t < nm * N; t += nthr) {
-            const int mt = t / N, i = t - mt * N;
+        for (int t = tid; t < nm * ni; t += nthr) {
+            const int mt = t / ni, i = i0 + t - mt * ni;
             const TriShared s = tri_carve(smem64 + mt * stride, N);
             Eout[(b0 + mt) * N + i] = scalbn(s.lam[i], s.sc[0]);
-            if (VEC)
-                for (int w = i; w < 2 * W + 1; w += N) marks_of(Ain + (b0 + mt) * N * N, N)[w] = s.marks[w];
         }
+        if (VEC)
+            for (int t = tid; t < nm * (2 * W + 1); t += nthr) {
+                const int mt = t / (2 * W + 1), w = t - mt * (2 * W + 1);
+                const unsigned v = tri_carve(smem64 + mt * stride, N).marks[w];
+                unsigned* g = marks_of(Ain + (b0 + mt) * N * N, N) + w;
+                if (parts == 1)
+                    *g = v;
+                else if (w < 2 * W)
+                    atomicOr(g, v);
+                else
+                    atomicAdd(g, v);
+            }
+        __syncthreads();
+    }
+}
+
+// Eigenvalues of a matrix whose parts were found by different CTAs: neighbours
+// bisected from their own brackets may differ in the last bits in either order.
+__global__ void __launch_bounds__(256) tri64_order_kernel(int N, int64_t batch, double* __restrict__ E) {
+    for (int64_t b = blockIdx.x; b < batch; b += gridDim.x) {
+        double* e = E + b * N;
+        bool out = false;
+        for (int i = threadIdx.x; i < N - 1; i += blockDim.x) out = out || e[i] > e[i + 1];
+        if (__syncthreads_or(out) && threadIdx.x == 0)
+            for (int i = 1; i < N; ++i) {
+                const double v = e[i];
+                int p = i - 1;
+                for (; p >= 0 && e[p] > v; --p) e[p + 1] = e[p];
+                e[p + 1] = v;
+            }
         __syncthreads();
     }
 }
@@ -691,9 +685,11 @@ __device__ void tri_solve64(int N, const double* d, const double* e, double lam,
 
 // Vectors that tri64 left: clusters (runs of marked neighbours) and single
 // vectors that did not converge, one lane per cluster, inverse iteration with
-// modified Gram-Schmidt against the earlier members.  One warp per matrix;
-// a matrix without marks costs one read.
-__global__ void __launch_bounds__(32) tri64_cluster_kernel(int N, int64_t batch, int G, zc* __restrict__ Ain,
+// modified Gram-Schmidt against the earlier members.  One warp per matrix, or per
+// `len` eigenvalues of it (clusters that start there) when there are few matrices;
+// one without marks costs one read.
+__global__ void __launch_bounds__(32) tri64_cluster_kernel(int N, int64_t batch, int G, int parts, int len,
+                                                           const zc* __restrict__ Ain,
                                                            const double* __restrict__ Ein, zc* __restrict__ Uout) {
     extern __shared__ __align__(16) unsigned char smem64[];
     double* d = reinterpret_cast<double*>(smem64);
@@ -701,9 +697,11 @@ __global__ void __launch_bounds__(32) tri64_cluster_kernel(int N, int64_t batch,
     double* lam = e + N;
     double* scr = lam + N;  // 4 N G
     const int lane = threadIdx.x, W = (N + 31) / 32;
-    for (int64_t b = blockIdx.x; b < batch; b += gridDim.x) {
-        zc* A = Ain + b * N * N;
-        const unsigned* mk_ = marks_of(A, N);
+    for (int64_t unit = blockIdx.x; unit < batch * parts; unit += gridDim.x) {
+        const int64_t b = unit / parts;
+        const int i0 = (int)(unit % parts) * len, i1 = min(i0 + len, N);
+        const zc* A = Ain + b * N * N;
+        const unsigned* mk_ = marks_of(const_cast<zc*>(A), N);
         if (mk_[2 * W] == 0) continue;
         zc* U = Uout + b * N * N;
         double tn = 0.0;
@@ -733,9 +731,9 @@ __global__ void __launch_bounds__(32) tri64_cluster_kernel(int N, int64_t batch,
         __syncwarp();
         auto joined = [&](int i) { return (mk_[i >> 5] >> (i & 31)) & 1u; };
         auto redo = [&](int i) { return (mk_[W + (i >> 5)] >> (i & 31)) & 1u; };
-        for (int g0 = 0; g0 < N; g0 += G) {
+        for (int g0 = i0; g0 < i1; g0 += G) {
             const int i = g0 + lane;
-            if (lane < G && i < N && !(i > 0 && joined(i)) && redo(i)) {
+            if (lane < G && i < i1 && !(i > 0 && joined(i)) && redo(i)) {
                 int c1 = i;
                 while (c1 + 1 < N && joined(c1 + 1)) ++c1;
                 double* x = scr + lane;
@@ -888,18 +886,32 @@ int launch_bt(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U) {
 
 }  // namespace
 
+// Whether the back-transformation takes the blocked form.  Its FP64 work (T) is a
+// small part of the 4 N^3 FMA of bt64, which does not go beyond 256 bands; below
+// kWYWork the launches of a block cost more than that saves, and below kWYMinN
+// bands too little of a 128-row tile is used (1024 x 128 bands 6.8 against 17.5 ms,
+// 200 x 97 1.2 against 1.4; 30 x 128 0.65 against 0.51, 4032 x 64 7.8 against 8.2,
+// 200 x 64 0.58 against 0.42)
+constexpr int kWYMinN = 80;
+constexpr double kWYWork = 6e8;
+static bool use_wy(int N, int64_t batch) {
+    return N > 256 || (N >= kWYMinN && 4.0 * N * N * (double)N * batch >= kWYWork);
+}
+
 // Largest matrix whose packed triangle and vectors fit one CTA's shared memory.
 bool eig64_fits(int N) { return N <= kWarpMax || cta_smem_bytes(N, cta_threads(N)) <= kSmemCta; }
 
 // Eigenvalues E (ascending) and, when U is given, eigenvectors (columns) of
 // batch N x N matrices A (upper triangles read, destroyed), N >= 1 (>= 4 with
-// vectors).  Requires eig64_fits(N).
+// vectors), N <= kBigMaxN.  With timed = false nothing is allocated, which
+// requires eig64_fits(N) (and N <= 256 with vectors).
 int eig64(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* status_d, bool timed) {
     if (batch <= 0) return TBG_OK;
     const int nsm = sm_count();
     const double n3 = (double)N * N * N * batch;
     int rc = TBG_OK;
     auto reduce = [&]() -> int {
+        if (!eig64_fits(N)) return hetrd64_big(st, N, batch, A, status_d);
         if (N <= kWarpMax) {
             // one warp per CTA while that spreads a small batch over more SMs
             const int wpc = batch > (int64_t)nsm * 8 ? kWarpsPerCta : 1;
@@ -918,27 +930,48 @@ int eig64(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* s
     };
     auto tri = [&]() -> int {
         const int mpc = N <= 64 ? std::max(1, 128 / N) : 1;
-        const int thr = std::min(512, (mpc * N + 31) & ~31);
+        // few large matrices: the eigenvalues of each over several CTAs (12 matrices of
+        // 512: 1.3 ms over 16 CTAs each; with vectors, most of them in clusters, 12.0
+        // against 51.6 ms when one warp per matrix does the clusters)
+        int parts = 1, len = N;
+        if (N > 64 && batch < 2 * nsm) {
+            parts = (int)std::min<int64_t>((N + 31) / 32, (2 * nsm + batch - 1) / batch);
+            len = ((N + parts - 1) / parts + 31) & ~31;
+            parts = (N + len - 1) / len;
+        }
+        const int thr = std::min(512, (mpc * len + 31) & ~31);
         const size_t smem = mpc * ((tri_smem_bytes(N) + 15) & ~size_t(15));
-        const int64_t ctas = std::min<int64_t>((batch + mpc - 1) / mpc, (int64_t)nsm * 64);
+        const int64_t ctas = std::min<int64_t>((batch + mpc - 1) / mpc * parts, (int64_t)nsm * 64);
+        auto order = [&]() -> int {
+            if (parts == 1) return TBG_OK;
+            tri64_order_kernel<<<(unsigned)std::min<int64_t>(batch, nsm * 8), 256, 0, st>>>(N, batch, E);
+            TBG_LAUNCHED("tri64_order_kernel");
+            return TBG_OK;
+        };
         if (U) {
             if (int r = allow_smem(tri64_kernel<true>, smem)) return r;
-            tri64_kernel<true><<<(unsigned)ctas, thr, smem, st>>>(N, batch, mpc, A, E, U, status_d);
+            if (parts > 1)
+                TBG_CUDA(cudaMemset2DAsync(A + (size_t)(N - 1) * N, sizeof(zc) * (size_t)N * N, 0,
+                                           4 * (2 * (size_t)((N + 31) / 32) + 1), batch, st));
+            tri64_kernel<true><<<(unsigned)ctas, thr, smem, st>>>(N, batch, mpc, parts, len, A, E, U, status_d);
             TBG_LAUNCHED("tri64_kernel");
+            if (int r = order()) return r;
             const int G = (int)std::max<size_t>(1, std::min<size_t>(32, (64 * 1024) / (32 * (size_t)N)));
             const size_t csm = sizeof(double) * (size_t)N * (3 + 4 * G);
             if (int r = allow_smem(tri64_cluster_kernel, csm)) return r;
-            tri64_cluster_kernel<<<(unsigned)std::min<int64_t>(batch, (int64_t)nsm * 32), 32, csm, st>>>(N, batch, G,
-                                                                                                       A, E, U);
+            tri64_cluster_kernel<<<(unsigned)std::min<int64_t>(batch * parts, (int64_t)nsm * 32), 32, csm, st>>>(
+                N, batch, G, parts, len, A, E, U);
             TBG_LAUNCHED("tri64_cluster_kernel");
         } else {
             if (int r = allow_smem(tri64_kernel<false>, smem)) return r;
-            tri64_kernel<false><<<(unsigned)ctas, thr, smem, st>>>(N, batch, mpc, A, E, nullptr, status_d);
+            tri64_kernel<false><<<(unsigned)ctas, thr, smem, st>>>(N, batch, mpc, parts, len, A, E, nullptr, status_d);
             TBG_LAUNCHED("tri64_kernel");
+            if (int r = order()) return r;
         }
         return TBG_OK;
     };
     auto back = [&]() -> int {
+        if (timed && use_wy(N, batch)) return bt64_wy(st, N, batch, A, U, status_d);
         // 32 rows a lane (fewer shuffles per column) when that still gives every
         // sub-partition a warp, else 16: 128 bands 17.5 against 31.6 ms per 1024
         // matrices, 64 bands 8.5 against 14.4 per 4032; up to 32 bands 16 rows, whose
