@@ -20,8 +20,6 @@
 namespace tbg {
 namespace {
 
-constexpr double kTwoPiS = 6.283185307179586476925286766559;
-
 __device__ __forceinline__ double fermi_s(double e, double mu, double width) {
     if (width == 0.0) return (e < mu) ? 1.0 : ((e > mu) ? 0.0 : 0.5);
     const double x = (e - mu) / width;
@@ -30,17 +28,33 @@ __device__ __forceinline__ double fermi_s(double e, double mu, double width) {
     return 1.0 / (1.0 + exp(x));
 }
 
+// The rotation that annihilates a_pq: tan 2 theta = 2 |a_pq| / (a_pp - a_qq), theta
+// in [0, pi / 2].  Square roots of the half-angle formulas, the larger of cosine
+// and sine first (no cancellation); a third of the FP64 instructions of atan2 and
+// sincos.
+__device__ __forceinline__ void jacobi_angle(double mag, double d, double& cs, double& sn) {
+    const double h = sqrt(fma(d, d, 4.0 * mag * mag));
+    const double big = sqrt(0.5 * (1.0 + fabs(d) / h)), little = mag / (h * big);
+    cs = d >= 0.0 ? big : little;
+    sn = d >= 0.0 ? little : big;
+}
+
 // Cyclic complex Jacobi on the Hermitian NM x NM (active N) matrix A; W gets
 // the eigenvectors in columns.  Rotation: G = diag(1, e^{-i phi}) [[c,-s],[s,c]]
-// with e^{i phi} = a_pq / |a_pq|, tan 2 theta = 2 |a_pq| / (a_pp - a_qq).
+// with e^{i phi} = a_pq / |a_pq|.
 template <int NM, bool WANT_W>
-__device__ void jacobi(int N, zc (&A)[NM][NM], zc (&W)[NM][NM]) {
+__device__ __forceinline__ void jacobi(int N, zc (&A)[NM][NM], zc (&W)[NM][NM]) {
     if (WANT_W)
+#pragma unroll
         for (int i = 0; i < NM; ++i)
+#pragma unroll
             for (int j = 0; j < NM; ++j) W[i][j] = mk(i == j ? 1.0 : 0.0, 0.0);
+#pragma unroll 1
     for (int sweep = 0; sweep < 40; ++sweep) {
         double off = 0.0, dia = 0.0;
+#pragma unroll
         for (int i = 0; i < N; ++i)
+#pragma unroll
             for (int j = 0; j < N; ++j) {
                 if (i != j)
                     off += abs2(A[i][j]);
@@ -48,22 +62,25 @@ __device__ void jacobi(int N, zc (&A)[NM][NM], zc (&W)[NM][NM]) {
                     dia += abs2(A[i][j]);
             }
         if (off <= 1e-32 * dia || off == 0.0) break;
+#pragma unroll
         for (int p = 0; p < N - 1; ++p)
+#pragma unroll
             for (int q = p + 1; q < N; ++q) {
                 const zc apq = A[p][q];
                 const double mag = sqrt(abs2(apq));
                 if (mag == 0.0) continue;
-                const double app = A[p][p].re, aqq = A[q][q].re;
-                const zc ph = mk(apq.re / mag, apq.im / mag);
+                const double rm = 1.0 / mag;
+                const zc ph = mk(apq.re * rm, apq.im * rm);
                 const zc emi = conj(ph);
-                const double theta = 0.5 * atan2(2.0 * mag, app - aqq);
                 double sn, cs;
-                sincos(theta, &sn, &cs);
+                jacobi_angle(mag, A[p][p].re - A[q][q].re, cs, sn);
+#pragma unroll
                 for (int k = 0; k < N; ++k) {
                     const zc akp = A[k][p], akq = emi * A[k][q];
                     A[k][p] = cs * akp + sn * akq;
                     A[k][q] = cs * akq - sn * akp;
                 }
+#pragma unroll
                 for (int k = 0; k < N; ++k) {
                     const zc apk = A[p][k], aqk = ph * A[q][k];
                     A[p][k] = cs * apk + sn * aqk;
@@ -74,6 +91,7 @@ __device__ void jacobi(int N, zc (&A)[NM][NM], zc (&W)[NM][NM]) {
                 A[p][p].im = 0.0;
                 A[q][q].im = 0.0;
                 if (WANT_W)
+#pragma unroll
                     for (int k = 0; k < N; ++k) {
                         const zc wkp = W[k][p], wkq = emi * W[k][q];
                         W[k][p] = cs * wkp + sn * wkq;
@@ -83,95 +101,204 @@ __device__ void jacobi(int N, zc (&A)[NM][NM], zc (&W)[NM][NM]) {
     }
 }
 
+// Ascending order of E, f(i) exchanging what goes with entries i and i + 1 (bubble
+// network: constant indices keep the arrays in registers; ties stay as they are).
+template <int NM, typename F>
+__device__ __forceinline__ void sort_bands(int N, double (&E)[NM], F f) {
+#pragma unroll
+    for (int a = N - 1; a > 0; --a)
+#pragma unroll
+        for (int i = 0; i < a; ++i)
+            if (E[i] > E[i + 1]) {
+                const double t = E[i];
+                E[i] = E[i + 1];
+                E[i + 1] = t;
+                f(i);
+            }
+}
+__device__ __forceinline__ void swap_d(double& a, double& b) {
+    const double t = a;
+    a = b;
+    b = t;
+}
+
+// z^r for |z| = 1 (r uniform over the warp: no divergence)
+__device__ __forceinline__ void times_power(zc& u, bool& one, zc z, int r) {
+    if (r == 0) return;
+    if (r < 0) z.im = -z.im;
+    for (unsigned n = (unsigned)(r < 0 ? -r : r);;) {
+        if (n & 1) {
+            u = one ? z : u * z;
+            one = false;
+        }
+        n >>= 1;
+        if (!n) break;
+        z = z * z;
+    }
+}
+
+// e^{2 pi i i_d / n_d} along each axis of a mesh, axes one after the other.
+__global__ void mesh_phase_kernel(int64_t n0, int64_t n1, int64_t n2, zc* __restrict__ z) {
+    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n0 + n1 + n2;
+         t += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t n = t < n0 ? n0 : (t < n0 + n1 ? n1 : n2), i = t < n0 ? t : (t < n0 + n1 ? t - n0 : t - n0 - n1);
+        double sn, cs;
+        sincospi(2.0 * ((double)i / (double)n), &sn, &cs);
+        z[t] = mk(cs, sn);
+    }
+}
+
 // VALS: band energies only (E_out); no velocities, eigenvectors or curvature.
-template <int NM, bool VALS>
-__global__ void __launch_bounds__(128) small_fused_kernel(
-    int N, int norb, int dim, int nR, int64_t nk, const double* __restrict__ klist, int64_t k0, int64_t n0,
-    int64_t n1, int64_t n2, const zc* __restrict__ ham, const int* __restrict__ hamR, const double* __restrict__ Rcart,
-    const double* __restrict__ tau, const double* __restrict__ taucart, const double* __restrict__ dirs, int spin,
-    double eta, int nmu, const double* __restrict__ mu, double width, double* __restrict__ Om_out,
-    double* __restrict__ E_out, double* __restrict__ S_out, double* __restrict__ Met_out, double* __restrict__ SM_out) {
+// EXACT: N == NM, known to the compiler, so the matrices stay in registers (they
+// are indexed, in local memory, otherwise).  The FP64 pipe is the bound, so the
+// phase of R comes from the e^{2 pi i k_d} by R_d-fold products, one sincospi per
+// axis and k-point (none with ztab, the mesh's table) instead of one sincos per R,
+// and energies of two bands from the quadratic formula: 10^6 k-points of the
+// honeycomb model 0.92 -> 0.185 ms, 961 of the Haldane model's curvature 62 -> 45 us.
+template <int NM, bool VALS, bool EXACT>
+__global__ void __launch_bounds__(64) small_fused_kernel(
+    int Nrt, int norb, int dim, int nR, int64_t nk, const double* __restrict__ klist, int64_t k0, int64_t n0,
+    int64_t n1, int64_t n2, const zc* __restrict__ ztab, const zc* __restrict__ ham, const int* __restrict__ hamR,
+    const double* __restrict__ Rcart, const double* __restrict__ tau, const double* __restrict__ taucart,
+    const double* __restrict__ dirs, int spin, double eta, int nmu, const double* __restrict__ mu, double width,
+    double* __restrict__ Om_out, double* __restrict__ E_out, double* __restrict__ S_out, double* __restrict__ Met_out,
+    double* __restrict__ SM_out) {
+    const int N = EXACT ? NM : Nrt;
+    // the model in shared memory, all of it requested at once
+    extern __shared__ __align__(16) unsigned char small_smem[];
+    zc* s_ham = reinterpret_cast<zc*>(small_smem);                      // (nR, N, N)
+    double* s_c = reinterpret_cast<double*>(s_ham + (int64_t)nR * N * N);  // (nR, 2) w . R
+    double* s_tau = s_c + 2 * nR;                                       // (N, 5): tau, w . tau
+    int* s_R = reinterpret_cast<int*>(s_tau + 5 * N);                   // (nR, 3)
+    for (int i = threadIdx.x; i < nR * N * N; i += blockDim.x) s_ham[i] = ham[i];
+    for (int i = threadIdx.x; i < 3 * nR; i += blockDim.x) s_R[i] = hamR[i];
+    if (!VALS) {
+        auto along = [&](int d, const double* v) {  // w_d . v
+            const double* w = dirs + d * dim;
+            double c = w[0] * v[0];
+            if (dim > 1) c += w[1] * v[1];
+            if (dim > 2) c += w[2] * v[2];
+            return c;
+        };
+        for (int i = threadIdx.x; i < 2 * nR; i += blockDim.x) s_c[i] = along(i & 1, Rcart + 3 * (i >> 1));
+        for (int i = threadIdx.x; i < 5 * N; i += blockDim.x) {
+            const int a = i / 5, d = i % 5;
+            s_tau[i] = d < 3 ? tau[3 * a + d] : along(d - 3, taucart + 3 * a);
+        }
+    }
+    __syncthreads();
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= nk) return;
     double kv[3] = {0.0, 0.0, 0.0};
+    zc z[3];
     if (klist) {
         for (int d = 0; d < dim; ++d) kv[d] = klist[t * dim + d];
     } else {
-        const int64_t idx = k0 + t;  // gen_kmesh order (src/kpoints.rs:49-87)
-        if (dim == 1) {
-            kv[0] = (double)idx / (double)n0;
-        } else if (dim == 2) {
-            kv[0] = (double)(idx / n1) / (double)n0;
-            kv[1] = (double)(idx % n1) / (double)n1;
+        const int64_t idx = k0 + t;  // gen_kmesh order (src/kpoints.rs:49-87), n1 = n2 = 1 beyond dim
+        int64_t i0, i1, i2;
+        if (n0 * n1 * n2 <= 0xffffffffll) {  // 32-bit divisions
+            const unsigned u = (unsigned)idx, q = u / (unsigned)n2;
+            i2 = u - q * (unsigned)n2;
+            i0 = q / (unsigned)n1;
+            i1 = q - (unsigned)i0 * (unsigned)n1;
         } else {
-            kv[0] = (double)(idx / (n1 * n2)) / (double)n0;
-            kv[1] = (double)((idx / n2) % n1) / (double)n1;
-            kv[2] = (double)(idx % n2) / (double)n2;
+            i2 = idx % n2;
+            i1 = (idx / n2) % n1;
+            i0 = idx / (n1 * n2);
+        }
+        if (!VALS || !ztab) {
+            kv[0] = (double)i0 / (double)n0;
+            if (dim > 1) kv[1] = (double)i1 / (double)n1;
+            if (dim > 2) kv[2] = (double)i2 / (double)n2;
+        }
+        if (ztab) {
+            z[0] = ztab[i0];
+            z[1] = ztab[n0 + i1];
+            z[2] = ztab[n0 + n1 + i2];
+        }
+    }
+    if (!ztab) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            z[d] = mk(1.0, 0.0);
+            if (d < dim) sincospi(2.0 * kv[d], &z[d].im, &z[d].re);
         }
     }
     zc H[NM][NM], V0[NM][NM], V1[NM][NM];
+#pragma unroll
     for (int i = 0; i < NM; ++i)
+#pragma unroll
         for (int j = 0; j < NM; ++j) H[i][j] = V0[i][j] = V1[i][j] = mk(0.0, 0.0);
-    const double* w0 = dirs;
-    const double* w1 = dirs + dim;
     for (int r = 0; r < nR; ++r) {
-        const int* R = hamR + 3 * r;
-        double s = (double)R[0] * kv[0];
-        if (dim > 1) s += (double)R[1] * kv[1];
-        if (dim > 2) s += (double)R[2] * kv[2];
-        double sn, cs;
-        sincos(kTwoPiS * s, &sn, &cs);
-        const zc u = mk(cs, sn);
-        const zc* hr = ham + (int64_t)r * N * N;
+        const int* R = s_R + 3 * r;
+        zc u = mk(1.0, 0.0);
+        bool one = true;
+        times_power(u, one, z[0], R[0]);
+        if (dim > 1) times_power(u, one, z[1], R[1]);
+        if (dim > 2) times_power(u, one, z[2], R[2]);
+        const zc* hr = s_ham + r * N * N;
         if (VALS) {
+#pragma unroll
             for (int i = 0; i < N; ++i)
-                for (int j = 0; j < N; ++j) H[i][j] = H[i][j] + u * hr[i * N + j];
+#pragma unroll
+                for (int j = i; j < N; ++j) {  // upper triangle
+                    const zc h = hr[i * N + j];
+                    H[i][j].re = fma(u.re, h.re, fma(-u.im, h.im, H[i][j].re));
+                    if (j > i) H[i][j].im = fma(u.re, h.im, fma(u.im, h.re, H[i][j].im));
+                }
             continue;
         }
-        const double* rc = Rcart + 3 * r;
-        double c0 = w0[0] * rc[0], c1 = w1[0] * rc[0];
-        if (dim > 1) {
-            c0 += w0[1] * rc[1];
-            c1 += w1[1] * rc[1];
-        }
-        if (dim > 2) {
-            c0 += w0[2] * rc[2];
-            c1 += w1[2] * rc[2];
-        }
+        const double c0 = s_c[2 * r], c1 = s_c[2 * r + 1];
+#pragma unroll
         for (int i = 0; i < N; ++i)
+#pragma unroll
             for (int j = 0; j < N; ++j) {
                 const zc tt = u * hr[i * N + j];
                 H[i][j] = H[i][j] + tt;
-                V0[i][j] = V0[i][j] + mk(-c0 * tt.im, c0 * tt.re);  // i c0 t
-                V1[i][j] = V1[i][j] + mk(-c1 * tt.im, c1 * tt.re);
+                // i c t
+                V0[i][j] = mk(fma(-c0, tt.im, V0[i][j].re), fma(c0, tt.re, V0[i][j].im));
+                V1[i][j] = mk(fma(-c1, tt.im, V1[i][j].re), fma(c1, tt.re, V1[i][j].im));
             }
+    }
+    if (VALS) {
+        double E[NM];
+        if constexpr (EXACT && NM == 2) {
+            const double m = 0.5 * (H[0][0].re + H[1][1].re), d = 0.5 * (H[0][0].re - H[1][1].re);
+            const double h = sqrt(fma(d, d, abs2(H[0][1])));
+            E[0] = m - h;
+            E[1] = m + h;
+        } else {
+#pragma unroll
+            for (int i = 1; i < N; ++i)
+#pragma unroll
+                for (int j = 0; j < i; ++j) H[i][j] = conj(H[j][i]);
+            jacobi<NM, false>(N, H, V0);
+#pragma unroll
+            for (int i = 0; i < N; ++i) E[i] = H[i][i].re;
+            sort_bands<NM>(N, E, [](int) {});
+        }
+#pragma unroll
+        for (int i = 0; i < N; ++i) E_out[t * N + i] = E[i];
+        return;
     }
     // Atom gauge + tau term
     zc ph[NM];
     double tp0[NM], tp1[NM];
-    // energies only: the Atom-gauge phase is a unitary similarity and leaves them unchanged
-    for (int s = 0; s < (VALS ? 0 : N); ++s) {
-        const double* ts = tau + 3 * s;
+#pragma unroll
+    for (int s = 0; s < N; ++s) {
+        const double* ts = s_tau + 5 * s;
         double a = ts[0] * kv[0];
         if (dim > 1) a += ts[1] * kv[1];
         if (dim > 2) a += ts[2] * kv[2];
         double sn, cs;
-        sincos(kTwoPiS * a, &sn, &cs);
+        sincospi(2.0 * a, &sn, &cs);
         ph[s] = mk(cs, sn);
-        const double* tc = taucart + 3 * s;
-        double p0 = w0[0] * tc[0], p1 = w1[0] * tc[0];
-        if (dim > 1) {
-            p0 += w0[1] * tc[1];
-            p1 += w1[1] * tc[1];
-        }
-        if (dim > 2) {
-            p0 += w0[2] * tc[2];
-            p1 += w1[2] * tc[2];
-        }
-        tp0[s] = p0;
-        tp1[s] = p1;
+        tp0[s] = ts[3];
+        tp1[s] = ts[4];
     }
-    for (int m = 0; m < (VALS ? 0 : N); ++m)
+#pragma unroll
+    for (int m = 0; m < N; ++m)
+#pragma unroll
         for (int n = 0; n < N; ++n) {
             const zc g = cmul(ph[m], ph[n]);
             const zc hl = H[m][n];
@@ -180,7 +307,7 @@ __global__ void __launch_bounds__(128) small_fused_kernel(
             V1[m][n] = (V1[m][n] + mk(-d1 * hl.im, d1 * hl.re)) * g;
             H[m][n] = hl * g;
         }
-    if (!VALS && spin >= 0) {  // J = 1/2 (S V0 + V0 S), S = sigma (x) I / 2
+    if (spin >= 0) {  // J = 1/2 (S V0 + V0 S), S = sigma (x) I / 2
         zc J[NM][NM];
         for (int i = 0; i < N; ++i)
             for (int j = 0; j < N; ++j) {
@@ -202,56 +329,59 @@ __global__ void __launch_bounds__(128) small_fused_kernel(
                 ent(i, pi, si);
                 ent(j, pj, sj);
                 ent(pj, ppj, sj);  // (V S)[i][j] = V[i][pi(j)] S[pi(j)][j]
-                const zc a = si * V0[pi][j];
-                const zc c = V0[i][pj] * sj;
+                zc vi = V0[0][0], vj = V0[0][0];  // V0[pi][j], V0[i][pj] by constant indices
+#pragma unroll
+                for (int x = 0; x < N; ++x) {
+                    if (x == pi) vi = V0[x][j];
+                    if (x == pj) vj = V0[i][x];
+                }
+                const zc a = si * vi;
+                const zc c = vj * sj;
                 J[i][j] = mk(0.5 * (a.re + c.re), 0.5 * (a.im + c.im));
             }
+#pragma unroll
         for (int i = 0; i < N; ++i)
+#pragma unroll
             for (int j = 0; j < N; ++j) V0[i][j] = J[i][j];
     }
     zc W[NM][NM];
-    jacobi<NM, !VALS>(N, H, W);
+    jacobi<NM, true>(N, H, W);
     double E[NM];
-    int ord[NM];
-    for (int i = 0; i < N; ++i) {
-        E[i] = H[i][i].re;
-        ord[i] = i;
-    }
-    for (int i = 1; i < N; ++i) {  // ascending order (insertion sort of the index)
-        const int oi = ord[i];
-        int j = i - 1;
-        while (j >= 0 && E[ord[j]] > E[oi]) {
-            ord[j + 1] = ord[j];
-            --j;
-        }
-        ord[j + 1] = oi;
-    }
-    if (VALS) {
-        for (int i = 0; i < N; ++i) E_out[t * N + i] = E[ord[i]];
-        return;
-    }
-    // band-basis velocities B = W^H V W (H reused as scratch)
+#pragma unroll
+    for (int i = 0; i < N; ++i) E[i] = H[i][i].re;
+    // band-basis velocities B = W^H V W
     zc Bx[NM][NM], By[NM][NM];
-    for (int a = 0; a < N; ++a)
-        for (int b = 0; b < N; ++b) {
+#pragma unroll
+    for (int b = 0; b < N; ++b) {
+        zc tx[NM], ty[NM];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            tx[i] = ty[i] = mk(0.0, 0.0);
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                fma_cx(tx[i], V0[i][j], W[j][b]);
+                fma_cx(ty[i], V1[i][j], W[j][b]);
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < N; ++a) {
             zc sx = mk(0.0, 0.0), sy = mk(0.0, 0.0);
+#pragma unroll
             for (int i = 0; i < N; ++i) {
-                zc tx = mk(0.0, 0.0), ty = mk(0.0, 0.0);
-                for (int j = 0; j < N; ++j) {
-                    fma_cx(tx, V0[i][j], W[j][b]);
-                    fma_cx(ty, V1[i][j], W[j][b]);
-                }
-                fma_cjx(sx, W[i][a], tx);
-                fma_cjx(sy, W[i][a], ty);
+                fma_cjx(sx, W[i][a], tx[i]);
+                fma_cjx(sy, W[i][a], ty[i]);
             }
             Bx[a][b] = sx;
             By[a][b] = sy;
         }
+    }
     const double eta2 = eta * eta;
     const bool met = Met_out || SM_out;
     double Om[NM], G[NM];
+#pragma unroll
     for (int a = 0; a < N; ++a) {
         double v = 0.0, g = 0.0;
+#pragma unroll
         for (int b = 0; b < N; ++b) {
             if (a == b) continue;
             const double im = Bx[a][b].re * By[b][a].im + Bx[a][b].im * By[b][a].re;
@@ -263,18 +393,24 @@ __global__ void __launch_bounds__(128) small_fused_kernel(
         Om[a] = v;
         G[a] = g;
     }
+    sort_bands<NM>(N, E, [&](int i) {
+        swap_d(Om[i], Om[i + 1]);
+        swap_d(G[i], G[i + 1]);
+    });
+#pragma unroll
     for (int i = 0; i < N; ++i) {
-        if (Om_out) Om_out[t * N + i] = Om[ord[i]];
-        if (E_out) E_out[t * N + i] = E[ord[i]];
-        if (Met_out) Met_out[t * N + i] = G[ord[i]];
+        if (Om_out) Om_out[t * N + i] = Om[i];
+        if (E_out) E_out[t * N + i] = E[i];
+        if (Met_out) Met_out[t * N + i] = G[i];
     }
     if (S_out) {
         for (int j = 0; j < nmu; ++j) {
             double s = 0.0, sg = 0.0;
+#pragma unroll
             for (int i = 0; i < N; ++i) {
-                const double f = fermi_s(E[ord[i]], mu[j], width);
-                s += Om[ord[i]] * f;
-                sg += G[ord[i]] * f;
+                const double f = fermi_s(E[i], mu[j], width);
+                s += Om[i] * f;
+                sg += G[i] * f;
             }
             S_out[t * nmu + j] = s;
             if (SM_out) SM_out[t * nmu + j] = sg;
@@ -286,41 +422,43 @@ __global__ void __launch_bounds__(128) small_fused_kernel(
 // matrix: cyclic Jacobi in registers, E ascending, U with the eigenvectors in
 // columns (row-major, the layout of the batched solver); U may be null.
 // Non-finite input sets bit 0 of *status, as the batched solver does.
-template <int NM>
-__global__ void __launch_bounds__(128) small_eig_kernel(int N, int64_t batch, const zc* __restrict__ H,
-                                                       double* __restrict__ E_out, zc* __restrict__ U_out,
-                                                       int* __restrict__ status) {
+template <int NM, bool EXACT>
+__global__ void __launch_bounds__(64) small_eig_kernel(int Nrt, int64_t batch, const zc* __restrict__ H,
+                                                      double* __restrict__ E_out, zc* __restrict__ U_out,
+                                                      int* __restrict__ status) {
+    const int N = EXACT ? NM : Nrt;
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= batch) return;
     const int64_t NN = (int64_t)N * N;
     zc A[NM][NM], W[NM][NM];
+#pragma unroll
     for (int i = 0; i < NM; ++i)
+#pragma unroll
         for (int j = 0; j < NM; ++j) A[i][j] = (i < N && j < N) ? H[t * NN + i * N + j] : mk(0.0, 0.0);
     jacobi<NM, true>(N, A, W);
     double E[NM];
-    int ord[NM];
+    bool bad = false;
+#pragma unroll
     for (int i = 0; i < N; ++i) {
         E[i] = A[i][i].re;
-        ord[i] = i;
-    }
-    for (int i = 1; i < N; ++i) {  // ascending (insertion sort of the index)
-        const int oi = ord[i];
-        int j = i - 1;
-        while (j >= 0 && E[ord[j]] > E[oi]) {
-            ord[j + 1] = ord[j];
-            --j;
-        }
-        ord[j + 1] = oi;
-    }
-    bool bad = false;
-    for (int i = 0; i < N; ++i) {
-        E_out[t * N + i] = E[ord[i]];
         bad = bad || !isfinite(E[i]);
     }
     if (bad && status) atomicOr(status, 1);
+    sort_bands<NM>(N, E, [&](int i) {
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            const zc w = W[r][i];
+            W[r][i] = W[r][i + 1];
+            W[r][i + 1] = w;
+        }
+    });
+#pragma unroll
+    for (int i = 0; i < N; ++i) E_out[t * N + i] = E[i];
     if (U_out)
+#pragma unroll
         for (int r = 0; r < N; ++r)
-            for (int c = 0; c < N; ++c) U_out[t * NN + r * N + c] = W[r][ord[c]];
+#pragma unroll
+            for (int c = 0; c < N; ++c) U_out[t * NN + r * N + c] = W[r][c];
 }
 
 }  // namespace
@@ -332,31 +470,47 @@ int small_fused(const ModelDev& m, cudaStream_t st, int64_t nk, const double* kl
     const int N = (int)m.nsta;
     const int64_t n0 = kmesh ? kmesh[0] : 1, n1 = (kmesh && m.dim > 1) ? kmesh[1] : 1,
                   n2 = (kmesh && m.dim > 2) ? kmesh[2] : 1;
-    const unsigned blocks = (unsigned)((nk + 127) / 128);
     KTimer kt(st, "small_fused_kernel");
     // energies only when nothing else is asked for
     const bool vals = !Om && !S && !Met && !SM;
     if (vals && !E) return TBG_OK;
-#define SMALL_LAUNCH(NM)                                                                                             \
+    // a table of the mesh's phases once it saves more than its launch takes
+    zc* ztab = nullptr;
+    if (kmesh && !klist_d && nk >= 65536) {
+        const int64_t n = n0 + n1 + n2;
+        TBG_CUDA(cudaMallocAsync(&ztab, sizeof(zc) * n, st));
+        mesh_phase_kernel<<<(unsigned)std::min<int64_t>((n + 127) / 128, 152LL * 8), 128, 0, st>>>(n0, n1, n2, ztab);
+        TBG_LAUNCHED("mesh_phase_kernel");
+    }
+    // one warp per block while that spreads a small mesh over more SMs
+    const int thr = nk <= 152 * 64 ? 32 : 64;
+    const unsigned blocks = (unsigned)((nk + thr - 1) / thr);
+    const size_t smem = sizeof(zc) * m.nR * N * N + sizeof(double) * (2 * m.nR + 5 * N) + sizeof(int) * 3 * m.nR;
+#define SMALL_LAUNCH(NM, EX)                                                                                         \
     do {                                                                                                             \
         if (vals)                                                                                                    \
-            small_fused_kernel<NM, true><<<blocks, 128, 0, st>>>(                                                    \
-                N, (int)m.norb, m.dim, (int)m.nR, nk, klist_d, k0, n0, n1, n2, m.ham, m.hamR_d, m.Rcart_d, m.tau_d, \
-                m.taucart_d, dirs_d, spin, eta, nmu, mu_d, width, Om, E, S, Met, SM);                               \
+            small_fused_kernel<NM, true, EX><<<blocks, thr, smem, st>>>(                                             \
+                N, (int)m.norb, m.dim, (int)m.nR, nk, klist_d, k0, n0, n1, n2, ztab, m.ham, m.hamR_d, m.Rcart_d,    \
+                m.tau_d, m.taucart_d, dirs_d, spin, eta, nmu, mu_d, width, Om, E, S, Met, SM);                      \
         else                                                                                                         \
-            small_fused_kernel<NM, false><<<blocks, 128, 0, st>>>(                                                   \
-                N, (int)m.norb, m.dim, (int)m.nR, nk, klist_d, k0, n0, n1, n2, m.ham, m.hamR_d, m.Rcart_d, m.tau_d, \
-                m.taucart_d, dirs_d, spin, eta, nmu, mu_d, width, Om, E, S, Met, SM);                               \
+            small_fused_kernel<NM, false, EX><<<blocks, thr, smem, st>>>(                                            \
+                N, (int)m.norb, m.dim, (int)m.nR, nk, klist_d, k0, n0, n1, n2, ztab, m.ham, m.hamR_d, m.Rcart_d,    \
+                m.tau_d, m.taucart_d, dirs_d, spin, eta, nmu, mu_d, width, Om, E, S, Met, SM);                      \
     } while (0)
-    if (N <= 2)
-        SMALL_LAUNCH(2);
-    else if (N <= 4)
-        SMALL_LAUNCH(4);
+    if (N == 2)
+        SMALL_LAUNCH(2, true);
+    else if (N <= 2)
+        SMALL_LAUNCH(2, false);
+    else if (N == 3)
+        SMALL_LAUNCH(3, true);
+    else if (N == 4)
+        SMALL_LAUNCH(4, true);
     else if (N <= 8)
-        SMALL_LAUNCH(8);
+        SMALL_LAUNCH(8, false);
     else
         return set_error(TBG_E_UNSUPPORTED, "small_fused: nsta > 8");
 #undef SMALL_LAUNCH
+    if (ztab) cudaFreeAsync(ztab, st);
     TBG_LAUNCHED("small_fused_kernel");
     return TBG_OK;
 }
@@ -366,13 +520,16 @@ int small_fused(const ModelDev& m, cudaStream_t st, int64_t nk, const double* kl
 namespace tbg {
 int eig_small(cudaStream_t st, int N, int64_t batch, const zc* H, double* E, zc* U, int* status) {
     if (batch <= 0) return TBG_OK;
-    const unsigned blocks = (unsigned)((batch + 127) / 128);
-    if (N <= 2)
-        small_eig_kernel<2><<<blocks, 128, 0, st>>>(N, batch, H, E, U, status);
-    else if (N <= 4)
-        small_eig_kernel<4><<<blocks, 128, 0, st>>>(N, batch, H, E, U, status);
+    const int thr = batch <= 152 * 64 ? 32 : 64;
+    const unsigned blocks = (unsigned)((batch + thr - 1) / thr);
+    if (N == 2)
+        small_eig_kernel<2, true><<<blocks, thr, 0, st>>>(N, batch, H, E, U, status);
+    else if (N == 3)
+        small_eig_kernel<3, true><<<blocks, thr, 0, st>>>(N, batch, H, E, U, status);
+    else if (N == 4)
+        small_eig_kernel<4, true><<<blocks, thr, 0, st>>>(N, batch, H, E, U, status);
     else
-        small_eig_kernel<8><<<blocks, 128, 0, st>>>(N, batch, H, E, U, status);
+        small_eig_kernel<8, false><<<blocks, thr, 0, st>>>(N, batch, H, E, U, status);
     TBG_LAUNCHED("small_eig_kernel");
     return TBG_OK;
 }

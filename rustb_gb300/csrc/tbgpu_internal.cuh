@@ -322,7 +322,8 @@ constexpr int kSmallMaxN = 8;
 // whose Fourier sum spreads each k-point's R sum over many threads.
 int small_max_nr();
 inline bool use_small_fused(const ModelDev& m) {
-    return m.nsta <= kSmallMaxN && m.n_rmat == 0 && m.nR <= small_max_nr();
+    return m.nsta <= kSmallMaxN && m.n_rmat == 0 && m.nR <= small_max_nr() &&
+           m.nR * (m.nsta * m.nsta + 2) <= 2600;  // its shared-memory copy stays below 48 KB
 }
 // Eigenpairs of N <= kSmallMaxN matrices by per-thread Jacobi (E ascending,
 // U columns; U may be null; non-finite input sets bit 0 of *status).
