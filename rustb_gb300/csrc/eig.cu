@@ -35,7 +35,6 @@
 #include <cstdlib>
 #include <vector>
 
-#include "eig64.cuh"
 #include "tbgpu_internal.cuh"
 
 namespace tbg {
@@ -1294,11 +1293,7 @@ int eig_batched(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, 
     if (batch <= 0) return TBG_OK;
     if (N <= kSmallMaxN) return eig_small(st, N, batch, A, E, U, status_d);  // one thread per matrix
     if (N <= jacobi_max_n()) return eig_jacobi(st, N, batch, A, E, U, status_d);  // one warp per matrix
-    if (N <= kBigMaxN) return eig64(st, N, batch, A, E, U, status_d);
-    int G, PB;
-    choose_g_pb<double>(N, false, 16, 16, G, PB);
-    return launch_heev<double, false>(st, N, batch, A, E, U, work, work_bytes, status_d, "heev_kernel<double>", G,
-                                      PB);
+    return eig64(st, N, batch, A, E, U, status_d);
 }
 
 // Eigenvalues only, FP64, of `batch` matrices held in caller-provided device
@@ -1439,16 +1434,9 @@ extern "C" int tbg_internal_eig_f64(int n, int64_t nk, const double* H, double* 
             else if (n <= kSmallMaxN)
                 rc = eig_small(0, n, nk, static_cast<zc*>(dA), static_cast<double*>(dE), static_cast<zc*>(dU),
                                static_cast<int*>(dS));
-            else if (n <= kBigMaxN)
+            else
                 rc = eig64(0, n, nk, static_cast<zc*>(dA), static_cast<double*>(dE), static_cast<zc*>(dU),
                            static_cast<int*>(dS));
-            else {
-                int G, PB;
-                choose_g_pb<double>(n, false, 16, 16, G, PB);
-                rc = launch_heev<double, false>(0, n, nk, static_cast<zc*>(dA), static_cast<double*>(dE),
-                                                static_cast<zc*>(dU), nullptr, 0, static_cast<int*>(dS),
-                                                "heev_kernel<double>", G, PB);
-            }
             cudaEventRecord(e1, 0);
             cudaError_t e = cudaEventSynchronize(e1);
             if (!rc && e != cudaSuccess) rc = cuda_error(e, "eig test");

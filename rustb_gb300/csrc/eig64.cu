@@ -903,7 +903,7 @@ bool eig64_fits(int N) { return N <= kWarpMax || cta_smem_bytes(N, cta_threads(N
 
 // Eigenvalues E (ascending) and, when U is given, eigenvectors (columns) of
 // batch N x N matrices A (upper triangles read, destroyed), N >= 1 (>= 4 with
-// vectors), N <= kBigMaxN.  With timed = false nothing is allocated, which
+// vectors).  With timed = false nothing is allocated, which
 // requires eig64_fits(N) (and N <= 256 with vectors).
 int eig64(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* status_d, bool timed) {
     if (batch <= 0) return TBG_OK;

@@ -57,9 +57,9 @@ __device__ __forceinline__ void reflector_scalars64(zc alpha, double xn, zc& tau
     }
 }
 
-// Reduction by a cluster of CTAs per matrix (eig64_big.cu).
+// Reduction by a cluster of CTAs per matrix (eig64_big.cu); a column stays in
+// shared memory (models have at most 4096 bands).
 int hetrd64_big(cudaStream_t st, int N, int64_t batch, zc* A, int* status_d);
-constexpr int kBigMaxN = 4096;  // columns in shared memory
 // Back-transformation with blocked reflectors on the tensor cores (eig64_big.cu).
 int bt64_wy(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U, int* status_d);
 

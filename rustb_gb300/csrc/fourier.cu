@@ -169,169 +169,149 @@ int launch_gemm(cudaStream_t st, int64_t nk, int nR, int ldph, int N, const zc* 
 // 2 pi k . R_q,
 //   H += c A_q + s B_q,   V_p += c_p(R_q) (c B_q - s A_q)   (c_p(R_0) = 0),
 // 8 + 2 NP FMAs per pair and element for two R (10 + 2 NP per R unpaired).
-// The velocity accumulators already hold V_p (no factor i).
+//
+// The form for little work (large sums go to the tensor cores), where latency and
+// launches count: one launch, no scratch.  A block has 32 consecutive (k, element)
+// outputs, one per lane, and deals the pairs to G warps; phases and projection
+// coefficients of kPairChunk pairs at a time are made in shared memory.  One k-point
+// of 18 bands, 125 R and three projections 490 -> 22 us, 10201 k-points of two
+// bands 186 -> 32 us, against 32 k x 64 element tiles (mostly padding there)
+// behind three launches for the phases.
+constexpr int kPairChunk = 64;
 template <int NP>
-__global__ void __launch_bounds__(256) fourier_pair_kernel(
-    int64_t nk, int Kc, int N, const zc* __restrict__ cs, const zc* __restrict__ T, const int* __restrict__ pair,
-    int nR, const double* __restrict__ coef, const zc* __restrict__ orbph, const double* __restrict__ taup,
-    int gauge, zc* __restrict__ H, int64_t ldH, zc* __restrict__ V, int64_t ldV) {
-    __shared__ zc s_A[RC][TE], s_B[RC][TE];
-    __shared__ zc s_cs[RC][TK];
-    __shared__ double s_coef[NP > 0 ? NP : 1][RC];
-    const int tid = threadIdx.x;
-    const int te = tid & 15;  // element lane: e = te + 16 j
-    const int tk = tid >> 4;  // k lane: k = tk + 16 i
-    const int64_t NN = (int64_t)N * N;
-    const int64_t e0 = (int64_t)blockIdx.x * TE;
-    const int64_t k0 = (int64_t)blockIdx.y * TK;
-
-    zc accH[2][4];
-    zc accV[NP > 0 ? NP : 1][2][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            accH[i][j] = mk(0.0, 0.0);
-#pragma unroll
-            for (int p = 0; p < NP; ++p) accV[p][i][j] = mk(0.0, 0.0);
-        }
-
-    for (int q0 = 0; q0 < Kc; q0 += RC) {
-        for (int idx = tid; idx < RC * TE; idx += 256) {
-            const int r = idx / TE, e = idx % TE;
-            zc a = mk(0.0, 0.0), b = mk(0.0, 0.0);
-            if (q0 + r < Kc && e0 + e < NN) {
-                a = T[(int64_t)(2 * (q0 + r)) * NN + e0 + e];
-                b = T[(int64_t)(2 * (q0 + r) + 1) * NN + e0 + e];
-            }
-            s_A[r][e] = a;
-            s_B[r][e] = b;
-        }
-        {
-            const int r = tid / TK, kk = tid % TK;  // 256 == RC*TK
-            zc u = mk(0.0, 0.0);
-            if (q0 + r < Kc && k0 + kk < nk) u = cs[(k0 + kk) * Kc + q0 + r];
-            s_cs[r][kk] = u;
-        }
-        if (NP > 0 && tid < NP * RC) {
-            const int p = tid / RC, r = tid % RC, q = q0 + r;
-            s_coef[p][r] = (q > 0 && q < Kc) ? coef[(int64_t)p * nR + pair[q - 1]] : 0.0;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < RC; ++r) {
-            zc a[4], b[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                a[j] = s_A[r][te + 16 * j];
-                b[j] = s_B[r][te + 16 * j];
-            }
-            double cp[NP > 0 ? NP : 1];
-#pragma unroll
-            for (int p = 0; p < NP; ++p) cp[p] = s_coef[p][r];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const zc u = s_cs[r][tk + 16 * i];  // (cos, sin)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    accH[i][j].re = fma(u.re, a[j].re, accH[i][j].re);
-                    accH[i][j].re = fma(u.im, b[j].re, accH[i][j].re);
-                    accH[i][j].im = fma(u.re, a[j].im, accH[i][j].im);
-                    accH[i][j].im = fma(u.im, b[j].im, accH[i][j].im);
-                    if (NP > 0) {
-                        const double wr = fma(u.re, b[j].re, -u.im * a[j].re);
-                        const double wi = fma(u.re, b[j].im, -u.im * a[j].im);
-#pragma unroll
-                        for (int p = 0; p < NP; ++p) {
-                            accV[p][i][j].re = fma(cp[p], wr, accV[p][i][j].re);
-                            accV[p][i][j].im = fma(cp[p], wi, accV[p][i][j].im);
-                        }
-                    }
-                }
-            }
-        }
-        __syncthreads();
-    }
-
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int64_t kk = k0 + tk + 16 * i;
-        if (kk >= nk) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int64_t e = e0 + te + 16 * j;
-            if (e >= NN) continue;
-            const int mrow = (int)(e / N), ncol = (int)(e % N);
-            const zc hl = accH[i][j];
-            zc g = mk(1.0, 0.0);
-            if (gauge == TBG_GAUGE_ATOM) g = cmul(orbph[kk * N + mrow], orbph[kk * N + ncol]);
-            if (H) H[kk * ldH + e] = hl * g;
-#pragma unroll
-            for (int p = 0; p < NP; ++p) {
-                zc v = accV[p][i][j];
-                if (gauge == TBG_GAUGE_ATOM) {
-                    const double diff = taup[p * N + ncol] - taup[p * N + mrow];
-                    v.re -= diff * hl.im;
-                    v.im += diff * hl.re;
-                    v = v * g;
-                }
-                V[kk * ldV + p * NN + e] = v;
-            }
-        }
-    }
-}
-
-// (cos, sin) of 2 pi k . R_q per k-point and pair (pair 0: R = 0), from the
-// same operation order as phases_kernel.
-__global__ void phases_pair_kernel(int64_t nk, int dim, const double* __restrict__ k, int np,
-                                   const int* __restrict__ pair, const int* __restrict__ hamR, zc* __restrict__ cs) {
+__global__ void __launch_bounds__(256) fourier_few_kernel(
+    int64_t nk, int dim, const double* __restrict__ k, int np, const int* __restrict__ pair,
+    const int* __restrict__ hamR, const double* __restrict__ Rcart, const zc* __restrict__ T, int N,
+    const double* __restrict__ tau, const double* __restrict__ taucart, const double* __restrict__ dirs, int gauge,
+    zc* __restrict__ H, int64_t ldH, zc* __restrict__ V, int64_t ldV) {
+    constexpr int NV = NP > 0 ? NP : 1;
+    extern __shared__ __align__(16) unsigned char few_smem[];
+    __shared__ double s_coef[NV][kPairChunk];
+    const int lane = threadIdx.x, g = threadIdx.y, G = blockDim.y, tid = g * 32 + lane;
+    const int64_t NN = (int64_t)N * N, total = nk * NN, first = blockIdx.x * (int64_t)32;
+    const int64_t kf = first / NN, idx = min(first + lane, total - 1), kk = idx / NN;
+    const int nks = (int)(min(first + 31, total - 1) / NN - kf) + 1;
+    const int64_t e = idx - kk * NN;
+    zc* s_cs = reinterpret_cast<zc*>(few_smem);       // (nks, kPairChunk)
+    zc* s_red = s_cs;                                 // then (G, 1 + NP, 32)
     const int Kc = np + 1;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < nk * Kc;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t kk = idx / Kc;
-        const int q = (int)(idx % Kc);
-        if (q == 0) {
-            cs[idx] = mk(1.0, 0.0);
-            continue;
+    zc accH = mk(0.0, 0.0), accV[NV];
+#pragma unroll
+    for (int p = 0; p < NV; ++p) accV[p] = mk(0.0, 0.0);
+    for (int q0 = 0; q0 < Kc; q0 += kPairChunk) {
+        const int nq = min(kPairChunk, Kc - q0);
+        __syncthreads();
+        for (int t = tid; t < nks * nq; t += 32 * G) {
+            const int kl = t / nq, q = t - kl * nq;
+            zc u = mk(1.0, 0.0);
+            if (q0 + q > 0) {
+                const int* r = hamR + 3 * pair[q0 + q - 1];
+                const double* kv = k + (kf + kl) * dim;
+                double s = (double)r[0] * kv[0];
+                if (dim > 1) s += (double)r[1] * kv[1];
+                if (dim > 2) s += (double)r[2] * kv[2];
+                sincospi(2.0 * s, &u.im, &u.re);
+            }
+            s_cs[kl * kPairChunk + q] = u;
         }
-        const int* r = hamR + 3 * pair[q - 1];
-        const double* kv = k + kk * dim;
-        double s = (double)r[0] * kv[0];
-        if (dim > 1) s += (double)r[1] * kv[1];
-        if (dim > 2) s += (double)r[2] * kv[2];
-        double sn, c;
-        sincos(kTwoPi * s, &sn, &c);
-        cs[idx] = mk(c, sn);
+        if (NP > 0)
+            for (int t = tid; t < NP * nq; t += 32 * G) {
+                const int p = t / nq, q = t - p * nq;
+                double c = 0.0;
+                if (q0 + q > 0) {
+                    const double *r = Rcart + 3 * pair[q0 + q - 1], *w = dirs + p * dim;
+                    c = w[0] * r[0];
+                    if (dim > 1) c += w[1] * r[1];
+                    if (dim > 2) c += w[2] * r[2];
+                }
+                s_coef[p][q] = c;
+            }
+        __syncthreads();
+        const zc* cs = s_cs + (kk - kf) * kPairChunk;
+        const zc* t0 = T + (int64_t)(2 * q0) * NN + e;
+#pragma unroll 4
+        for (int q = g; q < nq; q += G) {
+            const zc a = t0[(2 * q) * NN], b = t0[(2 * q + 1) * NN], u = cs[q];  // (cos, sin)
+            accH.re = fma(u.re, a.re, accH.re);
+            accH.re = fma(u.im, b.re, accH.re);
+            accH.im = fma(u.re, a.im, accH.im);
+            accH.im = fma(u.im, b.im, accH.im);
+            if (NP > 0) {
+                const double wr = fma(u.re, b.re, -u.im * a.re), wi = fma(u.re, b.im, -u.im * a.im);
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    accV[p].re = fma(s_coef[p][q], wr, accV[p].re);
+                    accV[p].im = fma(s_coef[p][q], wi, accV[p].im);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    // sums over the G warps: warp p takes output p
+    s_red[(g * (1 + NP)) * 32 + lane] = accH;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) s_red[(g * (1 + NP) + 1 + p) * 32 + lane] = accV[p];
+    __syncthreads();
+    const bool on = first + lane < total;
+    const int m = (int)(e / N), n = (int)(e - (int64_t)m * N);
+    for (int o = g; o <= NP; o += G) {
+        auto sum = [&](int i) {
+            zc t = s_red[i * 32 + lane];
+            for (int w = 1; w < G; ++w) t = t + s_red[(w * (1 + NP) + i) * 32 + lane];
+            return t;
+        };
+        const zc hl = sum(0);
+        zc ph = mk(1.0, 0.0), v = o > 0 ? sum(o) : hl;
+        if (gauge == TBG_GAUGE_ATOM) {
+            // conj(phi_m) phi_n
+            const double *kv = k + kk * dim, *tm = tau + 3 * m, *tn = tau + 3 * n;
+            double sm = tm[0] * kv[0], sn = tn[0] * kv[0];
+            if (dim > 1) sm += tm[1] * kv[1], sn += tn[1] * kv[1];
+            if (dim > 2) sm += tm[2] * kv[2], sn += tn[2] * kv[2];
+            zc fm, fn;
+            sincospi(2.0 * sm, &fm.im, &fm.re);
+            sincospi(2.0 * sn, &fn.im, &fn.re);
+            ph = cmul(fm, fn);
+            if (o > 0) {
+                const double* w = dirs + (o - 1) * dim;
+                const double *cm = taucart + 3 * m, *cn = taucart + 3 * n;
+                double pm = w[0] * cm[0], pn = w[0] * cn[0];
+                if (dim > 1) pm += w[1] * cm[1], pn += w[1] * cn[1];
+                if (dim > 2) pm += w[2] * cm[2], pn += w[2] * cn[2];
+                const double diff = pn - pm;
+                v.re -= diff * hl.im;
+                v.im += diff * hl.re;
+            }
+            v = v * ph;
+        }
+        if (!on) continue;
+        if (o > 0)
+            V[kk * ldV + (o - 1) * NN + e] = v;
+        else if (H)
+            H[kk * ldH + e] = v;
     }
 }
 
 template <int NP>
-int launch_pair(cudaStream_t st, int64_t nk, int Kc, int N, const zc* cs, const zc* T, const int* pair, int nR,
-                const double* coef, const zc* orbph, const double* taup, int gauge, zc* H, int64_t ldH, zc* V,
-                int64_t ldV) {
+int launch_few(cudaStream_t st, const ModelDev& m, int64_t nk, const double* k_d, const double* dirs, int gauge, zc* H,
+               int64_t ldH, zc* V, int64_t ldV) {
+    const int N = (int)m.nsta, Kc = m.hop_K;
     const int64_t NN = (int64_t)N * N;
     // algorithmic work as for the unpaired sum (8 nR N^2 per output matrix)
-    KTimer kt(st, "fourier_gemm_kernel", 8.0 * nR * (double)NN * nk * ((H ? 1 : 0) + NP));
-    for (int64_t kb = 0; kb < nk; kb += (int64_t)TK * 65535) {
-        const int64_t nkb = std::min<int64_t>(nk - kb, (int64_t)TK * 65535);
-        dim3 grid((unsigned)((NN + TE - 1) / TE), (unsigned)((nkb + TK - 1) / TK));
-        fourier_pair_kernel<NP><<<grid, 256, 0, st>>>(nkb, Kc, N, cs + kb * Kc, T, pair, nR, coef, orbph + kb * N,
-                                                        taup, gauge, H ? H + kb * ldH : nullptr, ldH,
-                                                        V ? V + kb * ldV : nullptr, ldV);
-        TBG_LAUNCHED("fourier_pair_kernel");
+    KTimer kt(st, "fourier_gemm_kernel", 8.0 * m.nR * (double)NN * nk * ((H ? 1 : 0) + NP));
+    int G = 1;
+    while (G < 8 && 4 * G < Kc) G *= 2;
+    const int64_t nks = std::min<int64_t>(nk, 31 / NN + 2);
+    const size_t smem = sizeof(zc) * std::max<size_t>((size_t)nks * kPairChunk, (size_t)G * (1 + NP) * 32);
+    const int64_t step = std::max<int64_t>(1, (int64_t(1) << 35) / NN);  // blocks within a grid's limit
+    for (int64_t kb = 0; kb < nk; kb += step) {
+        const int64_t n = std::min(step, nk - kb);
+        fourier_few_kernel<NP><<<(unsigned)((n * NN + 31) / 32), dim3(32, G), smem, st>>>(
+            n, m.dim, k_d + kb * m.dim, m.hop_np, m.hop_pair_d, m.hamR_d, m.Rcart_d, m.pair_T, N, m.tau_d, m.taucart_d,
+            dirs, gauge, H ? H + kb * ldH : nullptr, ldH, V ? V + kb * ldV : nullptr, ldV);
+        TBG_LAUNCHED("fourier_few_kernel");
     }
     return TBG_OK;
-}
-
-int dispatch_pair(cudaStream_t st, int np, int64_t nk, int Kc, int N, const zc* cs, const zc* T, const int* pair,
-                  int nR, const double* coef, const zc* orbph, const double* taup, int gauge, zc* H, int64_t ldH,
-                  zc* V, int64_t ldV) {
-    switch (np) {
-        case 0: return launch_pair<0>(st, nk, Kc, N, cs, T, pair, nR, coef, orbph, taup, gauge, H, ldH, V, ldV);
-        case 1: return launch_pair<1>(st, nk, Kc, N, cs, T, pair, nR, coef, orbph, taup, gauge, H, ldH, V, ldV);
-        case 2: return launch_pair<2>(st, nk, Kc, N, cs, T, pair, nR, coef, orbph, taup, gauge, H, ldH, V, ldV);
-        default: return launch_pair<3>(st, nk, Kc, N, cs, T, pair, nR, coef, orbph, taup, gauge, H, ldH, V, ldV);
-    }
 }
 
 // i A of the rmatrix Fourier sum, with the gauge transform and the zeroed
@@ -1101,7 +1081,7 @@ int fourier_oz64(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k
 int fourier_direct(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k_d, int gauge, int nproj,
                    const double* dirs_d, zc* H, zc* V, int64_t ldH, int64_t ldV, int* status_d) {
     if (nk <= 0) return TBG_OK;
-    const int N = (int)m.nsta, nR = (int)m.nR;
+    const int N = (int)m.nsta;
     bool oz = false;
     {
         // the +-R paired table, built once per model (a cache: logically const)
@@ -1113,48 +1093,19 @@ int fourier_direct(const ModelDev& m, cudaStream_t st, int64_t nk, const double*
         oz = oz && m.oz_img;
     }
     if (oz) return fourier_oz64(m, st, nk, k_d, gauge, nproj, dirs_d, H, V, ldH, ldV, status_d);
-    const int Kc = m.hop_K;
-    zc *cs = nullptr, *orbph = nullptr;
-    double *coef = nullptr, *taup = nullptr;
-    TBG_CUDA(cudaMallocAsync(&cs, sizeof(zc) * nk * Kc, st));
-    TBG_CUDA(cudaMallocAsync(&orbph, sizeof(zc) * nk * N, st));
-    const int npc = std::max(nproj, 1);
-    TBG_CUDA(cudaMallocAsync(&coef, sizeof(double) * npc * nR, st));
-    TBG_CUDA(cudaMallocAsync(&taup, sizeof(double) * npc * N, st));
-    int rc = TBG_OK;
-    {
-        KTimer kt(st, "phases_kernel");
-        const int64_t t1 = nk * (int64_t)N;  // orbital phases only
-        phases_kernel<<<(unsigned)std::min<int64_t>((t1 + 255) / 256, 65535 * 8), 256, 0, st>>>(
-            nk, m.dim, k_d, 0, m.hamR_d, N, m.tau_d, cs, orbph);
-        const int64_t t2 = nk * (int64_t)Kc;
-        phases_pair_kernel<<<(unsigned)std::min<int64_t>((t2 + 255) / 256, 65535 * 8), 256, 0, st>>>(
-            nk, m.dim, k_d, m.hop_np, m.hop_pair_d, m.hamR_d, cs);
-        count_launch(2);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = cuda_error(e, "phases_kernel");
-    }
-    if (rc == TBG_OK && nproj > 0) {
-        const int total = nproj * (nR + N);
-        proj_coef_kernel<<<(total + 255) / 256, 256, 0, st>>>(nproj, m.dim, dirs_d, nR, m.Rcart_d, N,
-                                                              m.taucart_d, coef, taup);
-        count_launch();
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) rc = cuda_error(e, "proj_coef_kernel");
-    }
     // H together with up to 3 projections per pass
-    for (int p0 = 0; rc == TBG_OK && (p0 < nproj || (p0 == 0 && nproj == 0)); p0 += 3) {
-        const int np = std::min(3, std::max(0, nproj - p0));
-        zc* Hout = (p0 == 0) ? H : nullptr;
-        if (!Hout && np == 0) break;
-        rc = dispatch_pair(st, np, nk, Kc, N, cs, m.pair_T, m.hop_pair_d, nR, coef + (int64_t)p0 * nR, orbph,
-                           taup + (int64_t)p0 * N, gauge, Hout, ldH, V ? V + (int64_t)p0 * N * N : nullptr, ldV);
-        if (nproj == 0) break;
+    int rc = TBG_OK;
+    for (int p0 = 0; rc == TBG_OK && (p0 < nproj || p0 == 0); p0 += 3) {
+        const double* w = dirs_d + (int64_t)p0 * m.dim;
+        zc* Ho = p0 == 0 ? H : nullptr;
+        zc* Vo = V ? V + (int64_t)p0 * N * N : nullptr;
+        switch (std::min(3, nproj - p0)) {
+            case 0: rc = launch_few<0>(st, m, nk, k_d, w, gauge, Ho, ldH, Vo, ldV); break;
+            case 1: rc = launch_few<1>(st, m, nk, k_d, w, gauge, Ho, ldH, Vo, ldV); break;
+            case 2: rc = launch_few<2>(st, m, nk, k_d, w, gauge, Ho, ldH, Vo, ldV); break;
+            default: rc = launch_few<3>(st, m, nk, k_d, w, gauge, Ho, ldH, Vo, ldV);
+        }
     }
-    cudaFreeAsync(cs, st);
-    cudaFreeAsync(orbph, st);
-    cudaFreeAsync(coef, st);
-    cudaFreeAsync(taup, st);
     return rc;
 }
 
