@@ -1388,7 +1388,9 @@ int tbg_hall_energy_cut(const tbg_model* m, const int64_t* kmesh, const double* 
     double* Om_all = ctx.alloc<double>(nk * N);
     zc* U_all = ctx.alloc<zc>(nk * NN);
     zc* K_all = ctx.alloc<zc>(nk * NN);
-    double* Rd = ctx.alloc<double>(J.chunk * NN);
+    const bool track_gpu = N <= kEcTrackMaxN && nk > 1 && nk < (int64_t(1) << 30);
+    double* Rd = ctx.alloc<double>(track_gpu ? nk * dim * NN : J.chunk * NN);
+    unsigned* lev = track_gpu ? ctx.alloc<unsigned>(2 * (dim == 3 ? kmesh[0] * kmesh[1] : kmesh[0])) : nullptr;
     int* perm_d = ctx.alloc<int>(nk * N);
     if (ctx.rc) return ctx.rc;
     if ((rc = alloc_berry(ctx, J))) return rc;
@@ -1407,7 +1409,7 @@ int tbg_hall_energy_cut(const tbg_model* m, const int64_t* kmesh, const double* 
     // 2. squared overlaps of the forward mesh edges, per dimension
     const int64_t n3[3] = {n0, n1, n2};
     const int64_t stride[3] = {n3[1] * n3[2], n3[2], 1};
-    std::vector<double> R_h((size_t)nk * dim * NN, 0.0);
+    std::vector<double> R_h(track_gpu ? 0 : (size_t)nk * dim * NN, 0.0);
     for (int d = 0; d < dim; ++d) {
         const int64_t sd = stride[d];
         for (int64_t a0 = 0; a0 + sd < nk; a0 += J.chunk) {
@@ -1415,17 +1417,24 @@ int tbg_hall_energy_cut(const tbg_model* m, const int64_t* kmesh, const double* 
             if ((rc = zgemm_batched(ctx.st, N, na, true, U_all + a0 * NN, NN, U_all + (a0 + sd) * NN, NN, J.scratch,
                                     NN, J.status_d)))
                 return rc;
-            if ((rc = ec_abs2(ctx.st, na * NN, J.scratch, Rd))) return rc;
+            if ((rc = ec_abs2(ctx.st, na * NN, J.scratch, track_gpu ? Rd + (d * nk + a0) * NN : Rd))) return rc;
+            if (track_gpu) continue;
             TBG_CUDA(cudaMemcpy2DAsync(R_h.data() + ((size_t)a0 * dim + d) * NN, sizeof(double) * dim * NN, Rd,
                                        sizeof(double) * NN, sizeof(double) * NN, na, cudaMemcpyDeviceToHost, ctx.st));
             if (ctx.sync("tbg_hall_energy_cut overlaps")) return ctx.rc;
         }
     }
-    if ((rc = check_status(J.status_d, ctx.st))) return rc;
-    // 3. band tracking on the host, permutations to the device
-    std::vector<int> perm_h((size_t)nk * N);
-    ec_track(dim, kmesh, N, R_h.data(), perm_h.data());
-    TBG_CUDA(cudaMemcpyAsync(perm_d, perm_h.data(), sizeof(int) * nk * N, cudaMemcpyHostToDevice, ctx.st));
+    // 3. band tracking
+    if (track_gpu) {
+        if ((rc = ec_track_gpu(ctx.st, dim, kmesh, N, Rd, perm_d, lev))) return rc;
+    } else {
+        if ((rc = check_status(J.status_d, ctx.st))) return rc;
+        // on the host, permutations to the device
+        std::vector<int> perm_h((size_t)nk * N);
+        ec_track(dim, kmesh, N, R_h.data(), perm_h.data());
+        TBG_CUDA(cudaMemcpyAsync(perm_d, perm_h.data(), sizeof(int) * nk * N, cudaMemcpyHostToDevice, ctx.st));
+        if (ctx.sync("tbg_hall_energy_cut permutations")) return ctx.rc;  // perm_h goes
+    }
     // 4. the mu grid: the chemical potentials, or the extended fine grid of the thermal convolution
     const double width = (T <= 0.0) ? 0.0 : T * 8.617333262145e-5;
     std::vector<double> grid;
@@ -1465,6 +1474,7 @@ int tbg_hall_energy_cut(const tbg_model* m, const int64_t* kmesh, const double* 
     TBG_CUDA(cudaMemcpyAsync(acc_h.data(), acc_d, sizeof(double) * ng, cudaMemcpyDeviceToHost, ctx.st));
     TBG_CUDA(cudaMemcpyAsync(full_h.data(), full_d, sizeof(double) * ng, cudaMemcpyDeviceToHost, ctx.st));
     if (ctx.sync("tbg_hall_energy_cut")) return ctx.rc;
+    if ((rc = check_status(J.status_d, ctx.st))) return rc;
     std::vector<double> s0(ng);
     for (int w0 = 0; w0 < ng; w0 += window) {  // the full-occupancy difference array restarts per window
         double run = 0.0;
