@@ -64,21 +64,106 @@ void configure_pool() {
     });
 }
 
-// Per-call context: stream + stream-ordered allocations released at the end.
+// What a call borrows: a stream, a slab of device memory for its small buffers
+// and a page of pinned host memory for small results.  Idle lanes are kept (at most
+// kIdleLanes, 1.1 MB each) while a model exists and released with the last one; a
+// lane serves one call at a time.  Creating and destroying the stream, some fifteen
+// stream-ordered allocations and a synchronous copy per small result took half of
+// the smallest calls (Hall conductivity of 961 k-points 235 -> 101 us, gen_v at one
+// k-point 122 -> 57 us).
+struct Lane {
+    int device = 0;
+    cudaStream_t st = nullptr;
+    unsigned char* slab = nullptr;
+    unsigned char* host = nullptr;
+};
+constexpr size_t kSlabBytes = 1 << 20, kSlabItem = 128 << 10, kHostBytes = 64 << 10;
+constexpr size_t kIdleLanes = 8;
+std::mutex g_lane_mu;
+std::vector<Lane> g_lanes;
+int64_t g_models = 0;
+
+void destroy_lane(Lane& l) {
+    if (l.slab) cudaFree(l.slab);
+    if (l.host) cudaFreeHost(l.host);
+    if (l.st) cudaStreamDestroy(l.st);
+    l = Lane();
+}
+int acquire_lane(Lane& l) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return cuda_error(e, "cudaGetDevice");
+    {
+        std::lock_guard<std::mutex> lk(g_lane_mu);
+        for (size_t i = g_lanes.size(); i-- > 0;)
+            if (g_lanes[i].device == dev) {
+                l = g_lanes[i];
+                g_lanes.erase(g_lanes.begin() + (std::ptrdiff_t)i);
+                return TBG_OK;
+            }
+    }
+    l.device = dev;
+    e = cudaStreamCreateWithFlags(&l.st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMalloc(&l.slab, kSlabBytes);
+    if (e == cudaSuccess) e = cudaMallocHost(&l.host, kHostBytes);
+    if (e == cudaSuccess) return TBG_OK;
+    destroy_lane(l);
+    return cuda_error(e, "call context");
+}
+void release_lane(Lane& l, bool healthy) {
+    if (healthy) {
+        std::lock_guard<std::mutex> lk(g_lane_mu);
+        if (g_models > 0 && g_lanes.size() < kIdleLanes) {
+            g_lanes.push_back(l);
+            return;
+        }
+    }
+    destroy_lane(l);
+}
+// Live models; with the last one the idle lanes go.
+void count_models(int d) {
+    std::vector<Lane> drop;
+    {
+        std::lock_guard<std::mutex> lk(g_lane_mu);
+        g_models += d;
+        if (g_models <= 0) drop.swap(g_lanes);
+    }
+    int dev = 0;
+    if (drop.empty() || cudaGetDevice(&dev) != cudaSuccess) return;
+    for (Lane& l : drop) {
+        cudaSetDevice(l.device);
+        destroy_lane(l);
+    }
+    cudaSetDevice(dev);
+}
+
+// Per-call context: a lane, small buffers from its slab, large ones stream-ordered;
+// everything is given back at the end, after the stream has drained.
 struct Ctx {
+    Lane lane;
     cudaStream_t st = nullptr;
     std::vector<void*> bufs;
+    size_t slab_at = 0, host_at = 64;  // the first 64 bytes of host take the status word
     int rc = TBG_OK;
     Ctx() {
         configure_pool();
-        cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-        if (e != cudaSuccess) rc = cuda_error(e, "cudaStreamCreate");
+        rc = acquire_lane(lane);
+        st = lane.st;
+        if (rc == TBG_OK) std::memset(lane.host, 0, 64);
     }
+    Ctx(const Ctx&) = delete;
+    Ctx& operator=(const Ctx&) = delete;
     template <typename T>
     T* alloc(size_t count) {
         if (rc != TBG_OK) return nullptr;
+        const size_t bytes = (std::max<size_t>(count, 1) * sizeof(T) + 255) & ~size_t(255);
+        if (bytes <= kSlabItem && slab_at + bytes <= kSlabBytes) {
+            T* p = reinterpret_cast<T*>(lane.slab + slab_at);
+            slab_at += bytes;
+            return p;
+        }
         void* p = nullptr;
-        cudaError_t e = cudaMallocAsync(&p, std::max<size_t>(count, 1) * sizeof(T), st);
+        cudaError_t e = cudaMallocAsync(&p, bytes, st);
         if (e != cudaSuccess) {
             rc = cuda_error(e, "cudaMallocAsync");
             return nullptr;
@@ -86,6 +171,24 @@ struct Ctx {
         bufs.push_back(p);
         return static_cast<T*>(p);
     }
+    // Device -> pinned host copy of count values, readable after sync(); null when
+    // the page is full (the caller then copies to its own memory).
+    template <typename T>
+    const T* fetch(const T* d, size_t count) {
+        const size_t bytes = (count * sizeof(T) + 15) & ~size_t(15);
+        if (host_at + bytes > kHostBytes) return nullptr;
+        T* h = reinterpret_cast<T*>(lane.host + host_at);
+        const cudaError_t e = cudaMemcpyAsync(h, d, count * sizeof(T), cudaMemcpyDeviceToHost, st);
+        if (e != cudaSuccess && rc == TBG_OK) rc = cuda_error(e, "result copy");
+        host_at += bytes;
+        return h;
+    }
+    // The status word: queued behind the kernels, read after the next sync().
+    void fetch_status(const int* status_d) {
+        const cudaError_t e = cudaMemcpyAsync(lane.host, status_d, sizeof(int), cudaMemcpyDeviceToHost, st);
+        if (e != cudaSuccess && rc == TBG_OK) rc = cuda_error(e, "status readback");
+    }
+    int status() const { return *reinterpret_cast<const volatile int*>(lane.host); }
     int sync(const char* where) {
         cudaError_t e = cudaStreamSynchronize(st);
         if (e != cudaSuccess && rc == TBG_OK) rc = cuda_error(e, where);
@@ -93,12 +196,11 @@ struct Ctx {
         return rc;
     }
     ~Ctx() {
-        if (st) {
-            for (void* p : bufs) cudaFreeAsync(p, st);
-            cudaStreamSynchronize(st);
-            timing_flush();
-            cudaStreamDestroy(st);
-        }
+        if (!st) return;
+        for (void* p : bufs) cudaFreeAsync(p, st);
+        const bool healthy = cudaStreamSynchronize(st) == cudaSuccess;
+        timing_flush();
+        release_lane(lane, healthy);
     }
 };
 
@@ -134,6 +236,9 @@ int64_t choose_chunk(int64_t nk, int64_t per_k_bytes) {
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || nsm < 1) nsm = 1;
     const int64_t q = 2 * (int64_t)nsm;
     per_k_bytes = std::max<int64_t>(per_k_bytes, 1);
+    // the budget is never below 6 GB: no need to ask for work that fits it
+    if (!std::getenv("TBG_CHUNK_BYTES") && !std::getenv("TBG_MAX_CHUNK") && nk <= 65535 && nk <= (6LL << 30) / per_k_bytes)
+        return std::max<int64_t>(1, nk);
     int64_t budget = chunk_budget_bytes();
     if (!std::getenv("TBG_CHUNK_BYTES") && budget / per_k_bytes < std::min<int64_t>(nk, q)) {
         // large matrices: room for one full wave of the per-matrix kernels
@@ -306,7 +411,7 @@ struct BerryJob {
     double* k_d;
     zc *H, *V, *U, *scratch, *Hcopy;
     double *E, *Om;
-    int* status_d;
+    int* status_d = nullptr;  // the caller's (zeroed), or allocated with the buffers
     void* work;
     size_t work_bytes;
     void* fwork;
@@ -331,7 +436,8 @@ int alloc_berry(Ctx& ctx, BerryJob& J) {
     J.E = ctx.alloc<double>(c * N);
     J.Om = ctx.alloc<double>(c * N);
     J.Met = J.want_metric ? ctx.alloc<double>(c * N) : nullptr;
-    J.status_d = ctx.alloc<int>(1);
+    const bool own_status = !J.status_d;
+    if (own_status) J.status_d = ctx.alloc<int>(1);
     J.Hcopy = nullptr;
     J.U32 = nullptr;
     J.work = nullptr;
@@ -347,7 +453,7 @@ int alloc_berry(Ctx& ctx, BerryJob& J) {
         J.pairs = ctx.alloc<float4>(3 * c * NN);
         J.rexp = ctx.alloc<int>(3 * c * N);
     }
-    if (ctx.rc == TBG_OK) {
+    if (ctx.rc == TBG_OK && own_status) {
         cudaError_t e = cudaMemsetAsync(J.status_d, 0, sizeof(int), ctx.st);
         if (e != cudaSuccess) ctx.rc = cuda_error(e, "memset status");
     }
@@ -543,6 +649,7 @@ int tbg_model_create(int dim, int spin, int64_t norb, int64_t nR, const int64_t*
                 return set_error(TBG_E_INVALID_MODEL, "R component out of range");
     }
     tbg_model* m = new tbg_model();
+    count_models(1);
     ModelDev& M = m->d;
     cudaGetDevice(&M.device);
     M.dim = dim;
@@ -629,6 +736,7 @@ int tbg_model_destroy(tbg_model* m) {
     cudaFree(M.oz_EB);
     M.ham = nullptr;
     delete m;
+    count_models(-1);
     return TBG_OK;
 }
 
@@ -662,7 +770,6 @@ int tbg_gen_v_projected(const tbg_model* m, int64_t nk, const double* k, int gau
     int* status_d = ctx.alloc<int>(1);
     if (ctx.rc) return ctx.rc;
     TBG_CUDA(cudaMemsetAsync(status_d, 0, sizeof(int), ctx.st));
-    int status_h = 0;
     if (n_proj) TBG_CUDA(cudaMemcpyAsync(dirs_d, dirs, sizeof(double) * n_proj * M.dim, cudaMemcpyHostToDevice, ctx.st));
     for (int64_t c0 = 0; c0 < nk; c0 += chunk) {
         const int64_t nkc = std::min(chunk, nk - c0);
@@ -674,16 +781,15 @@ int tbg_gen_v_projected(const tbg_model* m, int64_t nk, const double* k, int gau
             rc = rmatrix_term(M, ctx.st, nkc, k_d, gauge, (int)n_proj, dirs_d, H, V, status_d);
             if (rc) return rc;
         }
+        ctx.fetch_status(status_d);
         if (H_out)
             TBG_CUDA(cudaMemcpyAsync(H_out + c0 * NN * 2, H, sizeof(zc) * nkc * NN, cudaMemcpyDeviceToHost, ctx.st));
         if (n_proj)
             TBG_CUDA(cudaMemcpyAsync(V_out + c0 * n_proj * NN * 2, V, sizeof(zc) * nkc * n_proj * NN,
                                      cudaMemcpyDeviceToHost, ctx.st));
-        if (c0 + nkc >= nk)
-            TBG_CUDA(cudaMemcpyAsync(&status_h, status_d, sizeof(int), cudaMemcpyDeviceToHost, ctx.st));
         if (ctx.sync("tbg_gen_v_projected")) return ctx.rc;
     }
-    return status_error(status_h);
+    return status_error(ctx.status());
 }
 
 int tbg_gen_ham(const tbg_model* m, int64_t nk, const double* k, int gauge, double* H_out) {
@@ -726,6 +832,7 @@ static int solve_impl(const tbg_model* m, int64_t nk, const double* k, double* E
         if (rc) return rc;
         rc = eig_batched(ctx.st, N, nkc, H, E, U, nullptr, 0, status_d);
         if (rc) return rc;
+        ctx.fetch_status(status_d);
         TBG_CUDA(cudaMemcpyAsync(E_out + c0 * N, E, sizeof(double) * nkc * N, cudaMemcpyDeviceToHost, ctx.st));
         if (U_out) {
             const zc* src = U;
@@ -738,8 +845,7 @@ static int solve_impl(const tbg_model* m, int64_t nk, const double* k, double* E
         }
         if (ctx.sync("tbg_solve")) return ctx.rc;
     }
-    if ((rc = check_status(status_d, ctx.st))) return rc;
-    return ctx.sync("tbg_solve");
+    return status_error(ctx.status());
 }
 
 int tbg_solve_band(const tbg_model* m, int64_t nk, const double* k, double* E_out) {
@@ -788,11 +894,11 @@ static int solve_band_mixed(const tbg_model* m, int64_t nk, const double* k, dou
         if (rc) return rc;
         if ((rc = mixed_berry(ctx.st, N, nkc, P, nullptr, nullptr, 0.0, E, nullptr, work, wb, status_d, clusters_d)))
             return rc;
+        ctx.fetch_status(status_d);
         TBG_CUDA(cudaMemcpyAsync(E_out + c0 * N, E, sizeof(double) * nkc * N, cudaMemcpyDeviceToHost, ctx.st));
     }
     if (ctx.sync("tbg_solve_band_prec")) return ctx.rc;
-    if ((rc = check_status(status_d, ctx.st))) return rc;
-    return ctx.sync("tbg_solve_band_prec");
+    return status_error(ctx.status());
 }
 
 int tbg_solve_band_prec(const tbg_model* m, int64_t nk, const double* k, int precision, double* E_out) {
@@ -856,6 +962,7 @@ static int berry_common(const tbg_model* m, int64_t nk, const double* k, const d
             if ((rc = small_fused(M, ctx.st, nkc, J.k_d, 0, nullptr, dirs_d, spin, eta, occ_out ? nmu : 0, mu_d, width,
                                   J.Om, J.E, occ_out ? S : nullptr, J.Met)))
                 return rc;
+            ctx.fetch_status(J.status_d);
             if (Met_out)
                 TBG_CUDA(cudaMemcpyAsync(Met_out + c0 * N, J.Met, sizeof(double) * nkc * N, cudaMemcpyDeviceToHost,
                                          ctx.st));
@@ -870,6 +977,7 @@ static int berry_common(const tbg_model* m, int64_t nk, const double* k, const d
             continue;
         }
         if ((rc = run_berry_chunk(ctx, J, nkc, nullptr))) return rc;
+        ctx.fetch_status(J.status_d);
         if (Met_out)
             TBG_CUDA(cudaMemcpyAsync(Met_out + c0 * N, J.Met, sizeof(double) * nkc * N, cudaMemcpyDeviceToHost, ctx.st));
         if (Omega_out)
@@ -882,8 +990,7 @@ static int berry_common(const tbg_model* m, int64_t nk, const double* k, const d
         }
         if (ctx.sync("berry")) return ctx.rc;
     }
-    if ((rc = check_status(J.status_d, ctx.st))) return rc;
-    return ctx.sync("berry");
+    return status_error(ctx.status());
 }
 
 int tbg_berry_curvature(const tbg_model* m, int64_t nk, const double* k, const double* dirs2, int spin, double eta,
@@ -1019,6 +1126,7 @@ int tbg_berry_curvature_multi(int64_t n_models, const tbg_model* const* models, 
         }
         // the rest once for the whole chunk
         if ((rc = berry_tail(ctx, J, nkc, nullptr))) return rc;
+        ctx.fetch_status(J.status_d);
         for (const Seg& g : segs) {
             const int64_t o = (off[g.model] + g.pos) * N;
             if (Omega_out)
@@ -1031,8 +1139,7 @@ int tbg_berry_curvature_multi(int64_t n_models, const tbg_model* const* models, 
         if (ctx.sync("berry multi")) return ctx.rc;
         done += nkc;
     }
-    if ((rc = check_status(J.status_d, ctx.st))) return rc;
-    return ctx.sync("berry multi");
+    return status_error(ctx.status());
 }
 
 static int hall_impl(const tbg_model* m, const int64_t* kmesh, int64_t k_begin, int64_t k_count, bool whole,
@@ -1089,22 +1196,22 @@ static int hall_impl(const tbg_model* m, const int64_t* kmesh, int64_t k_begin, 
     J.chunk = choose_chunk(std::max<int64_t>(k_count, 1),
                            sizeof(zc) * NN * (precision == TBG_PREC_MIXED ? 15 : 5) + 64 * N + 16 * nmu +
                                (precision == TBG_PREC_MIXED ? 48 * (int64_t)M.nR : 0));
-    double* dirs_d = ctx.alloc<double>(2 * M.dim);
-    J.dirs_d = dirs_d;
-    double* mu_d = ctx.alloc<double>(nmu);
+    // one block: directions, mu, then what starts from zero: the running compensated
+    // totals (those of the metric behind), the cluster count and the status word
+    const int64_t nacc = met ? 4 * nmu : 2 * nmu, nhead = 2 * M.dim + nmu, ntail = nacc + 2;
+    double* block = ctx.alloc<double>(nhead + ntail);
     double* S = ctx.alloc<double>(J.chunk * nmu);
-    double* acc = ctx.alloc<double>(2 * nmu);
-    // metric: occupation sums and running compensated totals
     double* SG = met ? ctx.alloc<double>(J.chunk * nmu) : nullptr;
-    double* accg = met ? ctx.alloc<double>(2 * nmu) : nullptr;
-    int64_t* clusters_d = ctx.alloc<int64_t>(1);
     if (ctx.rc) return ctx.rc;
+    double *dirs_d = block, *mu_d = block + 2 * M.dim, *acc = block + nhead, *accg = acc + 2 * nmu;
+    int64_t* clusters_d = reinterpret_cast<int64_t*>(acc + nacc);
+    J.dirs_d = dirs_d;
+    J.status_d = reinterpret_cast<int*>(acc + nacc + 1);
+    std::vector<double> block_h((size_t)(nhead + ntail), 0.0);
+    std::copy(dirs2, dirs2 + 2 * M.dim, block_h.begin());
+    std::copy(mu, mu + nmu, block_h.begin() + 2 * M.dim);
+    TBG_CUDA(cudaMemcpyAsync(block, block_h.data(), sizeof(double) * block_h.size(), cudaMemcpyHostToDevice, ctx.st));
     if ((rc = alloc_berry(ctx, J))) return rc;
-    TBG_CUDA(cudaMemcpyAsync(dirs_d, dirs2, sizeof(double) * 2 * M.dim, cudaMemcpyHostToDevice, ctx.st));
-    TBG_CUDA(cudaMemcpyAsync(mu_d, mu, sizeof(double) * nmu, cudaMemcpyHostToDevice, ctx.st));
-    TBG_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * 2 * nmu, ctx.st));
-    if (met) TBG_CUDA(cudaMemsetAsync(accg, 0, sizeof(double) * 2 * nmu, ctx.st));
-    TBG_CUDA(cudaMemsetAsync(clusters_d, 0, sizeof(int64_t), ctx.st));
     const double width = (T <= 0.0) ? 0.0 : T * 8.617333262145e-5;
     const int64_t n0 = kmesh[0], n1 = M.dim > 1 ? kmesh[1] : 1, n2 = M.dim > 2 ? kmesh[2] : 1;
     const bool small = use_small_fused(M);
@@ -1142,15 +1249,20 @@ static int hall_impl(const tbg_model* m, const int64_t* kmesh, int64_t k_begin, 
         if ((rc = kahan_column_sums(ctx.st, nkc, (int)nmu, S, acc))) return rc;
         if (met && (rc = kahan_column_sums(ctx.st, nkc, (int)nmu, SG, accg))) return rc;
     }
-    std::vector<double> acc_h(2 * nmu), accg_h(met ? 2 * nmu : 0);
-    int64_t clusters_h = 0;
-    TBG_CUDA(cudaMemcpyAsync(acc_h.data(), acc, sizeof(double) * 2 * nmu, cudaMemcpyDeviceToHost, ctx.st));
-    if (met)
-        TBG_CUDA(cudaMemcpyAsync(accg_h.data(), accg, sizeof(double) * 2 * nmu, cudaMemcpyDeviceToHost, ctx.st));
-    TBG_CUDA(cudaMemcpyAsync(&clusters_h, clusters_d, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx.st));
+    // the totals, the cluster count and the status word in one copy
     cudaEventRecord(ev1, ctx.st);
+    const double* acc_h = ctx.fetch(acc, (size_t)ntail);
+    if (!acc_h) {
+        TBG_CUDA(cudaMemcpyAsync(block_h.data(), acc, sizeof(double) * ntail, cudaMemcpyDeviceToHost, ctx.st));
+        acc_h = block_h.data();
+    }
     if (ctx.sync("tbg_hall_conductivity")) return ctx.rc;
-    if ((rc = check_status(J.status_d, ctx.st))) return rc;
+    const double* accg_h = acc_h + 2 * nmu;
+    int64_t clusters_h = 0;
+    int status_h = 0;
+    std::memcpy(&clusters_h, acc_h + nacc, sizeof(clusters_h));
+    std::memcpy(&status_h, acc_h + nacc + 1, sizeof(status_h));
+    if ((rc = status_error(status_h))) return rc;
     for (int64_t j = 0; j < nmu; ++j) {
         const double s = acc_h[2 * j] - acc_h[2 * j + 1];
         out[j] = whole ? s / (double)nk / det : s;
@@ -1229,10 +1341,16 @@ int tbg_dos(const tbg_model* m, const int64_t* kmesh, double E_min, double E_max
         if ((rc = me.run(ctx, c0, nkc))) return rc;
         if ((rc = dos_accumulate(ctx.st, nkc * N, me.E, E_n, E_min, step, sigma, part, slices, acc))) return rc;
     }
-    std::vector<double> acc_h(2 * E_n);
-    TBG_CUDA(cudaMemcpyAsync(acc_h.data(), acc, sizeof(double) * 2 * E_n, cudaMemcpyDeviceToHost, ctx.st));
+    std::vector<double> own;
+    ctx.fetch_status(me.status_d);
+    const double* acc_h = ctx.fetch(acc, (size_t)(2 * E_n));
+    if (!acc_h) {
+        own.resize((size_t)(2 * E_n));
+        TBG_CUDA(cudaMemcpyAsync(own.data(), acc, sizeof(double) * 2 * E_n, cudaMemcpyDeviceToHost, ctx.st));
+        acc_h = own.data();
+    }
     if (ctx.sync("tbg_dos")) return ctx.rc;
-    if ((rc = check_status(me.status_d, ctx.st))) return rc;
+    if ((rc = status_error(ctx.status()))) return rc;
     for (int64_t i = 0; i < E_n; ++i) dos_out[i] = (acc_h[2 * i] - acc_h[2 * i + 1]) / (double)nk;
     return TBG_OK;
 }
@@ -1251,11 +1369,11 @@ int tbg_bands_mesh(const tbg_model* m, const int64_t* kmesh, double* E_out) {
     for (int64_t c0 = 0; c0 < nk; c0 += me.chunk) {
         const int64_t nkc = std::min(me.chunk, nk - c0);
         if ((rc = me.run(ctx, c0, nkc))) return rc;
+        ctx.fetch_status(me.status_d);
         TBG_CUDA(cudaMemcpyAsync(E_out + c0 * N, me.E, sizeof(double) * nkc * N, cudaMemcpyDeviceToHost, ctx.st));
         if (ctx.sync("tbg_bands_mesh")) return ctx.rc;
     }
-    if ((rc = check_status(me.status_d, ctx.st))) return rc;
-    return ctx.sync("tbg_bands_mesh");
+    return status_error(ctx.status());
 }
 
 int tbg_wilson_loops(const tbg_model* m, int64_t n_loops, int64_t n_k, const double* kvec, int64_t n_occ,
@@ -1340,12 +1458,12 @@ int tbg_wilson_loops(const tbg_model* m, int64_t n_loops, int64_t n_k, const dou
         if ((rc = wilson_from_vectors(ctx.st, M, nl, (int)n_k, kv_d, U, (int)n_occ, occ_d, svd, out_d, work, wb,
                                       status_d)))
             return rc;
+        ctx.fetch_status(status_d);
         TBG_CUDA(cudaMemcpyAsync(out + l0 * (svd ? n_occ : 1), out_d, sizeof(double) * nl * (svd ? n_occ : 1),
                                  cudaMemcpyDeviceToHost, ctx.st));
         if (ctx.sync("tbg_wilson_loops")) return ctx.rc;
     }
-    if ((rc = check_status(status_d, ctx.st))) return rc;
-    return ctx.sync("tbg_wilson_loops");
+    return status_error(ctx.status());
 }
 
 int tbg_hall_energy_cut(const tbg_model* m, const int64_t* kmesh, const double* dirs2, int64_t nmu, const double* mu,
@@ -1462,19 +1580,25 @@ int tbg_hall_energy_cut(const tbg_model* m, const int64_t* kmesh, const double* 
     double* grid_d = ctx.alloc<double>(ng);
     double* part = ctx.alloc<double>((int64_t)nblocks * window);
     double* fpart = ctx.alloc<double>((int64_t)nblocks * window);
-    double* acc_d = ctx.alloc<double>(ng);
-    double* full_d = ctx.alloc<double>(ng);
+    double* acc_d = ctx.alloc<double>(2 * (size_t)ng);
+    double* full_d = acc_d + ng;
     if (ctx.rc) return ctx.rc;
     TBG_CUDA(cudaMemcpyAsync(grid_d, grid.data(), sizeof(double) * ng, cudaMemcpyHostToDevice, ctx.st));
     // 5. occupancy cut of every simplex
     if ((rc = ec_integrate(ctx.st, dim, kmesh, N, E_all, K_all, Om_all, perm_d, ng, grid_d, eta, part, fpart, nblocks,
                            window, acc_d, full_d)))
         return rc;
-    std::vector<double> acc_h(ng), full_h(ng);
-    TBG_CUDA(cudaMemcpyAsync(acc_h.data(), acc_d, sizeof(double) * ng, cudaMemcpyDeviceToHost, ctx.st));
-    TBG_CUDA(cudaMemcpyAsync(full_h.data(), full_d, sizeof(double) * ng, cudaMemcpyDeviceToHost, ctx.st));
+    std::vector<double> own;
+    ctx.fetch_status(J.status_d);
+    const double* acc_h = ctx.fetch(acc_d, 2 * (size_t)ng);
+    if (!acc_h) {
+        own.resize(2 * (size_t)ng);
+        TBG_CUDA(cudaMemcpyAsync(own.data(), acc_d, sizeof(double) * 2 * ng, cudaMemcpyDeviceToHost, ctx.st));
+        acc_h = own.data();
+    }
+    const double* full_h = acc_h + ng;
     if (ctx.sync("tbg_hall_energy_cut")) return ctx.rc;
-    if ((rc = check_status(J.status_d, ctx.st))) return rc;
+    if ((rc = status_error(ctx.status()))) return rc;
     std::vector<double> s0(ng);
     for (int w0 = 0; w0 < ng; w0 += window) {  // the full-occupancy difference array restarts per window
         double run = 0.0;
