@@ -1433,6 +1433,10 @@ int tbg_wilson_loops(const tbg_model* m, int64_t n_loops, int64_t n_k, const dou
     void* mwork = mixed ? ctx.alloc<unsigned char>(mwb) : nullptr;
     if (ctx.rc) return ctx.rc;
     std::vector<int> occ32(occ, occ + n_occ);
+    // only the vectors of the range that holds the occupied bands are needed
+    const int occ_lo = *std::min_element(occ32.begin(), occ32.end()), occ_hi = *std::max_element(occ32.begin(), occ32.end());
+    bool run = true;
+    for (int64_t i = 0; i < n_occ; ++i) run = run && occ32[i] == occ_lo + i;
     TBG_CUDA(cudaMemcpyAsync(occ_d, occ32.data(), sizeof(int) * n_occ, cudaMemcpyHostToDevice, ctx.st));
     TBG_CUDA(cudaMemsetAsync(status_d, 0, sizeof(int), ctx.st));
     for (int64_t l0 = 0; l0 < n_loops; l0 += chunk) {
@@ -1451,12 +1455,12 @@ int tbg_wilson_loops(const tbg_model* m, int64_t n_loops, int64_t n_k, const dou
                 if ((rc = mixed_berry(ctx.st, N, np, Hp, nullptr, nullptr, 0.0, E, nullptr, mwork, mwb, status_d,
                                       nullptr, nullptr, U)))
                     return rc;
-            } else if ((rc = eig_batched(ctx.st, N, np, H, E, U, nullptr, 0, status_d))) {
+            } else if ((rc = eig_batched(ctx.st, N, np, H, E, U, nullptr, 0, status_d, occ_lo, occ_hi - occ_lo + 1))) {
                 return rc;
             }
         }
-        if ((rc = wilson_from_vectors(ctx.st, M, nl, (int)n_k, kv_d, U, (int)n_occ, occ_d, svd, out_d, work, wb,
-                                      status_d)))
+        if ((rc = wilson_from_vectors(ctx.st, M, nl, (int)n_k, kv_d, U, (int)n_occ, occ_d, run ? occ_lo : -1, svd, out_d,
+                                      work, wb, status_d)))
             return rc;
         ctx.fetch_status(status_d);
         TBG_CUDA(cudaMemcpyAsync(out + l0 * (svd ? n_occ : 1), out_d, sizeof(double) * nl * (svd ? n_occ : 1),

@@ -1289,11 +1289,11 @@ int jacobi_max_n() { return jacobi_max_n_ref().load(std::memory_order_relaxed); 
 
 // FP64 driver (plain path): A destroyed, U complex<double>.
 int eig_batched(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, void* work,
-                size_t work_bytes, int* status_d) {
+                size_t work_bytes, int* status_d, int first, int ncol) {
     if (batch <= 0) return TBG_OK;
     if (N <= kSmallMaxN) return eig_small(st, N, batch, A, E, U, status_d);  // one thread per matrix
     if (N <= jacobi_max_n()) return eig_jacobi(st, N, batch, A, E, U, status_d);  // one warp per matrix
-    return eig64(st, N, batch, A, E, U, status_d);
+    return eig64(st, N, batch, A, E, U, status_d, true, first, ncol);
 }
 
 // Eigenvalues only, FP64, of `batch` matrices held in caller-provided device

@@ -782,18 +782,18 @@ __global__ void __launch_bounds__(32) tri64_cluster_kernel(int N, int64_t batch,
 // ---------------------------------------------------- back-transformation --
 // U <- H_0 ... H_{N-2} U, in place, RS lanes per column (rows q, q + RS, ...,
 // at most T each, in registers; the reflector is read twice, the second time
-// from L1).  Columns of consecutive matrices follow each other, so warps are
-// full for any N.
+// from L1).  Columns first .. first + ncol - 1 of consecutive matrices follow each
+// other, so warps are full for any N.
 template <int T, int RS>
 __global__ void __launch_bounds__(128, T <= 16 ? 5 : 3) bt64_kernel(int N, int64_t batch, const zc* __restrict__ Ain,
-                                                      zc* __restrict__ Uout) {
+                                                      zc* __restrict__ Uout, int first, int ncol) {
     const int lane = threadIdx.x & 31, q = lane & (RS - 1);
-    const int64_t cols = batch * N;
+    const int64_t cols = batch * ncol;
     const int64_t col0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / RS;
     const bool on = col0 < cols;
     const int64_t col = on ? col0 : cols - 1;
-    const int64_t b = col / N;
-    const int c = (int)(col - b * N);
+    const int64_t b = col / ncol;
+    const int c = first + (int)(col - b * ncol);
     const zc* A = Ain + b * (int64_t)N * N + q;
     zc* U = Uout + b * (int64_t)N * N + c;
     zc u[T];
@@ -877,9 +877,9 @@ int launch_cta(cudaStream_t st, int N, int64_t batch, zc* A, int nsm) {
 }
 
 template <int T, int RS>
-int launch_bt(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U) {
+int launch_bt(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U, int first, int ncol) {
     const int64_t cols = 128 / RS;
-    bt64_kernel<T, RS><<<(unsigned)((batch * N + cols - 1) / cols), 128, 0, st>>>(N, batch, A, U);
+    bt64_kernel<T, RS><<<(unsigned)((batch * ncol + cols - 1) / cols), 128, 0, st>>>(N, batch, A, U, first, ncol);
     TBG_LAUNCHED("bt64_kernel");
     return TBG_OK;
 }
@@ -894,8 +894,8 @@ int launch_bt(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U) {
 // 200 x 64 0.58 against 0.42)
 constexpr int kWYMinN = 80;
 constexpr double kWYWork = 6e8;
-static bool use_wy(int N, int64_t batch) {
-    return N > 256 || (N >= kWYMinN && 4.0 * N * N * (double)N * batch >= kWYWork);
+static bool use_wy(int N, int64_t batch, int ncol) {
+    return N > 256 || (N >= kWYMinN && 4.0 * N * N * (double)ncol * batch >= kWYWork);
 }
 
 // Largest matrix whose packed triangle and vectors fit one CTA's shared memory.
@@ -904,9 +904,12 @@ bool eig64_fits(int N) { return N <= kWarpMax || cta_smem_bytes(N, cta_threads(N
 // Eigenvalues E (ascending) and, when U is given, eigenvectors (columns) of
 // batch N x N matrices A (upper triangles read, destroyed), N >= 1 (>= 4 with
 // vectors).  With timed = false nothing is allocated, which
-// requires eig64_fits(N) (and N <= 256 with vectors).
-int eig64(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* status_d, bool timed) {
+// requires eig64_fits(N) (and N <= 256 with vectors).  Only the vectors first ..
+// first + ncol - 1 (all for ncol < 0) are finished; the other columns hold scratch.
+int eig64(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* status_d, bool timed, int first,
+          int ncol) {
     if (batch <= 0) return TBG_OK;
+    if (ncol < 0) ncol = N - first;
     const int nsm = sm_count();
     const double n3 = (double)N * N * N * batch;
     int rc = TBG_OK;
@@ -971,18 +974,23 @@ int eig64(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* s
         return TBG_OK;
     };
     auto back = [&]() -> int {
-        if (timed && use_wy(N, batch)) return bt64_wy(st, N, batch, A, U, status_d);
+        if (timed && use_wy(N, batch, ncol)) return bt64_wy(st, N, batch, A, U, status_d, first, ncol);
         // 32 rows a lane (fewer shuffles per column) when that still gives every
         // sub-partition a warp, else 16: 128 bands 17.5 against 31.6 ms per 1024
         // matrices, 64 bands 8.5 against 14.4 per 4032; up to 32 bands 16 rows, whose
         // shorter warps leave a shorter last wave (26 bands 0.65 against 0.92 ms per 2304)
-        const int64_t warps32 = batch * N * ((N + 31) / 32) / 32;
+        const int64_t warps32 = batch * ncol * ((N + 31) / 32) / 32;
         const bool wide = warps32 >= 4 * (int64_t)nsm;
-        if (N <= 16) return launch_bt<16, 1>(st, N, batch, A, U);
-        if (N <= 32) return launch_bt<16, 2>(st, N, batch, A, U);
-        if (N <= 64) return wide ? launch_bt<32, 2>(st, N, batch, A, U) : launch_bt<16, 4>(st, N, batch, A, U);
-        if (N <= 128) return wide ? launch_bt<32, 4>(st, N, batch, A, U) : launch_bt<16, 8>(st, N, batch, A, U);
-        return wide ? launch_bt<32, 8>(st, N, batch, A, U) : launch_bt<16, 16>(st, N, batch, A, U);
+        if (N <= 16) return launch_bt<16, 1>(st, N, batch, A, U, first, ncol);
+        if (N <= 32) return launch_bt<16, 2>(st, N, batch, A, U, first, ncol);
+        if (N <= 64)
+            return wide ? launch_bt<32, 2>(st, N, batch, A, U, first, ncol)
+                        : launch_bt<16, 4>(st, N, batch, A, U, first, ncol);
+        if (N <= 128)
+            return wide ? launch_bt<32, 4>(st, N, batch, A, U, first, ncol)
+                        : launch_bt<16, 8>(st, N, batch, A, U, first, ncol);
+        return wide ? launch_bt<32, 8>(st, N, batch, A, U, first, ncol)
+                    : launch_bt<16, 16>(st, N, batch, A, U, first, ncol);
     };
     if (!timed) {
         if ((rc = reduce()) || (rc = tri())) return rc;
@@ -997,7 +1005,7 @@ int eig64(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* s
         if ((rc = tri())) return rc;
     }
     if (!U) return TBG_OK;
-    KTimer kt(st, "bt64_kernel", 8.0 * n3);
+    KTimer kt(st, "bt64_kernel", 8.0 * n3 * ncol / N);
     return back();
 }
 

@@ -61,6 +61,6 @@ __device__ __forceinline__ void reflector_scalars64(zc alpha, double xn, zc& tau
 // shared memory (models have at most 4096 bands).
 int hetrd64_big(cudaStream_t st, int N, int64_t batch, zc* A, int* status_d);
 // Back-transformation with blocked reflectors on the tensor cores (eig64_big.cu).
-int bt64_wy(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U, int* status_d);
+int bt64_wy(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U, int* status_d, int first, int ncol);
 
 }  // namespace tbg

@@ -387,9 +387,9 @@ __global__ void __launch_bounds__(4 * kWY) wy_t_kernel(int N, int64_t batch, int
 
 }  // namespace
 
-// U <- H_0 ... H_{N-2} U in blocks of kWY reflectors, last block first:
+// U <- H_0 ... H_{N-2} U (columns first .. first + ncol - 1) in blocks of kWY reflectors, last block first:
 // U -= Y (T (Y^H U)), all products on the tensor cores.
-int bt64_wy(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U, int* status_d) {
+int bt64_wy(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U, int* status_d, int first, int ncol) {
     int nsm = 0, dev = 0;
     TBG_CUDA(cudaGetDevice(&dev));
     TBG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -401,7 +401,7 @@ int bt64_wy(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U, int* stat
     };
     const size_t nb = (size_t)batch;
     const size_t oY = take(sizeof(zc) * nb * kWY * (N - 1)), oG = take(sizeof(zc) * nb * kWY * kWY);
-    const size_t o1 = take(sizeof(zc) * nb * kWY * N), o2 = take(sizeof(zc) * nb * kWY * N);
+    const size_t o1 = take(sizeof(zc) * nb * kWY * ncol), o2 = take(sizeof(zc) * nb * kWY * ncol);
     const size_t oE = take(sizeof(int) * nb * (3 * kWY + 4 * N));
     unsigned char* buf = nullptr;
     TBG_CUDA(cudaMallocAsync(&buf, off, st));
@@ -413,8 +413,8 @@ int bt64_wy(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U, int* stat
     const int last = (N - 2) / kWY * kWY;
     for (int j0 = last; j0 >= 0 && !rc; j0 -= kWY) {
         const int w = std::min(kWY, N - 1 - j0), m = N - 1 - j0;
-        const int64_t sY = (int64_t)kWY * m, sG = kWY * kWY, sX = (int64_t)kWY * N, sU = (int64_t)N * N;
-        zc* Ut = U + (int64_t)(j0 + 1) * N;
+        const int64_t sY = (int64_t)kWY * m, sG = kWY * kWY, sX = (int64_t)kWY * ncol, sU = (int64_t)N * N;
+        zc* Ut = U + (int64_t)(j0 + 1) * N + first;
         wy_rows_kernel<<<(unsigned)std::min<int64_t>(batch * w, nsm * 64), 256, 0, st>>>(N, batch, j0, w, A, Y);
         TBG_LAUNCHED("wy_rows_kernel");
         if ((rc = oz64_row_exps(st, batch, w, m, Y, m, sY, ey))) break;
@@ -422,15 +422,16 @@ int bt64_wy(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U, int* stat
         if ((rc = oz64_gemm(st, batch, w, w, m, yh, {Y, m, 1, sY, 0, ey}, G, kWY, sG, 0, status_d))) break;
         wy_t_kernel<<<(unsigned)std::min<int64_t>(batch, nsm * 64), 4 * kWY, 0, st>>>(N, batch, j0, w, A, G);
         TBG_LAUNCHED("wy_t_kernel");
-        if ((rc = oz64_row_exps(st, batch, w, w, G, kWY, sG, et)) || (rc = oz64_col_exps(st, batch, m, N, Ut, N, sU, eu)) ||
+        if ((rc = oz64_row_exps(st, batch, w, w, G, kWY, sG, et)) || (rc = oz64_col_exps(st, batch, m, ncol, Ut, N, sU, eu)) ||
             (rc = oz64_col_exps(st, batch, w, m, Y, m, sY, ec)))
             break;
-        if ((rc = oz64_gemm(st, batch, w, N, m, yh, {Ut, 1, N, sU, 0, eu}, X1, N, sX, 0, status_d))) break;
-        if ((rc = oz64_col_exps(st, batch, w, N, X1, N, sX, e1))) break;
-        if ((rc = oz64_gemm(st, batch, w, N, w, {G, kWY, 1, sG, 0, et}, {X1, 1, N, sX, 0, e1}, X2, N, sX, 0, status_d)))
+        if ((rc = oz64_gemm(st, batch, w, ncol, m, yh, {Ut, 1, N, sU, 0, eu}, X1, ncol, sX, 0, status_d))) break;
+        if ((rc = oz64_col_exps(st, batch, w, ncol, X1, ncol, sX, e1))) break;
+        if ((rc = oz64_gemm(st, batch, w, ncol, w, {G, kWY, 1, sG, 0, et}, {X1, 1, ncol, sX, 0, e1}, X2, ncol, sX, 0,
+                            status_d)))
             break;
-        if ((rc = oz64_col_exps(st, batch, w, N, X2, N, sX, e2))) break;
-        rc = oz64_gemm(st, batch, m, N, w, {Y, 1, m, sY, 0, ec}, {X2, 1, N, sX, 0, e2}, Ut, N, sU, -1, status_d);
+        if ((rc = oz64_col_exps(st, batch, w, ncol, X2, ncol, sX, e2))) break;
+        rc = oz64_gemm(st, batch, m, ncol, w, {Y, 1, m, sY, 0, ec}, {X2, 1, ncol, sX, 0, e2}, Ut, N, sU, -1, status_d);
     }
     cudaFreeAsync(buf, st);
     return rc;

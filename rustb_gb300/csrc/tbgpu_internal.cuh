@@ -277,15 +277,17 @@ int fourier_mixed_packed(ModelDev& m, cudaStream_t st, bool* packed);
 
 // Batched Hermitian eigensolver: A (batch, N, N) FP64 input (destroyed),
 // E (batch, N) ascending, U (batch, N, N) eigenvectors in columns (may be
-// null).  precision: 0 = FP64, 1 = FP32 solve (U32 out, FP32 values) used by
+// null); only the vectors first .. first + ncol - 1 when ncol >= 0 (the other
+// columns are then undefined).  precision: 0 = FP64, 1 = FP32 solve (U32 out, FP32 values) used by
 // the mixed path.
 size_t eig_workspace_bytes(int N, int64_t batch, int precision);
 int eig_batched(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, void* work,
-                size_t work_bytes, int* status_d);
+                size_t work_bytes, int* status_d, int first = 0, int ncol = -1);
 // The FP64 solver behind it (eig64.cu): A destroyed, U may be null, nothing
 // allocated; timed = false launches the kernels without event records.
 bool eig64_fits(int N);
-int eig64(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* status_d, bool timed = true);
+int eig64(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* status_d, bool timed = true,
+          int first = 0, int ncol = -1);
 
 // Spin-current dressing J = 1/2 {S, V} (in place through scratch).
 int spin_dress(cudaStream_t st, int N, int64_t norb, int64_t batch, int spin, zc* V, int64_t ldV,
@@ -389,7 +391,7 @@ int ec_integrate(cudaStream_t st, int dim, const int64_t* kmesh, int N, const do
 constexpr int kWilsonMaxOcc = 64;
 size_t wilson_workspace_bytes(int N, int64_t n_loops, int n_k, int n_occ);
 int wilson_from_vectors(cudaStream_t st, const ModelDev& m, int64_t n_loops, int n_k, const double* kv_d, const zc* U,
-                        int n_occ, const int* occ_d, int svd, double* out, void* work, size_t work_bytes,
+                        int n_occ, const int* occ_d, int first_occ, int svd, double* out, void* work, size_t work_bytes,
                         int* status_d);
 
 int dos_slices(int64_t E_n, int64_t count);

@@ -79,6 +79,56 @@ __global__ void __launch_bounds__(256) wl_overlap_kernel(int N, int n_occ, int T
     }
 }
 
+// The closing points of the loops: columns first .. first + n - 1 of U at t = 0 with
+// the end phase, (n_loops, N, n).
+__global__ void wl_close_kernel(int64_t n_loops, int N, int n, int first, int T, const zc* __restrict__ U,
+                                const zc* __restrict__ endphase, zc* __restrict__ B) {
+    const int64_t per = (int64_t)N * n;
+    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n_loops * per;
+         idx += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t l = idx / per;
+        const int a = (int)(idx % per) / n, j = (int)(idx % per) % n;
+        B[idx] = endphase[l * N + a] * U[l * T * (int64_t)N * N + (int64_t)a * N + first + j];
+    }
+}
+
+// The overlaps of consecutive occupied bands first .. first + n - 1 as products on
+// the tensor cores (oz64.cu): every point with the one behind it, then the closing
+// segments over what that left for them.
+int wl_overlap_oz64(cudaStream_t st, int64_t n_loops, int T, int N, int n, int first, const zc* U, const zc* endphase,
+                    zc* O, int* status_d) {
+    const int64_t NN = (int64_t)N * N, nn = (int64_t)n * n, segs = n_loops * T, bn = (int64_t)N * n;
+    const size_t bytes = sizeof(zc) * n_loops * bn;
+    unsigned char* buf = nullptr;
+    TBG_CUDA(cudaMallocAsync(&buf, bytes + sizeof(int) * (segs + n_loops) * n, st));
+    zc* B = reinterpret_cast<zc*>(buf);
+    int *eu = reinterpret_cast<int*>(buf + bytes), *eb = eu + segs * n, *ea = nullptr;
+    wl_close_kernel<<<(unsigned)std::min<int64_t>((n_loops * bn + 255) / 256, 152LL * 64), 256, 0, st>>>(
+        n_loops, N, n, first, T, U, endphase, B);
+    TBG_LAUNCHED("wl_close_kernel");
+    const zc* Uo = U + first;
+    int rc = oz64_col_exps(st, segs, N, n, Uo, N, NN, eu);
+    if (!rc) rc = oz64_col_exps(st, n_loops, N, n, B, n, bn, eb);
+    if (!rc)
+        rc = oz64_gemm(st, segs - 1, n, n, N, {Uo, 1, N, NN, 1, eu}, {Uo + NN, 1, N, NN, 0, eu + n}, O, n, nn, 0,
+                       status_d);
+    // the left vectors of the closing segments lie T points apart: their exponents are gathered
+    if (!rc && cudaMallocAsync(&ea, sizeof(int) * n_loops * n, st) != cudaSuccess)
+        rc = set_error(TBG_E_OOM, "Wilson overlaps");
+    if (!rc && cudaMemcpy2DAsync(ea, sizeof(int) * n, eu + (int64_t)(T - 1) * n, sizeof(int) * n * T, sizeof(int) * n,
+                                 n_loops, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+        rc = set_error(TBG_E_CUDA, "Wilson overlaps");
+    if (!rc)
+        rc = oz64_gemm(st, n_loops, n, n, N, {Uo + (T - 1) * NN, 1, N, T * NN, 1, ea}, {B, 1, n, bn, 0, eb},
+                       O + (T - 1) * nn, n, T * nn, 0, status_d);
+    if (ea) cudaFreeAsync(ea, st);
+    cudaFreeAsync(buf, st);
+    return rc;
+}
+// Fewest bands (of which n_occ wanted) for which that beats one output per thread
+// from L1: 4032 overlaps of 32 of 64 bands 0.64 against 3.9 ms
+constexpr int kOverlapMinN = 32, kOverlapMinOcc = 12;
+
 // C = A B (n x n, shared memory), all threads of the block.
 __device__ void smem_mm(int n, const zc* A, const zc* B, zc* C) {
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
@@ -104,12 +154,17 @@ __global__ void __launch_bounds__(256) wl_polar_kernel(int n, zc* __restrict__ O
     __syncthreads();
     double err = 1.0;
     for (int it = 0; it < kMaxNS; ++it) {
-        // Y = X^dagger X
-        for (int e = threadIdx.x; e < nn; e += blockDim.x) {
-            const int i = e / n, j = e % n;
+        // Y = X^dagger X: the upper triangle, rows i and n - 1 - i side by side, mirrored
+        const int w = n + 1, half = (n + 1) / 2;
+        for (int e = threadIdx.x; e < half * w; e += blockDim.x) {
+            const int p = e / w, c = e - p * w;
+            const int i = c < n - p ? p : n - 1 - p, j = c < n - p ? p + c : i + c - (n - p);
+            if (c >= n - p && i == p) continue;  // the middle row of an odd n stands alone
             zc s = mk(0.0, 0.0);
             for (int k = 0; k < n; ++k) fma_cjx(s, X[k * n + i], X[k * n + j]);
-            Y[e] = s;
+            if (i == j) s.im = 0.0;
+            Y[i * n + j] = s;
+            Y[j * n + i] = conj(s);
         }
         if (threadIdx.x == 0) s_err = 0.0;
         __syncthreads();
@@ -140,17 +195,22 @@ __global__ void __launch_bounds__(256) wl_polar_kernel(int n, zc* __restrict__ O
     if (threadIdx.x == 0 && err > 1e-8) atomicOr(status, 4);
 }
 
-// P[l] = O[l][0] ... O[l][T-1] (unitary factors in SVD mode, raw overlaps in det mode).
-__global__ void __launch_bounds__(256) wl_chain_kernel(int n, int T, const zc* __restrict__ O, zc* __restrict__ P) {
+// P[l][g] = product of O[l][t] over the g-th run of len (unitary factors in SVD mode,
+// raw overlaps in det mode).  A chain is serial, so with fewer loops than SMs each
+// is cut into G runs whose products are chained by a second launch: 64 loops of 63
+// factors of 32 bands 1.3 ms in 5 runs, 2.1 in one.
+__global__ void __launch_bounds__(256) wl_chain_kernel(int n, int T, int G, int len, const zc* __restrict__ O,
+                                                       zc* __restrict__ P) {
     extern __shared__ zc wsm[];
     zc* X = wsm;
     zc* Z = X + n * n;
     zc* Pc = Z + n * n;
-    const int64_t l = blockIdx.x;
-    const int nn = n * n;
-    for (int e = threadIdx.x; e < nn; e += blockDim.x) Pc[e] = mk((e / n == e % n) ? 1.0 : 0.0, 0.0);
+    const int64_t l = blockIdx.x / G;
+    const int nn = n * n, t0 = (int)(blockIdx.x % G) * len, t1 = min(T, t0 + len);
+    for (int e = threadIdx.x; e < nn; e += blockDim.x)
+        Pc[e] = t0 < t1 ? O[(l * T + t0) * (int64_t)nn + e] : mk((e / n == e % n) ? 1.0 : 0.0, 0.0);
     __syncthreads();
-    for (int t = 0; t < T; ++t) {
+    for (int t = t0 + 1; t < t1; ++t) {
         const zc* Ot = O + (l * T + t) * (int64_t)nn;
         for (int e = threadIdx.x; e < nn; e += blockDim.x) X[e] = Ot[e];
         __syncthreads();
@@ -159,7 +219,7 @@ __global__ void __launch_bounds__(256) wl_chain_kernel(int n, int T, const zc* _
         for (int e = threadIdx.x; e < nn; e += blockDim.x) Pc[e] = Z[e];
         __syncthreads();
     }
-    for (int e = threadIdx.x; e < nn; e += blockDim.x) P[l * nn + e] = Pc[e];
+    for (int e = threadIdx.x; e < nn; e += blockDim.x) P[blockIdx.x * (int64_t)nn + e] = Pc[e];
 }
 
 // Hz[l] = (e^{-i phi} P + e^{i phi} P^dagger) / 2
@@ -286,10 +346,11 @@ inline unsigned nblk(int64_t total) {
 size_t wilson_chain_smem(int n_occ) { return sizeof(zc) * 3 * (size_t)n_occ * n_occ; }
 
 // kv_d: (n_loops, n_k, dim) k-points; U: eigenvectors at points t < n_k - 1 of
-// every loop, (n_loops * (n_k - 1), N, N).  out: (n_loops, n_occ) or (n_loops).
+// every loop, (n_loops * (n_k - 1), N, N); first_occ: the first occupied band when
+// they are consecutive, else -1.  out: (n_loops, n_occ) or (n_loops).
 int wilson_from_vectors(cudaStream_t st, const ModelDev& m, int64_t n_loops, int n_k, const double* kv_d, const zc* U,
-                        int n_occ, const int* occ_d, int svd, double* out, void* work, size_t work_bytes,
-                        int* status_d) {
+                        int n_occ, const int* occ_d, int first_occ, int svd, double* out, void* work,
+                        size_t work_bytes, int* status_d) {
     if (n_loops <= 0) return TBG_OK;
     const int N = (int)m.nsta, T = n_k - 1;
     const int64_t nn = (int64_t)n_occ * n_occ;
@@ -312,8 +373,12 @@ int wilson_from_vectors(cudaStream_t st, const ModelDev& m, int64_t n_loops, int
         wl_endphase_kernel<<<nblk(n_loops * N), 256, 0, st>>>(n_loops, n_k, m.dim, kv_d, N, m.tau_d, endph);
         TBG_LAUNCHED("wl_endphase_kernel");
         KTimer kt(st, "wl_overlap_kernel");
-        wl_overlap_kernel<<<(unsigned)(n_loops * T), 256, 0, st>>>(N, n_occ, T, U, occ_d, endph, O);
-        TBG_LAUNCHED("wl_overlap_kernel");
+        if (first_occ >= 0 && N >= kOverlapMinN && n_occ >= kOverlapMinOcc) {
+            if (int rc = wl_overlap_oz64(st, n_loops, T, N, n_occ, first_occ, U, endph, O, status_d)) return rc;
+        } else {
+            wl_overlap_kernel<<<(unsigned)(n_loops * T), 256, 0, st>>>(N, n_occ, T, U, occ_d, endph, O);
+            TBG_LAUNCHED("wl_overlap_kernel");
+        }
     }
     const size_t smem = wilson_chain_smem(n_occ);
     if (svd && T > 0) {
@@ -325,8 +390,18 @@ int wilson_from_vectors(cudaStream_t st, const ModelDev& m, int64_t n_loops, int
     {
         KTimer kt(st, "wl_chain_kernel");
         if (int rc = wl_allow_smem(wl_chain_kernel, smem)) return rc;
-        wl_chain_kernel<<<(unsigned)n_loops, 256, smem, st>>>(n_occ, T, O, P);
+        // about two blocks per SM, runs of at least four factors
+        const int want = (int)std::min<int64_t>(T / 4, (2 * 152 + n_loops - 1) / n_loops);
+        const int len = want > 1 ? (T + want - 1) / want : std::max(T, 1), G = std::max(1, (T + len - 1) / len);
+        zc* part = P;
+        if (G > 1) TBG_CUDA(cudaMallocAsync(&part, sizeof(zc) * n_loops * G * nn, st));
+        wl_chain_kernel<<<(unsigned)(n_loops * G), 256, smem, st>>>(n_occ, T, G, len, O, part);
         TBG_LAUNCHED("wl_chain_kernel");
+        if (G > 1) {
+            wl_chain_kernel<<<(unsigned)n_loops, 256, smem, st>>>(n_occ, G, 1, G, part, P);
+            cudaFreeAsync(part, st);
+            TBG_LAUNCHED("wl_chain_kernel");
+        }
     }
     if (!svd) {
         wl_det_kernel<<<nblk(n_loops), 256, 0, st>>>(n_loops, n_occ, P, out);
