@@ -11,7 +11,9 @@
 // 16 CTAs, rows dealt cyclically so that the shares stay equal as the block
 // shrinks); two cluster barriers a step.
 //
-// 12 matrices of 512 bands (eigenvalues) 176 -> 17.7 ms, against one CTA per matrix.
+// 12 matrices of 512 bands (eigenvalues) 176 -> 15.5 ms, against one CTA per matrix; a
+// step is 12.5 us of A v (10 at the pipe's rate, ten CTAs) and about as much of
+// exchange, reductions and the panel's products.
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -32,6 +34,7 @@ constexpr int kPW = 2 * kNB;
 constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMaxCluster = 16;
+constexpr int kRows = 4;         // rows of A v that a warp takes together
 
 // Published by the CTAs of a matrix to each other, per matrix.
 struct Exchange {
@@ -39,10 +42,10 @@ struct Exchange {
     zc* p;         // (N) A v
     zc* gh;        // (C, kPW) partial [V W]^H v
     double* norm;  // (C, kWarps) partial |a|^2 without the first entry
-    double* s;     // (C) partial v^H A v
+    double* s;     // (C, kWarps) partial v^H A v
 };
 __host__ __device__ inline size_t exchange_bytes(int N, int C) {
-    return sizeof(zc) * (2 * (size_t)N + (size_t)C * kPW) + sizeof(double) * ((size_t)C * kWarps + C + (C & 1));
+    return sizeof(zc) * (2 * (size_t)N + (size_t)C * kPW) + sizeof(double) * 2 * (size_t)C * kWarps;
 }
 __device__ __forceinline__ Exchange exchange_of(unsigned char* base, int N, int C) {
     Exchange x;
@@ -58,8 +61,8 @@ __device__ __forceinline__ zc ldcg(const zc* p) {
     return mk(t.x, t.y);
 }
 
-// Sums over the warp of R complex values per lane (R = 4 or 8): lane l ends with
-// the sum of value l mod R, in R - 1 + (5 - log2 R) additions per component
+// Sums over the warp of R complex values per lane: lane l ends with the sum of
+// value l mod R, in R - 1 + (5 - log2 R) additions per component
 // instead of 5 R.
 template <int R>
 __device__ __forceinline__ zc warp_sums(zc (&v)[R], int lane) {
@@ -80,6 +83,30 @@ __device__ __forceinline__ zc warp_sums(zc (&v)[R], int lane) {
         r.im += __shfl_xor_sync(all, r.im, o);
     }
     return r;
+}
+
+// Sum of n values in pairs (FP64 latency is long here: log2 n steps, not n).
+template <int n>
+__device__ __forceinline__ zc pair_sum(zc (&v)[n]) {
+#pragma unroll
+    for (int h = n / 2; h > 0; h >>= 1)
+#pragma unroll
+        for (int i = 0; i < h; ++i) v[i] = v[i] + v[i + h];
+    return v[0];
+}
+// Sum over the C CTAs' warps of a published partial, by one warp; all requested at once.
+__device__ __forceinline__ double sum_published(const double* x, int C, int lane) {
+    constexpr int n = kMaxCluster * kWarps / 32;
+    double v[n];
+#pragma unroll
+    for (int w = 0; w < n; ++w) v[w] = lane + 32 * w < C * kWarps ? __ldcg(x + lane + 32 * w) : 0.0;
+#pragma unroll
+    for (int h = n / 2; h > 0; h >>= 1)
+#pragma unroll
+        for (int i = 0; i < h; ++i) v[i] += v[i + h];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
 }
 
 // One panel: columns j0 .. j0 + steps - 1 of every matrix.  Writes the reflectors,
@@ -103,10 +130,11 @@ __global__ void __launch_bounds__(kThreads) panel64_kernel(int N, int j0, int st
     extern __shared__ __align__(16) unsigned char smem_p[];
     zc* sa = reinterpret_cast<zc*>(smem_p);  // (N) column below the diagonal
     zc* sq = sa + N;                         // (own rows) A a, then p
+    zc* sx = sq + (N + C - 1) / C;           // (own rows) part of the next column
     __shared__ zc s_part[kWarps][kPW];       // partial [V W]^H a per warp
     __shared__ zc s_mul[kPW], s_row[kPW];    // coefficients of V, W; the next row of [W V]
     __shared__ zc s_scal, s_tau, s_u1;
-    __shared__ double s_beta, s_ca, s_d, s_sw[kWarps];
+    __shared__ double s_beta, s_ca, s_d;
     __shared__ int s_next;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     auto first_own = [&](int r) { return r + ((rank - r) % C + C) % C; };  // own row at or after r
@@ -136,10 +164,7 @@ __global__ void __launch_bounds__(kThreads) panel64_kernel(int N, int j0, int st
         __syncthreads();
         if (warp == 0) {
             // reflector of the column: H^H x = beta e_0 with beta real
-            double xn = 0.0;
-            for (int t = lane; t < C * kWarps; t += 32) xn += __ldcg(X.norm + t);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) xn += __shfl_xor_sync(0xffffffffu, xn, o);
+            const double xn = sum_published(X.norm, C, lane);
             if (lane == 0) {
                 const zc alpha = sa[0];
                 zc tau, scal;
@@ -151,33 +176,33 @@ __global__ void __launch_bounds__(kThreads) panel64_kernel(int N, int j0, int st
             }
         }
         // q = A a without the first column, partial [V W]^H a without the first row;
-        // four own rows at a time
+        // kRows own rows at a time
         zc gh = mk(0.0, 0.0);
         const bool on = (lane & (kNB - 1)) < i;
         for (;;) {
             int g = 0;
-            if (lane == 0) g = atomicAdd(&s_next, 4);
+            if (lane == 0) g = atomicAdd(&s_next, kRows);
             g = __shfl_sync(0xffffffffu, g, 0);
             if (g >= nrows) break;
-            zc acc[4] = {};
-            const zc* row[4];
+            zc acc[kRows] = {};
+            const zc* row[kRows];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) row[k] = A + (size_t)(r0 + C * min(g + k, nrows - 1)) * N + f;
+            for (int k = 0; k < kRows; ++k) row[k] = A + (size_t)(r0 + C * min(g + k, nrows - 1)) * N + f;
 #pragma unroll 2
             for (int c = lane; c < N - f; c += 32) {
                 const zc x = c > 0 ? sa[c] : mk(0.0, 0.0);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) fma_cx(acc[k], row[k][c], x);
+                for (int k = 0; k < kRows; ++k) fma_cx(acc[k], row[k][c], x);
             }
             if (on) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
+                for (int k = 0; k < kRows; ++k) {
                     const int r = r0 + C * (g + k);
                     if (g + k < nrows && r > f) fma_cjx(gh, P[(size_t)r * kPW + lane], sa[r - f]);
                 }
             }
-            const zc q = warp_sums<4>(acc, lane);
-            if (lane < 4 && g + lane < nrows) sq[g + lane] = q;
+            const zc q = warp_sums<kRows>(acc, lane);
+            if (lane < kRows && g + lane < nrows) sq[g + lane] = q;
         }
         s_part[warp][lane] = gh;
         __syncthreads();
@@ -194,103 +219,121 @@ __global__ void __launch_bounds__(kThreads) panel64_kernel(int N, int j0, int st
             X.p[r] = p;
             s += fma(v.re, p.re, v.im * p.im);
         }
+        if (warp * 32 < nrows)  // the others have no row
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) s_sw[warp] = s;
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) X.s[rank * kWarps + warp] = s;
         if (warp == kWarps - 1) {
-            zc t = mk(0.0, 0.0);
+            zc part[kWarps];
 #pragma unroll
-            for (int w = 0; w < kWarps; ++w) t = t + s_part[w][lane];
-            t = scal * t;
+            for (int w = 0; w < kWarps; ++w) part[w] = s_part[w][lane];
+            zc t = scal * pair_sum(part);
             if (r0 == f && on) t = t + conj(P[(size_t)f * kPW + lane]);
             X.gh[rank * kPW + lane] = t;
         }
-        __syncthreads();
-        if (tid == 0) {
-            double t = 0.0;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) t += s_sw[w];
-            X.s[rank] = t;
-        }
         cl.sync();
-        if (warp == 0) {
-            // h = V^H v (lanes 0 ..), g = W^H v (lanes kNB ..)
-            zc t = mk(0.0, 0.0);
-            double st = 0.0;
-            for (int c = 0; c < C; ++c) {
-                t = t + ldcg(X.gh + c * kPW + lane);
-                st += __ldcg(X.s + c);
-            }
+        if (warp < 2) {
+            // h = V^H v (lanes 0 ..), g = W^H v (lanes kNB ..), both by two warps
+            zc part[kMaxCluster];  // all requested at once
+#pragma unroll
+            for (int c = 0; c < kMaxCluster; ++c) part[c] = c < C ? ldcg(X.gh + c * kPW + lane) : mk(0.0, 0.0);
+            const zc pf = ldcg(X.p + f), pr = on ? P[(size_t)f * kPW + lane] : mk(0.0, 0.0);
+            zc t = pair_sum(part);
             if (!on) t = mk(0.0, 0.0);
             const zc o = mk(__shfl_xor_sync(0xffffffffu, t.re, kNB), __shfl_xor_sync(0xffffffffu, t.im, kNB));
-            // v^H A_true v = v^H p - 2 Re sum conj(h) g; each pair is seen by two lanes
-            double cr = fma(t.re, o.re, t.im * o.im);
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) cr += __shfl_xor_sync(0xffffffffu, cr, d);
-            st -= cr;
             const zc tau = s_tau;
-            const double ca = -0.5 * fma(tau.re, tau.re, tau.im * tau.im) * st;
-            // A_true v = p - V g - W h
-            const zc pr = on ? P[(size_t)f * kPW + lane] : mk(0.0, 0.0);
-            zc d1[4] = {pr * o, mk(0.0, 0.0), mk(0.0, 0.0), mk(0.0, 0.0)};
-            const zc dot0 = warp_sums<4>(d1, lane);
-            const zc dot = mk(__shfl_sync(0xffffffffu, dot0.re, 0), __shfl_sync(0xffffffffu, dot0.im, 0));
-            zc u1 = tau * (ldcg(X.p + f) - dot);
-            u1.re += ca;
-            s_mul[lane] = o;
-            const zc sw = mk(__shfl_xor_sync(0xffffffffu, pr.re, kNB), __shfl_xor_sync(0xffffffffu, pr.im, kNB));
-            s_row[lane] = sw;  // row f of [W | V], columns before i
-            if (lane == 0) {
-                s_ca = ca;
-                s_u1 = u1;
-                if (rank == j % C) A[(size_t)j * N + j] = mk(s_d, s_beta);
-                if (rank == 0) A[(size_t)f * N + j] = tau;
+            if (warp == 0) {
+                // A_true v = p - V g - W h; its row f and row f of [W | V], columns before i
+                zc dot = pr * o;
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) {
+                    dot.re += __shfl_xor_sync(0xffffffffu, dot.re, d);
+                    dot.im += __shfl_xor_sync(0xffffffffu, dot.im, d);
+                }
+                s_mul[lane] = o;
+                s_row[lane] = mk(__shfl_xor_sync(0xffffffffu, pr.re, kNB), __shfl_xor_sync(0xffffffffu, pr.im, kNB));
+                if (lane == 0) {
+                    s_u1 = tau * (pf - dot);
+                    if (rank == j % C) A[(size_t)j * N + j] = mk(s_d, s_beta);
+                    if (rank == 0) A[(size_t)f * N + j] = tau;
+                }
+            } else {
+                // v^H A_true v = v^H p - 2 Re sum conj(h) g; each pair is seen by two lanes
+                double cr = fma(t.re, o.re, t.im * o.im);
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) cr += __shfl_xor_sync(0xffffffffu, cr, d);
+                const double st = sum_published(X.s, C, lane) - cr;
+                if (lane == 0) s_ca = -0.5 * fma(tau.re, tau.re, tau.im * tau.im) * st;
             }
         }
         __syncthreads();
-        // own rows: u = tau A_true v + ca v, and the next column
-        const zc tau = s_tau, mul = s_mul[lane], nrow = conj(s_row[lane]), u1 = s_u1;
-        const double ca = s_ca;
+        // own rows: u = tau A_true v + ca v, and the next column.  Four lanes a row
+        // for the two products with its [V W], then one lane a row.
         const bool more = i + 1 < steps || f == N - 1;
-        double nrm = 0.0;
-        for (int g = 4 * warp; g < nrows; g += 4 * kWarps) {
-            zc acc[8];
+        for (int t0 = tid >> 2; (t0 & ~7) < nrows; t0 += kThreads / 4) {  // whole warps
+            const int r = r0 + C * min(t0, nrows - 1);
+            const zc* Pr = P + (size_t)r * kPW;
+            zc q1 = mk(0.0, 0.0), q2 = mk(0.0, 0.0);
+            zc v[kNB / 4], w[kNB / 4], z1 = mk(0.0, 0.0), z2 = mk(0.0, 0.0);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int r = r0 + C * min(g + k, nrows - 1);
-                const zc x = on ? P[(size_t)r * kPW + lane] : mk(0.0, 0.0);
-                acc[k] = x * mul;
-                acc[4 + k] = x * nrow;
+            for (int kk = 0; kk < kNB / 4; ++kk) {  // all requested at once
+                const int k = (tid & 3) + 4 * kk;
+                v[kk] = k < i ? Pr[k] : mk(0.0, 0.0);
+                w[kk] = k < i ? Pr[kNB + k] : mk(0.0, 0.0);
             }
-            const zc q = warp_sums<8>(acc, lane);
-            const zc q2 = mk(__shfl_down_sync(0xffffffffu, q.re, 4), __shfl_down_sync(0xffffffffu, q.im, 4));
-            if (lane < 4 && g + lane < nrows) {
-                const int r = r0 + C * (g + lane);
-                const zc v = r == f ? mk(1.0, 0.0) : scal * sa[r - f];
-                zc u = tau * (sq[g + lane] - q);
-                u = mk(fma(ca, v.re, u.re), fma(ca, v.im, u.im));
-                const zc vs = up * v, us = down * u;
-                P[(size_t)r * kPW + i] = vs;
-                P[(size_t)r * kPW + kNB + i] = us;
-                Q[(size_t)r * kPW + i] = us;
-                Q[(size_t)r * kPW + kNB + i] = vs;
-                A[(size_t)j * N + r] = v;
-                if (more) {
-                    // column f of A_true: a - [V W] conj(row f of [W V]) - v conj(u_f) - u
-                    zc x = A[(size_t)r * N + f] - q2 - u;
-                    x = x - mulc(v, u1);
-                    if (r == f) {
-                        s_d = x.re;
-                        if (f == N - 1) A[(size_t)f * N + f] = mk(x.re, 0.0);
-                    } else {
-                        X.a[r] = x;
-                        if (r > f + 1) nrm += abs2(x);
-                    }
+#pragma unroll
+            for (int kk = 0; kk < kNB / 4; ++kk) {
+                const int k = (tid & 3) + 4 * kk;
+                if (4 * kk >= i) break;
+                fma_cx(q1, v[kk], s_mul[k]);
+                fma_cx(z1, w[kk], s_mul[kNB + k]);
+                fma_cx(q2, v[kk], conj(s_row[k]));
+                fma_cx(z2, w[kk], conj(s_row[kNB + k]));
+            }
+            q1 = q1 + z1;
+            q2 = q2 + z2;
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                q1.re += __shfl_xor_sync(0xffffffffu, q1.re, o);
+                q1.im += __shfl_xor_sync(0xffffffffu, q1.im, o);
+                q2.re += __shfl_xor_sync(0xffffffffu, q2.re, o);
+                q2.im += __shfl_xor_sync(0xffffffffu, q2.im, o);
+            }
+            if ((tid & 3) == 0 && t0 < nrows) {
+                sq[t0] = sq[t0] - q1;
+                sx[t0] = q2;
+            }
+        }
+        __syncthreads();
+        const zc tau = s_tau, u1 = mk(s_u1.re + s_ca, s_u1.im);
+        const double ca = s_ca;
+        double nrm = 0.0;
+        for (int t = tid; t < nrows; t += kThreads) {
+            const int r = r0 + C * t;
+            const zc v = r == f ? mk(1.0, 0.0) : scal * sa[r - f];
+            zc u = tau * sq[t];
+            u = mk(fma(ca, v.re, u.re), fma(ca, v.im, u.im));
+            const zc vs = up * v, us = down * u;
+            P[(size_t)r * kPW + i] = vs;
+            P[(size_t)r * kPW + kNB + i] = us;
+            Q[(size_t)r * kPW + i] = us;
+            Q[(size_t)r * kPW + kNB + i] = vs;
+            A[(size_t)j * N + r] = v;
+            if (more) {
+                // column f of A_true: a - [V W] conj(row f of [W V]) - v conj(u_f) - u
+                const zc x = A[(size_t)r * N + f] - sx[t] - u - mulc(v, u1);
+                if (r == f) {
+                    s_d = x.re;
+                    if (f == N - 1) A[(size_t)f * N + f] = mk(x.re, 0.0);
+                } else {
+                    X.a[r] = x;
+                    if (r > f + 1) nrm += abs2(x);
                 }
             }
         }
+        if (warp * 32 < nrows)
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+            for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
         if (lane == 0) X.norm[rank * kWarps + warp] = nrm;
         __syncthreads();
     }
@@ -455,7 +498,7 @@ int hetrd64_big(cudaStream_t st, int N, int64_t batch, zc* A, int* status_d) {
     cfg.numAttrs = 1;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    auto smem_of = [&](int c) { return sizeof(zc) * ((size_t)N + (N + c - 1) / c + 1); };
+    auto smem_of = [&](int c) { return sizeof(zc) * ((size_t)N + 2 * ((N + c - 1) / c)); };
     for (;; --C) {
         const size_t smem = smem_of(C);
         TBG_CUDA(cudaFuncSetAttribute(panel64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
