@@ -499,7 +499,8 @@ __global__ void tau_pairs_kernel(int64_t nk, int N, float4* __restrict__ C, cons
 // multiple of 32 dividing 256) each warp's maximum goes through shared memory
 // and the row's exponent is stored; otherwise rexp is preset below every
 // exponent and the maxima are folded in by atomicMax, one per warp when N is
-// a multiple of 32 (a warp then lies in one row), else per lane.
+// a multiple of 32 (a warp then lies in one row), one or two from 32 bands on (304
+// k-points of 251 bands 2.06 -> 0.39 ms, against one per lane), else per lane.
 constexpr int kUnpackThreads = 256;
 __host__ __device__ constexpr bool unpack_block_rows(int N) { return (N & 31) == 0 && kUnpackThreads % N == 0; }
 
@@ -561,6 +562,17 @@ __global__ void __launch_bounds__(kUnpackThreads) unpack_tau_kernel(int64_t nk, 
                 for (int c = 0; c < 3; ++c) {
                     const int v = __reduce_max_sync(0xffffffffu, __float_as_int(mag[c]));
                     if (valid && lane == 0) atomicMax(&rexp[(c * nk + kk) * N + mrow], line_exp_of(__int_as_float(v)));
+                }
+            } else if (N >= 32) {  // a warp lies in at most two rows
+                const int r0 = __shfl_sync(0xffffffffu, mrow, 0);
+                const bool second = valid && mrow != r0, two = __any_sync(0xffffffffu, second);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const int bits = __float_as_int(mag[c]);
+                    const int v = __reduce_max_sync(0xffffffffu, second ? 0 : bits);
+                    const int w = two ? __reduce_max_sync(0xffffffffu, second ? bits : 0) : 0;
+                    if (lane == 0 && valid) atomicMax(&rexp[(c * nk + kk) * N + r0], line_exp_of(__int_as_float(v)));
+                    if (lane == 0 && two) atomicMax(&rexp[(c * nk + kk) * N + r0 + 1], line_exp_of(__int_as_float(w)));
                 }
             } else if (valid) {
 #pragma unroll
@@ -1001,9 +1013,15 @@ int ensure_table_image(ModelDev& m, cudaStream_t st) {
     return TBG_OK;
 }
 
-// FP64 instructions (per lane) of the direct sum above which the tensor-core form
-// is taken: 2e7 keep the FP64 pipe for 40 us, about what its launches take
-constexpr double kOzFourierWork = 2e7;
+// Whether M x NN sums over Kc pairs (work: FP64 instructions of the direct form, per
+// output lane) take the tensor-core form.  Both sides in us: the launches and, per
+// round of tiles over the SMs, 8 and 1.6 a stage, against the direct form at 0.6 of
+// the FP64 pipe's rate (60 instructions an element for its gauge phases).  301 k-points
+// of 14 bands, 125 R: 34 against 64 us; 12 of 512 bands, 9 R: 0.41 against 0.73 ms.
+bool oz64_sum_pays(int64_t M, int64_t NN, int Kc, double work) {
+    const int64_t rounds = ((M + 127) / 128 * ((NN + 39) / 40) + 151) / 152;
+    return 25.0 + (double)rounds * (8.0 + 1.6 * ((Kc + 15) / 16)) < work / 3.2e5;
+}
 constexpr int64_t kOzFourierBytes = 512LL << 20;  // sums held at a time
 
 // H and nproj projections on the tensor cores at FP64 accuracy (oz64.cu): the
@@ -1088,7 +1106,8 @@ int fourier_direct(const ModelDev& m, cudaStream_t st, int64_t nk, const double*
         std::lock_guard<std::mutex> lk(g_hop_mu);
         int rc = ensure_pair_table(const_cast<ModelDev&>(m), st);
         if (rc) return rc;
-        oz = status_d && (double)nk * N * N * m.hop_K * (nproj > 0 ? 8 + 2 * nproj : 4) >= kOzFourierWork;
+        oz = status_d && oz64_sum_pays(nk * (1 + nproj), (int64_t)N * N, m.hop_K,
+                                       (double)nk * N * N * (m.hop_K * (nproj > 0 ? 8 + 2 * nproj : 4) + 60));
         if (oz && (rc = ensure_table_image(const_cast<ModelDev&>(m), st))) return rc;
         oz = oz && m.oz_img;
     }
@@ -1116,7 +1135,7 @@ int rmatrix_term(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k
     const int N = (int)m.nsta, nR = (int)m.nR, nr = (int)m.n_rmat;
     const int64_t NN = (int64_t)N * N;
     // the same forms as fourier_direct's for the sums, as the rotation's for the products
-    const bool oz = (double)nk * NN * nr * 4.0 >= kOzFourierWork, tc = N > kCommSmemMaxN;
+    const bool oz = oz64_sum_pays(nk, NN, nr, (double)nk * NN * nr * 4.0), tc = N > kCommSmemMaxN;
     const int step = oz ? 2 : 1;
     size_t off = 0;
     auto take = [&](size_t bytes) {
