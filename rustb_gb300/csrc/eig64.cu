@@ -889,11 +889,11 @@ int launch_bt(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U, int fir
 // Whether the back-transformation takes the blocked form.  Its FP64 work (T) is a
 // small part of the 4 N^3 FMA of bt64, which does not go beyond 256 bands; below
 // kWYWork the launches of a block cost more than that saves, and below kWYMinN
-// bands too little of a 128-row tile is used (1024 x 128 bands 6.8 against 17.5 ms,
-// 200 x 97 1.2 against 1.4; 30 x 128 0.65 against 0.51, 4032 x 64 7.8 against 8.2,
-// 200 x 64 0.58 against 0.42)
-constexpr int kWYMinN = 80;
-constexpr double kWYWork = 6e8;
+// bands too little of a 128-row tile is used (1024 x 128 bands 4.6 against 17.5 ms,
+// 4032 x 64 5.7 against 7.9, 200 x 64 0.49 against 0.67, 50 x 97 0.55 against 0.53,
+// 460 x 48 0.61 against 0.50)
+constexpr int kWYMinN = 56;
+constexpr double kWYWork = 1.8e8;
 static bool use_wy(int N, int64_t batch, int ncol) {
     return N > 256 || (N >= kWYMinN && 4.0 * N * N * (double)ncol * batch >= kWYWork);
 }

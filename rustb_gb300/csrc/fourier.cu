@@ -1015,12 +1015,12 @@ int ensure_table_image(ModelDev& m, cudaStream_t st) {
 
 // Whether M x NN sums over Kc pairs (work: FP64 instructions of the direct form, per
 // output lane) take the tensor-core form.  Both sides in us: the launches and, per
-// round of tiles over the SMs, 8 and 1.6 a stage, against the direct form at 0.6 of
+// round of tiles over the SMs, 8 and 1 a stage, against the direct form at 0.6 of
 // the FP64 pipe's rate (60 instructions an element for its gauge phases).  301 k-points
 // of 14 bands, 125 R: 34 against 64 us; 12 of 512 bands, 9 R: 0.41 against 0.73 ms.
 bool oz64_sum_pays(int64_t M, int64_t NN, int Kc, double work) {
-    const int64_t rounds = ((M + 127) / 128 * ((NN + 39) / 40) + 151) / 152;
-    return 25.0 + (double)rounds * (8.0 + 1.6 * ((Kc + 15) / 16)) < work / 3.2e5;
+    const int64_t rounds = ((M + 127) / 128 * ((NN + 31) / 32) + 151) / 152;
+    return 25.0 + (double)rounds * (8.0 + (Kc + 15) / 16) < work / 3.2e5;
 }
 constexpr int64_t kOzFourierBytes = 512LL << 20;  // sums held at a time
 

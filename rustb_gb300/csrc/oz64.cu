@@ -14,21 +14,29 @@
 // levels 4 to 6 in one the error of a 128-term product was 300 x 2^-54 of the
 // scale, against 10 x for an FP64 sum and 6.8 x now.
 //
-// CTA = 14 (13) warps, one output tile of 128 rows x 40 (32) complex columns:
-//   warps 0..7    digits of A, thread = (row, 8 consecutive k); afterwards the
-//                 epilogue, one TMEM lane = one row
-//   next 5 (4)    digits of B, thread = (column, 8 consecutive k, component); for
-//                 operands cut beforehand one thread copies the stage images of
-//                 both with cp.async.bulk
-//   last          allocates TMEM and issues the MMAs (M = 128, N = 80 or 64, K = 16)
-// 40 columns fill 480 of the 512 TMEM columns with six accumulators (levels 5 and 6
-// share the last), 32 columns 448 with seven.  Complex products keep the blocks
-// -Im B, Re B, Im B, so [Re B; Im B] and [-Im B; Re B] are the same memory at two
-// offsets.  Stage hand-off by mbarriers; every wait is bounded, as in the
-// float-pair products (ozaki_tc.cu).
+// Shared memory feeds the tensor cores 128 bytes a clock, so an MMA of 128 rows pays
+// 32 clocks for A and 16 per 64 columns of B, against 16 of arithmetic: digit pairs
+// (s, t), (s, t + 1), ... are one MMA, the digits of B side by side as its columns and
+// the accumulators of the levels side by side as its output (10 MMAs for the 28
+// pairs; one each took 55 clocks a pair).
 //
-// 1024 products of 128 bands: one of the four of the rotation 13.8 -> 0.93 ms
-// against 64 x 64 tiles on the FP64 pipe.
+// A's digits are cut into stage images first (a_image_kernel: one pass, not one per
+// column tile, and with every SM's issue slots).  A CTA then walks output tiles of
+// 128 rows x 32 complex columns (seven accumulators of 64 of the 512 TMEM columns):
+//   warps 0..15    epilogue, one TMEM lane = one row
+//   warps 16..23   digits of B, thread = (column, 8 consecutive k, component), two
+//                  groups that fill the two stage buffers in turn; idle when B too
+//                  comes as images
+//   warp 24        copies the images with cp.async.bulk
+//   warp 25        allocates TMEM and issues the MMAs (M = 128, N <= 256, K = 16)
+// so a tile's epilogue runs beside the next tile's copies and cutting.  A k step of
+// complex operands is [Re A] with [Re B; Im B], then [Im A] with [-Im B; Re B].
+// Stage hand-off by mbarriers; every wait is bounded, as in the float-pair products
+// (ozaki_tc.cu).
+//
+// 1024 products of 128 bands: one of the four of the rotation 13.8 ms on the FP64
+// pipe in 64 x 64 tiles, @ROT@ here (0.93 with one MMA per pair and A cut by the
+// tiles' own warps).
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -48,25 +56,21 @@ constexpr int S = 7;        // digits per value
 constexpr int TM = 128;     // rows of a tile
 constexpr int TK = 16;      // complex k per stage
 constexpr int APLANE = TM * 2 * TK * 2;  // bytes of one digit plane of A in a stage
-constexpr int A_THREADS = 256;
+constexpr int TNC = 32;     // complex columns of a tile
+constexpr int NR = 2 * TNC; // real columns: of a digit of B, and of a level's accumulator
+constexpr int BBLK = NR * TK * 2;            // bytes of one digit of B for one k step: NR rows x 16 k
+constexpr int BKS = S * BBLK;                // the digits side by side
+constexpr int ABYTES = S * APLANE, BBYTES = 2 * BKS, STAGE = ABYTES + BBYTES;
+constexpr int E_THREADS = 512;               // epilogue
+constexpr int B_THREADS = TNC * 4;           // (column, half of the 16 k, component), per group
+constexpr int THREADS = E_THREADS + 2 * B_THREADS + 64;
+constexpr int EPI = E_THREADS / 32 * 32 * 5 * 16;  // 4 columns of 32 rows per warp, rows padded to 5
+constexpr int SMEM = 2 * STAGE + EPI + 1024;
 constexpr int kMaxK = 256;  // complex k that one launch keeps exact
-enum { CPLX = 0, REALC = 1 };  // blocks of a B plane: complex product, or real coefficients (pre-cut)
-
-template <int TNC>
-struct Shape {
-    static constexpr int NR = 2 * TNC;               // real columns of a tile
-    static constexpr int NLEV = TNC > 32 ? 6 : 7;    // accumulators (level 6 with level 5 in the first case)
-    static_assert(NLEV * NR <= 512, "TMEM columns");
-    static constexpr int BLK = TNC * TK * 2;         // one block: TNC rows x 16 k
-    static constexpr int B_THREADS = TNC * 4;        // (column, half of the 16 k, component)
-    static constexpr int THREADS = A_THREADS + B_THREADS + 32;
-    static constexpr uint32_t IDESC =
-        (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NR >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
-    static constexpr int bplane(int mode) { return (mode == REALC ? 4 : 3) * BLK; }
-    static constexpr int stage(int mode) { return S * (APLANE + bplane(mode)); }
-    static constexpr int EPI = 8 * 32 * 5 * 16;      // 4 columns of 32 rows per warp, rows padded to 5
-    static constexpr int smem(int mode) { return 2 * stage(mode) + EPI + 1024; }
-};
+// kind::f16: D = F32, A = B = BF16, K-major, M = 128, N = n NR
+__host__ __device__ constexpr uint32_t idesc(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n * NR >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+}
 
 // byte offset of (row, half of the 16 k) in a block of core matrices (8 rows x 16 bytes)
 __host__ __device__ __forceinline__ int blk_off(int row, int half) {
@@ -79,23 +83,12 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
                  : "memory");
 }
 
-// One MMA; COL: use of the collector buffer for A (0 none, 1 fill, 2 use, 3 last use).
-template <int COL>
 __device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-#define TBG_MMA(Q)                                                                                          \
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16" Q    \
-                 " [%0], %1, %2, %3, p;\n\t}" ::"r"(d),                                                      \
-                 "l"(a), "l"(b), "r"(idesc), "r"(acc)                                                        \
-                 : "memory")
-    if constexpr (COL == 1)
-        TBG_MMA(".collector::a::fill");
-    else if constexpr (COL == 2)
-        TBG_MMA(".collector::a::use");
-    else if constexpr (COL == 3)
-        TBG_MMA(".collector::a::lastuse");
-    else
-        TBG_MMA("");
-#undef TBG_MMA
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, "
+        "p;\n\t}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
 }
 
 // Biased exponent of |x| (0x7ff: NaN or Inf); a line's largest one, at least 1,
@@ -133,14 +126,13 @@ __device__ __forceinline__ void digits(long long F, float (&P)[S]) {
     P[5] = fmaf(__uint_as_float(__byte_perm(lo, 0x4B000000, 0x7441)), 0x1p-40f, -C * 0x1p-40f);
     P[6] = fmaf(__uint_as_float(__byte_perm(lo, 0x4B000000, 0x7440)), 0x1p-48f, -C * 0x1p-48f);
 }
-template <int PART>
-__device__ __forceinline__ void planes(const zc (&v)[8], int e, bool neg, uint4 (&out)[S]) {
+__device__ __forceinline__ void planes(const double (&v)[8], int e, bool neg, uint4 (&out)[S]) {
     uint32_t pk[S][4];
 #pragma unroll
     for (int i = 0; i < 8; i += 2) {
         float P0[S], P1[S];
-        digits(fixed55(PART ? v[i].im : v[i].re, e), P0);
-        digits(fixed55(PART ? v[i + 1].im : v[i + 1].re, e), P1);
+        digits(fixed55(v[i], e), P0);
+        digits(fixed55(v[i + 1], e), P1);
 #pragma unroll
         for (int s = 0; s < S; ++s) pk[s][i >> 1] = bf16x2(P0[s], P1[s]);
     }
@@ -153,21 +145,26 @@ __device__ __forceinline__ uint4 neg8(uint4 v) {
     return make_uint4(v.x ^ m, v.y ^ m, v.z ^ m, v.w ^ m);
 }
 
-__device__ __forceinline__ void ld8(const zc* p, int64_t stride, int nvalid, zc (&r)[8]) {
+// 8 consecutive-k elements (stride in elements), and the same of one component.
+__device__ __forceinline__ void ld8(const zc* p, int64_t stride, int nvalid, double (&re)[8], double (&im)[8]) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         double2 t = make_double2(0.0, 0.0);
         if (i < nvalid) t = __ldg(reinterpret_cast<const double2*>(p + i * stride));
-        r[i] = mk(t.x, t.y);
+        re[i] = t.x;
+        im[i] = t.y;
     }
+}
+__device__ __forceinline__ void ld8(const zc* p, int part, int64_t stride, int nvalid, double (&v)[8]) {
+    const double* d = reinterpret_cast<const double*>(p) + part;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = i < nvalid ? __ldg(d + 2 * i * stride) : 0.0;
 }
 
 // The level sums -> their FP64 value times 2^(ea + eb - 2058) (e - 1022 - 7 per operand).
-template <int NLEV>
-__device__ __forceinline__ double combine(const uint32_t (&a)[NLEV], int ea, int eb) {
+__device__ __forceinline__ double combine(const uint32_t (&a)[S], int ea, int eb) {
     if (ea == kNonFinite || eb == kNonFinite) return __longlong_as_double(0x7ff8000000000000ll);
-    float tail = __uint_as_float(a[5]);  // levels 5 and 6, below 2^-14
-    if (NLEV == 7) tail += __uint_as_float(a[NLEV - 1]);
+    const float tail = __uint_as_float(a[5]) + __uint_as_float(a[6]);  // below 2^-14
     const long long I = ((long long)__float2int_rn(__uint_as_float(a[0])) << 39) +
                         ((long long)__float2int_rn(__uint_as_float(a[1]) * 0x1p8f) << 31) +
                         ((long long)__float2int_rn(__uint_as_float(a[2]) * 0x1p16f) << 23) +
@@ -188,18 +185,16 @@ __device__ __forceinline__ double combine(const uint32_t (&a)[NLEV], int ea, int
     return sg ? -r : r;
 }
 
-// C (M x Nc per matrix) = / += / -= op(A) op(B).  Element (i, k) of op(A) is at
-// A + b sA + i ai + k ak (conjugated when conjA), (k, j) of op(B) at
-// B + b sB + k bk + j bj.  EA, EB: line exponents per (matrix, row) and (matrix,
-// column).  PRE: A and B are stage images (row tile, nst_img stages) and (column
-// tile, nst_img stages), from stage it0 on.
+// C (M x Nc per matrix) = / += / -= A op(B).  A: stage images, nst_img stages per
+// (matrix, row tile), from stage it0 on.  Element (k, j) of op(B) is at
+// B + b sB + k bk + j bj (conjugated when conjB); PRE: B is images too, per column
+// tile.  EA, EB: line exponents per (matrix, row) and (matrix, column).
 struct OzArgs {
     int M, Nc, K;
-    const void* A;
-    int64_t ai, ak, sA;
+    const unsigned char* A;
     const void* B;
     int64_t bk, bj, sB;
-    int conjA, conjB;
+    int conjB;
     const int *EA, *EB;
     zc* C;
     int64_t ldc, sC;
@@ -226,46 +221,40 @@ __device__ __forceinline__ Tile tile_at(const OzArgs& p, int64_t L) {
     return t;
 }
 __device__ __forceinline__ int kleft(int K, int k) { return max(0, min(8, K - k)); }
-// OR over the eight epilogue warps
-__device__ __forceinline__ bool any256(bool v) {
+// OR over the epilogue warps
+__device__ __forceinline__ bool any_epilogue(bool v) {
     uint32_t r;
     asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, 1, 256, q;\n\tselp.u32 %0, 1, 0, "
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, 1, %2, q;\n\tselp.u32 %0, 1, 0, "
         "p;\n\t}"
         : "=r"(r)
-        : "r"((uint32_t)v)
+        : "r"((uint32_t)v), "n"(E_THREADS)
         : "memory");
     return r != 0;
 }
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(taddr));
+__device__ __forceinline__ void tmem_ld2(uint32_t taddr, uint32_t& a, uint32_t& b) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(a), "=r"(b) : "r"(taddr));
 }
 
-template <int TNC, bool PRE>
-__global__ void __launch_bounds__(Shape<TNC>::THREADS, 1) oz64_kernel(OzArgs p) {
-    using Sh = Shape<TNC>;
-    constexpr int MODE = PRE ? REALC : CPLX;
-    constexpr int BPLANE = Sh::bplane(MODE), ABYTES = S * APLANE, STAGE = Sh::stage(MODE), NR = Sh::NR, BLK = Sh::BLK;
-    constexpr int NLEV = Sh::NLEV;
+template <bool PRE>
+__global__ void __launch_bounds__(THREADS, 1) oz64_kernel(OzArgs p) {
     extern __shared__ __align__(1024) unsigned char oz_smem[];
     unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)oz_smem + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t bar_full[2], bar_empty[2], bar_done, bar_tmem;
     __shared__ uint32_t tmem_sh;
     __shared__ volatile int abort_sh;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr int MMA_WARP = (A_THREADS + Sh::B_THREADS) / 32;
+    constexpr int MMA_WARP = THREADS / 32 - 1, COPY_WARP = MMA_WARP - 1;
     const int nst = (p.K + TK - 1) / TK;
     const uint32_t sbase = su32(base);
     if (tid == 0) {
-        const uint32_t nfull = PRE ? 1 : A_THREADS + Sh::B_THREADS;
+        const uint32_t nfull = PRE ? 1 : 1 + B_THREADS;
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bar_full[i], nfull);
             mbar_init(&bar_empty[i], 1);
         }
         mbar_init(&bar_done, 1);
-        mbar_init(&bar_tmem, 8);
+        mbar_init(&bar_tmem, E_THREADS / 32);
         abort_sh = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -302,26 +291,16 @@ __global__ void __launch_bounds__(Shape<TNC>::THREADS, 1) oz64_kernel(OzArgs p) 
                     const uint32_t sa = sbase + bi * STAGE, sb = sa + ABYTES;
 #pragma unroll
                     for (int ks = 0; ks < 2; ++ks) {
-                        // [Re B; Im B] then [-Im B; Re B] (blocks -Im, Re, Im), or the
-                        // even then the odd rows of a real-coefficient table
-                        const int boff = MODE == CPLX ? (ks == 0 ? BLK : 0) : ks * 2 * BLK;
 #pragma unroll
                         for (int s = 0; s < S; ++s) {
+                            const uint64_t ad = smem_desc(sa + s * APLANE + ks * (APLANE / 2), 128, 256);
 #pragma unroll
-                            for (int t = 0; t < S - s; ++t) {
-                                const int lv = s + t < NLEV - 1 ? s + t : NLEV - 1;
-                                const uint64_t ad = smem_desc(sa + s * APLANE + ks * (APLANE / 2), 128, 256);
-                                const uint64_t bd = smem_desc(sb + t * BPLANE + boff, 128, 256);
-                                const uint32_t acc = (it == 0 && ks == 0 && s == 0 && t < NLEV) ? 0u : 1u;
-                                const uint32_t dst = tmem + (uint32_t)(lv * NR);
-                                if (s == S - 1)
-                                    mma<0>(dst, ad, bd, Sh::IDESC, acc);
-                                else if (t == 0)
-                                    mma<1>(dst, ad, bd, Sh::IDESC, acc);
-                                else if (t == S - 1 - s)
-                                    mma<3>(dst, ad, bd, Sh::IDESC, acc);
-                                else
-                                    mma<2>(dst, ad, bd, Sh::IDESC, acc);
+                            for (int t = 0; t < S - s; t += 4) {
+                                const int n = S - s - t < 4 ? S - s - t : 4;  // pairs (s, t) .. (s, t + n - 1)
+                                const uint64_t bd = smem_desc(sb + ks * BKS + t * BBLK, 128, 256);
+                                // digit 0 of A meets every level first
+                                const uint32_t acc = (it == 0 && ks == 0 && s == 0) ? 0u : 1u;
+                                mma(tmem + (uint32_t)((s + t) * NR), ad, bd, idesc(n), acc);
                             }
                         }
                     }
@@ -333,69 +312,59 @@ __global__ void __launch_bounds__(Shape<TNC>::THREADS, 1) oz64_kernel(OzArgs p) 
             }
         }
         __syncwarp();
-    } else if (tid < A_THREADS) {
-        // rows of consecutive threads when op(A) is stored by columns, else pairs of threads per row
-        const bool bycol = p.ak != 1;
-        const int r = bycol ? (tid & 127) : (tid >> 1);
-        const int g = bycol ? (tid >> 7) : (tid & 1);
-        const int q = warp & 3, h = warp >> 2;
-        const uint32_t lane_addr = tmem + ((uint32_t)(32 * q) << 16);
-        double2* epi = reinterpret_cast<double2*>(base + 2 * STAGE) + warp * (32 * 5);
-        zc nxt[8];
-        auto load = [&](int64_t L, int it) {
-            const Tile t = tile_at(p, L);
-            const int gi = t.rt * TM + r, k = it * TK + 8 * g;
-            ld8(static_cast<const zc*>(p.A) + t.b * p.sA + gi * p.ai + k * p.ak, p.ak, gi < p.M ? kleft(p.K, k) : 0, nxt);
-        };
-        if constexpr (!PRE)
-            if (blockIdx.x < p.ntiles) load(blockIdx.x, 0);
-        int tn = 0;
-        for (int64_t L = blockIdx.x; L < p.ntiles; L += gridDim.x, ++tn) {
-            const Tile t = tile_at(p, L);
-            if constexpr (!PRE) {
-                const int gi = t.rt * TM + r;
-                const int e = gi < p.M ? p.EA[t.b * p.M + gi] : 1;
+    } else if (warp == COPY_WARP) {
+        if (lane == 0) {
+            const int nrt = p.rows_fast ? p.gx : p.gy;
+            int64_t last[2] = {-1, -1};
+            int tn = 0;
+            bool stop = false;
+            for (int64_t L = blockIdx.x; L < p.ntiles && !stop; L += gridDim.x, ++tn) {
+                const Tile t = tile_at(p, L);
+                const unsigned char* ia = p.A + ((t.b * nrt + t.rt) * p.nst_img + p.it0) * ABYTES;
+                const unsigned char* ib =
+                    static_cast<const unsigned char*>(p.B) + ((int64_t)t.ct * p.nst_img + p.it0) * BBYTES;
                 for (int it = 0; it < nst; ++it) {
                     const int64_t gs = (int64_t)tn * nst + it;
                     const int bi = (int)(gs & 1);
-                    zc cur[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) cur[i] = nxt[i];
-                    if (it + 1 < nst)
-                        load(L, it + 1);
-                    else if (L + gridDim.x < p.ntiles)
-                        load(L + gridDim.x, 0);
-                    uint4 d[S];
-                    const bool live = gi < p.M;
-#pragma unroll
-                    for (int s = 0; s < S; ++s) d[s] = make_uint4(0, 0, 0, 0);
-                    if (live) planes<0>(cur, e, false, d);
-                    if (gs >= 2 && !mbar_wait(&bar_empty[bi], (uint32_t)(((gs >> 1) - 1) & 1), &abort_sh, p.wait_limit)) {
+                    if (abort_sh || (gs >= 2 && !mbar_wait(&bar_empty[bi], (uint32_t)(((gs >> 1) - 1) & 1), &abort_sh,
+                                                           p.wait_limit))) {
                         abort_sh = 1;
+                        stop = true;
                         break;
                     }
-                    if (abort_sh) break;
-                    const uint32_t sa = sbase + bi * STAGE + blk_off(r, g);
-#pragma unroll
-                    for (int s = 0; s < S; ++s) st_shared_v4(sa + s * APLANE, d[s]);
-                    if (live) planes<1>(cur, e, p.conjA != 0, d);
-#pragma unroll
-                    for (int s = 0; s < S; ++s) st_shared_v4(sa + s * APLANE + APLANE / 2, d[s]);
-                    fence_async_smem();
-                    mbar_arrive(&bar_full[bi]);
+                    mbar_arrive_tx(&bar_full[bi], PRE ? STAGE : ABYTES);
+                    bulk_copy(sbase + bi * STAGE, ia + (int64_t)it * ABYTES, ABYTES, &bar_full[bi]);
+                    if (PRE) bulk_copy(sbase + bi * STAGE + ABYTES, ib + (int64_t)it * BBYTES, BBYTES, &bar_full[bi]);
+                    last[bi] = gs;
                 }
             }
-            // epilogue: a tile is written whole or not at all
+            // every copy has landed before the CTA can leave (after an abort the other
+            // producers may not arrive: the bounded wait then outlasts the copies)
+            for (int bi = 0; bi < 2; ++bi)
+                if (last[bi] >= 0) mbar_wait_plain(&bar_full[bi], (uint32_t)((last[bi] >> 1) & 1));
+        }
+        __syncwarp();
+    } else if (tid < E_THREADS) {
+        // warp: TMEM lanes 32 q .. and complex columns 8 h ..
+        const int q = warp & 3, h = warp >> 2;
+        constexpr int CW = TNC / (E_THREADS / 128);
+        const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(CW * h);
+        double2* epi = reinterpret_cast<double2*>(base + 2 * STAGE) + warp * (32 * 5);
+        int tn = 0;
+        for (int64_t L = blockIdx.x; L < p.ntiles; L += gridDim.x, ++tn) {
+            const Tile t = tile_at(p, L);
+            const int row = t.rt * TM + 32 * q + lane;
+            const int ea = row < p.M ? p.EA[t.b * p.M + row] : 1;
+            const int col0 = t.ct * TNC + CW * h;
+            const int* EBt = p.EB + t.b * p.Nc;
+            // a tile is written whole or not at all
             bool bad = abort_sh != 0;
             if (!bad && !mbar_wait(&bar_done, tn & 1, &abort_sh, p.wait_limit)) {
                 abort_sh = 1;
                 bad = true;
             }
-            if (any256(bad)) break;
+            if (any_epilogue(bad)) break;
             tc_fence_after();
-            const int row = t.rt * TM + 32 * q + lane;
-            const int ea = row < p.M ? p.EA[t.b * p.M + row] : 1;
-            const int col0 = t.ct * TNC + h * (TNC / 2);
             zc* Cb = p.C + t.b * p.sC;
             if (t.rt * TM + 32 * q >= p.M || col0 >= p.Nc) {  // nothing of the tile in this warp
                 tc_fence_before();
@@ -404,30 +373,25 @@ __global__ void __launch_bounds__(Shape<TNC>::THREADS, 1) oz64_kernel(OzArgs p) 
                 continue;
             }
 #pragma unroll 1
-            for (int c0 = 0; c0 < TNC / 2; c0 += 4) {
-                uint32_t re[NLEV][4], im[NLEV][4];
+            for (int c0 = 0; c0 < CW; c0 += 4) {
 #pragma unroll
-                for (int lv = 0; lv < NLEV; ++lv) {
-                    tmem_ld4(lane_addr + (uint32_t)(lv * NR + h * (TNC / 2) + c0), re[lv]);
-                    tmem_ld4(lane_addr + (uint32_t)(lv * NR + TNC + h * (TNC / 2) + c0), im[lv]);
-                }
-                tmem_wait_ld();
-                if (c0 + 4 >= TNC / 2) {  // the accumulators are in registers: the next tile may have them
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bar_tmem);
-                }
+                for (int c2 = 0; c2 < 4; c2 += 2) {
+                    uint32_t x0[S], x1[S], y0[S], y1[S];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const int j = col0 + c0 + c;
-                    const int eb = j < p.Nc ? p.EB[t.b * p.Nc + j] : 1;
-                    uint32_t x[NLEV], y[NLEV];
-#pragma unroll
-                    for (int lv = 0; lv < NLEV; ++lv) {
-                        x[lv] = re[lv][c];
-                        y[lv] = im[lv][c];
+                    for (int lv = 0; lv < S; ++lv) {
+                        tmem_ld2(taddr + (uint32_t)(lv * NR + c0 + c2), x0[lv], x1[lv]);
+                        tmem_ld2(taddr + (uint32_t)(lv * NR + TNC + c0 + c2), y0[lv], y1[lv]);
                     }
-                    epi[lane * 5 + c] = make_double2(combine<NLEV>(x, ea, eb), combine<NLEV>(y, ea, eb));
+                    const int j = col0 + c0 + c2;
+                    const int e0 = j < p.Nc ? EBt[j] : 1, e1 = j + 1 < p.Nc ? EBt[j + 1] : 1;
+                    tmem_wait_ld();
+                    if (c0 + 4 >= CW && c2 == 2) {  // the accumulators are in registers: the next tile may have them
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&bar_tmem);
+                    }
+                    epi[lane * 5 + c2] = make_double2(combine(x0, ea, e0), combine(y0, ea, e0));
+                    epi[lane * 5 + c2 + 1] = make_double2(combine(x1, ea, e1), combine(y1, ea, e1));
                 }
                 __syncwarp();
                 // 8 rows of 4 columns (64 bytes) at a time
@@ -448,87 +412,43 @@ __global__ void __launch_bounds__(Shape<TNC>::THREADS, 1) oz64_kernel(OzArgs p) 
                 __syncwarp();
             }
         }
-    } else {
-        const int tb = tid - A_THREADS;
-        if constexpr (PRE) {
-            if (tb == 0) {
-                int64_t last[2] = {-1, -1};
-                int tn = 0;
-                bool stop = false;
-                for (int64_t L = blockIdx.x; L < p.ntiles && !stop; L += gridDim.x, ++tn) {
-                    const Tile t = tile_at(p, L);
-                    const unsigned char* ia =
-                        static_cast<const unsigned char*>(p.A) + ((int64_t)t.rt * p.nst_img + p.it0) * ABYTES;
-                    const unsigned char* ib =
-                        static_cast<const unsigned char*>(p.B) + ((int64_t)t.ct * p.nst_img + p.it0) * (S * BPLANE);
-                    for (int it = 0; it < nst; ++it) {
-                        const int64_t gs = (int64_t)tn * nst + it;
-                        const int bi = (int)(gs & 1);
-                        if (abort_sh || (gs >= 2 && !mbar_wait(&bar_empty[bi], (uint32_t)(((gs >> 1) - 1) & 1), &abort_sh,
-                                                               p.wait_limit))) {
-                            abort_sh = 1;
-                            stop = true;
-                            break;
-                        }
-                        mbar_arrive_tx(&bar_full[bi], STAGE);
-                        bulk_copy(sbase + bi * STAGE, ia + (int64_t)it * ABYTES, ABYTES, &bar_full[bi]);
-                        bulk_copy(sbase + bi * STAGE + ABYTES, ib + (int64_t)it * (S * BPLANE), S * BPLANE, &bar_full[bi]);
-                        last[bi] = gs;
-                    }
-                }
-                // every copy has landed before the CTA can leave
-                for (int bi = 0; bi < 2; ++bi)
-                    if (last[bi] >= 0) mbar_wait_plain(&bar_full[bi], (uint32_t)((last[bi] >> 1) & 1));
+    } else if constexpr (!PRE) {
+        // group grp fills buffer grp: stages grp, grp + 2, ... of the CTA's sequence
+        const int grp = (tid - E_THREADS) / B_THREADS, tb = (tid - E_THREADS) % B_THREADS;
+        const int j = tb % TNC, g = (tb / TNC) & 1, part = tb / (2 * TNC);
+        double nxt[8];
+        int en = 1;
+        auto load = [&](int gs) -> bool {
+            const int tn = gs / nst, it = gs - tn * nst;
+            const int64_t L = blockIdx.x + (int64_t)tn * gridDim.x;
+            if (L >= p.ntiles) return false;
+            const Tile t = tile_at(p, L);
+            const int gj = t.ct * TNC + j, k = it * TK + 8 * g;
+            en = gj < p.Nc ? p.EB[t.b * p.Nc + gj] : 1;
+            ld8(static_cast<const zc*>(p.B) + t.b * p.sB + k * p.bk + gj * p.bj, part, p.bk,
+                gj < p.Nc ? kleft(p.K, k) : 0, nxt);
+            return true;
+        };
+        bool more = load(grp);
+        for (int gs = grp; more; gs += 2) {
+            uint4 d[S];
+            planes(nxt, en, part && p.conjB, d);
+            more = load(gs + 2);
+            if (abort_sh ||
+                (gs >= 2 && !mbar_wait(&bar_empty[grp], (uint32_t)(((gs >> 1) - 1) & 1), &abort_sh, p.wait_limit))) {
+                abort_sh = 1;
+                break;
             }
-        } else {
-            const int j = tb % TNC, g = (tb / TNC) & 1, part = tb / (2 * TNC);
-            zc nxt[8];
-            auto load = [&](int64_t L, int it) {
-                const Tile t = tile_at(p, L);
-                const int gj = t.ct * TNC + j, k = it * TK + 8 * g;
-                ld8(static_cast<const zc*>(p.B) + t.b * p.sB + k * p.bk + gj * p.bj, p.bk, gj < p.Nc ? kleft(p.K, k) : 0,
-                    nxt);
-            };
-            if (blockIdx.x < p.ntiles) load(blockIdx.x, 0);
-            int tn = 0;
-            bool stop = false;
-            for (int64_t L = blockIdx.x; L < p.ntiles && !stop; L += gridDim.x, ++tn) {
-                const Tile t = tile_at(p, L);
-                const int gj = t.ct * TNC + j;
-                const int e = gj < p.Nc ? p.EB[t.b * p.Nc + gj] : 1;
-                for (int it = 0; it < nst; ++it) {
-                    const int64_t gs = (int64_t)tn * nst + it;
-                    const int bi = (int)(gs & 1);
-                    uint4 d[S];
-                    if (part == 0)
-                        planes<0>(nxt, e, false, d);
-                    else
-                        planes<1>(nxt, e, p.conjB != 0, d);
-                    if (it + 1 < nst)
-                        load(L, it + 1);
-                    else if (L + gridDim.x < p.ntiles)
-                        load(L + gridDim.x, 0);
-                    if (abort_sh || (gs >= 2 && !mbar_wait(&bar_empty[bi], (uint32_t)(((gs >> 1) - 1) & 1), &abort_sh,
-                                                           p.wait_limit))) {
-                        abort_sh = 1;
-                        stop = true;
-                        break;
-                    }
-                    const uint32_t sb = sbase + bi * STAGE + ABYTES + blk_off(j, g);
-                    if (part == 0) {
+            // Re to [Re; .] and [.; Re], Im to [.; Im] and [-Im; .]
+            const uint32_t sb = sbase + grp * STAGE + ABYTES;
+            const uint32_t d0 = sb + blk_off(part ? TNC + j : j, g), d1 = sb + BKS + blk_off(part ? j : TNC + j, g);
 #pragma unroll
-                        for (int s = 0; s < S; ++s) st_shared_v4(sb + s * BPLANE + BLK, d[s]);
-                    } else {
-#pragma unroll
-                        for (int s = 0; s < S; ++s) {
-                            st_shared_v4(sb + s * BPLANE + 2 * BLK, d[s]);
-                            st_shared_v4(sb + s * BPLANE, neg8(d[s]));
-                        }
-                    }
-                    fence_async_smem();
-                    mbar_arrive(&bar_full[bi]);
-                }
+            for (int s = 0; s < S; ++s) {
+                st_shared_v4(d0 + s * BBLK, d[s]);
+                st_shared_v4(d1 + s * BBLK, part ? neg8(d[s]) : d[s]);
             }
+            fence_async_smem();
+            mbar_arrive(&bar_full[grp]);
         }
     }
     tc_fence_before();
@@ -578,37 +498,37 @@ __global__ void __launch_bounds__(256) col_exp64_kernel(int64_t batch, int K, in
     }
 }
 
-// Stage images of A (M x K row-major, row exponents EA): thread = (row, 8 k).
-__global__ void __launch_bounds__(256) a_image_kernel(int64_t M, int K, const zc* __restrict__ A, int64_t ld,
-                                                      const int* __restrict__ EA, unsigned char* __restrict__ img) {
-    const int nst = (K + TK - 1) / TK;
-    const int64_t total = ((M + TM - 1) / TM) * nst * 256;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        const int q = (int)(idx & 255), r = q >> 1, g = q & 1;
-        const int64_t blk = idx >> 8, gi = blk / nst * TM + r;
-        const int k = (int)(blk % nst) * TK + 8 * g;
-        const int e = gi < M ? EA[gi] : 1;
-        zc v[8];
-        ld8(A + gi * ld + k, 1, gi < M ? kleft(K, k) : 0, v);
+// Stage images of op(A) (batch matrices of M x K, element (i, k) at
+// A + b sA + i ai + k ak, row exponents EA): thread = (row, 8 k), rows of consecutive
+// threads when op(A) is stored by columns, else pairs of threads per row.
+__global__ void __launch_bounds__(256) a_image_kernel(int64_t batch, int M, int K, const zc* __restrict__ A, int64_t ai,
+                                                      int64_t ak, int64_t sA, int conj_a, const int* __restrict__ EA,
+                                                      unsigned char* __restrict__ img) {
+    const int nst = (K + TK - 1) / TK, nrt = (M + TM - 1) / TM;
+    const int q = threadIdx.x, r = ak != 1 ? (q & 127) : (q >> 1), g = ak != 1 ? (q >> 7) : (q & 1);
+    for (int64_t blk = blockIdx.x; blk < batch * nrt * nst; blk += gridDim.x) {
+        const int it = (int)(blk % nst);
+        const int64_t br = blk / nst, b = br / nrt;
+        const int gi = (int)(br % nrt) * TM + r, k = it * TK + 8 * g;
         unsigned char* dst = img + blk * (int64_t)(S * APLANE) + blk_off(r, g);
+        if (gi >= M) continue;  // rows beyond the matrix only meet rows of the tile that are not stored
+        const int e = EA[b * M + gi];
+        double re[8], im[8];
+        ld8(A + b * sA + gi * ai + k * ak, ak, kleft(K, k), re, im);
         uint4 d[S];
-        planes<0>(v, e, false, d);
+        planes(re, e, false, d);
 #pragma unroll
         for (int s = 0; s < S; ++s) *reinterpret_cast<uint4*>(dst + s * APLANE) = d[s];
-        planes<1>(v, e, false, d);
+        planes(im, e, conj_a != 0, d);
 #pragma unroll
         for (int s = 0; s < S; ++s) *reinterpret_cast<uint4*>(dst + s * APLANE + APLANE / 2) = d[s];
     }
 }
-// Stage images of a real-coefficient table (2 Kc rows of Nc complex entries):
-// blocks Re even, Im even, Re odd, Im odd rows; thread = (column, 8 kappa, even / odd).
-template <int TNC>
-__global__ void __launch_bounds__(TNC * 4) table_image_kernel(int Kc, int64_t Nc, const zc* __restrict__ T,
-                                                              const int* __restrict__ EB,
-                                                              unsigned char* __restrict__ img) {
-    using Sh = Shape<TNC>;
-    constexpr int BPLANE = Sh::bplane(REALC);
+// Stage images of a real-coefficient table (2 Kc rows of Nc complex entries): k step 0
+// the even rows, k step 1 the odd ones, [Re; Im]; thread = (column, 8 kappa, even / odd).
+__global__ void __launch_bounds__(B_THREADS) table_image_kernel(int Kc, int64_t Nc, const zc* __restrict__ T,
+                                                                const int* __restrict__ EB,
+                                                                unsigned char* __restrict__ img) {
     const int nst = (Kc + TK - 1) / TK;
     const int64_t nblk = ((Nc + TNC - 1) / TNC) * nst;
     const int j = threadIdx.x % TNC, g = (threadIdx.x / TNC) & 1, odd = threadIdx.x / (2 * TNC);
@@ -616,16 +536,16 @@ __global__ void __launch_bounds__(TNC * 4) table_image_kernel(int Kc, int64_t Nc
         const int64_t gj = blk / nst * TNC + j;
         const int k = (int)(blk % nst) * TK + 8 * g;
         const int e = gj < Nc ? EB[gj] : 1;
-        zc v[8];
-        ld8(T + (int64_t)(2 * k + odd) * Nc + gj, 2 * Nc, gj < Nc ? kleft(Kc, k) : 0, v);
-        unsigned char* dst = img + blk * (int64_t)(S * BPLANE) + odd * 2 * Sh::BLK + blk_off(j, g);
+        double re[8], im[8];
+        ld8(T + (int64_t)(2 * k + odd) * Nc + gj, 2 * Nc, gj < Nc ? kleft(Kc, k) : 0, re, im);
+        unsigned char* dst = img + blk * (int64_t)BBYTES + odd * BKS;
         uint4 d[S];
-        planes<0>(v, e, false, d);
+        planes(re, e, false, d);
 #pragma unroll
-        for (int s = 0; s < S; ++s) *reinterpret_cast<uint4*>(dst + s * BPLANE) = d[s];
-        planes<1>(v, e, false, d);
+        for (int s = 0; s < S; ++s) *reinterpret_cast<uint4*>(dst + s * BBLK + blk_off(j, g)) = d[s];
+        planes(im, e, false, d);
 #pragma unroll
-        for (int s = 0; s < S; ++s) *reinterpret_cast<uint4*>(dst + s * BPLANE + Sh::BLK) = d[s];
+        for (int s = 0; s < S; ++s) *reinterpret_cast<uint4*>(dst + s * BBLK + blk_off(TNC + j, g)) = d[s];
     }
 }
 
@@ -640,11 +560,10 @@ int sms() {
 }
 inline unsigned blocks(int64_t n) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(n, 152LL * 64)); }
 
-template <int TNC, bool PRE>
+template <bool PRE>
 int launch(cudaStream_t st, OzArgs p, int64_t batch, int rows_fast) {
-    const int smem = Shape<TNC>::smem(PRE ? REALC : CPLX);
-    auto kern = oz64_kernel<TNC, PRE>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    auto kern = oz64_kernel<PRE>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(oz64)");
     const int nr = (p.M + TM - 1) / TM, nc = (p.Nc + TNC - 1) / TNC;
     p.rows_fast = rows_fast;
@@ -652,7 +571,7 @@ int launch(cudaStream_t st, OzArgs p, int64_t batch, int rows_fast) {
     p.gy = rows_fast ? nc : nr;
     p.ntiles = (int64_t)nr * nc * batch;
     p.wait_limit = tc_wait_limit();
-    kern<<<(unsigned)std::min<int64_t>(p.ntiles, sms()), Shape<TNC>::THREADS, smem, st>>>(p);
+    kern<<<(unsigned)std::min<int64_t>(p.ntiles, sms()), THREADS, SMEM, st>>>(p);
     TBG_LAUNCHED("oz64_kernel");
     return TBG_OK;
 }
@@ -671,53 +590,62 @@ int oz64_col_exps(cudaStream_t st, int64_t batch, int K, int64_t Nc, const zc* B
     return TBG_OK;
 }
 
+size_t oz64_row_image_bytes(int64_t M, int K) {
+    return (size_t)((M + TM - 1) / TM) * ((K + TK - 1) / TK) * S * APLANE;
+}
+constexpr int64_t kImageBytes = 512LL << 20;  // images of A held at a time
+
 int oz64_gemm(cudaStream_t st, int64_t batch, int M, int Nc, int K, const Oz64Operand& A, const Oz64Operand& B, zc* C,
               int64_t ldc, int64_t sC, int mode, int* err) {
     if (batch <= 0 || M <= 0 || Nc <= 0) return TBG_OK;
     if (K <= 0) return set_error(TBG_E_INVALID_ARGUMENT, "oz64_gemm: empty contraction");
     KTimer kt(st, "oz64_kernel", 8.0 * M * Nc * (double)K * batch);
-    OzArgs p = {};
-    p.M = M;
-    p.Nc = Nc;
-    p.ai = A.line;
-    p.ak = A.k;
-    p.sA = A.batch;
-    p.conjA = A.conj;
-    p.EA = A.exps;
-    p.bj = B.line;
-    p.bk = B.k;
-    p.sB = B.batch;
-    p.conjB = B.conj;
-    p.EB = B.exps;
-    p.C = C;
-    p.ldc = ldc;
-    p.sC = sC;
-    p.err = err;
-    for (int k0 = 0; k0 < K; k0 += kMaxK) {
-        p.K = std::min(kMaxK, K - k0);
-        p.A = A.p + k0 * A.k;
-        p.B = B.p + k0 * B.k;
-        p.mode = k0 ? (mode < 0 ? -1 : 1) : mode;
-        // 40 columns a tile unless 32 leave fewer idle ones
-        const int w40 = (Nc + 39) / 40 * 40, w32 = (Nc + 31) / 32 * 32;
-        const int rc = w32 <= w40 ? launch<32, false>(st, p, batch, 0) : launch<40, false>(st, p, batch, 0);
-        if (rc) return rc;
+    const int64_t per = (int64_t)oz64_row_image_bytes(M, K), sub = std::min(batch, std::max<int64_t>(1, kImageBytes / per));
+    unsigned char* img = nullptr;
+    TBG_CUDA(cudaMallocAsync(&img, per * sub, st));
+    int rc = TBG_OK;
+    for (int64_t b0 = 0; b0 < batch && !rc; b0 += sub) {
+        const int64_t nb = std::min(sub, batch - b0);
+        a_image_kernel<<<blocks(nb * ((M + TM - 1) / TM) * ((K + TK - 1) / TK)), 256, 0, st>>>(
+            nb, M, K, A.p + b0 * A.batch, A.line, A.k, A.batch, A.conj, A.exps + b0 * M, img);
+        count_launch();
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) rc = cuda_error(e, "a_image_kernel");
+        OzArgs p = {};
+        p.M = M;
+        p.Nc = Nc;
+        p.A = img;
+        p.EA = A.exps + b0 * M;
+        p.bj = B.line;
+        p.bk = B.k;
+        p.sB = B.batch;
+        p.conjB = B.conj;
+        p.EB = B.exps + b0 * Nc;
+        p.C = C + b0 * sC;
+        p.ldc = ldc;
+        p.sC = sC;
+        p.err = err;
+        p.nst_img = (K + TK - 1) / TK;
+        for (int k0 = 0; k0 < K && !rc; k0 += kMaxK) {
+            p.K = std::min(kMaxK, K - k0);
+            p.it0 = k0 / TK;
+            p.B = B.p + b0 * B.batch + k0 * B.k;
+            p.mode = k0 ? (mode < 0 ? -1 : 1) : mode;
+            rc = launch<false>(st, p, nb, 0);
+        }
     }
-    return TBG_OK;
+    cudaFreeAsync(img, st);
+    return rc;
 }
 
-constexpr int kTab = 40;  // columns of a table image's tiles
 size_t oz64_table_image_bytes(int Kc, int64_t Nc) {
-    return (size_t)((Nc + kTab - 1) / kTab) * ((Kc + TK - 1) / TK) * S * Shape<kTab>::bplane(REALC);
-}
-size_t oz64_row_image_bytes(int64_t M, int Kc) {
-    return (size_t)((M + TM - 1) / TM) * ((Kc + TK - 1) / TK) * S * APLANE;
+    return (size_t)((Nc + TNC - 1) / TNC) * ((Kc + TK - 1) / TK) * BBYTES;
 }
 // Image of a table of 2 Kc rows x Nc entries and its column exponents EB (Nc).
 int oz64_table_image(cudaStream_t st, int Kc, int64_t Nc, const zc* T, int* EB, void* img) {
     if (int rc = oz64_col_exps(st, 1, 2 * Kc, Nc, T, Nc, 0, EB)) return rc;
-    const int64_t nblk = ((Nc + kTab - 1) / kTab) * ((Kc + TK - 1) / TK);
-    table_image_kernel<kTab><<<blocks(nblk), kTab * 4, 0, st>>>(Kc, Nc, T, EB, static_cast<unsigned char*>(img));
+    const int64_t nblk = ((Nc + TNC - 1) / TNC) * ((Kc + TK - 1) / TK);
+    table_image_kernel<<<blocks(nblk), B_THREADS, 0, st>>>(Kc, Nc, T, EB, static_cast<unsigned char*>(img));
     TBG_LAUNCHED("table_image_kernel");
     return TBG_OK;
 }
@@ -731,7 +659,7 @@ int oz64_table_product(cudaStream_t st, int64_t M, int64_t Nc, int Kc, const zc*
     {
         KTimer kt(st, "oz64_image_kernel");
         if (int rc = oz64_row_exps(st, 1, (int)M, Kc, coef, ld, 0, EA)) return rc;
-        a_image_kernel<<<blocks((M + TM - 1) / TM * nst), 256, 0, st>>>(M, Kc, coef, ld, EA,
+        a_image_kernel<<<blocks((M + TM - 1) / TM * nst), 256, 0, st>>>(1, (int)M, Kc, coef, ld, 1, 0, 0, EA,
                                                                         static_cast<unsigned char*>(aimg));
         TBG_LAUNCHED("a_image_kernel");
     }
@@ -739,8 +667,7 @@ int oz64_table_product(cudaStream_t st, int64_t M, int64_t Nc, int Kc, const zc*
     OzArgs p = {};
     p.M = (int)M;
     p.Nc = (int)Nc;
-    p.A = aimg;
-    p.ak = 1;
+    p.A = static_cast<const unsigned char*>(aimg);
     p.B = img;
     p.EA = EA;
     p.EB = EB;
@@ -753,7 +680,7 @@ int oz64_table_product(cudaStream_t st, int64_t M, int64_t Nc, int Kc, const zc*
         p.it0 = k0 / TK;
         p.mode = k0 ? 1 : 0;
         // row tiles fastest: CTAs running together share a column tile's image in L2
-        if (int rc = launch<kTab, true>(st, p, 1, 1)) return rc;
+        if (int rc = launch<true>(st, p, 1, 1)) return rc;
     }
     return TBG_OK;
 }

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,nk", [(165, 1), (177, 40), (192, 2), (193, 160), (256, 3), (257, 2), (300, 9), (512, 2),
-                                  (80, 300), (97, 170), (128, 72), (129, 75), (161, 38)])
+                                  (56, 260), (63, 180), (65, 170), (97, 60), (128, 24), (129, 30), (161, 12)])
 def test_random(n, nk):
     check(random_hermitian(np.random.default_rng(n), nk, n))
 
