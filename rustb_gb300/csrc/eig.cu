@@ -249,6 +249,49 @@ __device__ bool twisted_vector(int N, const T* __restrict__ d, const T* __restri
     return true;
 }
 
+// Vectors c0 .. c1 of a cluster by inverse iteration with Gram-Schmidt against its
+// earlier members, into columns of U (N x N); x, u0, u1, u2: N values each, G apart.
+template <typename T>
+__device__ void inverse_iteration(int N, const T* d, const T* e, const T* lam, int c0, int c1, T tnorm, T pert, T* x,
+                                  T* u0, T* u1, T* u2, int G, cx<T>* U) {
+    T shift_prev = -INFINITY;
+    for (int jj = c0; jj <= c1; ++jj) {
+        T shift = lam[jj];
+        // separate coincident shifts inside a cluster
+        const T pertol = T(10) * Lim<T>::eps() * max(fabs(shift), tnorm * T(1e-3));
+        if (jj > c0 && shift - shift_prev < pertol) shift = shift_prev + pertol;
+        shift_prev = shift;
+        for (int r = 0; r < N; ++r) {
+            const unsigned h = hash32((unsigned)(r * 7919 + jj * 104729 + 12345));
+            x[(size_t)r * G] = T(1) + T(0.5) * ((T)(h & 0xffff) / T(65535) - T(0.5));
+        }
+        for (int iter = 0; iter < (sizeof(T) == sizeof(float) ? 2 : 3); ++iter) {
+            tri_solve<T>(N, d, e, shift, pert, x, u0, u1, u2, G);
+            // Gram-Schmidt against earlier cluster members (stored in U, real parts)
+            for (int pp = c0; pp < jj; ++pp) {
+                T dot = 0;
+                for (int r = 0; r < N; ++r) dot += U[(size_t)r * N + pp].re * x[(size_t)r * G];
+                for (int r = 0; r < N; ++r) x[(size_t)r * G] -= dot * U[(size_t)r * N + pp].re;
+            }
+            T nrm = 0, amax = 0;
+            for (int r = 0; r < N; ++r) amax = max(amax, fabs(x[(size_t)r * G]));
+            if (!(amax > T(0)) || isinf(amax)) {
+                for (int r = 0; r < N; ++r) x[(size_t)r * G] = (r == (jj % N)) ? T(1) : T(0);
+                amax = 1;
+            }
+            const T sc = T(1) / amax;
+            for (int r = 0; r < N; ++r) {
+                const T xv = x[(size_t)r * G] * sc;
+                x[(size_t)r * G] = xv;
+                nrm += xv * xv;
+            }
+            const T inv = T(1) / sqrt(nrm);
+            for (int r = 0; r < N; ++r) x[(size_t)r * G] *= inv;
+        }
+        for (int r = 0; r < N; ++r) U[(size_t)r * N + jj] = mk<T>(x[(size_t)r * G], T(0));
+    }
+}
+
 template <typename T>
 struct EigShared {
     cx<T>* A;   // N*N (shared or global)
@@ -733,42 +776,7 @@ __global__ void __launch_bounds__(MINB == 3 ? 320 : 512, MINB) heev_kernel(int N
                     T* u0 = x + (size_t)N * G;
                     T* u1 = u0 + (size_t)N * G;
                     T* u2 = u1 + (size_t)N * G;
-                    T shift_prev = -INFINITY;
-                    for (int jj = i; jj <= c1; ++jj) {
-                        T shift = sh.lam[jj];
-                        // separate coincident shifts inside a cluster
-                        const T pertol = T(10) * Lim<T>::eps() * max(fabs(shift), tnorm * T(1e-3));
-                        if (jj > i && shift - shift_prev < pertol) shift = shift_prev + pertol;
-                        shift_prev = shift;
-                        for (int r = 0; r < N; ++r) {
-                            const unsigned h = hash32((unsigned)(r * 7919 + jj * 104729 + 12345));
-                            x[(size_t)r * G] = T(1) + T(0.5) * ((T)(h & 0xffff) / T(65535) - T(0.5));
-                        }
-                        for (int iter = 0; iter < (sizeof(T) == sizeof(float) ? 2 : 3); ++iter) {
-                            tri_solve<T>(N, sh.d, sh.e, shift, pert, x, u0, u1, u2, G);
-                            // Gram-Schmidt against earlier cluster members (stored in U, real parts)
-                            for (int pp = i; pp < jj; ++pp) {
-                                T dot = 0;
-                                for (int r = 0; r < N; ++r) dot += U[(size_t)r * N + pp].re * x[(size_t)r * G];
-                                for (int r = 0; r < N; ++r) x[(size_t)r * G] -= dot * U[(size_t)r * N + pp].re;
-                            }
-                            T nrm = 0, amax = 0;
-                            for (int r = 0; r < N; ++r) amax = max(amax, fabs(x[(size_t)r * G]));
-                            if (!(amax > T(0)) || isinf(amax)) {
-                                for (int r = 0; r < N; ++r) x[(size_t)r * G] = (r == (jj % N)) ? T(1) : T(0);
-                                amax = 1;
-                            }
-                            const T sc = T(1) / amax;
-                            for (int r = 0; r < N; ++r) {
-                                const T xv = x[(size_t)r * G] * sc;
-                                x[(size_t)r * G] = xv;
-                                nrm += xv * xv;
-                            }
-                            const T inv = T(1) / sqrt(nrm);
-                            for (int r = 0; r < N; ++r) x[(size_t)r * G] *= inv;
-                        }
-                        for (int r = 0; r < N; ++r) U[(size_t)r * N + jj] = mk<T>(x[(size_t)r * G], T(0));
-                    }
+                    inverse_iteration<T>(N, sh.d, sh.e, sh.lam, i, c1, tnorm, pert, x, u0, u1, u2, G, U);
                 }
             }
             __syncthreads();
@@ -1107,6 +1115,196 @@ int allow_max_smem(K kern, size_t need) {
     return TBG_OK;
 }
 
+// Back-transformation pass of the FP32 solver (reflectors and tau in work).
+int launch_bt32(cudaStream_t st, int N, int64_t batch, const void* work, cc* U, int PB) {
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const size_t bsm = bt_tiled_smem_bytes(N, PB);
+    auto bk = PB >= ((N + 3) & ~3) ? heev_bt_tiled_kernel<false> : heev_bt_tiled_kernel<true>;
+    if (int rc = allow_max_smem(bk, bsm)) return rc;
+    KTimer kt(st, "heev_bt_kernel", 8.0 * (double)N * N * N * batch);
+    bk<<<(unsigned)std::min<int64_t>(nsm, batch), 512, bsm, st>>>(N, batch, static_cast<const cc*>(work), U, PB);
+    TBG_LAUNCHED("heev_bt_kernel");
+    return TBG_OK;
+}
+
+// Tridiagonal stage of the FP32 solver for the given forms of matrices beyond the
+// TMEM-resident sizes (de: d then e): eigenvalues by bisection, vectors of isolated
+// ones by the twisted factorisation, as heev_kernel does.  There the stage ran in
+// the reduction's launch shape, one CTA per SM around the matrix's shared memory;
+// it needs little of that, so here `len` eigenvalues (a thread each, their outer
+// neighbours too) make a CTA and many share an SM: 304 matrices of 251 bands
+// 2.06 -> 1.03 ms with the clusters below.  The factorisation's scratch is the
+// imaginary part of the column that the vector then fills; a column left to
+// tri32_cluster_kernel has a 1 there in row 0.
+struct Tri32Bounds {
+    float lo, hi, tnorm, pivmin;
+    bool bad;
+};
+__device__ __forceinline__ Tri32Bounds tri32_bounds(int N, const float* d, const float* e, const float* e2, int lane) {
+    Tri32Bounds t;
+    float lo = INFINITY, hi = -INFINITY, em = 0;
+    bool bad = false;
+    for (int i = lane; i < N; i += 32) {
+        const float r = ((i > 0) ? fabsf(e[i - 1]) : 0.f) + ((i < N - 1) ? fabsf(e[i]) : 0.f);
+        lo = fminf(lo, d[i] - r);
+        hi = fmaxf(hi, d[i] + r);
+        em = fmaxf(em, e2[i]);
+        bad = bad || !isfinite(d[i]) || !isfinite(e[i]);
+    }
+    lo = -warp_max(-lo);
+    hi = warp_max(hi);
+    em = warp_max(em);
+    t.bad = __any_sync(0xffffffffu, bad);
+    t.tnorm = fmaxf(fabsf(lo), fabsf(hi));
+    if (!(t.tnorm == t.tnorm) || isinf(t.tnorm)) {
+        t.bad = true;
+        t.tnorm = 1.f;
+        lo = -1.f;
+        hi = 1.f;
+    }
+    t.pivmin = FLT_MIN * fmaxf(1.f, em);
+    const float pad = 2.f * FLT_EPSILON * t.tnorm + 4.f * t.pivmin;
+    t.lo = lo - pad - 2.f * FLT_EPSILON * t.tnorm;
+    t.hi = hi + pad + 2.f * FLT_EPSILON * t.tnorm;
+    if (t.tnorm == 0.f) {
+        t.lo = -t.pivmin;
+        t.hi = t.pivmin;
+    }
+    return t;
+}
+// off-diagonals below eps (|d_i| + |d_i+1|) are set to zero (decoupled blocks)
+__device__ __forceinline__ float tri32_deflate(int N, const float* src, int i) {
+    const float ei = i < N - 1 ? src[N + i] : 0.f;
+    return (i < N - 1 && fabsf(ei) <= FLT_EPSILON * (fabsf(src[i]) + fabsf(src[i + 1]))) ? 0.f : ei;
+}
+__global__ void __launch_bounds__(128) tri32_kernel(int N, int64_t batch, int parts, int len,
+                                                    const float* __restrict__ de, double* __restrict__ Eout,
+                                                    cc* __restrict__ Uout, int* __restrict__ status) {
+    extern __shared__ float tri32_smem[];
+    float *d = tri32_smem, *e = d + N, *e2 = e + N, *lam = e2 + N;  // lam: len + 2
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (int64_t unit = blockIdx.x; unit < batch * parts; unit += gridDim.x) {
+        const int64_t b = unit / parts;
+        const int i0 = (int)(unit % parts) * len, i1 = min(i0 + len, N), h0 = max(i0 - 1, 0), h1 = min(i1 + 1, N);
+        const float* src = de + b * 2 * N;
+        for (int i = tid; i < N; i += blockDim.x) {
+            d[i] = src[i];
+            e[i] = tri32_deflate(N, src, i);
+            e2[i] = e[i] * e[i];
+        }
+        __syncthreads();
+        const Tri32Bounds t = tri32_bounds(N, d, e, e2, lane);
+        if (t.bad && tid == 0 && i0 == 0 && status) atomicOr(status, 1);
+        const float atol = 2.f * FLT_EPSILON * t.tnorm + 2.f * t.pivmin;
+        for (int i = h0 + tid; i < h1; i += blockDim.x) {
+            float a = t.lo, c = t.hi;
+            for (int it = 0; it < 200 && !(c - a <= atol + 2.f * FLT_EPSILON * fmaxf(fabsf(a), fabsf(c))); ++it) {
+                const float x = a + 0.5f * (c - a);
+                if (sturm_count<float>(N, d, e2, x, t.pivmin) > i)
+                    c = x;
+                else
+                    a = x;
+            }
+            float l = 0.5f * (a + c);
+            // an isolated diagonal entry inside the final bracket is the exact eigenvalue
+            for (int j = 0; j < N; ++j) {
+                const bool one = (j == 0 || e[j - 1] == 0.f) && (j == N - 1 || e[j] == 0.f);
+                if (one && d[j] >= a && d[j] <= c) {
+                    l = d[j];
+                    break;
+                }
+            }
+            lam[i - h0] = l;
+            if (i >= i0 && i < i1) Eout[b * N + i] = (double)l;
+        }
+        __syncthreads();
+        const float ctol = 1e-3f * fmaxf(t.tnorm, FLT_MIN), pert = fmaxf(FLT_EPSILON * t.tnorm, t.pivmin);
+        if (Uout)
+            for (int i = i0 + tid; i < i1; i += blockDim.x) {
+                const float* l = lam + (i - h0);
+                const bool iso = (i == 0 || l[0] - l[-1] > ctol) && (i == N - 1 || l[1] - l[0] > ctol);
+                cc* u = Uout + b * N * N + i;
+                if (!iso || !twisted_vector<float>(N, d, e, e2, l[0], pert, &u->im, 2 * N, u, N)) *u = mk(0.f, 1.f);
+            }
+        __syncthreads();
+    }
+}
+// The columns tri32_kernel left: a lane per cluster among `len` eigenvalues of a
+// matrix, inverse iteration with Gram-Schmidt against the earlier members.
+__global__ void __launch_bounds__(32) tri32_cluster_kernel(int N, int64_t batch, int parts, int len, int G,
+                                                           const float* __restrict__ de,
+                                                           const double* __restrict__ Ein, cc* __restrict__ Uout) {
+    extern __shared__ float tri32_smem[];
+    float *d = tri32_smem, *e = d + N, *e2 = e + N, *lam = e2 + N, *scr = lam + N;  // scr: 4 N G
+    const int lane = threadIdx.x;
+    for (int64_t unit = blockIdx.x; unit < batch * parts; unit += gridDim.x) {
+        const int64_t b = unit / parts;
+        const int i0 = (int)(unit % parts) * len, i1 = min(i0 + len, N);
+        cc* U = Uout + b * N * N;
+        bool any = false;
+        for (int i = i0 + lane; i < i1; i += 32) any = any || U[i].im != 0.f;
+        if (!__any_sync(0xffffffffu, any)) continue;
+        __syncwarp();
+        const float* src = de + b * 2 * N;
+        for (int i = lane; i < N; i += 32) {
+            d[i] = src[i];
+            e[i] = tri32_deflate(N, src, i);
+            e2[i] = e[i] * e[i];
+            lam[i] = (float)Ein[b * N + i];
+        }
+        __syncwarp();
+        const Tri32Bounds t = tri32_bounds(N, d, e, e2, lane);
+        const float ctol = 1e-3f * fmaxf(t.tnorm, FLT_MIN), pert = fmaxf(FLT_EPSILON * t.tnorm, t.pivmin);
+        // the clusters that start here, G lanes at a time
+        for (int g0 = i0; g0 < i1; g0 += 32) {
+            const int ic = g0 + lane;
+            const bool mine = ic < i1 && (ic == 0 || lam[ic] - lam[ic - 1] > ctol) && U[ic].im != 0.f;
+            unsigned todo = __ballot_sync(0xffffffffu, mine);
+            while (todo) {
+                // lane l < G takes the l-th remaining start
+                unsigned rest = todo;
+                int start = -1;
+                for (int l = 0; l < G && rest; ++l) {
+                    const int bit = __ffs(rest) - 1;
+                    rest &= rest - 1;
+                    if (l == lane) start = g0 + bit;
+                }
+                todo = rest;
+                if (start >= 0) {
+                    int c1 = start;
+                    while (c1 + 1 < N && lam[c1 + 1] - lam[c1] <= ctol) ++c1;
+                    float* x = scr + lane;
+                    float *u0 = x + (size_t)N * G, *u1 = u0 + (size_t)N * G, *u2 = u1 + (size_t)N * G;
+                    inverse_iteration<float>(N, d, e, lam, start, c1, t.tnorm, pert, x, u0, u1, u2, G, U);
+                }
+                __syncwarp();
+            }
+        }
+    }
+}
+// E and U (vectors of the tridiagonal forms) from de.
+int tri32(cudaStream_t st, int N, int64_t batch, const float* de, double* E, cc* U, int* status) {
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    KTimer kt(st, "tri32_kernel");
+    const int parts = (N + 125) / 126, len = (N + parts - 1) / parts;
+    const int64_t ctas = std::min<int64_t>(batch * parts, (int64_t)nsm * 64);
+    tri32_kernel<<<(unsigned)ctas, 128, sizeof(float) * (3 * (size_t)N + len + 2), st>>>(N, batch, parts, len, de, E, U,
+                                                                                         status);
+    TBG_LAUNCHED("tri32_kernel");
+    if (!U) return TBG_OK;
+    const int G = (int)std::max<size_t>(1, std::min<size_t>(16, (48 * 1024 / sizeof(float) - 4 * (size_t)N) / (4 * (size_t)N)));
+    const int cparts = (N + 31) / 32;
+    const int64_t cctas = std::min<int64_t>(batch * cparts, (int64_t)nsm * 64);
+    tri32_cluster_kernel<<<(unsigned)cctas, 32, sizeof(float) * (4 * (size_t)N + 4 * (size_t)N * G), st>>>(
+        N, batch, cparts, 32, G, de, E, U);
+    TBG_LAUNCHED("tri32_cluster_kernel");
+    return TBG_OK;
+}
+
 template <typename T, bool A_SMEM, int MINB = (A_SMEM ? 2 : 1), bool HYB = false>
 int launch_heev(cudaStream_t st, int N, int64_t batch, zc* H, double* E, cx<T>* U, void* work,
                 size_t work_bytes, int* status_d, const char* name, int G, int PB, const float4* Hpair = nullptr,
@@ -1158,15 +1356,8 @@ int launch_heev(cudaStream_t st, int N, int64_t batch, zc* H, double* E, cx<T>* 
         TBG_LAUNCHED(name);
     }
     if constexpr (A_SMEM) {
-        if (!U || skip_bt || stop > 0) return TBG_OK;
         static_assert(sizeof(T) == sizeof(float), "the shared-memory solver is the FP32 one");
-        const size_t bsm = bt_tiled_smem_bytes(N, PB);
-        auto bk = PB >= ((N + 3) & ~3) ? heev_bt_tiled_kernel<false> : heev_bt_tiled_kernel<true>;
-        if (int rc = allow_max_smem(bk, bsm)) return rc;
-        KTimer kt(st, "heev_bt_kernel", 8.0 * (double)N * N * N * batch);
-        bk<<<(unsigned)std::min<int64_t>(nsm, batch), 512, bsm, st>>>(N, batch, reinterpret_cast<const cc*>(work),
-                                                                      reinterpret_cast<cc*>(U), PB);
-        TBG_LAUNCHED("heev_bt_kernel");
+        if (U && !skip_bt && stop == 0) return launch_bt32(st, N, batch, work, U, PB);
     }
     return TBG_OK;
 }
@@ -1359,30 +1550,27 @@ int eig_batched_f32(cudaStream_t st, int N, int64_t batch, zc* H, double* E, cc*
         auto finish = [&]() {
             return hetrd_tc(st, 128, batch, nullptr, nullptr, static_cast<cc*>(work), de, status_d, Tb, N, stop);
         };
+        auto tri = [&]() {
+            if (int r = tri32(st, N, batch, de, E, U, status_d)) return r;
+            return U ? launch_bt32(st, N, batch, work, U, tp.PB) : TBG_OK;
+        };
         if (tp.r0 > 0) {
             rc = launch_heev<float, true, 2, true>(st, N, batch, H, E, U, work, work_bytes, status_d,
                                                    "heev_kernel<float,hybrid>", tp.G, tp.PB, Hpair, nullptr, false,
                                                    tp.r0, stop, Tb, de, tp.off_ag);
             if (!rc) rc = finish();
-            if (!rc)
-                rc = launch_heev<float, true, 2, true>(st, N, batch, H, E, U, work, work_bytes, status_d,
-                                                       "heev_tri_kernel<float>", tp.G, tp.PB, Hpair, de, false, tp.r0,
-                                                       0, nullptr, nullptr, tp.off_ag);
+            if (!rc) rc = tri();
         } else if (tp.ctas == 3) {
             rc = launch_heev<float, true, 3>(st, N, batch, H, E, U, work, work_bytes, status_d,
                                              "heev_kernel<float,smem>", tp.G, tp.PB, Hpair, nullptr, false, 0, stop, Tb,
                                              de);
             if (!rc) rc = finish();
-            if (!rc)
-                rc = launch_heev<float, true, 3>(st, N, batch, H, E, U, work, work_bytes, status_d,
-                                                 "heev_tri_kernel<float>", tp.G, tp.PB, Hpair, de);
+            if (!rc) rc = tri();
         } else {
             rc = launch_heev<float, true>(st, N, batch, H, E, U, work, work_bytes, status_d, "heev_kernel<float,smem>",
                                           tp.G, tp.PB, Hpair, nullptr, false, 0, stop, Tb, de);
             if (!rc) rc = finish();
-            if (!rc)
-                rc = launch_heev<float, true>(st, N, batch, H, E, U, work, work_bytes, status_d,
-                                              "heev_tri_kernel<float>", tp.G, tp.PB, Hpair, de);
+            if (!rc) rc = tri();
         }
         return rc;
     }
