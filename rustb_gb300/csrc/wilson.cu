@@ -33,7 +33,7 @@ namespace tbg {
 namespace {
 
 constexpr double kTwoPiW = 6.283185307179586476925286766559;
-constexpr int kMaxNS = 80;  // Newton-Schulz steps (quadratic from sigma_min >= 1e-6 needs ~45)
+constexpr int kMaxNS = 52;  // Newton-Schulz steps: 1.875^52, so singular values from about 1e-14 on reach 1
 
 // endphase[l][a] = exp(-2 pi i (k_T - k_0) . tau_a)
 __global__ void wl_endphase_kernel(int64_t n_loops, int n_k, int dim, const double* __restrict__ kv, int N,
@@ -139,9 +139,30 @@ __device__ void smem_mm(int n, const zc* A, const zc* B, zc* C) {
     }
 }
 
-// O[seg] <- its unitary factor U V^dagger, one block per segment, by the
-// Newton-Schulz iteration: stop when X is unitary to rounding, or one step
-// after the error fell below 1e-8 (that step squares it).
+// C (Hermitian) = f(i, j) over the upper triangle, rows i and n - 1 - i side by side so
+// that no thread's round is padding, mirrored; all threads of the block.
+template <typename F>
+__device__ __forceinline__ void smem_hermitian(int n, zc* C, F f) {
+    const int w = n + 1, half = (n + 1) / 2;
+    for (int e = threadIdx.x; e < half * w; e += blockDim.x) {
+        const int p = e / w, c = e - p * w;
+        const int i = c < n - p ? p : n - 1 - p, j = c < n - p ? p + c : i + c - (n - p);
+        if (c >= n - p && i == p) continue;  // the middle row of an odd n stands alone
+        zc s = f(i, j);
+        if (i == j) s.im = 0.0;
+        C[i * n + j] = s;
+        C[j * n + i] = conj(s);
+    }
+}
+
+// O[seg] <- its unitary factor U V^dagger, one block per segment, by the third-order
+// member of the Newton-Schulz family, X <- X (15 I - 10 Y + 3 Y^2) / 8 with
+// Y = X^dagger X (singular values s <- s (15 - 10 s^2 + 3 s^4) / 8, from (0, 1] as
+// overlaps have them): the FP64 pipe bounds it, and Y and Y^2 are Hermitian, so a step
+// costs two products against one and a half for the second-order X (3 I - Y) / 2 but
+// takes 1 - s^2 = e to 5 e^3 / 16 instead of 3 e^2 / 4 (4032 segments of 32 bands
+// 5.9 ms, 6.3 with that).  Stop when X is unitary to rounding, or one step after
+// the error fell below 1e-6 (that step cubes it).
 __global__ void __launch_bounds__(256) wl_polar_kernel(int n, zc* __restrict__ O, int* __restrict__ status) {
     extern __shared__ zc wsm[];
     zc* X = wsm;
@@ -154,18 +175,11 @@ __global__ void __launch_bounds__(256) wl_polar_kernel(int n, zc* __restrict__ O
     __syncthreads();
     double err = 1.0;
     for (int it = 0; it < kMaxNS; ++it) {
-        // Y = X^dagger X: the upper triangle, rows i and n - 1 - i side by side, mirrored
-        const int w = n + 1, half = (n + 1) / 2;
-        for (int e = threadIdx.x; e < half * w; e += blockDim.x) {
-            const int p = e / w, c = e - p * w;
-            const int i = c < n - p ? p : n - 1 - p, j = c < n - p ? p + c : i + c - (n - p);
-            if (c >= n - p && i == p) continue;  // the middle row of an odd n stands alone
+        smem_hermitian(n, Y, [&](int i, int j) {  // Y = X^dagger X
             zc s = mk(0.0, 0.0);
             for (int k = 0; k < n; ++k) fma_cjx(s, X[k * n + i], X[k * n + j]);
-            if (i == j) s.im = 0.0;
-            Y[i * n + j] = s;
-            Y[j * n + i] = conj(s);
-        }
+            return s;
+        });
         if (threadIdx.x == 0) s_err = 0.0;
         __syncthreads();
         double m = 0.0;
@@ -178,15 +192,22 @@ __global__ void __launch_bounds__(256) wl_polar_kernel(int n, zc* __restrict__ O
         __syncthreads();
         err = s_err;
         if (err <= 4e-16 * n) break;  // uniform: every thread read the same s_err
-        // Y <- (3 I - Y) / 2, X <- X Y
+        smem_hermitian(n, Z, [&](int i, int j) {  // Z = Y^2
+            zc s = mk(0.0, 0.0);
+            for (int k = 0; k < n; ++k) fma_cjx(s, Y[k * n + i], Y[k * n + j]);
+            return s;
+        });
+        __syncthreads();
+        // Y <- (15 I - 10 Y + 3 Y^2) / 8, X <- X Y
         for (int e = threadIdx.x; e < nn; e += blockDim.x)
-            Y[e] = mk(((e / n == e % n) ? 1.5 : 0.0) - 0.5 * Y[e].re, -0.5 * Y[e].im);
+            Y[e] = mk(fma(0.375, Z[e].re, fma(-1.25, Y[e].re, (e / n == e % n) ? 1.875 : 0.0)),
+                      fma(0.375, Z[e].im, -1.25 * Y[e].im));
         __syncthreads();
         smem_mm(n, X, Y, Z);
         __syncthreads();
         for (int e = threadIdx.x; e < nn; e += blockDim.x) X[e] = Z[e];
         __syncthreads();
-        if (err <= 1e-8) {
+        if (err <= 1e-6) {
             err = 0.0;
             break;
         }
