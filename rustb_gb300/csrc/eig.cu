@@ -1133,11 +1133,12 @@ int launch_bt32(cudaStream_t st, int N, int64_t batch, const void* work, cc* U, 
 // TMEM-resident sizes (de: d then e): eigenvalues by bisection, vectors of isolated
 // ones by the twisted factorisation, as heev_kernel does.  There the stage ran in
 // the reduction's launch shape, one CTA per SM around the matrix's shared memory;
-// it needs little of that, so here `len` eigenvalues (a thread each, their outer
+// it needs little of that, so here `len` eigenvalues (S threads each, their outer
 // neighbours too) make a CTA and many share an SM: 304 matrices of 251 bands
-// 2.06 -> 1.03 ms with the clusters below.  The factorisation's scratch is the
-// imaginary part of the column that the vector then fills; a column left to
-// tri32_cluster_kernel has a 1 there in row 0.
+// 2.06 -> 1.04 ms with the clusters below.  The same steps in the same order, S as
+// there, so that the results are the same to the last bit.  The factorisation's
+// scratch is the imaginary part of the column that the vector then fills; a column
+// left to tri32_cluster_kernel has a 1 there in row 0.
 struct Tri32Bounds {
     float lo, hi, tnorm, pivmin;
     bool bad;
@@ -1179,7 +1180,7 @@ __device__ __forceinline__ float tri32_deflate(int N, const float* src, int i) {
     const float ei = i < N - 1 ? src[N + i] : 0.f;
     return (i < N - 1 && fabsf(ei) <= FLT_EPSILON * (fabsf(src[i]) + fabsf(src[i + 1]))) ? 0.f : ei;
 }
-__global__ void __launch_bounds__(128) tri32_kernel(int N, int64_t batch, int parts, int len,
+__global__ void __launch_bounds__(128) tri32_kernel(int N, int64_t batch, int parts, int len, int S,
                                                     const float* __restrict__ de, double* __restrict__ Eout,
                                                     cc* __restrict__ Uout, int* __restrict__ status) {
     extern __shared__ float tri32_smem[];
@@ -1198,26 +1199,42 @@ __global__ void __launch_bounds__(128) tri32_kernel(int N, int64_t batch, int pa
         const Tri32Bounds t = tri32_bounds(N, d, e, e2, lane);
         if (t.bad && tid == 0 && i0 == 0 && status) atomicOr(status, 1);
         const float atol = 2.f * FLT_EPSILON * t.tnorm + 2.f * t.pivmin;
-        for (int i = h0 + tid; i < h1; i += blockDim.x) {
+        // multisection, S = 1 or 2 threads per eigenvalue, as in heev_kernel (one pass:
+        // (len + 2) S <= threads)
+        {
+            const int i = h0 + tid / S, q = tid % S;
+            const int gbase = (lane / S) * S;
+            const unsigned gmask = (1u << S) - 1u;
             float a = t.lo, c = t.hi;
-            for (int it = 0; it < 200 && !(c - a <= atol + 2.f * FLT_EPSILON * fmaxf(fabsf(a), fabsf(c))); ++it) {
-                const float x = a + 0.5f * (c - a);
-                if (sturm_count<float>(N, d, e2, x, t.pivmin) > i)
-                    c = x;
-                else
-                    a = x;
-            }
-            float l = 0.5f * (a + c);
-            // an isolated diagonal entry inside the final bracket is the exact eigenvalue
-            for (int j = 0; j < N; ++j) {
-                const bool one = (j == 0 || e[j - 1] == 0.f) && (j == N - 1 || e[j] == 0.f);
-                if (one && d[j] >= a && d[j] <= c) {
-                    l = d[j];
-                    break;
+            bool done = i >= h1;
+            for (int it = 0; it < 200; ++it) {
+                done = done || (c - a <= atol + float(2) * FLT_EPSILON * max(fabs(a), fabs(c)));
+                if (__all_sync(0xffffffffu, done)) break;
+                const float h = (c - a) / float(S + 1);
+                const float x = a + float(q + 1) * h;
+                const bool above = !done && sturm_count<float>(N, d, e2, x, t.pivmin) > i;
+                const unsigned g = (__ballot_sync(0xffffffffu, above) >> gbase) & gmask;
+                if (!done) {
+                    const int qs = g ? __ffs(g) - 1 : S;  // first inner point above the eigenvalue
+                    const float na = (qs == 0) ? a : a + float(qs) * h;
+                    const float nc = (qs == S) ? c : a + float(qs + 1) * h;
+                    a = na;
+                    c = nc;
                 }
             }
-            lam[i - h0] = l;
-            if (i >= i0 && i < i1) Eout[b * N + i] = (double)l;
+            if (i < h1 && q == 0) {
+                float l = float(0.5) * (a + c);
+                // an isolated diagonal entry inside the final bracket is the exact eigenvalue
+                for (int j = 0; j < N; ++j) {
+                    const bool one = (j == 0 || e[j - 1] == 0.f) && (j == N - 1 || e[j] == 0.f);
+                    if (one && d[j] >= a && d[j] <= c) {
+                        l = d[j];
+                        break;
+                    }
+                }
+                lam[i - h0] = l;
+                if (i >= i0 && i < i1) Eout[b * N + i] = (double)l;
+            }
         }
         __syncthreads();
         const float ctol = 1e-3f * fmaxf(t.tnorm, FLT_MIN), pert = fmaxf(FLT_EPSILON * t.tnorm, t.pivmin);
@@ -1284,16 +1301,18 @@ __global__ void __launch_bounds__(32) tri32_cluster_kernel(int N, int64_t batch,
         }
     }
 }
-// E and U (vectors of the tridiagonal forms) from de.
-int tri32(cudaStream_t st, int N, int64_t batch, const float* de, double* E, cc* U, int* status) {
+// E and U (vectors of the tridiagonal forms) from de; heev_threads: the launch shape
+// whose arithmetic is kept.
+int tri32(cudaStream_t st, int N, int64_t batch, const float* de, double* E, cc* U, int* status, int heev_threads) {
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     KTimer kt(st, "tri32_kernel");
-    const int parts = (N + 125) / 126, len = (N + parts - 1) / parts;
+    const int S = 2 * N <= heev_threads ? 2 : 1;  // heev_kernel's for N > 128
+    const int most = 128 / S - 2, parts = (N + most - 1) / most, len = (N + parts - 1) / parts;
     const int64_t ctas = std::min<int64_t>(batch * parts, (int64_t)nsm * 64);
-    tri32_kernel<<<(unsigned)ctas, 128, sizeof(float) * (3 * (size_t)N + len + 2), st>>>(N, batch, parts, len, de, E, U,
-                                                                                         status);
+    tri32_kernel<<<(unsigned)ctas, 128, sizeof(float) * (3 * (size_t)N + len + 2), st>>>(N, batch, parts, len, S, de, E,
+                                                                                         U, status);
     TBG_LAUNCHED("tri32_kernel");
     if (!U) return TBG_OK;
     const int G = (int)std::max<size_t>(1, std::min<size_t>(16, (48 * 1024 / sizeof(float) - 4 * (size_t)N) / (4 * (size_t)N)));
@@ -1551,7 +1570,8 @@ int eig_batched_f32(cudaStream_t st, int N, int64_t batch, zc* H, double* E, cc*
             return hetrd_tc(st, 128, batch, nullptr, nullptr, static_cast<cc*>(work), de, status_d, Tb, N, stop);
         };
         auto tri = [&]() {
-            if (int r = tri32(st, N, batch, de, E, U, status_d)) return r;
+            const int thr = eig_threads<float>(N, tp.r0 == 0 && tp.ctas == 3 ? 3 : 2);
+            if (int r = tri32(st, N, batch, de, E, U, status_d, thr)) return r;
             return U ? launch_bt32(st, N, batch, work, U, tp.PB) : TBG_OK;
         };
         if (tp.r0 > 0) {
