@@ -1,7 +1,7 @@
 // Fused path for small models (nsta <= 8): one thread per k-point runs the
 // whole of berry_curvature_at_impl (src/response/traits.rs:160-200) in
 // registers / local memory, FP64:
-//   H, V_0, V_1 by the Fourier sum over R with the Atom gauge and tau term
+//   H, V_0, V_1 by the Fourier sum over R with the tau term (lattice gauge)
 //   (src/velocity.rs:538-622), optional spin dressing (traits.rs:170-175),
 //   eigenpairs by cyclic complex Jacobi, U^H V U, Omega_n (and optionally
 //   the quantum metric, src/quantum_geometry.rs:160-187), and the
@@ -29,12 +29,14 @@ __device__ __forceinline__ double fermi_s(double e, double mu, double width) {
 }
 
 // The rotation that annihilates a_pq: tan 2 theta = 2 |a_pq| / (a_pp - a_qq), theta
-// in [0, pi / 2].  Square roots of the half-angle formulas, the larger of cosine
-// and sine first (no cancellation); a third of the FP64 instructions of atan2 and
-// sincos.
-__device__ __forceinline__ void jacobi_angle(double mag, double d, double& cs, double& sn) {
-    const double h = sqrt(fma(d, d, 4.0 * mag * mag));
-    const double big = sqrt(0.5 * (1.0 + fabs(d) / h)), little = mag / (h * big);
+// in [0, pi / 2], and a_pq / |a_pq|.  Half-angle formulas over reciprocal square
+// roots, the larger of cosine and sine first (no cancellation): a fraction of the
+// FP64 instructions of sqrt, division, atan2 and sincos.
+__device__ __forceinline__ void jacobi_rotation(zc apq, double m2, double d, zc& ph, double& cs, double& sn) {
+    const double rm = rsqrt(m2), mag = m2 * rm;
+    ph = mk(apq.re * rm, apq.im * rm);
+    const double rh = rsqrt(fma(d, d, 4.0 * m2)), q = fma(0.5 * fabs(d), rh, 0.5);
+    const double rb = rsqrt(q), big = q * rb, little = mag * rh * rb;
     cs = d >= 0.0 ? big : little;
     sn = d >= 0.0 ? little : big;
 }
@@ -67,13 +69,12 @@ __device__ __forceinline__ void jacobi(int N, zc (&A)[NM][NM], zc (&W)[NM][NM]) 
 #pragma unroll
             for (int q = p + 1; q < N; ++q) {
                 const zc apq = A[p][q];
-                const double mag = sqrt(abs2(apq));
-                if (mag == 0.0) continue;
-                const double rm = 1.0 / mag;
-                const zc ph = mk(apq.re * rm, apq.im * rm);
-                const zc emi = conj(ph);
+                const double m2 = abs2(apq);
+                if (m2 == 0.0) continue;
+                zc ph;
                 double sn, cs;
-                jacobi_angle(mag, A[p][p].re - A[q][q].re, cs, sn);
+                jacobi_rotation(apq, m2, A[p][p].re - A[q][q].re, ph, cs, sn);
+                const zc emi = conj(ph);
 #pragma unroll
                 for (int k = 0; k < N; ++k) {
                     const zc akp = A[k][p], akq = emi * A[k][q];
@@ -154,22 +155,21 @@ __global__ void mesh_phase_kernel(int64_t n0, int64_t n1, int64_t n2, zc* __rest
 // phase of R comes from the e^{2 pi i k_d} by R_d-fold products, one sincospi per
 // axis and k-point (none with ztab, the mesh's table) instead of one sincos per R,
 // and energies of two bands from the quadratic formula: 10^6 k-points of the
-// honeycomb model 0.92 -> 0.185 ms, 961 of the Haldane model's curvature 62 -> 45 us.
+// honeycomb model 0.92 -> 0.185 ms, 961 of the Haldane model's curvature 62 -> 35 us.
 template <int NM, bool VALS, bool EXACT>
 __global__ void __launch_bounds__(64) small_fused_kernel(
     int Nrt, int norb, int dim, int nR, int64_t nk, const double* __restrict__ klist, int64_t k0, int64_t n0,
     int64_t n1, int64_t n2, const zc* __restrict__ ztab, const zc* __restrict__ ham, const int* __restrict__ hamR,
-    const double* __restrict__ Rcart, const double* __restrict__ tau, const double* __restrict__ taucart,
-    const double* __restrict__ dirs, int spin, double eta, int nmu, const double* __restrict__ mu, double width,
-    double* __restrict__ Om_out, double* __restrict__ E_out, double* __restrict__ S_out, double* __restrict__ Met_out,
-    double* __restrict__ SM_out) {
+    const double* __restrict__ Rcart, const double* __restrict__ taucart, const double* __restrict__ dirs, int spin,
+    double eta, int nmu, const double* __restrict__ mu, double width, double* __restrict__ Om_out,
+    double* __restrict__ E_out, double* __restrict__ S_out, double* __restrict__ Met_out, double* __restrict__ SM_out) {
     const int N = EXACT ? NM : Nrt;
     // the model in shared memory, all of it requested at once
     extern __shared__ __align__(16) unsigned char small_smem[];
     zc* s_ham = reinterpret_cast<zc*>(small_smem);                      // (nR, N, N)
     double* s_c = reinterpret_cast<double*>(s_ham + (int64_t)nR * N * N);  // (nR, 2) w . R
-    double* s_tau = s_c + 2 * nR;                                       // (N, 5): tau, w . tau
-    int* s_R = reinterpret_cast<int*>(s_tau + 5 * N);                   // (nR, 3)
+    double* s_tau = s_c + 2 * nR;                                       // (N, 2) w . tau
+    int* s_R = reinterpret_cast<int*>(s_tau + 2 * N);                   // (nR, 3)
     for (int i = threadIdx.x; i < nR * N * N; i += blockDim.x) s_ham[i] = ham[i];
     for (int i = threadIdx.x; i < 3 * nR; i += blockDim.x) s_R[i] = hamR[i];
     if (!VALS) {
@@ -181,10 +181,7 @@ __global__ void __launch_bounds__(64) small_fused_kernel(
             return c;
         };
         for (int i = threadIdx.x; i < 2 * nR; i += blockDim.x) s_c[i] = along(i & 1, Rcart + 3 * (i >> 1));
-        for (int i = threadIdx.x; i < 5 * N; i += blockDim.x) {
-            const int a = i / 5, d = i % 5;
-            s_tau[i] = d < 3 ? tau[3 * a + d] : along(d - 3, taucart + 3 * a);
-        }
+        for (int i = threadIdx.x; i < 2 * N; i += blockDim.x) s_tau[i] = along(i & 1, taucart + 3 * (i >> 1));
     }
     __syncthreads();
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -281,31 +278,17 @@ __global__ void __launch_bounds__(64) small_fused_kernel(
         for (int i = 0; i < N; ++i) E_out[t * N + i] = E[i];
         return;
     }
-    // Atom gauge + tau term
-    zc ph[NM];
-    double tp0[NM], tp1[NM];
-#pragma unroll
-    for (int s = 0; s < N; ++s) {
-        const double* ts = s_tau + 5 * s;
-        double a = ts[0] * kv[0];
-        if (dim > 1) a += ts[1] * kv[1];
-        if (dim > 2) a += ts[2] * kv[2];
-        double sn, cs;
-        sincospi(2.0 * a, &sn, &cs);
-        ph[s] = mk(cs, sn);
-        tp0[s] = ts[3];
-        tp1[s] = ts[4];
-    }
+    // tau term.  The Atom gauge's phases conj(phi_m) phi_n are a diagonal unitary
+    // similarity of H and the velocities (one phase per orbital, both spins): E, Omega
+    // and the metric are the same without them.
 #pragma unroll
     for (int m = 0; m < N; ++m)
 #pragma unroll
         for (int n = 0; n < N; ++n) {
-            const zc g = cmul(ph[m], ph[n]);
             const zc hl = H[m][n];
-            const double d0 = tp0[n] - tp0[m], d1 = tp1[n] - tp1[m];
-            V0[m][n] = (V0[m][n] + mk(-d0 * hl.im, d0 * hl.re)) * g;
-            V1[m][n] = (V1[m][n] + mk(-d1 * hl.im, d1 * hl.re)) * g;
-            H[m][n] = hl * g;
+            const double d0 = s_tau[2 * n] - s_tau[2 * m], d1 = s_tau[2 * n + 1] - s_tau[2 * m + 1];
+            V0[m][n] = V0[m][n] + mk(-d0 * hl.im, d0 * hl.re);
+            V1[m][n] = V1[m][n] + mk(-d1 * hl.im, d1 * hl.re);
         }
     if (spin >= 0) {  // J = 1/2 (S V0 + V0 S), S = sigma (x) I / 2
         zc J[NM][NM];
@@ -485,17 +468,17 @@ int small_fused(const ModelDev& m, cudaStream_t st, int64_t nk, const double* kl
     // one warp per block while that spreads a small mesh over more SMs
     const int thr = nk <= 152 * 64 ? 32 : 64;
     const unsigned blocks = (unsigned)((nk + thr - 1) / thr);
-    const size_t smem = sizeof(zc) * m.nR * N * N + sizeof(double) * (2 * m.nR + 5 * N) + sizeof(int) * 3 * m.nR;
+    const size_t smem = sizeof(zc) * m.nR * N * N + sizeof(double) * (2 * m.nR + 2 * N) + sizeof(int) * 3 * m.nR;
 #define SMALL_LAUNCH(NM, EX)                                                                                         \
     do {                                                                                                             \
         if (vals)                                                                                                    \
             small_fused_kernel<NM, true, EX><<<blocks, thr, smem, st>>>(                                             \
                 N, (int)m.norb, m.dim, (int)m.nR, nk, klist_d, k0, n0, n1, n2, ztab, m.ham, m.hamR_d, m.Rcart_d,    \
-                m.tau_d, m.taucart_d, dirs_d, spin, eta, nmu, mu_d, width, Om, E, S, Met, SM);                      \
+                m.taucart_d, dirs_d, spin, eta, nmu, mu_d, width, Om, E, S, Met, SM);                      \
         else                                                                                                         \
             small_fused_kernel<NM, false, EX><<<blocks, thr, smem, st>>>(                                            \
                 N, (int)m.norb, m.dim, (int)m.nR, nk, klist_d, k0, n0, n1, n2, ztab, m.ham, m.hamR_d, m.Rcart_d,    \
-                m.tau_d, m.taucart_d, dirs_d, spin, eta, nmu, mu_d, width, Om, E, S, Met, SM);                      \
+                m.taucart_d, dirs_d, spin, eta, nmu, mu_d, width, Om, E, S, Met, SM);                      \
     } while (0)
     if (N == 2)
         SMALL_LAUNCH(2, true);
