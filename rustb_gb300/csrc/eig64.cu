@@ -32,9 +32,10 @@
 // diagonal, A(j, j) = (d_j, e_j), A(j + 1, j) = tau_j, and the cluster marks
 // sit in A(N - 1, 0 ..).  Nothing is allocated.
 //
-// Eigenpairs of 1024 matrices of 128 bands 82.9 -> 34.7 ms (reduction 14.5,
-// tridiagonal 2.7, back-transformation 17.5; the last two stages at 0.8 to 1.0
-// of the 1.06 TFLOP/s that the FP64 pipe does), 4032 of 64 bands 77 -> 18.7,
+// Eigenpairs of 1024 matrices of 128 bands 82.9 -> 20.7 ms (reduction 13.7,
+// tridiagonal 2.6, back-transformation 17.5 by single reflectors and 4.3 in
+// blocks on the tensor cores; the first two at 0.8 to 1.0 of the 1.06 TFLOP/s
+// that the FP64 pipe does), 4032 of 64 bands 77 -> 14.7,
 // 2304 of 26 bands 7.5 -> 1.14, against one kernel with FP64 bisection, the
 // matrix in L2 and reflectors applied by eight lanes per column.
 
@@ -189,9 +190,12 @@ __global__ void __launch_bounds__(32 * kWarpsPerCta) hetrd64_warp_kernel(int N, 
 // from the block's, so that the serial FP64 work of the blocks on an SM falls
 // on different sub-partitions) while the others update the rest of A22.
 __host__ __device__ inline size_t cta_smem_bytes(int N, int nthr) {
-    return sizeof(zc) * ((size_t)N * (N + 1) / 2 + 3 * (size_t)N + nthr) + 4 * sizeof(double);
+    return sizeof(zc) * ((size_t)N * (N + 1) / 2 + 3 * (size_t)N + nthr) + (4 + nthr / 32) * sizeof(double);
 }
 
+// Threads from which u is summed by all warps: equal times at 256 (70 - 112 bands),
+// 4 % slower at 128 (33 bands 0.69 -> 0.72 ms), where several CTAs share the SM.
+constexpr int kWideU = 512;
 template <int NT>
 __global__ void __launch_bounds__(NT) hetrd64_cta_kernel(int N, int64_t batch, zc* __restrict__ Ain) {
     extern __shared__ __align__(16) unsigned char smem64[];
@@ -200,6 +204,7 @@ __global__ void __launch_bounds__(NT) hetrd64_cta_kernel(int N, int64_t batch, z
     zc* su = svb + 2 * N;
     zc* part = su + N;
     double* sc = reinterpret_cast<double*>(part + NT);  // tau of even and odd steps
+    double* s_vav = sc + 4;                              // partial v^H A v per warp
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NW = NT / 32;
     for (int64_t b = blockIdx.x; b < batch; b += gridDim.x) {
@@ -237,23 +242,51 @@ __global__ void __launch_bounds__(NT) hetrd64_cta_kernel(int N, int64_t batch, z
                 part[t] = row_times(T22, m, i, q, Q, sv);
             }
             __syncthreads();
-            if (warp == lead) {
+            if constexpr (NT >= kWideU) {
+                // one CTA on the SM: u with one row per thread, as a lone warp would have a
+                // quarter of the FP64 rate (1024 x 128 bands 14.5 -> 13.7 ms)
                 const zc tau = mk(sc[2 * (j & 1)], sc[2 * (j & 1) + 1]);
-                double s = 0.0;
-                for (int i = lane; i < m; i += 32) {
-                    zc acc = part[i];
-                    for (int q = 1; q < Q; ++q) acc = acc + part[q * m + i];
-                    s = fma(sv[i].re, acc.re, fma(sv[i].im, acc.im, s));
-                    su[i] = tau * acc;
+                zc u = mk(0.0, 0.0), v = mk(0.0, 0.0);
+                if (warp * 32 < m) {
+                    double s = 0.0;
+                    if (tid < m) {
+                        zc acc = part[tid];
+                        for (int q = 1; q < Q; ++q) acc = acc + part[q * m + tid];
+                        v = sv[tid];
+                        s = fma(v.re, acc.re, v.im * acc.im);
+                        u = tau * acc;
+                    }
+                    s = wsum(s);
+                    if (lane == 0) s_vav[warp] = s;
                 }
-                s = wsum(s);
-                const double a2 = -0.5 * fma(tau.re, tau.re, tau.im * tau.im) * s;
-                for (int i = lane; i < m; i += 32) {
-                    const zc w = su[i];
-                    su[i] = mk(fma(a2, sv[i].re, w.re), fma(a2, sv[i].im, w.im));
+                __syncthreads();
+                if (tid < m) {
+                    double s = s_vav[0];  // v^H A v (real)
+                    for (int w = 1; w < (m + 31) / 32; ++w) s += s_vav[w];
+                    const double a2 = -0.5 * fma(tau.re, tau.re, tau.im * tau.im) * s;
+                    su[tid] = mk(fma(a2, v.re, u.re), fma(a2, v.im, u.im));
                 }
+                __syncthreads();
+            } else {
+                // the other CTAs of the SM fill the gap: one warp, one barrier less
+                if (warp == lead) {
+                    const zc tau = mk(sc[2 * (j & 1)], sc[2 * (j & 1) + 1]);
+                    double s = 0.0;
+                    for (int i = lane; i < m; i += 32) {
+                        zc acc = part[i];
+                        for (int q = 1; q < Q; ++q) acc = acc + part[q * m + i];
+                        s = fma(sv[i].re, acc.re, fma(sv[i].im, acc.im, s));
+                        su[i] = tau * acc;
+                    }
+                    s = wsum(s);
+                    const double a2 = -0.5 * fma(tau.re, tau.re, tau.im * tau.im) * s;
+                    for (int i = lane; i < m; i += 32) {
+                        const zc w = su[i];
+                        su[i] = mk(fma(a2, sv[i].re, w.re), fma(a2, sv[i].im, w.im));
+                    }
+                }
+                __syncthreads();
             }
-            __syncthreads();
             if (warp == lead) {
                 for (int l = lane; l < m; l += 32) rank2_elem(T22 + l, sv, su, 0, l);
                 __syncwarp();
