@@ -11,9 +11,10 @@
 //
 // CTA = 13 warps, one output tile of 128 rows x 64 complex columns:
 //   warps 0..7   A digit producers: thread = (row, 8 consecutive k); load the
-//                8 elements of the next stage into registers while converting
-//                the current one, write each digit plane as one 16-byte store
-//                (K-major core matrices of 8 rows x 16 bytes, no swizzle);
+//                8 elements of the next stage into registers (or, where A's rows
+//                are contiguous, copy the warp's rows to shared memory) while
+//                converting the current one, write each digit plane as one 16-byte
+//                store (K-major core matrices of 8 rows x 16 bytes, no swizzle);
 //   warps 8..11  B digit producers, same per (column, 8 consecutive k), or,
 //                for a pre-sliced operand, one thread that copies the stage
 //                image with cp.async.bulk (completion on an mbarrier);
@@ -55,8 +56,8 @@ template <> struct Class<6> { static constexpr int LMAX = 5, NLEV = 4, MIN_CTAS 
 //   MID : S = 5, LMAX = 4, NLEV = 4  (about 2^-35; the rotation into the eigenbasis)
 template <> struct Class<5> { static constexpr int LMAX = 4, NLEV = 4, MIN_CTAS = 1; };
 template <> struct Class<3> { static constexpr int LMAX = 2, NLEV = 1, MIN_CTAS = 2; };
-constexpr int tc_smem_bytes(int S) { return 2 * 2 * S * PLANE + 1024; }  // two stages of A and B planes + slack
-constexpr int TC_SMEM = tc_smem_bytes(TC_S);
+// two stages of A and B planes, the A elements of the next stage (raw_bytes) and slack
+constexpr int tc_smem_bytes(int S, int raw) { return 2 * 2 * S * PLANE + raw + 128; }
 // whether a class's two stage buffers can hold the 128 x 65 float-pair output tile
 constexpr bool tc_staged(int S) { return 2 * 2 * S * PLANE >= 128 * 65 * 16; }
 constexpr int TC_THREADS = 416;                 // 13 warps
@@ -72,6 +73,12 @@ enum { FMT_F64 = 0, FMT_F32 = 1, FMT_PAIR = 2, FMT_PRESLICED = 3 };
 
 // instruction descriptor, kind::f16: D = F32, A = B = BF16, K-major, N = 128, M = 128
 constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+
+// Bytes of one stage's A elements as they lie in memory (128 rows of 16), kept
+// where the rows of A are its lines; 0 where the producers load them directly.
+constexpr int raw_bytes(bool conj_a, int fmt_a) {
+    return conj_a || fmt_a == FMT_PRESLICED ? 0 : TC_TM * TC_TK * (fmt_a == FMT_F32 ? 8 : 16);
+}
 
 using namespace tc;
 
@@ -232,6 +239,56 @@ __device__ __forceinline__ void load8(const void* base, int64_t idx0, int64_t st
 #pragma unroll
     for (int i = 0; i < 8; ++i) r[i] = (i < nvalid) ? ld_elem<FMT>(base, idx0 + (int64_t)i * stride) : make_int4(0, 0, 0, 0);
 }
+// One warp's part of a stage of A whose rows are contiguous: 16 rows x 16 k as
+// 32 half rows of 8 elements, half row h = 2 row + g.  A thread slices one half
+// row, but 32 threads reading 32 half rows element by element touch 32 lines
+// per load (L1 then bounds the products: 2.33 ms per 8192 x 128^3 against 1.90
+// with A's columns as lines).  So the warp copies whole rows with cp.async,
+// and each thread reads its half row back; 16-byte units are permuted within a
+// half row so that neither direction has bank conflicts.
+template <int FMT>
+__device__ __forceinline__ void raw_copy(uint32_t raw, const void* base, int64_t row0, int64_t ld, int nrows, int kf,
+                                         int K, int lane) {
+    constexpr int EB = FMT == FMT_F32 ? 8 : 16;
+    const int e = lane & 7;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int h = 4 * i + (lane >> 3), rl = h >> 1, k = kf + 8 * (h & 1) + e;
+        const bool ok = rl < nrows && k < K;
+        const char* src = static_cast<const char*>(base) + (ok ? row0 + (int64_t)rl * ld + k : 0) * EB;
+        if constexpr (FMT == FMT_F32) {
+            const uint32_t dst = raw + 64 * h + ((((e >> 1) ^ ((h >> 1) & 3)) << 4) | ((e & 1) << 3));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(ok ? 8 : 0) : "memory");
+        } else {
+            const uint32_t dst = raw + 128 * h + ((e ^ (h & 7)) << 4);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0)
+                         : "memory");
+        }
+    }
+}
+// The lane's half row, after the warp's copies have landed.
+template <int FMT>
+__device__ __forceinline__ void raw_read(uint32_t raw, int lane, int4 (&r)[8]) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < (FMT == FMT_F32 ? 4 : 8); ++i) {
+        int4 v;
+        const uint32_t src = FMT == FMT_F32 ? raw + 64 * lane + ((i ^ ((lane >> 1) & 3)) << 4)
+                                            : raw + 128 * lane + ((i ^ (lane & 7)) << 4);
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                     : "r"(src)
+                     : "memory");
+        if constexpr (FMT == FMT_F32) {
+            r[2 * i] = make_int4(v.x, v.y, 0, 0);
+            r[2 * i + 1] = make_int4(v.z, v.w, 0, 0);
+        } else {
+            r[i] = v;
+        }
+    }
+    __syncwarp();  // before the next copies overwrite the buffer
+}
 // Digits of the real (part 0) or imaginary (part 1) component of one element.
 template <int FMT, int PART>
 __device__ __forceinline__ void elem_digits(const int4& r, int E, float s1, float s2, float* P) {
@@ -348,15 +405,16 @@ __global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
     constexpr int HS = S * PLANE;             // planes of one operand in a stage
     constexpr int SB = 2 * HS;                // stage bytes
     constexpr uint32_t TMEM_COLS = NLEV * 128;
-    extern __shared__ __align__(1024) unsigned char tc_smem[];
-    unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)tc_smem + 1023) & ~(uintptr_t)1023);
+    extern __shared__ __align__(128) unsigned char tc_smem[];
+    unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)tc_smem + 127) & ~(uintptr_t)127);
     __shared__ __align__(8) uint64_t bar_full[2], bar_bcopy[2], bar_empty[2], bar_done, bar_tmem, bar_stage;
     __shared__ uint32_t tmem_base_sh;
     __shared__ volatile int abort_sh;
-    __shared__ int emax[2][4][TC_TN];  // column maxima of a tile (float bits) by lane quarter
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nstages = (K + TC_TK - 1) / TC_TK;
     const uint32_t sbase = su32(base);
+    constexpr bool RAW = raw_bytes(CONJ_A, FMTA) > 0;  // A's rows come through the raw buffer
+    const uint32_t raw = sbase + 2 * SB + (warp & 7) * (raw_bytes(CONJ_A, FMTA) / 8);
     // With room in the stage buffers the 128 x 64 output tile is staged there
     // (rows padded to 65 entries: no bank conflicts either way).
     constexpr int TROW = TC_TN + 1;
@@ -464,8 +522,16 @@ __global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
             rv = gi < M;
             return CONJ_A ? (t.b * sA + gi) : (t.b * sA + (int64_t)gi * lda);
         };
+        // the warp's rows of a stage of tile L, on their way to its raw buffer
+        auto copy_rows = [&](int64_t L, int kf) {
+            const TileId t = tile_of(L, gx, gy, rows_fast);
+            const int g0 = t.rt * TC_TM + 16 * warp;
+            raw_copy<FMTA>(raw, A, t.b * sA + (int64_t)g0 * lda, lda, M - g0, kf, K, lane);
+        };
         int4 nxt[8];
-        if constexpr (!PRE_A) {
+        if constexpr (RAW) {
+            if (blockIdx.x < ntiles) copy_rows(blockIdx.x, 0);
+        } else if constexpr (!PRE_A) {
             bool rv0;
             const int64_t i0 = row_base(blockIdx.x, rv0);
             if (blockIdx.x < ntiles)
@@ -485,27 +551,36 @@ __global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
                 const int64_t gs = (int64_t)tn * nstages + it;
                 const int bi = (int)(gs & 1);
                 int4 cur[8];
+                // the next stage (of the next tile: in flight during this tile's epilogue)
+                const bool last = it + 1 == nstages;
+                if constexpr (RAW) {
+                    raw_read<FMTA>(raw, lane, cur);
+                    if (!last)
+                        copy_rows(L, (it + 1) * TC_TK);
+                    else if (L + gridDim.x < ntiles)
+                        copy_rows(L + gridDim.x, 0);
+                } else {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) cur[i] = nxt[i];
-                if (it + 1 < nstages) {
-                    const int kf = (it + 1) * TC_TK + 8 * g;
-                    load8<FMTA>(A, idx0 + (int64_t)kf * kstride, kstride, rv ? n_valid(K, kf) : 0, nxt);
-                } else if (L + gridDim.x < ntiles) {
-                    // the next tile's first stage, in flight during this tile's epilogue
-                    bool rvn;
-                    const int64_t in = row_base(L + gridDim.x, rvn);
-                    load8<FMTA>(A, in + (int64_t)(8 * g) * kstride, kstride, rvn ? n_valid(K, 8 * g) : 0, nxt);
+                    for (int i = 0; i < 8; ++i) cur[i] = nxt[i];
+                    if (!last) {
+                        const int kf = (it + 1) * TC_TK + 8 * g;
+                        load8<FMTA>(A, idx0 + (int64_t)kf * kstride, kstride, rv ? n_valid(K, kf) : 0, nxt);
+                    } else if (L + gridDim.x < ntiles) {
+                        bool rvn;
+                        const int64_t in = row_base(L + gridDim.x, rvn);
+                        load8<FMTA>(A, in + (int64_t)(8 * g) * kstride, kstride, rvn ? n_valid(K, 8 * g) : 0, nxt);
+                    }
                 }
                 // slice this stage while the MMAs of the two stages before it run; then
                 // wait only for the buffer and store
                 uint4 dre[S], dim[S];
                 item_planes<FMTA, 0, S>(cur, E, s1, s2, dre);
                 item_planes<FMTA, 1, S>(cur, E, s1, s2, dim);
-                if (gs >= 2 && !mbar_wait(&bar_empty[bi], (uint32_t)(((gs >> 1) - 1) & 1), &abort_sh, wait_limit)) {
-                    abort_sh = 1;
-                    break;
-                }
-                if (abort_sh) break;
+                bool quit = gs >= 2 && !mbar_wait(&bar_empty[bi], (uint32_t)(((gs >> 1) - 1) & 1), &abort_sh, wait_limit);
+                if (quit) abort_sh = 1;
+                quit = quit || abort_sh;
+                if (RAW) quit = __any_sync(0xffffffffu, quit);  // raw_read takes whole warps
+                if (quit) break;
                 const uint32_t sa = sbase + bi * SB;
 #pragma unroll
                 for (int s = 0; s < S; ++s) st_shared_v4(sa + s * PLANE + o_re, dre[s]);
@@ -528,7 +603,6 @@ __global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
             tc_fence_after();
             const int re_ = row0 + 32 * q + lane;
             const int ea = (re_ < M) ? EA[t.b * M + re_] : ZERO_EXP;
-            const int par = tn & 1;
             for (int cc = 0; cc < 4; ++cc) {
                 const int c0 = 32 * h + 8 * cc;
                 uint32_t v[2 * NLEV][8];  // [2 * level + (0 re, 1 im)][column]
@@ -588,14 +662,6 @@ __global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
                         }
                         *cp = out;
                     }
-                    if (Ecol) {
-                        // the column's largest magnitude over this warp's rows (>= 0,
-                        // NaN as 0: ordered as integers)
-                        float mg = in ? pair_mag(out) : 0.f;
-                        mg = (mg == mg) ? mg : 0.f;
-                        const int mv = __reduce_max_sync(0xffffffffu, __float_as_int(mg));
-                        if (lane == 0) emax[par][q][c0 + c] = mv;
-                    }
                 }
             }
             if (STAGE) {
@@ -632,15 +698,9 @@ __global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
                 }
                 asm volatile("bar.sync 1, 256;" ::: "memory");  // every read of the staged tile done
                 if (tid == 0) mbar_arrive(&bar_stage);
-            } else if (Ecol) {
-                // one row tile holds every row: the tile's column maxima are the columns'
-                asm volatile("bar.sync 1, 256;" ::: "memory");
-                if (tid < TC_TN && col0 + tid < Nc) {
-                    const int mx = max(max(emax[par][0][tid], emax[par][1][tid]), max(emax[par][2][tid], emax[par][3][tid]));
-                    Ecol[t.b * Nc + col0 + tid] = line_exp_of(__int_as_float(mx));
-                }
             }
         }
+        if (RAW) asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (tid < A_PRODUCERS + B_PRODUCERS) {
         const int qb = tid - A_PRODUCERS;
         if (PRE) {
@@ -881,7 +941,7 @@ static int launch_tc(cudaStream_t st, int64_t batch, int M, int Nc, int K, const
                      const void* B, int64_t ldb, int64_t sB, float4* C, int64_t ldc, int64_t sC, int* EA, int* EB,
                      int* err, const char* name, double work, int accumulate = 0, int* Ecol = nullptr) {
     auto kern = oz_tc_kernel<CJ, FA, FB, S>;
-    constexpr int smem = tc_smem_bytes(S);
+    constexpr int smem = tc_smem_bytes(S, raw_bytes(CJ, FA));
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(oz_tc)");
     KTimer kt(st, name, work);
@@ -1072,7 +1132,7 @@ static int fourier_tc_launch(cudaStream_t st, int64_t M, int64_t Nc, int K, cons
         TBG_LAUNCHED("phase_image_kernel");
     }
     auto kern = oz_tc_kernel<false, FMT_PRESLICED, FMT_PRESLICED, S>;
-    const int smem = tc_smem_bytes(S);
+    const int smem = tc_smem_bytes(S, 0);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(oz_tc fourier)");
     KTimer kt(st, S == TC_S ? "ozaki_tc_fourier_kernel" : "ozaki_tc_fourier_kernel<mid>", 8.0 * (double)M * Nc * K);
