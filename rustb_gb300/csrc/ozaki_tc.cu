@@ -9,15 +9,15 @@
 // FP32, M = 128, N = 128, K = 16) from shared-memory descriptors; the four
 // accumulation levels are 4 x 128 FP32 columns of tensor memory.
 //
-// CTA = 13 warps, one output tile of 128 rows x 64 complex columns:
-//   warps 0..7   A digit producers: thread = (row, 8 consecutive k); load the
-//                8 elements of the next stage into registers (or, where A's rows
-//                are contiguous, copy the warp's rows to shared memory) while
-//                converting the current one, write each digit plane as one 16-byte
-//                store (K-major core matrices of 8 rows x 16 bytes, no swizzle);
-//   warps 8..11  B digit producers, same per (column, 8 consecutive k), or,
-//                for a pre-sliced operand, one thread that copies the stage
-//                image with cp.async.bulk (completion on an mbarrier);
+// CTA = 13 working warps, an output tile of 128 rows x 64 complex columns at a time:
+//   warps 0..7   A digit producers: thread = (row, 8 consecutive k); cp.async
+//                brings the elements of the next stage to shared memory while the
+//                current one is converted; each digit plane is one 16-byte store
+//                (K-major core matrices of 8 rows x 16 bytes, no swizzle);
+//   warps 8..11  B digit producers, same per (column, 8 consecutive k) with the
+//                next elements in registers, or, for a pre-sliced operand, one
+//                thread that copies the stage image with cp.async.bulk
+//                (completion on an mbarrier);
 //   warp 12      allocates TMEM; lane 0 issues the MMAs and commits them;
 //   warps 0..7   after the K loop: read the four levels from TMEM (tcgen05.ld
 //                32x32b, one TMEM lane = one output row), combine them with
@@ -56,11 +56,12 @@ template <> struct Class<6> { static constexpr int LMAX = 5, NLEV = 4, MIN_CTAS 
 //   MID : S = 5, LMAX = 4, NLEV = 4  (about 2^-35; the rotation into the eigenbasis)
 template <> struct Class<5> { static constexpr int LMAX = 4, NLEV = 4, MIN_CTAS = 1; };
 template <> struct Class<3> { static constexpr int LMAX = 2, NLEV = 1, MIN_CTAS = 2; };
-// two stages of A and B planes, the A elements of the next stage (raw_bytes) and slack
-constexpr int tc_smem_bytes(int S, int raw) { return 2 * 2 * S * PLANE + raw + 128; }
-// whether a class's two stage buffers can hold the 128 x 65 float-pair output tile
-constexpr bool tc_staged(int S) { return 2 * 2 * S * PLANE >= 128 * 65 * 16; }
-constexpr int TC_THREADS = 416;                 // 13 warps
+// 13 warps; 16 where the producers take registers over from the last warpgroup
+// (its four warps must release together): 13 warps already cost as many, 128 a
+// thread, since one scheduler holds four of them.
+constexpr bool tc_split(int S) { return S > 3; }
+constexpr int tc_threads(int S) { return tc_split(S) ? 512 : 416; }
+constexpr int PRODUCER_REGS = 160, MMA_REGS = 32;  // 3 x 160 + 32 = 4 x 128
 constexpr int MMA_WARP = 12;
 constexpr int A_PRODUCERS = 256;
 constexpr int B_PRODUCERS = 128;
@@ -74,10 +75,24 @@ enum { FMT_F64 = 0, FMT_F32 = 1, FMT_PAIR = 2, FMT_PRESLICED = 3 };
 // instruction descriptor, kind::f16: D = F32, A = B = BF16, K-major, N = 128, M = 128
 constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 
-// Bytes of one stage's A elements as they lie in memory (128 rows of 16), kept
-// where the rows of A are its lines; 0 where the producers load them directly.
-constexpr int raw_bytes(bool conj_a, int fmt_a) {
-    return conj_a || fmt_a == FMT_PRESLICED ? 0 : TC_TM * TC_TK * (fmt_a == FMT_F32 ? 8 : 16);
+// Bytes of one stage's A elements as they lie in memory (128 rows of 16).
+constexpr int raw_bytes(int fmt_a) {
+    return fmt_a == FMT_PRESLICED ? 0 : TC_TM * TC_TK * (fmt_a == FMT_F32 ? 8 : 16);
+}
+
+// Epilogue: each of the eight warps passes its outputs, 32 rows x 4 columns of
+// float pairs at a time, through 2 KB of shared memory on the way to whole
+// sectors of C; its own where they fit beside the stage buffers (own_out), else
+// its part of the raw buffer, which then idles meanwhile.
+constexpr int OUT_BYTES = 8 * 2048;
+template <int S>
+constexpr bool own_out(int fmt_a) {
+    return Class<S>::MIN_CTAS == 1 && 4 * S * PLANE + raw_bytes(fmt_a) + OUT_BYTES <= 230000;
+}
+// two stages of A and B planes, the A elements of the next stage, the outputs and slack
+template <int S>
+constexpr int tc_smem_bytes(int fmt_a) {
+    return 4 * S * PLANE + raw_bytes(fmt_a) + (own_out<S>(fmt_a) ? OUT_BYTES : 0) + 128;
 }
 
 using namespace tc;
@@ -239,55 +254,81 @@ __device__ __forceinline__ void load8(const void* base, int64_t idx0, int64_t st
 #pragma unroll
     for (int i = 0; i < 8; ++i) r[i] = (i < nvalid) ? ld_elem<FMT>(base, idx0 + (int64_t)i * stride) : make_int4(0, 0, 0, 0);
 }
-// One warp's part of a stage of A whose rows are contiguous: 16 rows x 16 k as
-// 32 half rows of 8 elements, half row h = 2 row + g.  A thread slices one half
-// row, but 32 threads reading 32 half rows element by element touch 32 lines
-// per load (L1 then bounds the products: 2.33 ms per 8192 x 128^3 against 1.90
-// with A's columns as lines).  So the warp copies whole rows with cp.async,
-// and each thread reads its half row back; 16-byte units are permuted within a
-// half row so that neither direction has bank conflicts.
+// One warp's part of a stage of A on its way to the warp's raw buffer (cp.async):
+// the producers' registers hold the digits of the stage before it instead.
+//
+// Rows of A contiguous (16 rows x 16 k): 32 half rows of 8 elements, half row
+// h = 2 row + g.  A thread slices one half row, but 32 threads loading 32 half
+// rows element by element touch 32 lines per load (L1 then bounds the products:
+// 2.33 ms per 8192 x 128^3 against 1.90 with A's columns as lines).  So the warp
+// copies whole rows, and each thread reads its half row back; 16-byte units are
+// permuted within a half row so that neither direction has bank conflicts.
+//
+// Columns of A contiguous (conjugated; 32 rows x 8 k): every thread copies and
+// reads back its own row's elements, 32 neighbouring rows per k.
 template <int FMT>
-__device__ __forceinline__ void raw_copy(uint32_t raw, const void* base, int64_t row0, int64_t ld, int nrows, int kf,
+__device__ __forceinline__ void raw_put(uint32_t dst, const void* base, int64_t idx, bool ok) {
+    constexpr int EB = FMT == FMT_F32 ? 8 : 16;
+    const char* src = static_cast<const char*>(base) + (ok ? idx : 0) * EB;
+    if constexpr (FMT == FMT_F32)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(ok ? 8 : 0) : "memory");
+    else
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+template <bool COLS, int FMT>
+__device__ __forceinline__ void raw_copy(uint32_t raw, const void* base, int64_t first, int64_t ld, int nrows, int kf,
                                          int K, int lane) {
+    // first: element of the warp's first row at k = 0; kf: first k of the stage
+    // (of the warp's eight, COLS)
     constexpr int EB = FMT == FMT_F32 ? 8 : 16;
     const int e = lane & 7;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const int h = 4 * i + (lane >> 3), rl = h >> 1, k = kf + 8 * (h & 1) + e;
-        const bool ok = rl < nrows && k < K;
-        const char* src = static_cast<const char*>(base) + (ok ? row0 + (int64_t)rl * ld + k : 0) * EB;
-        if constexpr (FMT == FMT_F32) {
-            const uint32_t dst = raw + 64 * h + ((((e >> 1) ^ ((h >> 1) & 3)) << 4) | ((e & 1) << 3));
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(ok ? 8 : 0) : "memory");
+        if constexpr (COLS) {
+            raw_put<FMT>(raw + (32 * i + lane) * EB, base, first + (int64_t)(kf + i) * ld + lane,
+                         lane < nrows && kf + i < K);
         } else {
-            const uint32_t dst = raw + 128 * h + ((e ^ (h & 7)) << 4);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0)
-                         : "memory");
+            const int h = 4 * i + (lane >> 3), rl = h >> 1, k = kf + 8 * (h & 1) + e;
+            const uint32_t off = FMT == FMT_F32 ? 64 * h + ((((e >> 1) ^ ((h >> 1) & 3)) << 4) | ((e & 1) << 3))
+                                                : 128 * h + ((e ^ (h & 7)) << 4);
+            raw_put<FMT>(raw + off, base, first + (int64_t)rl * ld + k, rl < nrows && k < K);
         }
     }
 }
-// The lane's half row, after the warp's copies have landed.
-template <int FMT>
+// The thread's eight elements, after the warp's copies have landed.
+template <bool COLS, int FMT>
 __device__ __forceinline__ void raw_read(uint32_t raw, int lane, int4 (&r)[8]) {
     asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < (FMT == FMT_F32 ? 4 : 8); ++i) {
+    if constexpr (!COLS) __syncwarp();
+    auto ld16 = [](uint32_t src) {
         int4 v;
-        const uint32_t src = FMT == FMT_F32 ? raw + 64 * lane + ((i ^ ((lane >> 1) & 3)) << 4)
-                                            : raw + 128 * lane + ((i ^ (lane & 7)) << 4);
         asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
                      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                      : "r"(src)
                      : "memory");
-        if constexpr (FMT == FMT_F32) {
+        return v;
+    };
+    if constexpr (FMT == FMT_F32 && COLS) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            r[i] = make_int4(0, 0, 0, 0);
+            asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];"
+                         : "=r"(r[i].x), "=r"(r[i].y)
+                         : "r"(raw + (32 * i + lane) * 8)
+                         : "memory");
+        }
+    } else if constexpr (FMT == FMT_F32) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int4 v = ld16(raw + 64 * lane + ((i ^ ((lane >> 1) & 3)) << 4));
             r[2 * i] = make_int4(v.x, v.y, 0, 0);
             r[2 * i + 1] = make_int4(v.z, v.w, 0, 0);
-        } else {
-            r[i] = v;
         }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r[i] = ld16(COLS ? raw + (32 * i + lane) * 16 : raw + 128 * lane + ((i ^ (lane & 7)) << 4));
     }
-    __syncwarp();  // before the next copies overwrite the buffer
+    if constexpr (!COLS) __syncwarp();  // before the next copies overwrite the buffer
 }
 // Digits of the real (part 0) or imaginary (part 1) component of one element.
 template <int FMT, int PART>
@@ -385,12 +426,11 @@ __device__ __forceinline__ bool epilogue_any(bool v) {
 // Every role keeps the same tile order; a stage's buffer and barrier phase come
 // from the CTA's running stage count gs = (tiles before) * nstages + it.  The
 // epilogue warps (the A producers) drain the tile's accumulators from TMEM
-// (bar_tmem frees them for the next tile's MMAs), stage the tile of float
-// pairs in the idle stage buffers and write it out row by row, coalesced;
-// bar_stage then hands the buffers to the next tile's B stages.  The next
-// tile's first A and B stages are loaded into registers before the drain.
+// (bar_tmem frees them for the next tile's MMAs) and write them out a few columns
+// at a time; the stage buffers stay free for the next tile's B stages and images,
+// and its first A elements are on their way.
 template <bool CONJ_A, int FMTA, int FMTB, int S>
-__global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
+__global__ void __launch_bounds__(tc_threads(S), Class<S>::MIN_CTAS)
     oz_tc_kernel(int M, int Nc, int K, const void* __restrict__ A, int64_t lda, int64_t sA, const void* __restrict__ B,
                  int64_t ldb, int64_t sB, const int* __restrict__ EA, const int* __restrict__ EB,
                  float4* __restrict__ C, int64_t ldc, int64_t sC, int rows_fast, int* __restrict__ err,
@@ -407,19 +447,17 @@ __global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
     constexpr uint32_t TMEM_COLS = NLEV * 128;
     extern __shared__ __align__(128) unsigned char tc_smem[];
     unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)tc_smem + 127) & ~(uintptr_t)127);
-    __shared__ __align__(8) uint64_t bar_full[2], bar_bcopy[2], bar_empty[2], bar_done, bar_tmem, bar_stage;
+    __shared__ __align__(8) uint64_t bar_full[2], bar_bcopy[2], bar_empty[2], bar_done, bar_tmem;
     __shared__ uint32_t tmem_base_sh;
+    __shared__ int emax[4][S > 3 ? TC_TN : 1];  // column maxima of a tile (float bits) by lane quarter
     __shared__ volatile int abort_sh;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nstages = (K + TC_TK - 1) / TC_TK;
     const uint32_t sbase = su32(base);
-    constexpr bool RAW = raw_bytes(CONJ_A, FMTA) > 0;  // A's rows come through the raw buffer
-    const uint32_t raw = sbase + 2 * SB + (warp & 7) * (raw_bytes(CONJ_A, FMTA) / 8);
-    // With room in the stage buffers the 128 x 64 output tile is staged there
-    // (rows padded to 65 entries: no bank conflicts either way).
-    constexpr int TROW = TC_TN + 1;
-    constexpr bool STAGE = 2 * SB >= TC_TM * TROW * 16;
-    float4* tile = reinterpret_cast<float4*>(base);
+    const uint32_t raw = sbase + 2 * SB + (warp & 7) * (raw_bytes(FMTA) / 8);  // an A warp's part of the raw buffer
+    constexpr bool OWN = own_out<S>(FMTA);
+    // an A warp's 2 KB for its outputs
+    const uint32_t outb = OWN ? sbase + 2 * SB + raw_bytes(FMTA) + (warp & 7) * 2048 : raw;
 
     if (tid == 0) {
         const uint32_t nfull = PRE ? A_PRODUCERS : A_PRODUCERS + B_PRODUCERS;
@@ -431,7 +469,6 @@ __global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
         mbar_init(&bar_empty[1], 1);
         mbar_init(&bar_done, 1);
         mbar_init(&bar_tmem, 8);  // one arrival per epilogue warp
-        mbar_init(&bar_stage, 1);
         abort_sh = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -445,11 +482,15 @@ __global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_sh;
+    auto grow = []() {
+        if constexpr (tc_split(S)) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PRODUCER_REGS));
+    };
     int ndone = 0;  // MMA thread: tiles committed to bar_done
 
-    if (warp == MMA_WARP) {
+    if (warp >= MMA_WARP) {
         // ------------------------------------------------ MMA issuer (lane 0)
-        if (lane == 0) {
+        if constexpr (tc_split(S)) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(MMA_REGS));
+        if (warp == MMA_WARP && lane == 0) {
             int tn = 0;
             for (int64_t L = blockIdx.x; L < ntiles; L += gridDim.x, ++tn) {
                 // the previous tile's accumulators have been read out
@@ -509,108 +550,36 @@ __global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
         __syncwarp();
     } else if (tid < A_PRODUCERS) {
         // -------------------- A digit producers (row, 8 k), then the epilogue
+        grow();
         const int r = CONJ_A ? (tid & 127) : (tid >> 1);
         const int g = CONJ_A ? (tid >> 7) : (tid & 1);
-        const int64_t kstride = CONJ_A ? lda : 1;
         const uint32_t o_re = plane_off(r, 8 * g), o_im = plane_off(r, 16 + 8 * g);
         const int q = warp & 3, h = warp >> 2;  // epilogue: TMEM lanes 32q .. 32q+31; complex columns 32h .. 32h+31
         const uint32_t lane_addr = tmem + ((uint32_t)(32 * q) << 16);
-        // element index of (row gi of op(A), k = 0) for tile L, and whether the row exists
-        auto row_base = [&](int64_t L, bool& rv) -> int64_t {
+        // Drain tile L (the CTA's tn-th) from TMEM and write it; false: abort (of all
+        // eight warps: roles still running may set abort_sh at any time, so the
+        // verdict is one barrier reduction, and either the whole tile is written
+        // or none of it).
+        auto epilogue = [&](int64_t L, int tn) -> bool {
             const TileId t = tile_of(L, gx, gy, rows_fast);
-            const int gi = t.rt * TC_TM + r;
-            rv = gi < M;
-            return CONJ_A ? (t.b * sA + gi) : (t.b * sA + (int64_t)gi * lda);
-        };
-        // the warp's rows of a stage of tile L, on their way to its raw buffer
-        auto copy_rows = [&](int64_t L, int kf) {
-            const TileId t = tile_of(L, gx, gy, rows_fast);
-            const int g0 = t.rt * TC_TM + 16 * warp;
-            raw_copy<FMTA>(raw, A, t.b * sA + (int64_t)g0 * lda, lda, M - g0, kf, K, lane);
-        };
-        int4 nxt[8];
-        if constexpr (RAW) {
-            if (blockIdx.x < ntiles) copy_rows(blockIdx.x, 0);
-        } else if constexpr (!PRE_A) {
-            bool rv0;
-            const int64_t i0 = row_base(blockIdx.x, rv0);
-            if (blockIdx.x < ntiles)
-                load8<FMTA>(A, i0 + (int64_t)(8 * g) * kstride, kstride, rv0 ? n_valid(K, 8 * g) : 0, nxt);
-        }
-        int tn = 0;
-        for (int64_t L = blockIdx.x; L < ntiles; L += gridDim.x, ++tn) {
-            const TileId t = tile_of(L, gx, gy, rows_fast);
-            const int row0 = t.rt * TC_TM, col0 = t.ct * TC_TN;
-            const int gi = row0 + r;
-            const bool rv = gi < M;
-            const int E = rv ? EA[t.b * M + gi] : ZERO_EXP;
-            float s1, s2;
-            f32_scales(E, s1, s2);
-            const int64_t idx0 = CONJ_A ? (t.b * sA + gi) : (t.b * sA + (int64_t)gi * lda);
-            if constexpr (!PRE_A) for (int it = 0; it < nstages; ++it) {
-                const int64_t gs = (int64_t)tn * nstages + it;
-                const int bi = (int)(gs & 1);
-                int4 cur[8];
-                // the next stage (of the next tile: in flight during this tile's epilogue)
-                const bool last = it + 1 == nstages;
-                if constexpr (RAW) {
-                    raw_read<FMTA>(raw, lane, cur);
-                    if (!last)
-                        copy_rows(L, (it + 1) * TC_TK);
-                    else if (L + gridDim.x < ntiles)
-                        copy_rows(L + gridDim.x, 0);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) cur[i] = nxt[i];
-                    if (!last) {
-                        const int kf = (it + 1) * TC_TK + 8 * g;
-                        load8<FMTA>(A, idx0 + (int64_t)kf * kstride, kstride, rv ? n_valid(K, kf) : 0, nxt);
-                    } else if (L + gridDim.x < ntiles) {
-                        bool rvn;
-                        const int64_t in = row_base(L + gridDim.x, rvn);
-                        load8<FMTA>(A, in + (int64_t)(8 * g) * kstride, kstride, rvn ? n_valid(K, 8 * g) : 0, nxt);
-                    }
-                }
-                // slice this stage while the MMAs of the two stages before it run; then
-                // wait only for the buffer and store
-                uint4 dre[S], dim[S];
-                item_planes<FMTA, 0, S>(cur, E, s1, s2, dre);
-                item_planes<FMTA, 1, S>(cur, E, s1, s2, dim);
-                bool quit = gs >= 2 && !mbar_wait(&bar_empty[bi], (uint32_t)(((gs >> 1) - 1) & 1), &abort_sh, wait_limit);
-                if (quit) abort_sh = 1;
-                quit = quit || abort_sh;
-                if (RAW) quit = __any_sync(0xffffffffu, quit);  // raw_read takes whole warps
-                if (quit) break;
-                const uint32_t sa = sbase + bi * SB;
-#pragma unroll
-                for (int s = 0; s < S; ++s) st_shared_v4(sa + s * PLANE + o_re, dre[s]);
-#pragma unroll
-                for (int s = 0; s < S; ++s) st_shared_v4(sa + s * PLANE + o_im, CONJ_A ? neg_bf16x8(dim[s]) : dim[s]);
-                fence_async_smem();  // make the generic-proxy writes visible to the tensor core
-                mbar_arrive(&bar_full[bi]);
-            }
-            // ------------------------------------------------------ epilogue
-            // A time-out here is an abort too; either the whole tile is written
-            // or none of it
-            // (the verdict is one barrier reduction: roles still running may set
-            // abort_sh at any time, and the eight warps must agree)
+            const int row0 = t.rt * TC_TM + 32 * q, col0 = t.ct * TC_TN;
+            // exponents of the lane's row and of the warp's column h * 32 + lane
+            const int ea = (row0 + lane < M) ? EA[t.b * M + row0 + lane] : ZERO_EXP;
+            const int jl = col0 + 32 * h + lane;
+            const int ebl = jl < Nc ? EB[t.b * Nc + jl] : ZERO_EXP;
             bool bad = abort_sh != 0;
             if (!bad && !mbar_wait(&bar_done, tn & 1, &abort_sh, wait_limit)) {
                 abort_sh = 1;
                 bad = true;
             }
-            if (epilogue_any(bad)) break;
+            if (epilogue_any(bad)) return false;
             tc_fence_after();
-            const int re_ = row0 + 32 * q + lane;
-            const int ea = (re_ < M) ? EA[t.b * M + re_] : ZERO_EXP;
             for (int cc = 0; cc < 4; ++cc) {
                 const int c0 = 32 * h + 8 * cc;
                 uint32_t v[2 * NLEV][8];  // [2 * level + (0 re, 1 im)][column]
 #pragma unroll
-                for (int Lv = 0; Lv < NLEV; ++Lv) {
-                    tmem_ld8(lane_addr + (uint32_t)(Lv * 128 + c0), v[2 * Lv]);
-                    tmem_ld8(lane_addr + (uint32_t)(Lv * 128 + TC_TN + c0), v[2 * Lv + 1]);
-                }
+                for (int Lv = 0; Lv < 2 * NLEV; ++Lv)
+                    tmem_ld8(lane_addr + (uint32_t)((Lv >> 1) * 128 + (Lv & 1) * TC_TN + c0), v[Lv]);
                 tmem_wait_ld();
                 if (cc == 3) {
                     // every accumulator of this warp's lanes and columns is in registers
@@ -640,68 +609,121 @@ __global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
                         hl[2 * part] = hi;
                         hl[2 * part + 1] = (e1 + e2) + a3;
                     }
-                    const int eb = (j < Nc) ? EB[t.b * Nc + j] : ZERO_EXP;
+                    const int eb = __shfl_sync(0xffffffffu, ebl, 8 * cc + c);
                     float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (ea != ZERO_EXP && eb != ZERO_EXP) {
                         const int n = max(-126, min(127, ea + eb - 14));
                         const float sc = pow2f(n);
                         out = make_float4(hl[0] * sc, hl[1] * sc, hl[2] * sc, hl[3] * sc);
                     }
-                    if (STAGE) {
-                        tile[(32 * q + lane) * TROW + c0 + c] = out;
-                        continue;
+                    if (S > 3 && Ecol) {
+                        // the column's largest magnitude over this warp's rows (>= 0,
+                        // NaN as 0: ordered as integers; absent rows are 0)
+                        const float mg = fmaxf(pair_mag(out), 0.f);
+                        const int mv = __reduce_max_sync(0xffffffffu, __float_as_int(mg));
+                        if (lane == 0) emax[q][c0 + c] = mv;
                     }
-                    const bool in = re_ < M && j < Nc;
-                    if (in) {
-                        float4* cp = C + t.b * sC + (int64_t)re_ * ldc + j;
-                        if (accumulate) {  // a later K chunk: add to the stored pair
-                            const float4 prev = *cp;
-                            const float2 pre = pair_add(prev.x, prev.y, out.x, out.y);
-                            const float2 pim = pair_add(prev.z, prev.w, out.z, out.w);
-                            out = make_float4(pre.x, pre.y, pim.x, pim.y);
+                    // 16-byte units of a row's four columns permuted: no bank conflicts
+                    st_shared_v4(outb + 64 * lane + (((c & 3) ^ ((lane >> 1) & 3)) << 4),
+                                 make_uint4(__float_as_uint(out.x), __float_as_uint(out.y), __float_as_uint(out.z),
+                                            __float_as_uint(out.w)));
+                    if ((c & 3) == 3) {
+                        __syncwarp();
+                        const int jw = j - 3 + (lane & 3);
+#pragma unroll
+                        for (int p = 0; p < 4; ++p) {
+                            const int rl = 8 * p + (lane >> 2);
+                            float4 o;
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                         : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w)
+                                         : "r"(outb + 64 * rl + (((lane & 3) ^ ((rl >> 1) & 3)) << 4))
+                                         : "memory");
+                            if (row0 + rl >= M || jw >= Nc) continue;
+                            float4* cp = C + t.b * sC + (int64_t)(row0 + rl) * ldc + jw;
+                            if (accumulate) {  // a later K chunk: add to the stored pair
+                                const float4 prev = *cp;
+                                const float2 pre = pair_add(prev.x, prev.y, o.x, o.y);
+                                const float2 pim = pair_add(prev.z, prev.w, o.z, o.w);
+                                o = make_float4(pre.x, pre.y, pim.x, pim.y);
+                            }
+                            *cp = o;
                         }
-                        *cp = out;
+                        __syncwarp();
                     }
                 }
             }
-            if (STAGE) {
-                asm volatile("bar.sync 1, 256;" ::: "memory");  // the tile is staged
-                if (Ecol) {
-                    // exponents of the output's columns, as the line scan would take
-                    // them (one row tile holds all rows): warp w, columns w, w + 8, ...
-                    for (int cl = warp; cl < TC_TN; cl += 8) {
-                        float m = 0.f;
-                        for (int rl = lane; rl < TC_TM; rl += 32) m = fmaxf(m, pair_mag(tile[rl * TROW + cl]));
-#pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-                        if (lane == 0 && col0 + cl < Nc) Ecol[t.b * Nc + col0 + cl] = line_exp_of(m);
-                    }
+            if (S > 3 && Ecol) {
+                // exponents of the output's columns, as the line scan would take them
+                // (one row tile holds all rows)
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                if (tid < TC_TN && col0 + tid < Nc) {
+                    const int mx = max(max(emax[0][tid], emax[1][tid]), max(emax[2][tid], emax[3][tid]));
+                    Ecol[t.b * Nc + col0 + tid] = line_exp_of(__int_as_float(mx));
                 }
-                // warp w writes rows w, w + 8, ...; lanes over the 64 columns
-                for (int rl = warp; rl < TC_TM; rl += 8) {
-                    const int rr = row0 + rl;
-                    if (rr >= M) break;
-#pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        const int jl = lane + 32 * half, j = col0 + jl;
-                        if (j >= Nc) continue;
-                        float4 out = tile[rl * TROW + jl];
-                        float4* cp = C + t.b * sC + (int64_t)rr * ldc + j;
-                        if (accumulate) {  // a later K chunk: add to the stored pair
-                            const float4 prev = *cp;
-                            const float2 pre = pair_add(prev.x, prev.y, out.x, out.y);
-                            const float2 pim = pair_add(prev.z, prev.w, out.z, out.w);
-                            out = make_float4(pre.x, pre.y, pim.x, pim.y);
-                        }
-                        *cp = out;
-                    }
-                }
-                asm volatile("bar.sync 1, 256;" ::: "memory");  // every read of the staged tile done
-                if (tid == 0) mbar_arrive(&bar_stage);
             }
+            return true;
+        };
+        int tn = 0;
+        if constexpr (PRE_A) {
+            for (int64_t L = blockIdx.x; L < ntiles; L += gridDim.x, ++tn)
+                if (!epilogue(L, tn)) break;
+        } else {
+            // Stage (Ls, its) is the next to be sliced, its elements under way to the
+            // raw buffer unless the copy is held back; dre, dim hold the digits of the
+            // stage before it.
+            int64_t Ls = blockIdx.x;
+            int its = 0, Es = ZERO_EXP;
+            float s1 = 0.f, s2 = 0.f;
+            uint4 dre[S], dim[S];
+            auto copy = [&]() {
+                const TileId t = tile_of(Ls, gx, gy, rows_fast);
+                const int w0 = t.rt * TC_TM + (CONJ_A ? 32 * (warp & 3) : 16 * warp);
+                raw_copy<CONJ_A, FMTA>(raw, A, t.b * sA + (CONJ_A ? (int64_t)w0 : (int64_t)w0 * lda), lda, M - w0,
+                                       its * TC_TK + (CONJ_A ? 8 * g : 0), K, lane);
+                if (its == 0) Es = t.rt * TC_TM + r < M ? EA[t.b * M + t.rt * TC_TM + r] : ZERO_EXP;
+            };
+            auto slice = [&](bool hold) {
+                int4 cur[8];
+                raw_read<CONJ_A, FMTA>(raw, lane, cur);
+                if (its == 0) f32_scales(Es, s1, s2);
+                const int E = Es;
+                if (++its == nstages) {
+                    its = 0;
+                    Ls += gridDim.x;
+                }
+                if (!hold && Ls < ntiles) copy();
+                item_planes<FMTA, 0, S>(cur, E, s1, s2, dre);
+                item_planes<FMTA, 1, S>(cur, E, s1, s2, dim);
+            };
+            copy();
+            int64_t gs = 0;
+            for (int64_t L = blockIdx.x; L < ntiles; L += gridDim.x, ++tn) {
+                bool quit = false;
+                for (int it = 0; it < nstages; ++it, ++gs) {
+                    const int bi = (int)(gs & 1);
+                    // slice this stage while the MMAs of the two before it run; then wait
+                    // only for the buffer and store
+                    slice(!OWN && it + 1 == nstages);
+                    quit = gs >= 2 && !mbar_wait(&bar_empty[bi], (uint32_t)(((gs >> 1) - 1) & 1), &abort_sh, wait_limit);
+                    if (quit) abort_sh = 1;
+                    quit = __any_sync(0xffffffffu, quit || abort_sh);  // whole warps: raw_read
+                    if (quit) break;
+                    const uint32_t sa = sbase + bi * SB;
+#pragma unroll
+                    for (int s = 0; s < S; ++s) st_shared_v4(sa + s * PLANE + o_re, dre[s]);
+#pragma unroll
+                    for (int s = 0; s < S; ++s)
+                        st_shared_v4(sa + s * PLANE + o_im, CONJ_A ? neg_bf16x8(dim[s]) : dim[s]);
+                    fence_async_smem();  // make the generic-proxy writes visible to the tensor core
+                    mbar_arrive(&bar_full[bi]);
+                }
+                if (!epilogue(L, tn)) break;
+                if (!OWN && Ls < ntiles) copy();
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
         }
-        if (RAW) asm volatile("cp.async.wait_all;" ::: "memory");
     } else if (tid < A_PRODUCERS + B_PRODUCERS) {
+        grow();
         const int qb = tid - A_PRODUCERS;
         if (PRE) {
             // ------------------------- pre-sliced B: bulk copy of stage images
@@ -720,10 +742,8 @@ __global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
                     for (int it = 0; it < nstages; ++it) {
                         const int64_t gs = (int64_t)tn * nstages + it;
                         const int bi = (int)(gs & 1);
-                        if ((gs >= 2 &&
-                             !mbar_wait(&bar_empty[bi], (uint32_t)(((gs >> 1) - 1) & 1), &abort_sh, wait_limit)) ||
-                            (STAGE && tn > 0 && it < 2 &&
-                             !mbar_wait(&bar_stage, (uint32_t)((tn - 1) & 1), &abort_sh, wait_limit))) {
+                        if (gs >= 2 &&
+                            !mbar_wait(&bar_empty[bi], (uint32_t)(((gs >> 1) - 1) & 1), &abort_sh, wait_limit)) {
                             abort_sh = 1;
                             stop = true;
                             break;
@@ -788,10 +808,8 @@ __global__ void __launch_bounds__(TC_THREADS, Class<S>::MIN_CTAS)
                     uint4 dre[S], dim[S];
                     item_planes<FB, 0, S>(cur, E, s1, s2, dre);
                     item_planes<FB, 1, S>(cur, E, s1, s2, dim);
-                    if ((gs >= 2 &&
-                         !mbar_wait(&bar_empty[bi], (uint32_t)(((gs >> 1) - 1) & 1), &abort_sh, wait_limit)) ||
-                        (STAGE && tn > 0 && it < 2 &&
-                         !mbar_wait(&bar_stage, (uint32_t)((tn - 1) & 1), &abort_sh, wait_limit))) {
+                    if (gs >= 2 &&
+                        !mbar_wait(&bar_empty[bi], (uint32_t)(((gs >> 1) - 1) & 1), &abort_sh, wait_limit)) {
                         abort_sh = 1;
                         stop = true;
                         break;
@@ -941,21 +959,20 @@ static int launch_tc(cudaStream_t st, int64_t batch, int M, int Nc, int K, const
                      const void* B, int64_t ldb, int64_t sB, float4* C, int64_t ldc, int64_t sC, int* EA, int* EB,
                      int* err, const char* name, double work, int accumulate = 0, int* Ecol = nullptr) {
     auto kern = oz_tc_kernel<CJ, FA, FB, S>;
-    constexpr int smem = tc_smem_bytes(S, raw_bytes(CJ, FA));
+    constexpr int smem = tc_smem_bytes<S>(FA);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(oz_tc)");
     KTimer kt(st, name, work);
-    // tiles (column tile, row tile, matrix), column tiles fastest; persistent
-    // CTAs where the output is staged in shared memory (HIGH, MID: the
-    // per-CTA set-up and launch gap were ~12 % of a 128^3 tile), one tile per
-    // CTA for the LOW class (two CTAs per SM already overlap its epilogues)
+    // tiles (column tile, row tile, matrix), column tiles fastest; persistent CTAs
+    // (the set-up and launch gap were ~12 % of a 128^3 tile), but one tile per CTA
+    // for the LOW class, where two CTAs per SM overlap their epilogues
     const int gx = (Nc + TC_TN - 1) / TC_TN, gy = (M + TC_TM - 1) / TC_TM;
     const int64_t ntiles = (int64_t)gx * gy * batch;
     if (ntiles <= 0) return TBG_OK;  // nothing to compute
     if (K <= 0) return set_error(TBG_E_INVALID_ARGUMENT, "ozaki_zgemm_tc: empty contraction");
-    const int64_t grid = tc_staged(S) ? std::min<int64_t>(ntiles, (int64_t)sm_count() * Class<S>::MIN_CTAS)
+    const int64_t grid = Class<S>::MIN_CTAS == 1 ? std::min<int64_t>(ntiles, (int64_t)sm_count() * Class<S>::MIN_CTAS)
                                       : std::min<int64_t>(ntiles, 0x7fffffff);
-    kern<<<(unsigned)grid, TC_THREADS, smem, st>>>(M, Nc, K, A, lda, sA, B, ldb, sB, EA, EB, C, ldc, sC, 0, err,
+    kern<<<(unsigned)grid, tc_threads(S), smem, st>>>(M, Nc, K, A, lda, sA, B, ldb, sB, EA, EB, C, ldc, sC, 0, err,
                                                    accumulate, Ecol, tc_wait_limit(), gx, gy, ntiles);
     TBG_LAUNCHED(name);
     return TBG_OK;
@@ -1132,7 +1149,7 @@ static int fourier_tc_launch(cudaStream_t st, int64_t M, int64_t Nc, int K, cons
         TBG_LAUNCHED("phase_image_kernel");
     }
     auto kern = oz_tc_kernel<false, FMT_PRESLICED, FMT_PRESLICED, S>;
-    const int smem = tc_smem_bytes(S, 0);
+    const int smem = tc_smem_bytes<S>(FMT_PRESLICED);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(oz_tc fourier)");
     KTimer kt(st, S == TC_S ? "ozaki_tc_fourier_kernel" : "ozaki_tc_fourier_kernel<mid>", 8.0 * (double)M * Nc * K);
@@ -1142,7 +1159,7 @@ static int fourier_tc_launch(cudaStream_t st, int64_t M, int64_t Nc, int K, cons
     if (ntiles <= 0) return TBG_OK;
     if (K <= 0) return set_error(TBG_E_INVALID_ARGUMENT, "ozaki_fourier_tc: empty contraction");
     const int64_t grid = std::min<int64_t>(ntiles, (int64_t)sm_count() * Class<S>::MIN_CTAS);
-    kern<<<(unsigned)grid, TC_THREADS, smem, st>>>((int)M, (int)Nc, K, aimg, K, 0, img, Nc, 0, EA, EB, C, Nc, 0, 1,
+    kern<<<(unsigned)grid, tc_threads(S), smem, st>>>((int)M, (int)Nc, K, aimg, K, 0, img, Nc, 0, EA, EB, C, Nc, 0, 1,
                                                    err, 0, nullptr, tc_wait_limit(), gx, gy, ntiles);
     TBG_LAUNCHED(S == TC_S ? "ozaki_tc_fourier_kernel" : "ozaki_tc_fourier_kernel<mid>");
     return TBG_OK;
