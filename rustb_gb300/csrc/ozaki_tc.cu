@@ -136,21 +136,6 @@ __device__ __forceinline__ long long fx64(double x, int E) {
     const long long F = (sh >= 64) ? 0 : (long long)(M >> sh);
     return (b >> 63) ? -F : F;
 }
-// Fixed-point value trunc(x * 2^(42 - E)) of a float with |x| < 2^E.
-__device__ __forceinline__ long long fx32(float x, int E) {
-    const unsigned b = __float_as_uint(x);
-    const int ex = (int)((b >> 23) & 0xff);
-    if (ex == 0) return 0;
-    const unsigned long long M = (unsigned long long)((b & 0x7FFFFFu) | 0x800000u);
-    const int sh = (ex - 127) - 23 + 42 - E;
-    long long F;
-    if (sh >= 0)
-        F = (sh >= 40) ? 0 : (long long)(M << sh);
-    else
-        F = (-sh >= 64) ? 0 : (long long)(M >> (-sh));
-    return (b >> 31) ? -F : F;
-}
-
 // r rounded to the nearest multiple of 2^k (ties to even) by adding and
 // subtracting 1.5 * 2^(23 + k); exact for |r| < 2^(22 + k).
 constexpr double pow2c(int e) { return e == 0 ? 1.0 : (e > 0 ? 2.0 * pow2c(e - 1) : 0.5 * pow2c(e + 1)); }
@@ -179,25 +164,62 @@ __device__ __forceinline__ void digits_fixed(long long F, float* P) {
     P[4] = round_to_pow2<-28>(r2);
     P[5] = __fsub_rn(r2, P[4]);             // q_5 2^-35
 }
-// Six pre-scaled digits of u = x 2^(7 - E) in (-128, 128) for an FP32 x:
+// Two FP32 values in one instruction (add, sub, mul of .f32x2, each rounded to
+// nearest): the producers and the epilogue are bound by issue slots.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 a) {
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(a));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+template <int K>
+__device__ __forceinline__ f32x2 round_to_pow2(f32x2 r) {
+    constexpr float C = (float)(1.5 * pow2c(23 + K));
+    const f32x2 c = pack2(C, C);
+    return sub2(add2(r, c), c);
+}
+
+// Six pre-scaled digits of u = x 2^(7 - E) in (-128, 128) for an FP32 x (two
+// values at once):
 // P_s = u_s rounded to a multiple of 2^(-7s), u_{s+1} = u_s - P_s, every step
 // exact; the sum equals x rounded to the grid 2^(E-42).  |q_0| <= 128,
 // |q_s| <= 64.
-__device__ __forceinline__ void digits_float(float u, float* P) {
+__device__ __forceinline__ void digits_float(f32x2 u, f32x2* P) {
     P[0] = round_to_pow2<0>(u);
-    float r = __fsub_rn(u, P[0]);
+    f32x2 r = sub2(u, P[0]);
     P[1] = round_to_pow2<-7>(r);
-    r = __fsub_rn(r, P[1]);
+    r = sub2(r, P[1]);
     P[2] = round_to_pow2<-14>(r);
-    r = __fsub_rn(r, P[2]);
+    r = sub2(r, P[2]);
     P[3] = round_to_pow2<-21>(r);
-    r = __fsub_rn(r, P[3]);
+    r = sub2(r, P[3]);
     P[4] = round_to_pow2<-28>(r);
-    r = __fsub_rn(r, P[4]);
+    r = sub2(r, P[4]);
     P[5] = round_to_pow2<-35>(r);
 }
 // Six pre-scaled digits of u = (hi + lo) 2^(7 - E) in (-128, 128] for a
-// float pair, in FP32 arithmetic only.  The pair is first renormalised by an
+// float pair, in FP32 arithmetic only (two values at once).  The pair is first
+// renormalised by an
 // error-free two-sum (the producers' pairs need not have |lo| <= ulp(hi) / 2);
 // digits 0..2 then come from the leading part, whose remainder r (|r| <=
 // 2^-15, a subset of its bits) is exact; t = r + lo then needs the bits from
@@ -206,24 +228,24 @@ __device__ __forceinline__ void digits_float(float u, float* P) {
 // 2^-35 up to half a grid step plus t's rounding (the integer form truncates
 // each part: up to two grid steps).  |q_0| <= 128, |q_1|, |q_2|, |q_4|,
 // |q_5| <= 64, |q_3| <= 72.
-__device__ __forceinline__ void digits_pair(float uh, float ul, float* P) {
+__device__ __forceinline__ void digits_pair(f32x2 uh, f32x2 ul, f32x2* P) {
     {
-        const float sm = __fadd_rn(uh, ul);
-        const float v = __fsub_rn(sm, uh);
-        ul = __fadd_rn(__fsub_rn(uh, __fsub_rn(sm, v)), __fsub_rn(ul, v));
+        const f32x2 sm = add2(uh, ul);
+        const f32x2 v = sub2(sm, uh);
+        ul = add2(sub2(uh, sub2(sm, v)), sub2(ul, v));
         uh = sm;
     }
     P[0] = round_to_pow2<0>(uh);
-    float r = __fsub_rn(uh, P[0]);
+    f32x2 r = sub2(uh, P[0]);
     P[1] = round_to_pow2<-7>(r);
-    r = __fsub_rn(r, P[1]);
+    r = sub2(r, P[1]);
     P[2] = round_to_pow2<-14>(r);
-    r = __fsub_rn(r, P[2]);
-    float t = __fadd_rn(r, ul);
+    r = sub2(r, P[2]);
+    f32x2 t = add2(r, ul);
     P[3] = round_to_pow2<-21>(t);
-    t = __fsub_rn(t, P[3]);
+    t = sub2(t, P[3]);
     P[4] = round_to_pow2<-28>(t);
-    t = __fsub_rn(t, P[4]);
+    t = sub2(t, P[4]);
     P[5] = round_to_pow2<-35>(t);
 }
 __device__ __forceinline__ float pow2f(int n) { return __int_as_float((127 + n) << 23); }  // n in [-126, 127]
@@ -330,25 +352,28 @@ __device__ __forceinline__ void raw_read(uint32_t raw, int lane, int4 (&r)[8]) {
     }
     if constexpr (!COLS) __syncwarp();  // before the next copies overwrite the buffer
 }
-// Digits of the real (part 0) or imaginary (part 1) component of one element.
+// Digits of the real (part 0) or imaginary (part 1) component of two elements.
 template <int FMT, int PART>
-__device__ __forceinline__ void elem_digits(const int4& r, int E, float s1, float s2, float* P) {
+__device__ __forceinline__ void elem_digits(const int4& r0, const int4& r1, int E, float s1, float s2, f32x2* P) {
+    auto part = [](const int4& r, int lo) {
+        return __int_as_float(FMT == FMT_F32 ? (PART ? r.y : r.x) : lo ? (PART ? r.w : r.y) : (PART ? r.z : r.x));
+    };
+    const f32x2 ss = pack2(s2, s2);
     if (FMT == FMT_F32) {
-        const float x = __int_as_float(PART ? r.y : r.x);
-        digits_float((x * s1) * s2, P);
+        digits_float(mul2(pack2(part(r0, 0) * s1, part(r1, 0) * s1), ss), P);
     } else if (FMT == FMT_PAIR) {
-        const float hi = __int_as_float(PART ? r.z : r.x), lo = __int_as_float(PART ? r.w : r.y);
-        digits_pair(__fmul_rn(__fmul_rn(hi, s1), s2), __fmul_rn(__fmul_rn(lo, s1), s2), P);
+        digits_pair(mul2(pack2(part(r0, 0) * s1, part(r1, 0) * s1), ss),
+                    mul2(pack2(part(r0, 1) * s1, part(r1, 1) * s1), ss), P);
     } else {
-        long long F = 0;
-        if (E != ZERO_EXP) {
-            if (FMT == FMT_F64)
-                F = PART ? fx64(__hiloint2double(r.w, r.z), E) : fx64(__hiloint2double(r.y, r.x), E);
-            else
-                F = PART ? fx32(__int_as_float(r.z), E) + fx32(__int_as_float(r.w), E)
-                         : fx32(__int_as_float(r.x), E) + fx32(__int_as_float(r.y), E);
-        }
-        digits_fixed(F, P);
+        float P0[TC_S], P1[TC_S];
+        auto fixed = [&](const int4& r) {
+            if (E == ZERO_EXP) return 0ll;
+            return PART ? fx64(__hiloint2double(r.w, r.z), E) : fx64(__hiloint2double(r.y, r.x), E);
+        };
+        digits_fixed(fixed(r0), P0);
+        digits_fixed(fixed(r1), P1);
+#pragma unroll
+        for (int s = 0; s < TC_S; ++s) P[s] = pack2(P0[s], P1[s]);
     }
 }
 // (ah + al) + (bh + bl) as a float pair: two-sum of the leading parts, the
@@ -372,11 +397,13 @@ __device__ __forceinline__ void item_planes(const int4 (&r)[8], int E, float s1,
     uint32_t pk[S][4];
 #pragma unroll
     for (int i = 0; i < 8; i += 2) {
-        float P0[TC_S], P1[TC_S];
-        elem_digits<FMT, PART>(r[i], E, s1, s2, P0);
-        elem_digits<FMT, PART>(r[i + 1], E, s1, s2, P1);
+        f32x2 P[TC_S];
+        elem_digits<FMT, PART>(r[i], r[i + 1], E, s1, s2, P);
 #pragma unroll
-        for (int s = 0; s < S; ++s) pk[s][i >> 1] = pack_bf16x2(P0[s], P1[s]);
+        for (int s = 0; s < S; ++s) {
+            const float2 d = unpack2(P[s]);
+            pk[s][i >> 1] = pack_bf16x2(d.x, d.y);
+        }
     }
 #pragma unroll
     for (int s = 0; s < S; ++s) out[s] = make_uint4(pk[s][0], pk[s][1], pk[s][2], pk[s][3]);
@@ -577,6 +604,7 @@ __global__ void __launch_bounds__(tc_threads(S), Class<S>::MIN_CTAS)
             for (int cc = 0; cc < 4; ++cc) {
                 const int c0 = 32 * h + 8 * cc;
                 uint32_t v[2 * NLEV][8];  // [2 * level + (0 re, 1 im)][column]
+                float2 hl[4];
 #pragma unroll
                 for (int Lv = 0; Lv < 2 * NLEV; ++Lv)
                     tmem_ld8(lane_addr + (uint32_t)((Lv >> 1) * 128 + (Lv & 1) * TC_TN + c0), v[Lv]);
@@ -590,31 +618,38 @@ __global__ void __launch_bounds__(tc_threads(S), Class<S>::MIN_CTAS)
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                     const int j = col0 + c0 + c;
-                    float hl[4];
+                    // (re hi, re lo, im hi, im lo) of columns c and c + 1, two at a time.
+                    // Level 0 sums whole numbers and level 1 multiples of 2^-7 below 2^17,
+                    // level 2 multiples of 2^-14 below 2^10: the first addend of each sum
+                    // is a multiple of the second's ulp, so s - a is exact and the short
+                    // two-sum error free.
+                    if ((c & 1) == 0) {
 #pragma unroll
-                    for (int part = 0; part < 2; ++part) {
-                        if (NLEV == 1) {
-                            hl[2 * part] = __uint_as_float(v[part][c]);
-                            hl[2 * part + 1] = 0.f;
-                            continue;
+                        for (int part = 0; part < 2; ++part) {
+                            auto lvl = [&](int Lv) {
+                                return pack2(__uint_as_float(v[2 * Lv + part][c]), __uint_as_float(v[2 * Lv + part][c + 1]));
+                            };
+                            if (NLEV == 1) {
+                                hl[2 * part] = unpack2(lvl(0));
+                                hl[2 * part + 1] = make_float2(0.f, 0.f);
+                                continue;
+                            }
+                            const f32x2 a0 = lvl(0), a1 = lvl(1), a2 = lvl(2), a3 = lvl(3);
+                            const f32x2 sm = add2(a0, a1);
+                            const f32x2 e1 = sub2(a1, sub2(sm, a0));
+                            const f32x2 hi = add2(sm, a2);
+                            const f32x2 e2 = sub2(a2, sub2(hi, sm));
+                            hl[2 * part] = unpack2(hi);
+                            hl[2 * part + 1] = unpack2(add2(add2(e1, e2), a3));
                         }
-                        const float a0 = __uint_as_float(v[0 + part][c]), a1 = __uint_as_float(v[2 + part][c]);
-                        const float a2 = __uint_as_float(v[4 + part][c]), a3 = __uint_as_float(v[6 + part][c]);
-                        const float s1_ = a0 + a1;
-                        const float t1 = s1_ - a0;
-                        const float e1 = (a0 - (s1_ - t1)) + (a1 - t1);
-                        const float hi = s1_ + a2;
-                        const float t2 = hi - s1_;
-                        const float e2 = (s1_ - (hi - t2)) + (a2 - t2);
-                        hl[2 * part] = hi;
-                        hl[2 * part + 1] = (e1 + e2) + a3;
                     }
+                    auto at = [&](int i) { return c & 1 ? hl[i].y : hl[i].x; };
                     const int eb = __shfl_sync(0xffffffffu, ebl, 8 * cc + c);
                     float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (ea != ZERO_EXP && eb != ZERO_EXP) {
                         const int n = max(-126, min(127, ea + eb - 14));
                         const float sc = pow2f(n);
-                        out = make_float4(hl[0] * sc, hl[1] * sc, hl[2] * sc, hl[3] * sc);
+                        out = make_float4(at(0) * sc, at(1) * sc, at(2) * sc, at(3) * sc);
                     }
                     if (S > 3 && Ecol) {
                         // the column's largest magnitude over this warp's rows (>= 0,
