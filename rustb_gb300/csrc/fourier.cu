@@ -494,90 +494,77 @@ __global__ void tau_pairs_kernel(int64_t nk, int N, float4* __restrict__ C, cons
 // Packed upper-triangle contraction output -> full float-pair H, V_0, V_1
 // (P: three blocks of nk N^2 elements, blk elements apart) with the
 // orbital-position term V_p += i (tau_p,n - tau_p,m) H, in float-pair arithmetic.
-// With rexp (three blocks of nk N ints) the row exponents of the three written
-// matrices come out too: when a block of 256 threads holds whole rows (N a
-// multiple of 32 dividing 256) each warp's maximum goes through shared memory
-// and the row's exponent is stored; otherwise rexp is preset below every
-// exponent and the maxima are folded in by atomicMax, one per warp when N is
-// a multiple of 32 (a warp then lies in one row), one or two from 32 bands on (304
-// k-points of 251 bands 2.06 -> 0.39 ms, against one per lane), else per lane.
-constexpr int kUnpackThreads = 256;
-__host__ __device__ constexpr bool unpack_block_rows(int N) { return (N & 31) == 0 && kUnpackThreads % N == 0; }
+// A block writes 32 rows of one k-point's three matrices, 32 columns at a time, so
+// with rexp (three blocks of nk N ints) it has the rows' exponents as well.  Tiles
+// right of the diagonal are read as they lie; those below it are read as rows of
+// the upper triangle and turned over in shared memory, since element by element
+// a warp touched 32 lines per load (8192 k-points of 128 bands 2.36 -> 1.89 ms, 6.4 GB
+// written; 304 of 251 bands 0.38 -> 0.34).
+constexpr int kUnpackThreads = 256, kUnpackTile = 32;
 
 __global__ void __launch_bounds__(kUnpackThreads) unpack_tau_kernel(int64_t nk, int N, const float4* __restrict__ Cp,
                                                                    const float2* __restrict__ tau2,
                                                                    float4* __restrict__ P, int64_t blk,
                                                                    int* __restrict__ rexp) {
-    const int64_t NN = (int64_t)N * N;
-    const int e = blockIdx.x * kUnpackThreads + threadIdx.x;
-    const bool valid = e < NN;
-    const int mrow = valid ? e / N : 0, ncol = valid ? e - mrow * N : 0;
-    const bool warp_row = (N & 31) == 0, block_rows = unpack_block_rows(N);
+    constexpr int TL = kUnpackTile, NW = kUnpackThreads / 32, NR = TL / NW;  // NR rows per warp
+    // units of a row permuted by its low bits: no bank conflicts by rows or columns
+    __shared__ float4 tile[3][TL * TL];
+    const int64_t NN = (int64_t)N * N, np = (int64_t)N * (N + 1) / 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __shared__ int wmax[2][3][kUnpackThreads / 32];
-    float2 d[2];
+    const int R = blockIdx.x, T = (N + TL - 1) / TL;
+    for (int64_t kk = blockIdx.y; kk < nk; kk += gridDim.y) {
+        float mag[3][NR] = {};
+        for (int J = 0; J < T; ++J) {
+            const int n = J * TL + lane;
+            if (J <= R) {
+                __syncthreads();
 #pragma unroll
-    for (int p = 0; p < 2; ++p) d[p] = df_add(tau2[p * N + ncol], df_neg(tau2[p * N + mrow]));
-    int par = 0;  // alternates per k-point of this block
-    for (int64_t kk = blockIdx.y; kk < nk; kk += gridDim.y, par ^= 1) {
-        float mag[3] = {0.f, 0.f, 0.f};
-        if (valid) {
-            const float4 h = c_elem(Cp, true, nk, N, 0, kk, mrow, ncol);
-            P[kk * NN + e] = h;
-            mag[0] = pair_mag(h);
-            const float2 hr = make_float2(h.x, h.y), hi = make_float2(h.z, h.w);
+                for (int i = 0; i < NR; ++i) {
+                    const int r = warp + NW * i, gm = J * TL + r, gn = R * TL + lane;
+                    if (gm <= gn && gn < N)
 #pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const float4 v = c_elem(Cp, true, nk, N, 1 + p, kk, mrow, ncol);
-                const float2 vr = df_add(make_float2(v.x, v.y), df_neg(df_mul(d[p], hi)));
-                const float2 vi = df_add(make_float2(v.z, v.w), df_mul(d[p], hr));
-                const float4 o = make_float4(vr.x, vr.y, vi.x, vi.y);
-                P[(1 + p) * blk + kk * NN + e] = o;
-                mag[1 + p] = pair_mag(o);
+                        for (int c = 0; c < 3; ++c)
+                            tile[c][r * TL + (lane ^ (r & 7))] = Cp[(c * nk + kk) * np + upper_index(N, gm, gn)];
+                }
+                __syncthreads();
+            }
+#pragma unroll
+            for (int i = 0; i < NR; ++i) {
+                const int r = warp + NW * i, m = R * TL + r;
+                if (m >= N || n >= N) continue;
+                auto elem = [&](int c) {
+                    if (J > R) return Cp[(c * nk + kk) * np + upper_index(N, m, n)];
+                    if (m <= n) return tile[c][r * TL + (lane ^ (r & 7))];
+                    const float4 v = tile[c][lane * TL + (r ^ (lane & 7))];
+                    return make_float4(v.x, v.y, -v.z, -v.w);
+                };
+                const float4 h = elem(0);
+                float4* out = P + kk * NN + (int64_t)m * N + n;
+                out[0] = h;
+                // a NaN counts as 0, as fmaxf over a row would skip it
+                mag[0][i] = fmaxf(mag[0][i], pair_mag(h));
+                const float2 hr = make_float2(h.x, h.y), hi = make_float2(h.z, h.w);
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    const float4 v = elem(1 + p);
+                    const float2 d = df_add(tau2[p * N + n], df_neg(tau2[p * N + m]));
+                    const float2 vr = df_add(make_float2(v.x, v.y), df_neg(df_mul(d, hi)));
+                    const float2 vi = df_add(make_float2(v.z, v.w), df_mul(d, hr));
+                    const float4 o = make_float4(vr.x, vr.y, vi.x, vi.y);
+                    out[(1 + p) * blk] = o;
+                    mag[1 + p][i] = fmaxf(mag[1 + p][i], pair_mag(o));
+                }
             }
         }
         if (rexp) {
-            // magnitudes are >= 0 (NaN counts as 0, as fmaxf over a row would
-            // skip it), so their bit patterns order as integers
 #pragma unroll
-            for (int c = 0; c < 3; ++c) mag[c] = (mag[c] == mag[c]) ? mag[c] : 0.f;
-            if (block_rows) {
-                // every thread is valid (NN is a multiple of 256); the buffer
-                // alternates per k-point, so one barrier per k-point suffices
+            for (int c = 0; c < 3; ++c)
 #pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const int v = __reduce_max_sync(0xffffffffu, __float_as_int(mag[c]));
-                    if (lane == 0) wmax[par][c][warp] = v;
+                for (int i = 0; i < NR; ++i) {
+                    // magnitudes are >= 0: their bit patterns order as integers
+                    const int v = __reduce_max_sync(0xffffffffu, __float_as_int(mag[c][i])), m = R * TL + warp + NW * i;
+                    if (lane == 0 && m < N) rexp[(c * nk + kk) * N + m] = line_exp_of(__int_as_float(v));
                 }
-                __syncthreads();
-                const int rows = kUnpackThreads / N, wpr = N / 32;
-                if (threadIdx.x < 3 * rows) {
-                    const int c = threadIdx.x / rows, rr = threadIdx.x - c * rows;
-                    int v = 0;
-                    for (int w = rr * wpr; w < (rr + 1) * wpr; ++w) v = max(v, wmax[par][c][w]);
-                    rexp[(c * nk + kk) * N + blockIdx.x * rows + rr] = line_exp_of(__int_as_float(v));
-                }
-            } else if (warp_row) {  // NN and the warps' starts are multiples of 32: all lanes valid or none
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const int v = __reduce_max_sync(0xffffffffu, __float_as_int(mag[c]));
-                    if (valid && lane == 0) atomicMax(&rexp[(c * nk + kk) * N + mrow], line_exp_of(__int_as_float(v)));
-                }
-            } else if (N >= 32) {  // a warp lies in at most two rows
-                const int r0 = __shfl_sync(0xffffffffu, mrow, 0);
-                const bool second = valid && mrow != r0, two = __any_sync(0xffffffffu, second);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const int bits = __float_as_int(mag[c]);
-                    const int v = __reduce_max_sync(0xffffffffu, second ? 0 : bits);
-                    const int w = two ? __reduce_max_sync(0xffffffffu, second ? bits : 0) : 0;
-                    if (lane == 0 && valid) atomicMax(&rexp[(c * nk + kk) * N + r0], line_exp_of(__int_as_float(v)));
-                    if (lane == 0 && two) atomicMax(&rexp[(c * nk + kk) * N + r0 + 1], line_exp_of(__int_as_float(w)));
-                }
-            } else if (valid) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) atomicMax(&rexp[(c * nk + kk) * N + mrow], line_exp_of(mag[c]));
-            }
         }
     }
 }
@@ -936,13 +923,9 @@ int fourier_mixed_pairs(ModelDev& m, cudaStream_t st, int64_t nk, const double* 
     KTimer kt(st, "tau_pairs_kernel");
     dim3 grid((unsigned)((NN + 255) / 256), (unsigned)std::min<int64_t>(nk, 65535));
     if (m.hop_packed) {
-        if (rexp) {
-            // below every exponent (0x80808080), so each row's first atomicMax sets it
-            if (!unpack_block_rows(N))
-                TBG_CUDA(cudaMemsetAsync(rexp, 0x80, sizeof(int) * 3 * (size_t)nk * N, st));
-            if (rexp_filled) *rexp_filled = true;
-        }
-        unpack_tau_kernel<<<grid, kUnpackThreads, 0, st>>>(nk, N, Cg, tau2, out, blk, rexp);
+        if (rexp && rexp_filled) *rexp_filled = true;
+        const dim3 tiles((unsigned)((N + kUnpackTile - 1) / kUnpackTile), grid.y);
+        unpack_tau_kernel<<<tiles, kUnpackThreads, 0, st>>>(nk, N, Cg, tau2, out, blk, rexp);
         TBG_LAUNCHED("unpack_tau_kernel");
     } else {
         tau_pairs_kernel<<<grid, 256, 0, st>>>(nk, N, C, tau2);
