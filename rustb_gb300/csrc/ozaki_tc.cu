@@ -15,7 +15,8 @@
 //                current one is converted; each digit plane is one 16-byte store
 //                (K-major core matrices of 8 rows x 16 bytes, no swizzle);
 //   warps 8..11  B digit producers, same per (column, 8 consecutive k) with the
-//                next elements in registers, or, for a pre-sliced operand, one
+//                next elements in registers, and A's too in a tile's first stages
+//                (HELP), or, for a pre-sliced operand, one
 //                thread that copies the stage image with cp.async.bulk
 //                (completion on an mbarrier);
 //   warp 12      allocates TMEM; lane 0 issues the MMAs and commits them;
@@ -461,7 +462,14 @@ __device__ __forceinline__ bool epilogue_any(bool v) {
 // (bar_tmem frees them for the next tile's MMAs) and write them out a few columns
 // at a time; the stage buffers stay free for the next tile's B stages and images,
 // and its first A elements are on their way.
-template <bool CONJ_A, int FMTA, int FMTB, int S>
+//
+// The first HELP stages of a tile are sliced by the B warps alone, A's part too:
+// they fill the buffers while the A warps run the last tile's epilogue, which is
+// worth about eight stages.  Two stages where a tile has six or more, else one
+// (four MID products: 8192 x 128^3 8.19 ms with none, 7.77 with one, 7.59 with
+// two; 8000 x 64^3 2.53, 2.31, 2.73; three HIGH: 6.47, 6.18, 6.03 and 2.02, 1.85,
+// 1.82), none for LOW, whose CTAs run one tile each.
+template <bool CONJ_A, int FMTA, int FMTB, int S, int HELP>
 __global__ void __launch_bounds__(tc_threads(S), Class<S>::MIN_CTAS)
     oz_tc_kernel(int M, int Nc, int K, const void* __restrict__ A, int64_t lda, int64_t sA, const void* __restrict__ B,
                  int64_t ldb, int64_t sB, const int* __restrict__ EA, const int* __restrict__ EB,
@@ -472,6 +480,7 @@ __global__ void __launch_bounds__(tc_threads(S), Class<S>::MIN_CTAS)
     // sum's phases): the copy thread brings both operands, the A warps only run
     // the epilogue
     constexpr bool PRE_A = FMTA == FMT_PRESLICED;
+    static_assert(HELP <= 2 && (HELP == 0 || (!PRE && S > 3)), "the two buffers; persistent tiles");
     static_assert(!PRE_A || (PRE && !CONJ_A), "pre-sliced A goes with pre-sliced B, not conjugated");
     constexpr int LMAX = Class<S>::LMAX, NLEV = Class<S>::NLEV;
     constexpr int HS = S * PLANE;             // planes of one operand in a stage
@@ -712,7 +721,7 @@ __global__ void __launch_bounds__(tc_threads(S), Class<S>::MIN_CTAS)
             // raw buffer unless the copy is held back; dre, dim hold the digits of the
             // stage before it.
             int64_t Ls = blockIdx.x;
-            int its = 0, Es = ZERO_EXP;
+            int its = HELP, Es = ZERO_EXP;
             float s1 = 0.f, s2 = 0.f;
             uint4 dre[S], dim[S];
             auto copy = [&]() {
@@ -720,26 +729,26 @@ __global__ void __launch_bounds__(tc_threads(S), Class<S>::MIN_CTAS)
                 const int w0 = t.rt * TC_TM + (CONJ_A ? 32 * (warp & 3) : 16 * warp);
                 raw_copy<CONJ_A, FMTA>(raw, A, t.b * sA + (CONJ_A ? (int64_t)w0 : (int64_t)w0 * lda), lda, M - w0,
                                        its * TC_TK + (CONJ_A ? 8 * g : 0), K, lane);
-                if (its == 0) Es = t.rt * TC_TM + r < M ? EA[t.b * M + t.rt * TC_TM + r] : ZERO_EXP;
+                if (its == HELP) Es = t.rt * TC_TM + r < M ? EA[t.b * M + t.rt * TC_TM + r] : ZERO_EXP;
             };
             auto slice = [&](bool hold) {
                 int4 cur[8];
                 raw_read<CONJ_A, FMTA>(raw, lane, cur);
-                if (its == 0) f32_scales(Es, s1, s2);
+                if (its == HELP) f32_scales(Es, s1, s2);
                 const int E = Es;
                 if (++its == nstages) {
-                    its = 0;
+                    its = HELP;
                     Ls += gridDim.x;
                 }
                 if (!hold && Ls < ntiles) copy();
                 item_planes<FMTA, 0, S>(cur, E, s1, s2, dre);
                 item_planes<FMTA, 1, S>(cur, E, s1, s2, dim);
             };
-            copy();
-            int64_t gs = 0;
+            if (HELP < nstages) copy();
             for (int64_t L = blockIdx.x; L < ntiles; L += gridDim.x, ++tn) {
                 bool quit = false;
-                for (int it = 0; it < nstages; ++it, ++gs) {
+                for (int it = HELP; it < nstages; ++it) {
+                    const int64_t gs = (int64_t)tn * nstages + it;
                     const int bi = (int)(gs & 1);
                     // slice this stage while the MMAs of the two before it run; then wait
                     // only for the buffer and store
@@ -758,7 +767,7 @@ __global__ void __launch_bounds__(tc_threads(S), Class<S>::MIN_CTAS)
                     mbar_arrive(&bar_full[bi]);
                 }
                 if (!epilogue(L, tn)) break;
-                if (!OWN && Ls < ntiles) copy();
+                if (!OWN && HELP < nstages && Ls < ntiles) copy();
             }
             asm volatile("cp.async.wait_all;" ::: "memory");
         }
@@ -815,6 +824,20 @@ __global__ void __launch_bounds__(tc_threads(S), Class<S>::MIN_CTAS)
                 cv = gj < Nc;
                 return t.b * sB + gj;
             };
+            // A's first stage: two (row, 8 k) items a thread
+            auto help_r = [&](int u) { return CONJ_A ? qb : (qb + B_PRODUCERS * u) >> 1; };
+            auto help_g = [&](int u) { return CONJ_A ? u : qb & 1; };
+            int4 help[8];
+            int help_e = ZERO_EXP;
+            auto load_help = [&](const TileId& t, int it, int u) {
+                const int gi = t.rt * TC_TM + help_r(u), ga = help_g(u);
+                const bool rv = gi < M;
+                const int64_t ks = CONJ_A ? lda : 1;
+                help_e = rv ? EA[t.b * M + gi] : ZERO_EXP;
+                const int kf = it * TC_TK + 8 * ga;
+                load8<FMTA>(A, t.b * sA + (CONJ_A ? (int64_t)gi : (int64_t)gi * lda) + kf * ks, ks,
+                            rv ? n_valid(K, kf) : 0, help);
+            };
             int4 nxt[8];
             {
                 bool cv0;
@@ -845,6 +868,7 @@ __global__ void __launch_bounds__(tc_threads(S), Class<S>::MIN_CTAS)
                         const int64_t in = col_base(L + gridDim.x, cvn);
                         load8<FB>(B, in + (int64_t)(8 * g) * ldb, ldb, cvn ? n_valid(K, 8 * g) : 0, nxt);
                     }
+                    if (it < HELP) load_help(t, it, 0);
                     uint4 dre[S], dim[S];
                     item_planes<FB, 0, S>(cur, E, s1, s2, dre);
                     item_planes<FB, 1, S>(cur, E, s1, s2, dim);
@@ -869,8 +893,33 @@ __global__ void __launch_bounds__(tc_threads(S), Class<S>::MIN_CTAS)
                         st_shared_v4(sb + s * PLANE + o_kre, dim[s]);
                         st_shared_v4(sb + s * PLANE + o_jim, neg_bf16x8(dim[s]));
                     }
+                    if (it < HELP) {
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) cur[i] = help[i];
+                            const int Ea = help_e;
+                            if (u == 0) load_help(t, it, 1);
+                            float a1, a2;
+                            f32_scales(Ea, a1, a2);
+                            item_planes<FMTA, 0, S>(cur, Ea, a1, a2, dre);
+                            item_planes<FMTA, 1, S>(cur, Ea, a1, a2, dim);
+                            const int r = help_r(u), ga = help_g(u);
+                            const uint32_t sa = sbase + bi * SB;
+                            const uint32_t o_re = plane_off(r, 8 * ga), o_im = plane_off(r, 16 + 8 * ga);
+#pragma unroll
+                            for (int s = 0; s < S; ++s) {
+                                st_shared_v4(sa + s * PLANE + o_re, dre[s]);
+                                st_shared_v4(sa + s * PLANE + o_im, CONJ_A ? neg_bf16x8(dim[s]) : dim[s]);
+                            }
+                        }
+                    }
                     fence_async_smem();
                     mbar_arrive(&bar_full[bi]);
+                    if (it < HELP) {  // for the two A threads
+                        mbar_arrive(&bar_full[bi]);
+                        mbar_arrive(&bar_full[bi]);
+                    }
                 }
             }
         }
@@ -998,7 +1047,8 @@ template <bool CJ, int FA, int FB, int S>
 static int launch_tc(cudaStream_t st, int64_t batch, int M, int Nc, int K, const void* A, int64_t lda, int64_t sA,
                      const void* B, int64_t ldb, int64_t sB, float4* C, int64_t ldc, int64_t sC, int* EA, int* EB,
                      int* err, const char* name, double work, int accumulate = 0, int* Ecol = nullptr) {
-    auto kern = oz_tc_kernel<CJ, FA, FB, S>;
+    // six stages or more: the B warps slice two of them for A
+    auto kern = K > 5 * TC_TK ? oz_tc_kernel<CJ, FA, FB, S, (S > 3 ? 2 : 0)> : oz_tc_kernel<CJ, FA, FB, S, (S > 3 ? 1 : 0)>;
     constexpr int smem = tc_smem_bytes<S>(FA);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(oz_tc)");
@@ -1188,7 +1238,7 @@ static int fourier_tc_launch(cudaStream_t st, int64_t M, int64_t Nc, int K, cons
                                                                                                         aimg);
         TBG_LAUNCHED("phase_image_kernel");
     }
-    auto kern = oz_tc_kernel<false, FMT_PRESLICED, FMT_PRESLICED, S>;
+    auto kern = oz_tc_kernel<false, FMT_PRESLICED, FMT_PRESLICED, S, 0>;
     const int smem = tc_smem_bytes<S>(FMT_PRESLICED);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(oz_tc fourier)");
