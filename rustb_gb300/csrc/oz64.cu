@@ -5,14 +5,24 @@
 // splitting after Ozaki, Ogita, Oishi and Rump 2012): a row of A (column of B)
 // with |x| < 2^E is written on the grid 2^(E - 55) and cut into seven signed
 // digits of eight bits, which BF16 holds exactly.  Digit pairs of level
-// s + t <= 6 are kept (28 of 49), each level in an FP32 accumulator of its own: a
-// sum of up to 512 products of two digits is below 2^23, and what the last levels
-// may lose is below 2^-60 of the product's scale 2^(EA + EB).  The sums are put
+// s + t <= 6 are kept (28 of 49), each level in an FP32 accumulator of its own.
+// Digits are at most 128, so L + 1 pairs of level L sum to at most (L + 1) 2^15 a
+// complex term: FP32's 2^24 holds levels 0 to 4 exactly over 96 terms, level 0 over
+// 256.  So after every 96 terms at most the levels 4 .. 1 pass what exceeds a digit
+// on to the level before them, in tensor memory and exactly (carry), and after 256
+// the sums are drained and added in FP64.  (All 256 in one go lost the last bits of
+// levels 2 to 4 when the digits were large and their products did not cancel: 10^-9 of
+// the scale.)  Levels 5 and 6 may lose their last place, 2^-54 of the product's scale
+// 2^(EA + EB), but only where the sum itself is some 100 times the scale.  The level sums are put
 // together as 64-bit integers (an FP64 addition costs as much as dozens of integer
 // instructions here) and rounded once to FP64.  The tensor core truncates, so
 // levels with different last places must not share an accumulator early: with
 // levels 4 to 6 in one the error of a 128-term product was 300 x 2^-54 of the
 // scale, against 10 x for an FP64 sum and 6.8 x now.
+//
+// The error is relative to (largest of the line of A) x (largest of the line of B):
+// elements below an eighth of their line's largest keep fewer than 53 bits, where an
+// FP64 sum's error follows the sum of |a| |b|.
 //
 // Shared memory feeds the tensor cores 128 bytes a clock, so an MMA of 128 rows pays
 // 32 clocks for A and 16 per 64 columns of B, against 16 of arithmetic: digit pairs
@@ -66,7 +76,23 @@ constexpr int B_THREADS = TNC * 4;           // (column, half of the 16 k, compo
 constexpr int THREADS = E_THREADS + 2 * B_THREADS + 64;
 constexpr int EPI = E_THREADS / 32 * 32 * 5 * 16;  // 4 columns of 32 rows per warp, rows padded to 5
 constexpr int SMEM = 2 * STAGE + EPI + 1024;
-constexpr int kMaxK = 256;  // complex k that one launch keeps exact
+// How a contraction of nst stages is held exact: up to PLAIN_STAGES as it is; up to
+// SPLIT_STAGES with pair (4, 0) in an eighth accumulator (level 4 then has four pairs
+// in its own: 2^24 over 128 terms); beyond, in groups of at most GROUP stages, each in
+// parts of at most PLAIN_STAGES with a carry between them, cut evenly.  What it costs,
+// against the same kernel without: the 12 products of 128 bands, 1024 k-points (K = 64
+// and 128) 4.94 ms, 4.77; the Fourier sums of 172 pairs there 1.63, 1.35 (2.07 when drained
+// at 96 terms instead of carried).
+enum Form { PLAIN, SPLIT, CARRY };
+constexpr int PLAIN_STAGES = 6, SPLIT_STAGES = 8, GROUP = 16;  // 96, 128 and 256 complex k
+struct Cuts {
+    int group, part;  // stages
+};
+__host__ __device__ __forceinline__ Cuts cuts_of(int nst) {
+    const int groups = (nst + GROUP - 1) / GROUP, group = (nst + groups - 1) / groups;
+    const int parts = (group + PLAIN_STAGES - 1) / PLAIN_STAGES;
+    return {group, (group + parts - 1) / parts};
+}
 // kind::f16: D = F32, A = B = BF16, K-major, M = 128, N = n NR
 __host__ __device__ constexpr uint32_t idesc(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n * NR >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
@@ -162,14 +188,17 @@ __device__ __forceinline__ void ld8(const zc* p, int part, int64_t stride, int n
 }
 
 // The level sums -> their FP64 value times 2^(ea + eb - 2058) (e - 1022 - 7 per operand).
-__device__ __forceinline__ double combine(const uint32_t (&a)[S], int ea, int eb) {
+template <int N>
+__device__ __forceinline__ double combine(const uint32_t (&a)[N], int ea, int eb) {
     if (ea == kNonFinite || eb == kNonFinite) return __longlong_as_double(0x7ff8000000000000ll);
     const float tail = __uint_as_float(a[5]) + __uint_as_float(a[6]);  // below 2^-14
+    int l4 = __float2int_rn(__uint_as_float(a[4]) * 0x1p32f);
+    if (N > S) l4 += __float2int_rn(__uint_as_float(a[N - 1]) * 0x1p32f);  // pair (4, 0)
     const long long I = ((long long)__float2int_rn(__uint_as_float(a[0])) << 39) +
                         ((long long)__float2int_rn(__uint_as_float(a[1]) * 0x1p8f) << 31) +
                         ((long long)__float2int_rn(__uint_as_float(a[2]) * 0x1p16f) << 23) +
                         ((long long)__float2int_rn(__uint_as_float(a[3]) * 0x1p24f) << 15) +
-                        ((long long)__float2int_rn(__uint_as_float(a[4]) * 0x1p32f) << 7) +
+                        ((long long)l4 << 7) +
                         __float2int_rn(tail * 0x1p39f);
     if (I == 0) return 0.0;
     const unsigned long long sg = (unsigned long long)I & 0x8000000000000000ull;
@@ -185,8 +214,8 @@ __device__ __forceinline__ double combine(const uint32_t (&a)[S], int ea, int eb
     return sg ? -r : r;
 }
 
-// C (M x Nc per matrix) = / += / -= A op(B).  A: stage images, nst_img stages per
-// (matrix, row tile), from stage it0 on.  Element (k, j) of op(B) is at
+// C (M x Nc per matrix) = / += / -= A op(B).  A: stage images per (matrix, row
+// tile).  Element (k, j) of op(B) is at
 // B + b sB + k bk + j bj (conjugated when conjB); PRE: B is images too, per column
 // tile.  EA, EB: line exponents per (matrix, row) and (matrix, column).
 struct OzArgs {
@@ -203,7 +232,6 @@ struct OzArgs {
     int wait_limit;
     int gx, gy, rows_fast;
     int64_t ntiles;
-    int it0, nst_img;
 };
 
 struct Tile {
@@ -236,7 +264,29 @@ __device__ __forceinline__ void tmem_ld2(uint32_t taddr, uint32_t& a, uint32_t& 
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0,%1}, [%2];" : "=r"(a), "=r"(b) : "r"(taddr));
 }
 
-template <bool PRE>
+// Levels 4 .. 1 of 8 columns: what exceeds half a place of the level before goes
+// there, that of level 1 first, so that no level holds more than a digit when it
+// receives (level L counts in 2^(-8 L); |level| < 2^24 of that).
+__device__ __forceinline__ void carry_levels(uint32_t taddr) {
+    uint32_t v[5][8];
+#pragma unroll
+    for (int lv = 0; lv < 5; ++lv) tmem_ld8(taddr + (uint32_t)(lv * NR), v[lv]);
+    tmem_wait_ld();
+#pragma unroll
+    for (int lv = 1; lv < 5; ++lv) {
+        const float C = lv == 1 ? 0x1.8p23f : lv == 2 ? 0x1.8p15f : lv == 3 ? 0x1.8p7f : 0x1.8p-1f;  // 1.5 2^(31 - 8 lv)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float x = __uint_as_float(v[lv][i]), c = __fsub_rn(__fadd_rn(x, C), C);
+            v[lv - 1][i] = __float_as_uint(__fadd_rn(__uint_as_float(v[lv - 1][i]), c));
+            v[lv][i] = __float_as_uint(__fsub_rn(x, c));
+        }
+    }
+#pragma unroll
+    for (int lv = 0; lv < 5; ++lv) tmem_st8(taddr + (uint32_t)(lv * NR), v[lv]);
+}
+
+template <bool PRE, int FORM>
 __global__ void __launch_bounds__(THREADS, 1) oz64_kernel(OzArgs p) {
     extern __shared__ __align__(1024) unsigned char oz_smem[];
     unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)oz_smem + 1023) & ~(uintptr_t)1023);
@@ -246,6 +296,7 @@ __global__ void __launch_bounds__(THREADS, 1) oz64_kernel(OzArgs p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int MMA_WARP = THREADS / 32 - 1, COPY_WARP = MMA_WARP - 1;
     const int nst = (p.K + TK - 1) / TK;
+    const Cuts cut = FORM == CARRY ? cuts_of(nst) : Cuts{nst, nst};
     const uint32_t sbase = su32(base);
     if (tid == 0) {
         const uint32_t nfull = PRE ? 1 : 1 + B_THREADS;
@@ -267,19 +318,23 @@ __global__ void __launch_bounds__(THREADS, 1) oz64_kernel(OzArgs p) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_sh;
-    int ndone = 0;  // tiles committed to bar_done
+    int ndone = 0;  // parts committed to bar_done
 
     if (warp == MMA_WARP) {
         if (lane == 0) {
             int tn = 0;
-            for (int64_t L = blockIdx.x; L < p.ntiles; L += gridDim.x, ++tn) {
-                if (tn > 0 && !mbar_wait(&bar_tmem, (tn - 1) & 1, &abort_sh, p.wait_limit)) {
-                    abort_sh = 1;
-                    break;
-                }
-                tc_fence_after();
-                bool stop = false;
-                for (int it = 0; it < nst; ++it) {
+            bool stop = false, open = false;  // open: MMAs issued behind the last commit to bar_done
+            for (int64_t L = blockIdx.x; L < p.ntiles && !stop; L += gridDim.x, ++tn) {
+                for (int it = 0, ig = 0, ip = 0; it < nst; ++it) {  // ig, ip: stage of the group, of the part
+                    // the accumulators have been read out, or have carried
+                    if (ip == 0 && ndone > 0) {
+                        if (!mbar_wait(&bar_tmem, (uint32_t)((ndone - 1) & 1), &abort_sh, p.wait_limit)) {
+                            abort_sh = 1;
+                            stop = true;
+                            break;
+                        }
+                        tc_fence_after();
+                    }
                     const int64_t gs = (int64_t)tn * nst + it;
                     const int bi = (int)(gs & 1);
                     if (!mbar_wait(&bar_full[bi], (uint32_t)((gs >> 1) & 1), &abort_sh, p.wait_limit)) {
@@ -288,27 +343,40 @@ __global__ void __launch_bounds__(THREADS, 1) oz64_kernel(OzArgs p) {
                         break;
                     }
                     tc_fence_after();
+                    open = true;
                     const uint32_t sa = sbase + bi * STAGE, sb = sa + ABYTES;
 #pragma unroll
                     for (int ks = 0; ks < 2; ++ks) {
 #pragma unroll
                         for (int s = 0; s < S; ++s) {
                             const uint64_t ad = smem_desc(sa + s * APLANE + ks * (APLANE / 2), 128, 256);
-#pragma unroll
-                            for (int t = 0; t < S - s; t += 4) {
-                                const int n = S - s - t < 4 ? S - s - t : 4;  // pairs (s, t) .. (s, t + n - 1)
+                            // pairs (s, t) .. (s, t + n - 1) into the accumulators from `to` on
+                            auto pairs = [&](int t, int n, int to) {
                                 const uint64_t bd = smem_desc(sb + ks * BKS + t * BBLK, 128, 256);
                                 // digit 0 of A meets every level first
-                                const uint32_t acc = (it == 0 && ks == 0 && s == 0) ? 0u : 1u;
-                                mma(tmem + (uint32_t)((s + t) * NR), ad, bd, idesc(n), acc);
-                            }
+                                const uint32_t acc = (ig == 0 && ks == 0 && (s == 0 || to == S)) ? 0u : 1u;
+                                mma(tmem + (uint32_t)(to * NR), ad, bd, idesc(n), acc);
+                            };
+                            const bool apart = FORM == SPLIT && s == 4;
+                            if (apart) pairs(0, 1, S);
+#pragma unroll
+                            for (int t = apart ? 1 : 0; t < S - s; t += 4) pairs(t, S - s - t < 4 ? S - s - t : 4, s + t);
                         }
                     }
                     umma_commit(&bar_empty[bi]);
+                    ++ig;
+                    if (++ip == cut.part || ig == cut.group || it + 1 == nst) {
+                        umma_commit(&bar_done);
+                        ++ndone;
+                        open = false;
+                        ip = 0;
+                        if (ig == cut.group) ig = 0;
+                    }
                 }
+            }
+            if (open) {  // an abort: the part before has been read, so the wait below meets this commit
                 umma_commit(&bar_done);
                 ++ndone;
-                if (stop) break;
             }
         }
         __syncwarp();
@@ -320,9 +388,8 @@ __global__ void __launch_bounds__(THREADS, 1) oz64_kernel(OzArgs p) {
             bool stop = false;
             for (int64_t L = blockIdx.x; L < p.ntiles && !stop; L += gridDim.x, ++tn) {
                 const Tile t = tile_at(p, L);
-                const unsigned char* ia = p.A + ((t.b * nrt + t.rt) * p.nst_img + p.it0) * ABYTES;
-                const unsigned char* ib =
-                    static_cast<const unsigned char*>(p.B) + ((int64_t)t.ct * p.nst_img + p.it0) * BBYTES;
+                const unsigned char* ia = p.A + (t.b * nrt + t.rt) * nst * ABYTES;
+                const unsigned char* ib = static_cast<const unsigned char*>(p.B) + (int64_t)t.ct * nst * BBYTES;
                 for (int it = 0; it < nst; ++it) {
                     const int64_t gs = (int64_t)tn * nst + it;
                     const int bi = (int)(gs & 1);
@@ -350,46 +417,64 @@ __global__ void __launch_bounds__(THREADS, 1) oz64_kernel(OzArgs p) {
         constexpr int CW = TNC / (E_THREADS / 128);
         const uint32_t taddr = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(CW * h);
         double2* epi = reinterpret_cast<double2*>(base + 2 * STAGE) + warp * (32 * 5);
-        int tn = 0;
-        for (int64_t L = blockIdx.x; L < p.ntiles; L += gridDim.x, ++tn) {
+        int u = 0;  // parts so far
+        auto part_done = [&]() {  // whether the MMAs of part u are done; a group is written whole or not at all
+            bool bad = abort_sh != 0;
+            if (!bad && !mbar_wait(&bar_done, u & 1, &abort_sh, p.wait_limit)) {
+                abort_sh = 1;
+                bad = true;
+            }
+            ++u;
+            if (any_epilogue(bad)) return false;
+            tc_fence_after();
+            return true;
+        };
+        auto release = [&]() {  // the accumulators may be written again
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar_tmem);
+        };
+        int g0 = 0;  // first stage of the group (CARRY; the others have one)
+        for (int64_t L = blockIdx.x; L < p.ntiles; L += FORM == CARRY && g0 ? 0 : gridDim.x) {
+            const int glen = min(cut.group, nst - g0);
+            const int mode = FORM == CARRY && g0 ? (p.mode < 0 ? -1 : 1) : p.mode;
+            if constexpr (FORM == CARRY) g0 = g0 + glen < nst ? g0 + glen : 0;
             const Tile t = tile_at(p, L);
             const int row = t.rt * TM + 32 * q + lane;
             const int ea = row < p.M ? p.EA[t.b * p.M + row] : 1;
             const int col0 = t.ct * TNC + CW * h;
             const int* EBt = p.EB + t.b * p.Nc;
-            // a tile is written whole or not at all
-            bool bad = abort_sh != 0;
-            if (!bad && !mbar_wait(&bar_done, tn & 1, &abort_sh, p.wait_limit)) {
-                abort_sh = 1;
-                bad = true;
+            if constexpr (FORM == CARRY) {
+                bool go = true;
+                for (int i = cut.part; i < glen && (go = part_done()); i += cut.part) {
+                    carry_levels(taddr);
+                    carry_levels(taddr + TNC);
+                    tmem_wait_st();
+                    release();
+                }
+                if (!go) break;
             }
-            if (any_epilogue(bad)) break;
-            tc_fence_after();
+            if (!part_done()) break;
             zc* Cb = p.C + t.b * p.sC;
             if (t.rt * TM + 32 * q >= p.M || col0 >= p.Nc) {  // nothing of the tile in this warp
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bar_tmem);
+                release();
                 continue;
             }
 #pragma unroll 1
             for (int c0 = 0; c0 < CW; c0 += 4) {
 #pragma unroll
                 for (int c2 = 0; c2 < 4; c2 += 2) {
-                    uint32_t x0[S], x1[S], y0[S], y1[S];
+                    constexpr int NA = FORM == SPLIT ? S + 1 : S;
+                    uint32_t x0[NA], x1[NA], y0[NA], y1[NA];
 #pragma unroll
-                    for (int lv = 0; lv < S; ++lv) {
+                    for (int lv = 0; lv < NA; ++lv) {
                         tmem_ld2(taddr + (uint32_t)(lv * NR + c0 + c2), x0[lv], x1[lv]);
                         tmem_ld2(taddr + (uint32_t)(lv * NR + TNC + c0 + c2), y0[lv], y1[lv]);
                     }
                     const int j = col0 + c0 + c2;
                     const int e0 = j < p.Nc ? EBt[j] : 1, e1 = j + 1 < p.Nc ? EBt[j + 1] : 1;
                     tmem_wait_ld();
-                    if (c0 + 4 >= CW && c2 == 2) {  // the accumulators are in registers: the next tile may have them
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(&bar_tmem);
-                    }
+                    if (c0 + 4 >= CW && c2 == 2) release();  // all of them are in registers
                     epi[lane * 5 + c2] = make_double2(combine(x0, ea, e0), combine(y0, ea, e0));
                     epi[lane * 5 + c2 + 1] = make_double2(combine(x1, ea, e1), combine(y1, ea, e1));
                 }
@@ -402,9 +487,9 @@ __global__ void __launch_bounds__(THREADS, 1) oz64_kernel(OzArgs p) {
                     if (gi < p.M && j < p.Nc) {
                         double2 v = epi[rl * 5 + c];
                         double2* dst = reinterpret_cast<double2*>(Cb + gi * p.ldc + j);
-                        if (p.mode) {
+                        if (mode) {
                             const double2 o = *dst;
-                            v = p.mode > 0 ? make_double2(o.x + v.x, o.y + v.y) : make_double2(o.x - v.x, o.y - v.y);
+                            v = mode > 0 ? make_double2(o.x + v.x, o.y + v.y) : make_double2(o.x - v.x, o.y - v.y);
                         }
                         *dst = v;
                     }
@@ -562,7 +647,10 @@ inline unsigned blocks(int64_t n) { return (unsigned)std::max<int64_t>(1, std::m
 
 template <bool PRE>
 int launch(cudaStream_t st, OzArgs p, int64_t batch, int rows_fast) {
-    auto kern = oz64_kernel<PRE>;
+    const int nst = (p.K + TK - 1) / TK;
+    auto kern = nst <= PLAIN_STAGES   ? oz64_kernel<PRE, PLAIN>
+                : nst <= SPLIT_STAGES ? oz64_kernel<PRE, SPLIT>
+                                      : oz64_kernel<PRE, CARRY>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(oz64)");
     const int nr = (p.M + TM - 1) / TM, nc = (p.Nc + TNC - 1) / TNC;
@@ -625,14 +713,10 @@ int oz64_gemm(cudaStream_t st, int64_t batch, int M, int Nc, int K, const Oz64Op
         p.ldc = ldc;
         p.sC = sC;
         p.err = err;
-        p.nst_img = (K + TK - 1) / TK;
-        for (int k0 = 0; k0 < K && !rc; k0 += kMaxK) {
-            p.K = std::min(kMaxK, K - k0);
-            p.it0 = k0 / TK;
-            p.B = B.p + b0 * B.batch + k0 * B.k;
-            p.mode = k0 ? (mode < 0 ? -1 : 1) : mode;
-            rc = launch<false>(st, p, nb, 0);
-        }
+        p.K = K;
+        p.B = B.p + b0 * B.batch;
+        p.mode = mode;
+        if (!rc) rc = launch<false>(st, p, nb, 0);
     }
     cudaFreeAsync(img, st);
     return rc;
@@ -674,15 +758,9 @@ int oz64_table_product(cudaStream_t st, int64_t M, int64_t Nc, int Kc, const zc*
     p.C = C;
     p.ldc = Nc;
     p.err = err;
-    p.nst_img = nst;
-    for (int k0 = 0; k0 < Kc; k0 += kMaxK) {
-        p.K = std::min(kMaxK, Kc - k0);
-        p.it0 = k0 / TK;
-        p.mode = k0 ? 1 : 0;
-        // row tiles fastest: CTAs running together share a column tile's image in L2
-        if (int rc = launch<true>(st, p, 1, 1)) return rc;
-    }
-    return TBG_OK;
+    p.K = Kc;
+    // row tiles fastest: CTAs running together share a column tile's image in L2
+    return launch<true>(st, p, 1, 1);
 }
 
 }  // namespace tbg
