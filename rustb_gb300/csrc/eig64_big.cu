@@ -175,9 +175,8 @@ __global__ void __launch_bounds__(kThreads) panel64_kernel(int N, int j0, int st
                 s_beta = beta;
             }
         }
-        // q = A a without the first column, partial [V W]^H a without the first row;
-        // kRows own rows at a time
-        zc gh = mk(0.0, 0.0);
+        // q = A a without the first column, kRows own rows at a time by whichever warp is
+        // free: a row's sum does not depend on who takes it
         const bool on = (lane & (kNB - 1)) < i;
         for (;;) {
             int g = 0;
@@ -194,16 +193,17 @@ __global__ void __launch_bounds__(kThreads) panel64_kernel(int N, int j0, int st
 #pragma unroll
                 for (int k = 0; k < kRows; ++k) fma_cx(acc[k], row[k][c], x);
             }
-            if (on) {
-#pragma unroll
-                for (int k = 0; k < kRows; ++k) {
-                    const int r = r0 + C * (g + k);
-                    if (g + k < nrows && r > f) fma_cjx(gh, P[(size_t)r * kPW + lane], sa[r - f]);
-                }
-            }
             const zc q = warp_sums<kRows>(acc, lane);
             if (lane < kRows && g + lane < nrows) sq[g + lane] = q;
         }
+        // partial [V W]^H a without the first row: a sum over rows, which are dealt out
+        // in a fixed order so that a call's results are the same every time
+        zc gh = mk(0.0, 0.0);
+        if (on)
+            for (int t = warp; t < nrows; t += kWarps) {
+                const int r = r0 + C * t;
+                if (r > f) fma_cjx(gh, P[(size_t)r * kPW + lane], sa[r - f]);
+            }
         s_part[warp][lane] = gh;
         __syncthreads();
         // p = A v, v = (1, scal a); publish p, [V W]^H v and v^H p of the own rows
