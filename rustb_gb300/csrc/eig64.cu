@@ -881,20 +881,6 @@ int sm_count() {
     return n;
 }
 
-// The dynamic shared-memory limit is an attribute of the function, shared by
-// every host thread: it is set to the device's opt-in maximum.
-template <typename K>
-int allow_smem(K kern, size_t need) {
-    if (need <= 48 * 1024) return TBG_OK;
-    int dev = 0, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (need > (size_t)optin) return set_error(TBG_E_UNSUPPORTED, "FP64 eigensolver: shared memory beyond the limit");
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-    if (e != cudaSuccess) return cuda_error(e, "cudaFuncSetAttribute(eig64)");
-    return TBG_OK;
-}
-
 constexpr size_t kSmemCta = 226 * 1024;
 
 int cta_threads(int N) { return N <= 64 ? 128 : (N <= 112 ? 256 : 512); }

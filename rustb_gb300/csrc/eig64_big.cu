@@ -501,7 +501,7 @@ int hetrd64_big(cudaStream_t st, int N, int64_t batch, zc* A, int* status_d) {
     auto smem_of = [&](int c) { return sizeof(zc) * ((size_t)N + 2 * ((N + c - 1) / c)); };
     for (;; --C) {
         const size_t smem = smem_of(C);
-        TBG_CUDA(cudaFuncSetAttribute(panel64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (int r = allow_smem(panel64_kernel, smem)) return r;
         cfg.dynamicSmemBytes = smem;
         cfg.gridDim = dim3((unsigned)(batch * C));
         at[0].val.clusterDim.x = C;

@@ -847,8 +847,7 @@ int mixed_berry(cudaStream_t st, int N, int64_t batch, const float4* H, const fl
     {
         KTimer kt(st, "oa_kernel");
         const size_t smem = oa_smem_bytes(N);
-        cudaError_t ea = cudaFuncSetAttribute(oa_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (ea != cudaSuccess) return cuda_error(ea, "cudaFuncSetAttribute(oa_kernel)");
+        if ((rc = allow_smem(oa_pairs_kernel, smem))) return rc;
         TBG_CUDA(cudaMemsetAsync(clist, 0, sizeof(unsigned long long), st));
         oa_pairs_kernel<<<(unsigned)std::min<int64_t>(batch, 152 * 8), 256, smem, st>>>(
             N, batch, bA, bC, E, F, clusters_d, cinfo, Fcl, tc ? slot(FC) : nullptr, clist);

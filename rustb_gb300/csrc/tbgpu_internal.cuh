@@ -229,6 +229,24 @@ void timing_flush();  // resolve recorded event pairs (after a stream sync)
         if (_e != cudaSuccess) return cuda_error(_e, where);        \
     } while (0)
 
+// The dynamic shared-memory limit is an attribute of the function, shared by every
+// host thread: it is set to what the device allows beside the kernel's static
+// memory, never to one call's need (a smaller concurrent call would lower it under
+// the launches of a larger one).
+template <typename K>
+int allow_smem(K kern, size_t need) {
+    if (need <= 32 * 1024) return TBG_OK;  // with static memory, below the 48 KB that need no permission
+    int dev = 0, optin = 0;
+    cudaFuncAttributes fa;
+    TBG_CUDA(cudaGetDevice(&dev));
+    TBG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    TBG_CUDA(cudaFuncGetAttributes(&fa, kern));
+    const int most = optin - (int)fa.sharedSizeBytes;
+    if (need > (size_t)most) return set_error(TBG_E_UNSUPPORTED, "shared memory beyond the device limit");
+    TBG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    return TBG_OK;
+}
+
 // ---------------------------------------------------------- kernel drivers --
 // Fourier sum, direct form: for nk k-points (device k, (nk, dim)), outputs
 // H (nk, N, N) (may be null) and V (nk, nproj, N, N) (may be null when
