@@ -260,10 +260,16 @@ __global__ void __launch_bounds__(64) small_fused_kernel(
     if (VALS) {
         double E[NM];
         if constexpr (EXACT && NM == 2) {
-            const double m = 0.5 * (H[0][0].re + H[1][1].re), d = 0.5 * (H[0][0].re - H[1][1].re);
-            const double h = sqrt(fma(d, d, abs2(H[0][1])));
-            E[0] = m - h;
-            E[1] = m + h;
+            const double a = H[0][0].re, b = H[1][1].re, off = 2.0 * abs2(H[0][1]);
+            E[0] = a > b ? b : a;
+            E[1] = a > b ? a : b;
+            // coupled above the rounding of the diagonal, by the test of jacobi() (its squares
+            // out of range leave the diagonal as well)
+            if (!(off <= 1e-32 * fma(a, a, b * b) || off == 0.0)) {
+                const double m = 0.5 * (a + b), d = 0.5 * (a - b), h = sqrt(fma(d, d, 0.5 * off));
+                E[0] = m - h;
+                E[1] = m + h;
+            }
         } else {
 #pragma unroll
             for (int i = 1; i < N; ++i)
