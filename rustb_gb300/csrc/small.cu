@@ -186,10 +186,13 @@ __global__ void __launch_bounds__(64) small_fused_kernel(
     __syncthreads();
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= nk) return;
-    double kv[3] = {0.0, 0.0, 0.0};
+    double kv[3] = {0.0, 0.0, 0.0}, nan = 0.0;  // nan: NaN unless k is finite, also where no R reaches along an axis
     zc z[3];
     if (klist) {
-        for (int d = 0; d < dim; ++d) kv[d] = klist[t * dim + d];
+        for (int d = 0; d < dim; ++d) {
+            kv[d] = klist[t * dim + d];
+            nan = fma(0.0, kv[d], nan);
+        }
     } else {
         const int64_t idx = k0 + t;  // gen_kmesh order (src/kpoints.rs:49-87), n1 = n2 = 1 beyond dim
         int64_t i0, i1, i2;
@@ -219,6 +222,7 @@ __global__ void __launch_bounds__(64) small_fused_kernel(
         for (int d = 0; d < 3; ++d) {
             z[d] = mk(1.0, 0.0);
             if (d < dim) sincospi(2.0 * kv[d], &z[d].im, &z[d].re);
+            z[d].re += nan;
         }
     }
     zc H[NM][NM], V0[NM][NM], V1[NM][NM];
@@ -228,7 +232,7 @@ __global__ void __launch_bounds__(64) small_fused_kernel(
         for (int j = 0; j < NM; ++j) H[i][j] = V0[i][j] = V1[i][j] = mk(0.0, 0.0);
     for (int r = 0; r < nR; ++r) {
         const int* R = s_R + 3 * r;
-        zc u = mk(1.0, 0.0);
+        zc u = mk(1.0 + nan, 0.0);
         bool one = true;
         times_power(u, one, z[0], R[0]);
         if (dim > 1) times_power(u, one, z[1], R[1]);

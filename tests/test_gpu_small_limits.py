@@ -1,9 +1,10 @@
 """Small models at the limits of their fused path: entries near the ends of FP64's
-range and decoupled bands (GPU)."""
+range, decoupled bands, k-points that are not finite (GPU)."""
 
 import numpy as np
 import pytest
 
+from rustb_gb300 import Parameters
 from rustb_gb300.model import Model
 
 pytestmark = pytest.mark.gpu
@@ -31,3 +32,13 @@ def test_two_bands_match_the_closed_form():
         E = chain([d, -d], h).solve_band_mesh((3, 2)).reshape(-1, 2)
         r = np.hypot(d, h)
         assert np.max(np.abs(E - np.array([-r, r]))) <= 4 * np.finfo(float).eps * r
+
+
+@pytest.mark.parametrize("k", [[0.1, np.nan], [0.1, np.inf], [np.nan, 0.2]])
+def test_k_points_that_are_not_finite_give_no_numbers(k):
+    """Also along an axis that no hopping uses."""
+    m = chain([0.5, -0.5], 0.2)
+    p = Parameters.rank2((1, 1), [1.0, 0.0], [0.0, 1.0], [0.0])
+    Om, E = m.berry_curvature_on(np.array([k, [0.1, 0.2]]), p)
+    assert not np.any(np.isfinite(E[0])) and not np.any(np.isfinite(Om[0]))
+    assert np.all(np.isfinite(E[1])) and np.all(np.isfinite(Om[1]))
