@@ -564,6 +564,8 @@ __global__ void __launch_bounds__(512) tri64_kernel(int N, int64_t batch, int MP
                     }
                     const double g = qt + raw - (s.d[r] - x);
                     const double n2 = 1.0 + st + sum;
+                    // ratios that outgrow the range would pass for convergence (g / n2 = 0)
+                    if (hi_abs(n2) >= 0x7ff00000) break;
                     const double cor = g / n2;
                     x += cor;
                     if (!(fabs(x - (double)x0) <= kReach)) break;
