@@ -68,11 +68,24 @@ __device__ __forceinline__ void reflector64(const zc* row, int m, int lane, zc* 
     double part = 0.0;
     for (int i = lane; i < m; i += 32)
         if (i > 0) part += abs2(row[i]);
-    const double xn = wsum(part);
-    zc scal;
-    reflector_scalars64(conj(row[0]), xn, tau, scal, beta);
+    const Reflector64 r = reflector64_of(conj(row[0]), wsum(part), [&](double up) {
+        double p = 0.0;
+        for (int i = lane; i < m; i += 32)
+            if (i > 0) p += abs2(up * row[i]);
+        return wsum(p);
+    });
+    tau = r.tau;
+    beta = r.beta;
+    if (r.far) {
+        for (int i = lane; i < m; i += 32) {
+            const zc vi = (i == 0) ? mk(1.0, 0.0) : (r.up * conj(row[i])) * r.scal;
+            sv[i] = vi;
+            gv[i] = vi;
+        }
+        return;
+    }
     for (int i = lane; i < m; i += 32) {
-        const zc vi = (i == 0) ? mk(1.0, 0.0) : conj(row[i]) * scal;
+        const zc vi = (i == 0) ? mk(1.0, 0.0) : conj(row[i]) * r.scal;
         sv[i] = vi;
         gv[i] = vi;
     }
@@ -757,8 +770,9 @@ __global__ void __launch_bounds__(32) tri64_cluster_kernel(int N, int64_t batch,
         const int ex = (tn > 0.0 && tn < INFINITY) ? ilogb(tn) : 0;
         __syncwarp();
         for (int k = lane; k < N; k += 32) {
+            const double ek = scalbn(e[k], -ex);
             d[k] = scalbn(d[k], -ex);
-            e[k] = scalbn(e[k], -ex);
+            e[k] = hi_abs(ek) < 0x04000000 ? 0.0 : ek;  // 2^-959: a pivot of tri_solve64 has its reciprocal
             lam[k] = scalbn(lam[k], -ex);
         }
         tn = scalbn(tn, -ex);

@@ -27,34 +27,46 @@ __device__ __forceinline__ double flip_if(double x, bool f) {
 }
 __device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
 
-// Reflector H = I - tau v v^H, v = (1, scal x_1, ...), of a column with first
+// Reflector H = I - tau v v^H, v = (1, scal up x_1, ...), of a column with first
 // entry alpha and xn = sum of |x_i|^2 over the others: H^H x = beta e_0, beta real.
-__device__ __forceinline__ void reflector_scalars64(zc alpha, double xn, zc& tau, zc& scal, double& beta) {
-    if (xn == 0.0 && alpha.im == 0.0) {
-        tau = mk(0.0, 0.0);
-        scal = mk(0.0, 0.0);
-        beta = alpha.re;
-        return;
+// A column whose squares leave the range is taken times up = 2^900 or 2^-600
+// (rescaled(up): the sum of |up x_i|^2, by the same threads), else H would not be
+// unitary: the columns of a rank-deficient matrix fall by 10^16 a step, and vectors were
+// off by up to 10^-2 where one fell to 10^-160.
+struct Reflector64 {
+    zc tau, scal;
+    double beta, up;
+    bool far;  // up != 1
+};
+template <typename F>
+__device__ __forceinline__ Reflector64 reflector64_of(zc alpha, double xn, F rescaled) {
+    Reflector64 r;
+    r.up = 1.0;
+    double n2 = fma(alpha.re, alpha.re, fma(alpha.im, alpha.im, xn));
+    r.far = (unsigned)(__double2hiint(n2) - 0x05d00000) >= 0x74400000u;  // outside [2^-930, 2^930)
+    if (r.far) {
+        r.up = n2 < 1.0 ? 0x1p900 : 0x1p-600;
+        alpha = r.up * alpha;
+        xn = rescaled(r.up);
+        n2 = fma(alpha.re, alpha.re, fma(alpha.im, alpha.im, xn));
     }
-    const double n2 = fma(alpha.re, alpha.re, fma(alpha.im, alpha.im, xn));
-    if (n2 > 1e-280 && n2 < 1e280) {
+    if (xn == 0.0 && alpha.im == 0.0) {
+        r.tau = r.scal = mk(0.0, 0.0);
+        r.beta = alpha.re;
+    } else {
         const double y = fast_rsqrt(n2);
         double nrm = n2 * y;
         nrm = fma(fma(-nrm, nrm, n2), 0.5 * y, nrm);
         const bool neg = __double2hiint(alpha.re) >= 0;  // beta opposite in sign to Re(alpha)
-        beta = flip_if(nrm, neg);
+        r.beta = flip_if(nrm, neg);
         const double ib = flip_if(y, neg);
-        const double dr = alpha.re - beta;
-        tau = mk(-dr * ib, -alpha.im * ib);
-        const double r = fast_rcp(fma(dr, dr, alpha.im * alpha.im));
-        scal = mk(dr * r, -alpha.im * r);
-    } else {
-        const double nrm = sqrt(n2);
-        beta = (alpha.re >= 0.0) ? -nrm : nrm;
-        tau = mk((beta - alpha.re) / beta, -alpha.im / beta);
-        const double dr = alpha.re - beta, dd = dr * dr + alpha.im * alpha.im;
-        scal = mk(dr / dd, -alpha.im / dd);
+        const double dr = alpha.re - r.beta;
+        r.tau = mk(-dr * ib, -alpha.im * ib);
+        const double q = fast_rcp(fma(dr, dr, alpha.im * alpha.im));
+        r.scal = mk(dr * q, -alpha.im * q);
     }
+    if (r.far) r.beta *= r.up > 1.0 ? 0x1p-900 : 0x1p600;
+    return r;
 }
 
 // Reduction by a cluster of CTAs per matrix (eig64_big.cu); a column stays in

@@ -109,6 +109,11 @@ __device__ __forceinline__ double sum_published(const double* x, int C, int lane
     return v[0];
 }
 
+// Matrices whose largest entry lies beyond 2^-300 or 2^300 are reduced times a power
+// of two that brings it to 1 (products of their entries would leave the range); n: the
+// exponent field of the largest entry, 0x7ff for NaN and Inf.
+__device__ __forceinline__ int reduced_exp(int n) { return n == 0x7ff || (n >= 723 && n <= 1323) ? n : 1023; }
+
 // One panel: columns j0 .. j0 + steps - 1 of every matrix.  Writes the reflectors,
 // (d, e) and tau into A as hetrd64 does, and P = [V | W], Q = [W | V] (N x kPW),
 // with V times and W over a power of two near the root of A's largest entry
@@ -124,8 +129,8 @@ __global__ void __launch_bounds__(kThreads) panel64_kernel(int N, int j0, int st
     zc* A = Ain + b * (int64_t)N * N;
     zc* P = Pin + b * (int64_t)N * kPW;
     zc* Q = Qin + b * (int64_t)N * kPW;
-    const int half = (nexp[b] - 1022) / 2;
-    const double up = scalbn(1.0, half), down = scalbn(1.0, -half);
+    const int half = (reduced_exp(nexp[b]) - 1022) / 2;
+    const double vscale = scalbn(1.0, half), wscale = scalbn(1.0, -half);
     const Exchange X = exchange_of(xin + b * xbytes, N, C);
     extern __shared__ __align__(16) unsigned char smem_p[];
     zc* sa = reinterpret_cast<zc*>(smem_p);  // (N) column below the diagonal
@@ -134,7 +139,7 @@ __global__ void __launch_bounds__(kThreads) panel64_kernel(int N, int j0, int st
     __shared__ zc s_part[kWarps][kPW];       // partial [V W]^H a per warp
     __shared__ zc s_mul[kPW], s_row[kPW];    // coefficients of V, W; the next row of [W V]
     __shared__ zc s_scal, s_tau, s_u1;
-    __shared__ double s_beta, s_ca, s_d;
+    __shared__ double s_beta, s_ca, s_d, s_up;
     __shared__ int s_next;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     auto first_own = [&](int r) { return r + ((rank - r) % C + C) % C; };  // own row at or after r
@@ -165,14 +170,18 @@ __global__ void __launch_bounds__(kThreads) panel64_kernel(int N, int j0, int st
         if (warp == 0) {
             // reflector of the column: H^H x = beta e_0 with beta real
             const double xn = sum_published(X.norm, C, lane);
+            const Reflector64 r = reflector64_of(sa[0], xn, [&](double up) {
+                double p = 0.0;
+                for (int t = 1 + lane; t < N - f; t += 32) p += abs2(up * sa[t]);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+                return p;
+            });
             if (lane == 0) {
-                const zc alpha = sa[0];
-                zc tau, scal;
-                double beta;
-                reflector_scalars64(alpha, xn, tau, scal, beta);
-                s_tau = tau;
-                s_scal = scal;
-                s_beta = beta;
+                s_tau = r.tau;
+                s_scal = r.scal;
+                s_beta = r.beta;
+                s_up = r.up;
             }
         }
         // q = A a without the first column, kRows own rows at a time by whichever warp is
@@ -206,15 +215,16 @@ __global__ void __launch_bounds__(kThreads) panel64_kernel(int N, int j0, int st
             }
         s_part[warp][lane] = gh;
         __syncthreads();
-        // p = A v, v = (1, scal a); publish p, [V W]^H v and v^H p of the own rows
+        // p = A v, v = (1, scal up a); publish p, [V W]^H v and v^H p of the own rows
         double s = 0.0;
         const zc scal = s_scal;
+        const double up = s_up;
         for (int t = tid; t < nrows; t += kThreads) {
             const int r = r0 + C * t;
             zc p = A[(size_t)r * N + f];
             if (r == f) p.im = 0.0;
-            fma_cx(p, scal, sq[t]);
-            const zc v = r == f ? mk(1.0, 0.0) : scal * sa[r - f];
+            fma_cx(p, scal, up * sq[t]);
+            const zc v = r == f ? mk(1.0, 0.0) : scal * (up * sa[r - f]);
             sq[t] = p;
             X.p[r] = p;
             s += fma(v.re, p.re, v.im * p.im);
@@ -227,7 +237,7 @@ __global__ void __launch_bounds__(kThreads) panel64_kernel(int N, int j0, int st
             zc part[kWarps];
 #pragma unroll
             for (int w = 0; w < kWarps; ++w) part[w] = s_part[w][lane];
-            zc t = scal * pair_sum(part);
+            zc t = scal * (up * pair_sum(part));
             if (r0 == f && on) t = t + conj(P[(size_t)f * kPW + lane]);
             X.gh[rank * kPW + lane] = t;
         }
@@ -310,10 +320,10 @@ __global__ void __launch_bounds__(kThreads) panel64_kernel(int N, int j0, int st
         double nrm = 0.0;
         for (int t = tid; t < nrows; t += kThreads) {
             const int r = r0 + C * t;
-            const zc v = r == f ? mk(1.0, 0.0) : scal * sa[r - f];
+            const zc v = r == f ? mk(1.0, 0.0) : scal * (up * sa[r - f]);
             zc u = tau * sq[t];
             u = mk(fma(ca, v.re, u.re), fma(ca, v.im, u.im));
-            const zc vs = up * v, us = down * u;
+            const zc vs = vscale * v, us = wscale * u;
             P[(size_t)r * kPW + i] = vs;
             P[(size_t)r * kPW + kNB + i] = us;
             Q[(size_t)r * kPW + i] = us;
@@ -369,6 +379,21 @@ __global__ void __launch_bounds__(256) mirror64_kernel(int N, int64_t batch, zc*
                 M[(size_t)r2 * N + c2] = mk(v.re, 0.0);
         }
         __syncthreads();
+    }
+}
+
+// Matrices out of range: all entries before the reduction, the diagonal (d, e) after it.
+__global__ void __launch_bounds__(256) rescale64_kernel(int N, int64_t batch, zc* __restrict__ A,
+                                                        const int* __restrict__ nexp, bool back) {
+    for (int64_t b = blockIdx.y; b < batch; b += gridDim.y) {
+        const int sh = reduced_exp(nexp[b]) - nexp[b];
+        if (sh == 0) continue;
+        zc* M = A + b * (int64_t)N * N;
+        const int64_t n = back ? N : (int64_t)N * N, step = back ? N + 1 : 1;
+        for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+            const zc x = M[i * step];
+            M[i * step] = mk(scalbn(x.re, back ? -sh : sh), scalbn(x.im, back ? -sh : sh));
+        }
     }
 }
 
@@ -524,6 +549,9 @@ int hetrd64_big(cudaStream_t st, int N, int64_t batch, zc* A, int* status_d) {
     mirror64_kernel<<<(unsigned)std::min<int64_t>(batch * ((N + 15) / 16) * ((N + 15) / 16), nsm * 64), 256, 0, st>>>(
         N, batch, A, nexp);
     count_launch();
+    const dim3 rs(std::min(64, (N * N + 255) / 256), (unsigned)std::min<int64_t>(batch, 65535));
+    rescale64_kernel<<<rs, 256, 0, st>>>(N, batch, A, nexp, false);
+    count_launch();
     cudaError_t e = cudaGetLastError();
     for (int j0 = 0; j0 < N - 1 && e == cudaSuccess && !rc; j0 += kNB) {
         const int steps = std::min(kNB, N - 1 - j0);
@@ -538,6 +566,11 @@ int hetrd64_big(cudaStream_t st, int N, int64_t batch, zc* A, int* status_d) {
         if (!rc)
             rc = oz64_gemm(st, batch, m, m, kPW, {Pt, kPW, 1, sP, 0, ex}, {Qt, kPW, 1, sP, 1, ex},
                            A + (size_t)t * N + t, N, (int64_t)N * N, -1, status_d);
+    }
+    if (e == cudaSuccess && !rc) {
+        rescale64_kernel<<<dim3(1, rs.y), 256, 0, st>>>(N, batch, A, nexp, true);
+        count_launch();
+        e = cudaGetLastError();
     }
     if (e != cudaSuccess && !rc) rc = cuda_error(e, "panel64_kernel");
     cudaFreeAsync(buf, st);
