@@ -810,13 +810,24 @@ __global__ void __launch_bounds__(32) tri64_cluster_kernel(int N, int64_t batch,
                         }
                         const double sc = 1.0 / amax;
                         for (int r = 0; r < N; ++r) x[r * G] *= sc;
-                        for (int pp = i; pp < jj; ++pp) {
-                            double dot = 0.0;
-                            for (int r = 0; r < N; ++r) dot += U[(size_t)r * N + pp].re * x[r * G];
-                            for (int r = 0; r < N; ++r) x[r * G] -= dot * U[(size_t)r * N + pp].re;
+                        auto norm2 = [&]() {
+                            double s = 0.0;
+                            for (int r = 0; r < N; ++r) s += x[r * G] * x[r * G];
+                            return s;
+                        };
+                        // once more where little is left (eigenvalues that the shifts do not tell
+                        // apart give the earlier members again): what is left is then orthogonal
+                        double nrm = norm2();
+                        for (int pass = 0; pass < 2; ++pass) {
+                            const double before = nrm;
+                            for (int pp = i; pp < jj; ++pp) {
+                                double dot = 0.0;
+                                for (int r = 0; r < N; ++r) dot += U[(size_t)r * N + pp].re * x[r * G];
+                                for (int r = 0; r < N; ++r) x[r * G] -= dot * U[(size_t)r * N + pp].re;
+                            }
+                            nrm = norm2();
+                            if (!(nrm < 0.01 * before)) break;
                         }
-                        double nrm = 0.0;
-                        for (int r = 0; r < N; ++r) nrm += x[r * G] * x[r * G];
                         const double inv = (nrm > 0.0) ? 1.0 / sqrt(nrm) : 0.0;
                         for (int r = 0; r < N; ++r) x[r * G] *= inv;
                     }

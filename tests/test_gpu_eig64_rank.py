@@ -24,3 +24,17 @@ def test_rank_deficient(n):
 @pytest.mark.parametrize("scale", [1e-290, 1e-170, 1e-160, 1e-155, 1e155, 1e160, 1e200, 1e290])
 def test_scaled(n, scale):
     check(random_hermitian(np.random.default_rng(n), 3, n) * scale)
+
+
+@pytest.mark.parametrize("n", [20, 47, 64, 96, 128, 164, 200])
+@pytest.mark.parametrize("spread", [1e-15, 1e-14, 1e-12, 1e-10])
+def test_clusters_below_the_shifts(n, spread):
+    """Eigenvalues nearer than the shifts of the inverse iteration can tell apart."""
+    H = []
+    for seed in range(4):
+        rng = np.random.default_rng(seed)
+        h = random_hermitian(rng, 1, n)[0]
+        Q, _ = np.linalg.qr(h + 1j * np.eye(n))
+        H += [np.ones((n, n)) + spread * h, (Q * (np.arange(n) // (n // 2) + 1.0)) @ np.conj(Q.T) + spread * h]
+    H = np.stack(H)
+    check(0.5 * (H + np.conj(np.transpose(H, (0, 2, 1)))))
