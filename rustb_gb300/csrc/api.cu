@@ -1510,7 +1510,7 @@ int tbg_hall_energy_cut(const tbg_model* m, const int64_t* kmesh, const double* 
     double* Om_all = ctx.alloc<double>(nk * N);
     zc* U_all = ctx.alloc<zc>(nk * NN);
     zc* K_all = ctx.alloc<zc>(nk * NN);
-    const bool track_gpu = N <= kEcTrackMaxN && nk > 1 && nk < (int64_t(1) << 30);
+    const bool track_gpu = ec_track_pays(dim, kmesh, N);
     double* Rd = ctx.alloc<double>(track_gpu ? nk * dim * NN : J.chunk * NN);
     unsigned* lev = track_gpu ? ctx.alloc<unsigned>(2 * (dim == 3 ? kmesh[0] * kmesh[1] : kmesh[0])) : nullptr;
     int* perm_d = ctx.alloc<int>(nk * N);

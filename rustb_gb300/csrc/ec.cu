@@ -11,8 +11,8 @@
 // Omega) come from the FP64 per-chunk pipeline and stay resident; the squared
 // overlaps |<u_n(a)|u_m(b)>|^2 of every mesh edge are batched complex GEMMs
 // over strided vertex pairs; the breadth-first tracking composes permutations
-// instead of moving data (level by level on the GPU up to kEcTrackMaxN bands, on
-// the host above); one GPU thread
+// instead of moving data (level by level on the GPU for few bands and meshes that
+// are not too long or flat, on the host otherwise); one GPU thread
 // then integrates one (simplex, band) pair over the whole sorted mu grid,
 // reading the vertex data through the permutations, and adds into
 // shared-memory accumulators per mu (a difference array for the fully
@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <deque>
 #include <numeric>
@@ -699,7 +700,35 @@ void ec_track(int dim, const int64_t* kmesh, int N, const double* R, int* perm) 
     }
 }
 
-// The same on the GPU for up to kEcTrackMaxN bands, R on the device as (dim, nk, N, N);
+static std::atomic<int> g_ec_track_max{kEcTrackMaxN};
+
+// Both sides in us: the host 0.12 a vertex and 250 for the copies and the
+// synchronisation; the GPU one step a level and what a warp's items cost one SM, the
+// warps counted in which a level has a vertex (few lanes of each where a 3D mesh is
+// flat).  Whole calls GPU / host: 101 x 101 of 2, 3, 4 bands 0.55 / 1.5, 1.3 / 1.8,
+// 1.6 / 2.3 ms, 40^3 of 4 bands 13.0 / 17.2; 7 x 3000 of 4 bands 12.4 / 4.1, 200 x 200 x 3 of
+// 4 bands 111 / 67.  Above four bands a thread's matrices leave its registers: 101 x 101 of
+// 6 bands 6.9 / 4.0, 20^3 of 5 bands 19.1 / 13.6.
+bool ec_track_pays(int dim, const int64_t* kmesh, int N) {
+    const int64_t n0 = kmesh[0], n1 = kmesh[1], n2 = dim == 3 ? kmesh[2] : 1;
+    const int64_t nk = n0 * n1 * n2, items = dim == 2 ? n0 : n0 * n1;
+    if (N > g_ec_track_max.load(std::memory_order_relaxed) || N > kEcTrackMaxN || nk <= 1 || nk >= (int64_t(1) << 30))
+        return false;
+    const bool one_bit = N == 2 && items <= 1024;
+    const double levels = (double)(n0 + n1 + (dim == 3 ? n2 : 0) - dim + 1);
+    double warps, per;
+    if (dim == 2) {
+        warps = (double)nk / 32.0 + levels;
+        per = N <= 2 ? (one_bit ? 0.05 : 0.4) : (N == 3 ? 0.3 : 0.6);
+    } else {
+        warps = (double)n0 * (double)(n1 + n2) * ((double)std::min(n1, n2) / 32.0 + std::min(1.0, (double)n1 / 32.0));
+        per = N <= 2 ? (one_bit ? 0.16 : 0.38) : (N == 3 ? 1.0 : 0.85);
+    }
+    const double step = N <= 2 ? (one_bit ? 0.65 : 1.2) : (N == 3 ? 3.3 : 3.8);
+    return levels * step + warps * per < 250.0 + 0.12 * (double)nk;
+}
+
+// The tracking on the GPU for up to kEcTrackMaxN (4) bands, R on the device as (dim, nk, N, N);
 // lev: 2 n0 (n1 in 3D) words of scratch.
 int ec_track_gpu(cudaStream_t st, int dim, const int64_t* kmesh, int N, const double* R, int* perm, unsigned* lev) {
     const int n0 = (int)kmesh[0], n1 = (int)kmesh[1], n2 = dim == 3 ? (int)kmesh[2] : 1;
@@ -714,10 +743,8 @@ int ec_track_gpu(cudaStream_t st, int dim, const int64_t* kmesh, int N, const do
             ec_track2_kernel<3><<<1, thr, 0, st>>>(n0, n1, n2, R, perm);
     } else if (N <= 2)
         ec_track_kernel<2><<<1, thr, sm ? bytes : 0, st>>>(N, dim, n0, n1, n2, R, perm, lev, sm);
-    else if (N <= 4)
-        ec_track_kernel<4><<<1, thr, sm ? bytes : 0, st>>>(N, dim, n0, n1, n2, R, perm, lev, sm);
     else
-        ec_track_kernel<8><<<1, std::min(thr, 512), sm ? bytes : 0, st>>>(N, dim, n0, n1, n2, R, perm, lev, sm);
+        ec_track_kernel<4><<<1, thr, sm ? bytes : 0, st>>>(N, dim, n0, n1, n2, R, perm, lev, sm);
     TBG_LAUNCHED("ec_track_kernel");
     return TBG_OK;
 }
@@ -775,3 +802,9 @@ int ec_integrate(cudaStream_t st, int dim, const int64_t* kmesh, int N, const do
 }
 
 }  // namespace tbg
+
+// Internal test hook (not part of the public header): the bands up to which the GPU may
+// track (0: the host always; negative: the default).  Returns the previous value.
+extern "C" int tbg_internal_ec_track_max(int n) {
+    return tbg::g_ec_track_max.exchange(n < 0 ? tbg::kEcTrackMaxN : n);
+}

@@ -395,7 +395,9 @@ int oz64_table_product(cudaStream_t st, int64_t M, int64_t Nc, int Kc, const zc*
 // Energy-cut Hall integration (see ec.cu).
 constexpr int kEcWindow = 8192;  // mu points per integration launch
 void ec_track(int dim, const int64_t* kmesh, int N, const double* R, int* perm);
-constexpr int kEcTrackMaxN = 8;
+// Whether the GPU tracks the bands sooner than the host (at most kEcTrackMaxN of them).
+constexpr int kEcTrackMaxN = 4;
+bool ec_track_pays(int dim, const int64_t* kmesh, int N);
 int ec_track_gpu(cudaStream_t st, int dim, const int64_t* kmesh, int N, const double* R, int* perm, unsigned* lev);
 size_t ec_smem_max();
 int ec_vertex_data(cudaStream_t st, int N, int64_t batch, const zc* V, int64_t ldV, const double* E, double eta,
