@@ -478,7 +478,7 @@ int run_berry_chunk(Ctx& ctx, BerryJob& J, int64_t nkc, int64_t* clusters_d) {
                                      &J.rexp_ok);
             if (rc) return rc;
         } else {
-            rc = fourier_mixed(m, ctx.st, nkc, J.k_d, J.dirs_d, J.H, J.V, P, J.fwork, J.fwork_bytes);
+            rc = fourier_mixed(m, ctx.st, nkc, J.k_d, J.dirs_d, J.H, J.V, P, J.fwork, J.fwork_bytes, J.status_d);
             if (rc) return rc;
             if (m.n_rmat > 0) {
                 rc = rmatrix_term(m, ctx.st, nkc, J.k_d, TBG_GAUGE_ATOM, 2, J.dirs_d, J.H, J.V, J.status_d);

@@ -872,12 +872,12 @@ int fourier_mixed_gemm(ModelDev& m, cudaStream_t st, int64_t nk, const double* k
 }  // namespace
 
 int fourier_mixed(ModelDev& m, cudaStream_t st, int64_t nk, const double* k_d, const double* dirs_d, zc* H, zc* V,
-                  float4* C, void* scratch, size_t scratch_bytes) {
+                  float4* C, void* scratch, size_t scratch_bytes, int* status_d) {
     if (nk <= 0) return TBG_OK;
     const int N = (int)m.nsta;
     const int64_t NN = (int64_t)N * N;
     if (!fourier_mixed_ok(m) || !C || scratch_bytes < fourier_mixed_scratch_bytes(m, nk))
-        return fourier_direct(m, st, nk, k_d, TBG_GAUGE_ATOM, 2, dirs_d, H, V, NN, 2 * NN);
+        return fourier_direct(m, st, nk, k_d, TBG_GAUGE_ATOM, 2, dirs_d, H, V, NN, 2 * NN, status_d);
     zc* orbph;
     double* taup;
     float2* tau2;
@@ -941,7 +941,7 @@ int fourier_mixed_pairs(ModelDev& m, cudaStream_t st, int64_t nk, const double* 
 namespace {
 
 // Lattice-gauge sums G (1 + nproj blocks of nk N^2: H, V_p) -> H, V with the
-// orbital-position term and the gauge phases, as the epilogue of fourier_pair_kernel.
+// orbital-position term and the gauge phases, as the epilogue of fourier_few_kernel.
 __global__ void __launch_bounds__(256) gauge64_kernel(int64_t nk, int N, int nproj, const zc* __restrict__ G,
                                                       const zc* __restrict__ orbph, const double* __restrict__ taup,
                                                       int gauge, zc* __restrict__ H, int64_t ldH, zc* __restrict__ V,
@@ -1089,7 +1089,7 @@ int fourier_direct(const ModelDev& m, cudaStream_t st, int64_t nk, const double*
         std::lock_guard<std::mutex> lk(g_hop_mu);
         int rc = ensure_pair_table(const_cast<ModelDev&>(m), st);
         if (rc) return rc;
-        oz = status_d && oz64_sum_pays(nk * (1 + nproj), (int64_t)N * N, m.hop_K,
+        oz = oz64_sum_pays(nk * (1 + nproj), (int64_t)N * N, m.hop_K,
                                        (double)nk * N * N * (m.hop_K * (nproj > 0 ? 8 + 2 * nproj : 4) + 60));
         if (oz && (rc = ensure_table_image(const_cast<ModelDev&>(m), st))) return rc;
         oz = oz && m.oz_img;

@@ -251,10 +251,9 @@ int allow_smem(K kern, size_t need) {
 // Fourier sum, direct form: for nk k-points (device k, (nk, dim)), outputs
 // H (nk, N, N) (may be null) and V (nk, nproj, N, N) (may be null when
 // nproj == 0); dirs (nproj, dim) device (Cartesian weights).  Large sums run on
-// the tensor cores (oz64.cu) when the caller gives a status word for their
-// bounded waits.
+// the tensor cores (oz64.cu), whose bounded waits report to status_d.
 int fourier_direct(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k_d, int gauge,
-                   int nproj, const double* dirs_d, zc* H, zc* V, int64_t ldH, int64_t ldV, int* status_d = nullptr);
+                   int nproj, const double* dirs_d, zc* H, zc* V, int64_t ldH, int64_t ldV, int* status_d);
 
 // Position-matrix commutator term added to V (HasRMatrix models).
 int rmatrix_term(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k_d, int gauge,
@@ -276,7 +275,7 @@ bool fourier_mesh_supported(const ModelDev& m);
 size_t fourier_mixed_scratch_bytes(const ModelDev& m, int64_t nk);
 bool fourier_mixed_ok(const ModelDev& m);
 int fourier_mixed(ModelDev& m, cudaStream_t st, int64_t nk, const double* k_d, const double* dirs_d, zc* H,
-                  zc* V, float4* C, void* scratch, size_t scratch_bytes);
+                  zc* V, float4* C, void* scratch, size_t scratch_bytes, int* status_d);
 // Same contraction, left in C as float pairs in the lattice gauge with the
 // orbital-position term added to V_0, V_1 (blocks [0,nk), [nk,2nk), [2nk,3nk)
 // of N^2 elements).  Requires fourier_mixed_ok(m).  With `out` the three
