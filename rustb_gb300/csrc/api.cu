@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -42,6 +43,14 @@ int cuda_error(cudaError_t e, const char* where) {
 }
 
 void count_launch(int n) { g_launches += n; }
+
+static std::atomic<int64_t> g_scratch_cap{INT64_MAX};
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
+    if ((int64_t)bytes > g_scratch_cap.load(std::memory_order_relaxed)) return cudaErrorMemoryAllocation;
+    const cudaError_t e = cudaMallocAsync(p, bytes, st);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
 
 int zgemm_batched(cudaStream_t st, int N, int64_t batch, bool conj_a, const zc* A, int64_t sA, const zc* B,
                   int64_t sB, zc* C, int64_t sC, int* status_d);
@@ -163,7 +172,7 @@ struct Ctx {
             return p;
         }
         void* p = nullptr;
-        cudaError_t e = cudaMallocAsync(&p, bytes, st);
+        const cudaError_t e = scratch_alloc(&p, bytes, st);
         if (e != cudaSuccess) {
             rc = cuda_error(e, "cudaMallocAsync");
             return nullptr;
@@ -1651,3 +1660,9 @@ int tbg_quantum_geometry_mesh(const tbg_model* m, const int64_t* kmesh, const do
 }
 
 }  // extern "C"
+
+// Internal test hook (not part of the public header): scratch allocations beyond this
+// many bytes fail as if the device were full; bytes <= 0 lifts the limit.
+extern "C" void tbg_internal_scratch_cap(int64_t bytes) {
+    tbg::g_scratch_cap.store(bytes > 0 ? bytes : INT64_MAX);
+}

@@ -1005,11 +1005,13 @@ bool oz64_sum_pays(int64_t M, int64_t NN, int Kc, double work) {
     const int64_t rounds = ((M + 127) / 128 * ((NN + 31) / 32) + 151) / 152;
     return 25.0 + (double)rounds * (8.0 + (Kc + 15) / 16) < work / 3.2e5;
 }
-constexpr int64_t kOzFourierBytes = 512LL << 20;  // sums held at a time
+// Sums held at a time: about this much, but a row tile's 128 k-points at least, so that the
+// table's image is read once for full tiles; less where that does not fit.
+constexpr int64_t kOzFourierBytes = 512LL << 20;
 
 // H and nproj projections on the tensor cores at FP64 accuracy (oz64.cu): the
 // real coefficients of every output (rows: H, V_0, V_1, ... per k-point) times
-// the paired table.
+// the paired table.  TBG_E_OOM, with nothing done, when not even one k-point's scratch fits.
 int fourier_oz64(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k_d, int gauge, int nproj,
                  const double* dirs_d, zc* H, zc* V, int64_t ldH, int64_t ldV, int* status_d) {
     const int N = (int)m.nsta, nR = (int)m.nR, Kc = m.hop_K;
@@ -1017,20 +1019,26 @@ int fourier_oz64(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k
     int64_t sub = std::max<int64_t>(1, kOzFourierBytes / (int64_t)(sizeof(zc) * NN * (1 + nproj)));
     sub = sub >= 128 ? sub / 128 * 128 : std::min<int64_t>(128, nk);
     sub = std::min(sub, nk);
-    const int64_t M = sub * (1 + nproj);
     const int npc = std::max(nproj, 1);
-    size_t off = 0;
+    size_t off, o_phi, o_orb, o_coef, o_tau, o_ea, o_img, o_g;
     auto take = [&](size_t bytes) {
         const size_t o = off;
         off += (bytes + 255) & ~size_t(255);
         return o;
     };
-    const size_t o_phi = take(sizeof(zc) * M * Kc), o_orb = take(sizeof(zc) * sub * N);
-    const size_t o_coef = take(sizeof(double) * npc * nR), o_tau = take(sizeof(double) * npc * N);
-    const size_t o_ea = take(sizeof(int) * M), o_img = take(oz64_row_image_bytes(M, Kc));
-    const size_t o_g = take(sizeof(zc) * M * NN);
-    unsigned char* buf = nullptr;
-    TBG_CUDA(cudaMallocAsync(&buf, off, st));
+    void* mem = nullptr;
+    for (;; sub = (sub + 1) / 2) {
+        const int64_t M = sub * (1 + nproj);
+        off = 0;
+        o_phi = take(sizeof(zc) * M * Kc), o_orb = take(sizeof(zc) * sub * N);
+        o_coef = take(sizeof(double) * npc * nR), o_tau = take(sizeof(double) * npc * N);
+        o_ea = take(sizeof(int) * M), o_img = take(oz64_row_image_bytes(M, Kc));
+        o_g = take(sizeof(zc) * M * NN);
+        const cudaError_t e = scratch_alloc(&mem, off, st);
+        if (e == cudaSuccess) break;
+        if (sub == 1) return cuda_error(e, "fourier_oz64 scratch");
+    }
+    unsigned char* buf = static_cast<unsigned char*>(mem);
     zc* phi = reinterpret_cast<zc*>(buf + o_phi);
     zc* orbph = reinterpret_cast<zc*>(buf + o_orb);
     double* coef = reinterpret_cast<double*>(buf + o_coef);
@@ -1094,9 +1102,13 @@ int fourier_direct(const ModelDev& m, cudaStream_t st, int64_t nk, const double*
         if (oz && (rc = ensure_table_image(const_cast<ModelDev&>(m), st))) return rc;
         oz = oz && m.oz_img;
     }
-    if (oz) return fourier_oz64(m, st, nk, k_d, gauge, nproj, dirs_d, H, V, ldH, ldV, status_d);
-    // H together with up to 3 projections per pass
     int rc = TBG_OK;
+    if (oz) {
+        rc = fourier_oz64(m, st, nk, k_d, gauge, nproj, dirs_d, H, V, ldH, ldV, status_d);
+        if (rc != TBG_E_OOM) return rc;
+        rc = TBG_OK;  // the direct form needs no scratch
+    }
+    // H together with up to 3 projections per pass
     for (int p0 = 0; rc == TBG_OK && (p0 < nproj || p0 == 0); p0 += 3) {
         const double* w = dirs_d + (int64_t)p0 * m.dim;
         zc* Ho = p0 == 0 ? H : nullptr;

@@ -688,9 +688,15 @@ int oz64_gemm(cudaStream_t st, int64_t batch, int M, int Nc, int K, const Oz64Op
     if (batch <= 0 || M <= 0 || Nc <= 0) return TBG_OK;
     if (K <= 0) return set_error(TBG_E_INVALID_ARGUMENT, "oz64_gemm: empty contraction");
     KTimer kt(st, "oz64_kernel", 8.0 * M * Nc * (double)K * batch);
-    const int64_t per = (int64_t)oz64_row_image_bytes(M, K), sub = std::min(batch, std::max<int64_t>(1, kImageBytes / per));
-    unsigned char* img = nullptr;
-    TBG_CUDA(cudaMallocAsync(&img, per * sub, st));
+    const int64_t per = (int64_t)oz64_row_image_bytes(M, K);
+    int64_t sub = std::min(batch, std::max<int64_t>(1, kImageBytes / per));
+    void* mem = nullptr;
+    for (;; sub = (sub + 1) / 2) {  // fewer at a time where they do not fit
+        const cudaError_t e = scratch_alloc(&mem, (size_t)(per * sub), st);
+        if (e == cudaSuccess) break;
+        if (sub == 1) return cuda_error(e, "oz64_gemm images");
+    }
+    unsigned char* img = static_cast<unsigned char*>(mem);
     int rc = TBG_OK;
     for (int64_t b0 = 0; b0 < batch && !rc; b0 += sub) {
         const int64_t nb = std::min(sub, batch - b0);

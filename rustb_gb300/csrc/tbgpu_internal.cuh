@@ -247,6 +247,10 @@ int allow_smem(K kern, size_t need) {
     return TBG_OK;
 }
 
+// Stream-ordered allocation of scratch whose failure has a smaller form to fall back to
+// (tests lower what it grants: tbg_internal_scratch_cap).
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st);
+
 // ---------------------------------------------------------- kernel drivers --
 // Fourier sum, direct form: for nk k-points (device k, (nk, dim)), outputs
 // H (nk, N, N) (may be null) and V (nk, nproj, N, N) (may be null when
