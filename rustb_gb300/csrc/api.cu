@@ -1479,8 +1479,10 @@ int tbg_wilson_loops(const tbg_model* m, int64_t n_loops, int64_t n_k, const dou
     return status_error(ctx.status());
 }
 
-int tbg_hall_energy_cut(const tbg_model* m, const int64_t* kmesh, const double* dirs2, int64_t nmu, const double* mu,
-                        double T, double eta, int spin, double* sigma_out) {
+// track_gpu: in, whether the GPU may track the bands; out, whether it was to.
+static int hall_energy_cut_impl(const tbg_model* m, const int64_t* kmesh, const double* dirs2, int64_t nmu,
+                                const double* mu, double T, double eta, int spin, double* sigma_out,
+                                bool& track_gpu) {
     int rc = check_model(m);
     if (rc) return rc;
     const ModelDev& M = m->d;
@@ -1519,7 +1521,7 @@ int tbg_hall_energy_cut(const tbg_model* m, const int64_t* kmesh, const double* 
     double* Om_all = ctx.alloc<double>(nk * N);
     zc* U_all = ctx.alloc<zc>(nk * NN);
     zc* K_all = ctx.alloc<zc>(nk * NN);
-    const bool track_gpu = ec_track_pays(dim, kmesh, N);
+    track_gpu = track_gpu && ec_track_pays(dim, kmesh, N);
     double* Rd = ctx.alloc<double>(track_gpu ? nk * dim * NN : J.chunk * NN);
     unsigned* lev = track_gpu ? ctx.alloc<unsigned>(2 * (dim == 3 ? kmesh[0] * kmesh[1] : kmesh[0])) : nullptr;
     int* perm_d = ctx.alloc<int>(nk * N);
@@ -1642,6 +1644,19 @@ int tbg_hall_energy_cut(const tbg_model* m, const int64_t* kmesh, const double* 
         }
     }
     return TBG_OK;
+}
+
+int tbg_hall_energy_cut(const tbg_model* m, const int64_t* kmesh, const double* dirs2, int64_t nmu, const double* mu,
+                        double T, double eta, int spin, double* sigma_out) {
+    bool gpu = true;
+    int rc = hall_energy_cut_impl(m, kmesh, dirs2, nmu, mu, T, eta, spin, sigma_out, gpu);
+    // tracking on the GPU keeps the overlaps of the whole mesh, half as much again as the
+    // vertex data: without room for them the host tracks, a chunk of overlaps at a time
+    if (rc == TBG_E_OOM && gpu) {
+        gpu = false;
+        rc = hall_energy_cut_impl(m, kmesh, dirs2, nmu, mu, T, eta, spin, sigma_out, gpu);
+    }
+    return rc;
 }
 
 int tbg_quantum_geometry(const tbg_model* m, int64_t nk, const double* k, const double* dirs2, double eta,

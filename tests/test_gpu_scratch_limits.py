@@ -1,5 +1,5 @@
 """Calls whose scratch does not fit take their smaller forms: sums and images in
-parts, the direct Fourier sum (GPU).
+parts, the direct Fourier sum, band tracking on the host (GPU).
 
 Allocations beyond a limit set by the test fail as on a full device."""
 
@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 from rustb_gb300 import _lib, workloads as W
-from rustb_gb300.params import Parameters
+from rustb_gb300.params import Integration, Parameters
 
 pytestmark = pytest.mark.gpu
 
@@ -59,3 +59,17 @@ def test_product_images_in_parts():
     (Omx, Ex), names = limited(6 << 20, lambda: m.berry_curvature_on(k, p))
     assert "oz64_kernel" in names
     assert np.array_equal(Omx, Om) and np.array_equal(Ex, E)
+
+
+def test_energy_cut_overlaps(monkeypatch):
+    m = W.random_model(3, 4, False, 1, seed=8)
+    p = Parameters.rank2((12, 11, 10), [1.0, 0.0, 0.0], [0.0, 1.0, 0.0], list(np.linspace(-2, 2, 17)))
+    p.eta = 0.05
+    p.integration = Integration.EnergyCut
+    monkeypatch.setenv("TBG_MAX_CHUNK", "64")
+    ref, names = limited(0, lambda: m.hall_conductivity(p).conductivity)
+    assert "ec_track_kernel" in names
+    # vectors 338 KB, overlaps of the whole mesh 507 KB
+    got, names = limited(400000, lambda: m.hall_conductivity(p).conductivity)
+    assert "ec_track_kernel" not in names
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
