@@ -1259,12 +1259,12 @@ static int hall_impl(const tbg_model* m, const int64_t* kmesh, int64_t k_begin, 
         if (met && (rc = kahan_column_sums(ctx.st, nkc, (int)nmu, SG, accg))) return rc;
     }
     // the totals, the cluster count and the status word in one copy
-    cudaEventRecord(ev1, ctx.st);
     const double* acc_h = ctx.fetch(acc, (size_t)ntail);
     if (!acc_h) {
         TBG_CUDA(cudaMemcpyAsync(block_h.data(), acc, sizeof(double) * ntail, cudaMemcpyDeviceToHost, ctx.st));
         acc_h = block_h.data();
     }
+    cudaEventRecord(ev1, ctx.st);
     if (ctx.sync("tbg_hall_conductivity")) return ctx.rc;
     const double* accg_h = acc_h + 2 * nmu;
     int64_t clusters_h = 0;
