@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kBins) dos_center_kernel(int64_t count, int64_
     const int tile = (int)std::min<int64_t>(kBins, E_n - b0);
     const int64_t s0 = (int64_t)blockIdx.y * per_slice;
     const int64_t s1 = std::min<int64_t>(count, s0 + per_slice);
-    const double w = kCut * sigma, d = step * sigma0;
+    const double hw = kCut * sigma * inv_step, d = step * sigma0;
     for (int i = threadIdx.x; i <= half; i += kBins) {
         const double t = (double)i * d;
         Wt[i] = exp(-0.5 * t * t);
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kBins) dos_center_kernel(int64_t count, int64_
             if (threadIdx.x < nc) {
                 const double x = ev[c0 + threadIdx.x];
                 // bounds by the reciprocal step: a rounding shift of one bin stays inside the slack
-                const double u = (x - E_min) * inv_step, hw = w * inv_step;
+                const double s = E_min - x, u = -s * inv_step;
                 double a = ceil(u - hw) - 1.0;
                 double b = floor(u + hw) + 1.0;
                 a = fmax(a, (double)b0);
@@ -214,7 +214,10 @@ __global__ void __launch_bounds__(kBins) dos_center_kernel(int64_t count, int64_
                     lo = (int)(a - (double)b0);
                     len = min((int)(b - a) + 1, lmax);  // lmax holds the widest window; guard rounding
                     c = (int)(cr - (double)b0);
-                    a_c = (__dadd_rn(E_min, __dmul_rn(step, cr)) - x) * sigma0;
+                    // one rounding, of the energy's own; that of E_c would shift all energies
+                    // about a bin alike, for every bin of their windows (4.4e-15 of the DOS at 500
+                    // bins, against 1.5e-15)
+                    a_c = fma(step, cr, s) * sigma0;
                 }
             }
             // runs from the centre: bins c .. upward, c - 1 .. downward, those inside [lo, lo + len)
