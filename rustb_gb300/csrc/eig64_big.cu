@@ -400,8 +400,13 @@ __global__ void __launch_bounds__(256) rescale64_kernel(int N, int64_t batch, zc
 // ---------------------------------------------------- back-transformation --
 constexpr int kWY = 64;  // reflectors of a block
 
-// Reflectors j0 .. j0 + w - 1 of every matrix as rows of length m = N - 1 - j0
-// (zeros before the leading one), w = kWY rows held.
+// Reflectors j0 .. j0 + w - 1 of every matrix as rows of length m = N - 1 - j0 without
+// their leading ones (reflector jj has its at jj; zeros up to there), w = kWY rows held.
+//
+// The ones, and T's diagonal, are added apart in FP64 (wy_preset_kernel, wy_scale_kernel,
+// wy_ones_kernel): a digit product's error is relative to the largest entry of a line, and
+// beside them the rest is some ten times smaller (H U - U E of 128 bands 1.8e-13 in the
+// Frobenius norm with them in the products, 1.8e-14 by single reflectors).
 __global__ void __launch_bounds__(256) wy_rows_kernel(int N, int64_t batch, int j0, int w, const zc* __restrict__ A,
                                                       zc* __restrict__ Y) {
     const int m = N - 1 - j0;
@@ -411,13 +416,56 @@ __global__ void __launch_bounds__(256) wy_rows_kernel(int N, int64_t batch, int 
         const int jj = (int)(row % w);
         const zc* src = A + (b * N + j0 + jj) * (int64_t)N + j0 + 1;
         zc* dst = Y + (b * kWY + jj) * (int64_t)m;
-        for (int r = threadIdx.x; r < m; r += blockDim.x) dst[r] = r >= jj ? src[r] : mk(0.0, 0.0);
+        for (int r = threadIdx.x; r < m; r += blockDim.x) dst[r] = r > jj ? src[r] : mk(0.0, 0.0);
+    }
+}
+
+// What the leading ones add to G = Y^H Y above the diagonal (conj(Y(i, j))) and to Y^H U
+// (rows of U); ldu, sU: of U's rows and matrices.
+__global__ void __launch_bounds__(256) wy_preset_kernel(int64_t batch, int w, int m, int ncol,
+                                                        const zc* __restrict__ Y, const zc* __restrict__ U,
+                                                        int64_t ldu, int64_t sU, zc* __restrict__ G,
+                                                        zc* __restrict__ X) {
+    const int64_t total = batch * w;
+    for (int64_t row = blockIdx.x; row < total; row += gridDim.x) {
+        const int64_t b = row / w;
+        const int i = (int)(row % w);
+        const zc* y = Y + (b * kWY + i) * (int64_t)m;
+        zc* g = G + (b * kWY + i) * (int64_t)kWY;
+        for (int j = threadIdx.x; j < w; j += blockDim.x) g[j] = j > i ? conj(y[j]) : mk(0.0, 0.0);
+        const zc* u = U + b * sU + i * ldu;
+        zc* x = X + (b * kWY + i) * (int64_t)ncol;
+        for (int c = threadIdx.x; c < ncol; c += blockDim.x) x[c] = u[c];
+    }
+}
+// X2 = diag(tau) X1, and U's rows of the leading ones -= X2 (ones).
+__global__ void __launch_bounds__(256) wy_scale_kernel(int N, int64_t batch, int j0, int w, int ncol,
+                                                       const zc* __restrict__ A, const zc* __restrict__ X1,
+                                                       zc* __restrict__ X2) {
+    const int64_t total = batch * w;
+    for (int64_t row = blockIdx.x; row < total; row += gridDim.x) {
+        const int64_t b = row / w;
+        const int i = (int)(row % w);
+        const zc tau = A[(b * N + j0 + i + 1) * (int64_t)N + j0 + i];
+        const int64_t at = (b * kWY + i) * (int64_t)ncol;
+        for (int c = threadIdx.x; c < ncol; c += blockDim.x) X2[at + c] = tau * X1[at + c];
+    }
+}
+__global__ void __launch_bounds__(256) wy_ones_kernel(int64_t batch, int w, int ncol, const zc* __restrict__ X2,
+                                                      zc* __restrict__ U, int64_t ldu, int64_t sU) {
+    const int64_t total = batch * w;
+    for (int64_t row = blockIdx.x; row < total; row += gridDim.x) {
+        const int64_t b = row / w;
+        const int i = (int)(row % w);
+        zc* u = U + b * sU + i * ldu;
+        const zc* x = X2 + (b * kWY + i) * (int64_t)ncol;
+        for (int c = threadIdx.x; c < ncol; c += blockDim.x) u[c] = u[c] - x[c];
     }
 }
 
 // T of H_0 ... H_{w-1} = I - Y T Y^H from G = Y^H Y and tau (columns left to right:
-// T(0:j, j) = -tau_j T(0:j, 0:j) G(0:j, j)); T over G in place, one CTA per matrix,
-// four lanes per row.
+// T(0:j, j) = -tau_j T(0:j, 0:j) G(0:j, j)); T without its diagonal tau over G in place,
+// one CTA per matrix, four lanes per row.
 __global__ void __launch_bounds__(4 * kWY) wy_t_kernel(int N, int64_t batch, int j0, int w, const zc* __restrict__ A,
                                                        zc* __restrict__ G) {
     __shared__ zc T[kWY * (kWY + 1) / 2], g[kWY], s_tau[kWY];  // T by packed columns
@@ -447,7 +495,7 @@ __global__ void __launch_bounds__(4 * kWY) wy_t_kernel(int N, int64_t batch, int
         }
         for (int e = threadIdx.x; e < w * kWY; e += blockDim.x) {
             const int r = e / kWY, c = e - r * kWY;
-            Gb[e] = (c < w && r <= c) ? T[c * (c + 1) / 2 + r] : mk(0.0, 0.0);
+            Gb[e] = (c < w && r < c) ? T[c * (c + 1) / 2 + r] : mk(0.0, 0.0);
         }
         __syncthreads();
     }
@@ -485,19 +533,26 @@ int bt64_wy(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U, int* stat
         zc* Ut = U + (int64_t)(j0 + 1) * N + first;
         wy_rows_kernel<<<(unsigned)std::min<int64_t>(batch * w, nsm * 64), 256, 0, st>>>(N, batch, j0, w, A, Y);
         TBG_LAUNCHED("wy_rows_kernel");
+        const unsigned rows = (unsigned)std::min<int64_t>(batch * w, nsm * 64);
+        wy_preset_kernel<<<rows, 256, 0, st>>>(batch, w, m, ncol, Y, Ut, N, sU, G, X1);
+        TBG_LAUNCHED("wy_preset_kernel");
         if ((rc = oz64_row_exps(st, batch, w, m, Y, m, sY, ey))) break;
         const Oz64Operand yh{Y, m, 1, sY, 1, ey};
-        if ((rc = oz64_gemm(st, batch, w, w, m, yh, {Y, m, 1, sY, 0, ey}, G, kWY, sG, 0, status_d))) break;
+        if ((rc = oz64_gemm(st, batch, w, w, m, yh, {Y, m, 1, sY, 0, ey}, G, kWY, sG, 1, status_d))) break;
         wy_t_kernel<<<(unsigned)std::min<int64_t>(batch, nsm * 64), 4 * kWY, 0, st>>>(N, batch, j0, w, A, G);
         TBG_LAUNCHED("wy_t_kernel");
         if ((rc = oz64_row_exps(st, batch, w, w, G, kWY, sG, et)) || (rc = oz64_col_exps(st, batch, m, ncol, Ut, N, sU, eu)) ||
             (rc = oz64_col_exps(st, batch, w, m, Y, m, sY, ec)))
             break;
-        if ((rc = oz64_gemm(st, batch, w, ncol, m, yh, {Ut, 1, N, sU, 0, eu}, X1, ncol, sX, 0, status_d))) break;
+        if ((rc = oz64_gemm(st, batch, w, ncol, m, yh, {Ut, 1, N, sU, 0, eu}, X1, ncol, sX, 1, status_d))) break;
+        wy_scale_kernel<<<rows, 256, 0, st>>>(N, batch, j0, w, ncol, A, X1, X2);
+        TBG_LAUNCHED("wy_scale_kernel");
         if ((rc = oz64_col_exps(st, batch, w, ncol, X1, ncol, sX, e1))) break;
-        if ((rc = oz64_gemm(st, batch, w, ncol, w, {G, kWY, 1, sG, 0, et}, {X1, 1, ncol, sX, 0, e1}, X2, ncol, sX, 0,
+        if ((rc = oz64_gemm(st, batch, w, ncol, w, {G, kWY, 1, sG, 0, et}, {X1, 1, ncol, sX, 0, e1}, X2, ncol, sX, 1,
                             status_d)))
             break;
+        wy_ones_kernel<<<rows, 256, 0, st>>>(batch, w, ncol, X2, Ut, N, sU);
+        TBG_LAUNCHED("wy_ones_kernel");
         if ((rc = oz64_col_exps(st, batch, w, ncol, X2, ncol, sX, e2))) break;
         rc = oz64_gemm(st, batch, m, ncol, w, {Y, 1, m, sY, 0, ec}, {X2, 1, ncol, sX, 0, e2}, Ut, N, sU, -1, status_d);
     }
