@@ -626,11 +626,11 @@ __global__ void gather_exps_kernel(int64_t n, const int* __restrict__ idx, const
 //   A = t(R) + t(-R),  B = i (t(R) - t(-R))
 // (an R without its -R partner takes t(-R) = 0).  Rows: 0 = t(0), 1 = 0,
 // 2 + 2p = A_p, 3 + 2p = B_p.  pi[p] is the pair's R, pj[p] its -R or -1.
-// A non-finite entry sets *nonfinite (the exact-slice digits of the
+// A non-finite entry sets bit 0 of *flags (the exact-slice digits of the
 // tensor-core form cannot carry NaN or Inf, so the mixed path refuses such a
-// table up front).
+// table up front), one of 2^960 or more bit 1 (no room for the pairs' weights).
 __global__ void pair_table_kernel(int np, const int* __restrict__ pi, const int* __restrict__ pj, int z, int64_t NN,
-                                  const zc* __restrict__ ham, zc* __restrict__ T, int* __restrict__ nonfinite) {
+                                  const zc* __restrict__ ham, zc* __restrict__ T, int* __restrict__ flags) {
     const int64_t total = (int64_t)(np + 1) * NN;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
@@ -647,7 +647,11 @@ __global__ void pair_table_kernel(int np, const int* __restrict__ pi, const int*
             T[(2 + 2 * p) * NN + e] = mk(a.re + b.re, a.im + b.im);
             T[(3 + 2 * p) * NN + e] = mk(-(a.im - b.im), a.re - b.re);
         }
-        if (!(isfinite(a.re) && isfinite(a.im) && isfinite(b.re) && isfinite(b.im))) atomicOr(nonfinite, 1);
+        const double big = fmax(fmax(fabs(a.re), fabs(a.im)), fmax(fabs(b.re), fabs(b.im)));
+        if (!(isfinite(a.re) && isfinite(a.im) && isfinite(b.re) && isfinite(b.im)))
+            atomicOr(flags, 1);
+        else if (big >= 0x1p960)
+            atomicOr(flags, 2);
     }
 }
 
@@ -655,21 +659,23 @@ __global__ void pair_table_kernel(int np, const int* __restrict__ pi, const int*
 // imaginary parts are consecutive rows (Phi (1 + nproj, nk, Kc), Kc = 1 + np): H
 // row (1, 0 | cos, sin ...), V_p rows (0, 0 | -c_p(R) sin, c_p(R) cos ...), from
 //   i c_p(R) (t(R) e^{i theta} - t(-R) e^{-i theta}) = c_p(R) (B cos - A sin).
+// skip 1 leaves the R = 0 column out (Kc = np); wexp: columns over their pair's weight.
 __global__ void phases_real_kernel(int64_t nk, int dim, const double* __restrict__ k, int np,
                                    const int* __restrict__ pair, const int* __restrict__ hamR, int nR, int nproj,
-                                   const double* __restrict__ coef, zc* __restrict__ Phi) {
-    const int Kc = np + 1;
+                                   const double* __restrict__ coef, int skip, const int* __restrict__ wexp,
+                                   zc* __restrict__ Phi) {
+    const int Kc = np + 1 - skip;
     const int64_t total = nk * (int64_t)Kc;
     for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
         const int64_t kk = idx / Kc;
         const int c = (int)(idx % Kc);
-        if (c == 0) {
+        if (c + skip == 0) {
             Phi[idx] = mk(1.0, 0.0);
             for (int p = 0; p < nproj; ++p) Phi[(1 + p) * total + idx] = mk(0.0, 0.0);
             continue;
         }
-        const int j = pair[c - 1];
+        const int j = pair[c + skip - 1];
         const int* r = hamR + 3 * j;
         const double* kv = k + kk * dim;
         // same operation order as the reference: r0*k0 + r1*k1 + r2*k2
@@ -678,6 +684,11 @@ __global__ void phases_real_kernel(int64_t nk, int dim, const double* __restrict
         if (dim > 2) s += (double)r[2] * kv[2];
         double sn, cs;
         sincos(kTwoPi * s, &sn, &cs);
+        if (wexp) {
+            const double w = scalbn(1.0, -wexp[c + skip - 1]);
+            cs *= w;
+            sn *= w;
+        }
         Phi[idx] = mk(cs, sn);
         for (int p = 0; p < nproj; ++p) {
             const double cp = coef[(int64_t)p * nR + j];
@@ -712,11 +723,32 @@ int ensure_pair_table(ModelDev& m, cudaStream_t st) {
         pj.push_back(partner);
     }
     const int np = (int)pi.size(), Kc = np + 1;
-    int *pair_d = nullptr, *pj_d = nullptr;
+    // Weights of the pairs in the FP64-accurate products, whose error is relative to the
+    // largest coefficient and the largest table entry of a column: the velocities' c_p(R)
+    // grow with |R| while t(R) falls, so |R| (over the shortest, as a power of two) goes
+    // from the coefficients to the table.
+    std::vector<int> wexp((size_t)std::max(np, 1), 0);
+    std::vector<double> len((size_t)np, 0.0);
+    double shortest = 0.0;
+    for (int p = 0; p < np; ++p) {
+        double l2 = 0.0;
+        for (int c = 0; c < m.dim; ++c) {
+            double x = 0.0;
+            for (int d = 0; d < m.dim; ++d) x += (double)rvec(pi[p], d) * m.lat[(size_t)d * m.dim + c];
+            l2 += x * x;
+        }
+        len[p] = std::sqrt(l2);
+        if (len[p] > 0.0 && (shortest == 0.0 || len[p] < shortest)) shortest = len[p];
+    }
+    for (int p = 0; p < np; ++p)
+        if (len[p] > 0.0 && std::isfinite(len[p]))
+            wexp[p] = std::min(48, std::max(0, (int)std::lround(std::log2(len[p] / shortest))));
+    int *pair_d = nullptr, *pj_d = nullptr, *wexp_d = nullptr;
     zc* T = nullptr;
     int rc = TBG_OK;
     if (cudaMalloc(&T, sizeof(zc) * 2 * (size_t)Kc * NN) != cudaSuccess ||
         cudaMalloc(&pair_d, sizeof(int) * std::max(np, 1)) != cudaSuccess ||
+        cudaMalloc(&wexp_d, sizeof(int) * std::max(np, 1)) != cudaSuccess ||
         cudaMalloc(&pj_d, sizeof(int) * (std::max(np, 1) + 1)) != cudaSuccess)
         rc = set_error(TBG_E_OOM, "paired hop table");
     int* nonfinite_d = pj_d + std::max(np, 1);
@@ -730,18 +762,23 @@ int ensure_pair_table(ModelDev& m, cudaStream_t st) {
         pair_table_kernel<<<(unsigned)std::min<int64_t>(((int64_t)Kc * NN + 255) / 256, 152 * 64), 256, 0, st>>>(
             np, pair_d, pj_d, z, NN, m.ham, T, nonfinite_d);
         count_launch();
-        int nf = 0;
+        int nf = 0;  // flags of the table
         cudaError_t e = cudaMemcpyAsync(&nf, nonfinite_d, sizeof(int), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // other streams use the table next
         if (e != cudaSuccess) rc = cuda_error(e, "paired hop table");
-        m.nonfinite = nf != 0;
+        m.nonfinite = (nf & 1) != 0;
+        if (nf & 2) std::fill(wexp.begin(), wexp.end(), 0);
+        if (!rc && cudaMemcpy(wexp_d, wexp.data(), sizeof(int) * wexp.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+            rc = set_error(TBG_E_CUDA, "paired hop table weights");
     }
     cudaFree(pj_d);
     if (rc) {
         cudaFree(T);
         cudaFree(pair_d);
+        cudaFree(wexp_d);
         return rc;
     }
+    m.hop_wexp_d = wexp_d;
     m.pair_T = T;
     m.hop_pair_d = pair_d;
     m.hop_np = np;
@@ -842,7 +879,7 @@ int fourier_mixed_gemm(ModelDev& m, cudaStream_t st, int64_t nk, const double* k
                 nk, m.dim, k_d, 0, m.hamR_d, N, m.tau_d, ph3, orbph);
             const int64_t t2 = nk * (int64_t)m.hop_K;
             phases_real_kernel<<<(unsigned)std::min<int64_t>((t2 + 255) / 256, 65535 * 8), 256, 0, st>>>(
-                nk, m.dim, k_d, m.hop_np, m.hop_pair_d, m.hamR_d, nR, 2, coef, ph3);
+                nk, m.dim, k_d, m.hop_np, m.hop_pair_d, m.hamR_d, nR, 2, coef, 0, nullptr, ph3);
         } else {
             const int64_t t1 = nk * (int64_t)(nR + N);
             phases_kernel<<<(unsigned)std::min<int64_t>((t1 + 255) / 256, 65535 * 8), 256, 0, st>>>(
@@ -940,9 +977,10 @@ int fourier_mixed_pairs(ModelDev& m, cudaStream_t st, int64_t nk, const double* 
 
 namespace {
 
-// Lattice-gauge sums G (1 + nproj blocks of nk N^2: H, V_p) -> H, V with the
-// orbital-position term and the gauge phases, as the epilogue of fourier_few_kernel.
+// Lattice-gauge sums G (1 + nproj blocks of nk N^2: H without its R = 0 term t0, V_p) -> H, V
+// with the orbital-position term and the gauge phases, as the epilogue of fourier_few_kernel.
 __global__ void __launch_bounds__(256) gauge64_kernel(int64_t nk, int N, int nproj, const zc* __restrict__ G,
+                                                      const zc* __restrict__ t0,
                                                       const zc* __restrict__ orbph, const double* __restrict__ taup,
                                                       int gauge, zc* __restrict__ H, int64_t ldH, zc* __restrict__ V,
                                                       int64_t ldV) {
@@ -950,7 +988,7 @@ __global__ void __launch_bounds__(256) gauge64_kernel(int64_t nk, int N, int npr
     for (int64_t kk = blockIdx.y; kk < nk; kk += gridDim.y) {
         for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < (int)NN; e += gridDim.x * blockDim.x) {
             const int mrow = e / N, ncol = e - mrow * N;
-            const zc hl = G[kk * NN + e];
+            const zc hl = G[kk * NN + e] + t0[e];
             zc g = mk(1.0, 0.0);
             if (gauge == TBG_GAUGE_ATOM) g = cmul(orbph[kk * N + mrow], orbph[kk * N + ncol]);
             if (H) H[kk * ldH + e] = gauge == TBG_GAUGE_ATOM ? hl * g : hl;
@@ -969,19 +1007,21 @@ __global__ void __launch_bounds__(256) gauge64_kernel(int64_t nk, int N, int npr
 }
 
 // The digit image of the paired table for the tensor-core form, built once per
-// model; the caller holds g_hop_mu.  Without memory for it m.oz_img stays null.
+// model; the caller holds g_hop_mu.  R = 0 is left to gauge64_kernel: on-site energies are often
+// a thousand times the hoppings, and the velocities, which have no such term, would
+// carry errors relative to them.  Without memory for it m.oz_img stays null.
 int ensure_table_image(ModelDev& m, cudaStream_t st) {
-    if (m.oz_img || m.nonfinite) return TBG_OK;
+    if (m.oz_img || m.nonfinite || m.hop_np == 0) return TBG_OK;
     const int64_t NN = (int64_t)m.nsta * m.nsta;
     void* img = nullptr;
     int* eb = nullptr;
-    if (cudaMalloc(&img, oz64_table_image_bytes(m.hop_K, NN)) != cudaSuccess ||
+    if (cudaMalloc(&img, oz64_table_image_bytes(m.hop_np, NN)) != cudaSuccess ||
         cudaMalloc(&eb, sizeof(int) * NN) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(img);
         return TBG_OK;
     }
-    int rc = oz64_table_image(st, m.hop_K, NN, m.pair_T, eb, img);
+    int rc = oz64_table_image(st, m.hop_np, NN, m.pair_T + 2 * NN, m.hop_wexp_d, eb, img);
     if (!rc) {
         cudaError_t e = cudaStreamSynchronize(st);  // other streams use the image next
         if (e != cudaSuccess) rc = cuda_error(e, "table image");
@@ -1014,7 +1054,7 @@ constexpr int64_t kOzFourierBytes = 512LL << 20;
 // the paired table.  TBG_E_OOM, with nothing done, when not even one k-point's scratch fits.
 int fourier_oz64(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k_d, int gauge, int nproj,
                  const double* dirs_d, zc* H, zc* V, int64_t ldH, int64_t ldV, int* status_d) {
-    const int N = (int)m.nsta, nR = (int)m.nR, Kc = m.hop_K;
+    const int N = (int)m.nsta, nR = (int)m.nR, Kc = m.hop_np;  // R = 0 apart
     const int64_t NN = (int64_t)N * N;
     int64_t sub = std::max<int64_t>(1, kOzFourierBytes / (int64_t)(sizeof(zc) * NN * (1 + nproj)));
     sub = sub >= 128 ? sub / 128 * 128 : std::min<int64_t>(128, nk);
@@ -1068,7 +1108,7 @@ int fourier_oz64(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k
                 launched("phases_kernel");
             }
             phases_real_kernel<<<(unsigned)std::min<int64_t>((t2 + 255) / 256, 65535 * 8), 256, 0, st>>>(
-                nks, m.dim, k_d + k0 * m.dim, m.hop_np, m.hop_pair_d, m.hamR_d, nR, nproj, coef, phi);
+                nks, m.dim, k_d + k0 * m.dim, m.hop_np, m.hop_pair_d, m.hamR_d, nR, nproj, coef, 1, m.hop_wexp_d, phi);
             launched("phases_real_kernel");
         }
         if (!rc)
@@ -1077,7 +1117,7 @@ int fourier_oz64(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k
         if (rc) break;
         KTimer kt(st, "gauge64_kernel");
         const dim3 grid((unsigned)std::min<int64_t>((NN + 255) / 256, 1024), (unsigned)std::min<int64_t>(nks, 65535));
-        gauge64_kernel<<<grid, 256, 0, st>>>(nks, N, nproj, G, orbph, taup, gauge, H ? H + k0 * ldH : nullptr, ldH,
+        gauge64_kernel<<<grid, 256, 0, st>>>(nks, N, nproj, G, m.pair_T, orbph, taup, gauge, H ? H + k0 * ldH : nullptr, ldH,
                                              V ? V + k0 * ldV : nullptr, ldV);
         launched("gauge64_kernel");
     }
@@ -1172,7 +1212,7 @@ int rmatrix_term(const ModelDev& m, cudaStream_t st, int64_t nk, const double* k
         if (launched("rmat_combine_kernel")) break;
         // A = sum_{r < n_rmat} u(k,r) rm_p[r]   (lattice gauge)
         if (oz) {
-            rc = oz64_table_image(st, nr, NN, tab, EB, buf + o_tim);
+            rc = oz64_table_image(st, nr, NN, tab, nullptr, EB, buf + o_tim);
             if (!rc) rc = oz64_table_product(st, nk, NN, nr, ph, nR, EB, buf + o_tim, A, EA, buf + o_aim, status_d);
         } else {
             rc = launch_gemm(st, nk, nr, nR, N, ph, tab, A);

@@ -561,9 +561,10 @@ __global__ void row_exp64_kernel(int64_t rows, int M, int K, const zc* __restric
     }
 }
 // Column exponents: a warp takes 32 columns (lanes) of one matrix; the rows are
-// dealt to the block's warps.
+// dealt to the block's warps.  Rows 2 q, 2 q + 1 count times 2^wexp[q] when given.
 __global__ void __launch_bounds__(256) col_exp64_kernel(int64_t batch, int K, int64_t Nc, const zc* __restrict__ B,
-                                                        int64_t ld, int64_t sB, int* __restrict__ out) {
+                                                        int64_t ld, int64_t sB, const int* __restrict__ wexp,
+                                                        int* __restrict__ out) {
     __shared__ int part[8][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t nct = (Nc + 31) / 32;
@@ -571,7 +572,11 @@ __global__ void __launch_bounds__(256) col_exp64_kernel(int64_t batch, int K, in
         const int64_t b = w / nct, c = (w % nct) * 32 + lane;
         int e = 1;
         if (c < Nc)
-            for (int k = warp; k < K; k += 8) e = max(e, elem_exp(B[b * sB + (int64_t)k * ld + c]));
+            for (int k = warp; k < K; k += 8) {
+                zc x = B[b * sB + (int64_t)k * ld + c];
+                if (wexp) x = scalbn(1.0, wexp[k >> 1]) * x;
+                e = max(e, elem_exp(x));
+            }
         part[warp][lane] = e;
         __syncthreads();
         if (warp == 0) {
@@ -611,7 +616,9 @@ __global__ void __launch_bounds__(256) a_image_kernel(int64_t batch, int M, int 
 }
 // Stage images of a real-coefficient table (2 Kc rows of Nc complex entries): k step 0
 // the even rows, k step 1 the odd ones, [Re; Im]; thread = (column, 8 kappa, even / odd).
+// Row pair q times 2^wexp[q] when given.
 __global__ void __launch_bounds__(B_THREADS) table_image_kernel(int Kc, int64_t Nc, const zc* __restrict__ T,
+                                                                const int* __restrict__ wexp,
                                                                 const int* __restrict__ EB,
                                                                 unsigned char* __restrict__ img) {
     const int nst = (Kc + TK - 1) / TK;
@@ -623,6 +630,14 @@ __global__ void __launch_bounds__(B_THREADS) table_image_kernel(int Kc, int64_t 
         const int e = gj < Nc ? EB[gj] : 1;
         double re[8], im[8];
         ld8(T + (int64_t)(2 * k + odd) * Nc + gj, 2 * Nc, gj < Nc ? kleft(Kc, k) : 0, re, im);
+        if (wexp)
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (k + i < Kc) {
+                    const double w = scalbn(1.0, wexp[k + i]);
+                    re[i] *= w;
+                    im[i] *= w;
+                }
         unsigned char* dst = img + blk * (int64_t)BBYTES + odd * BKS;
         uint4 d[S];
         planes(re, e, false, d);
@@ -673,7 +688,7 @@ int oz64_row_exps(cudaStream_t st, int64_t batch, int M, int K, const zc* A, int
     return TBG_OK;
 }
 int oz64_col_exps(cudaStream_t st, int64_t batch, int K, int64_t Nc, const zc* B, int64_t ld, int64_t sB, int* out) {
-    col_exp64_kernel<<<blocks(batch * ((Nc + 31) / 32)), 256, 0, st>>>(batch, K, Nc, B, ld, sB, out);
+    col_exp64_kernel<<<blocks(batch * ((Nc + 31) / 32)), 256, 0, st>>>(batch, K, Nc, B, ld, sB, nullptr, out);
     TBG_LAUNCHED("col_exp64_kernel");
     return TBG_OK;
 }
@@ -731,11 +746,13 @@ int oz64_gemm(cudaStream_t st, int64_t batch, int M, int Nc, int K, const Oz64Op
 size_t oz64_table_image_bytes(int Kc, int64_t Nc) {
     return (size_t)((Nc + TNC - 1) / TNC) * ((Kc + TK - 1) / TK) * BBYTES;
 }
-// Image of a table of 2 Kc rows x Nc entries and its column exponents EB (Nc).
-int oz64_table_image(cudaStream_t st, int Kc, int64_t Nc, const zc* T, int* EB, void* img) {
-    if (int rc = oz64_col_exps(st, 1, 2 * Kc, Nc, T, Nc, 0, EB)) return rc;
+// Image of a table of 2 Kc rows x Nc entries, rows 2 q and 2 q + 1 times 2^wexp[q] (when
+// given), and its column exponents EB (Nc).
+int oz64_table_image(cudaStream_t st, int Kc, int64_t Nc, const zc* T, const int* wexp, int* EB, void* img) {
+    col_exp64_kernel<<<blocks((Nc + 31) / 32), 256, 0, st>>>(1, 2 * Kc, Nc, T, Nc, 0, wexp, EB);
+    TBG_LAUNCHED("col_exp64_kernel");
     const int64_t nblk = ((Nc + TNC - 1) / TNC) * ((Kc + TK - 1) / TK);
-    table_image_kernel<<<blocks(nblk), B_THREADS, 0, st>>>(Kc, Nc, T, EB, static_cast<unsigned char*>(img));
+    table_image_kernel<<<blocks(nblk), B_THREADS, 0, st>>>(Kc, Nc, T, wexp, EB, static_cast<unsigned char*>(img));
     TBG_LAUNCHED("table_image_kernel");
     return TBG_OK;
 }

@@ -194,7 +194,8 @@ struct ModelDev {
     int* hop_pair_d = nullptr;
     zc* pair_T = nullptr;          // the paired table (2 hop_K rows, nsta^2 columns)
     bool nonfinite = false;        // the table holds NaN or Inf (found when it is paired)
-    void* oz_img = nullptr;        // digit image of pair_T for the FP64-accurate products
+    int* hop_wexp_d = nullptr;     // per pair: its weight in the FP64-accurate products, 2^w
+    void* oz_img = nullptr;        // digit image of pair_T for the FP64-accurate products, R = 0 apart
     int* oz_EB = nullptr;          // its column exponents (nsta^2)
 };
 
@@ -388,7 +389,7 @@ int oz64_gemm(cudaStream_t st, int64_t batch, int M, int Nc, int K, const Oz64Op
               int64_t ldc, int64_t sC, int mode, int* err);
 size_t oz64_table_image_bytes(int Kc, int64_t Nc);
 size_t oz64_row_image_bytes(int64_t M, int Kc);
-int oz64_table_image(cudaStream_t st, int Kc, int64_t Nc, const zc* T, int* EB, void* img);
+int oz64_table_image(cudaStream_t st, int Kc, int64_t Nc, const zc* T, const int* wexp, int* EB, void* img);
 int oz64_table_product(cudaStream_t st, int64_t M, int64_t Nc, int Kc, const zc* coef, int64_t ld, const int* EB,
                        const void* img, zc* C, int* EA, void* aimg, int* err);
 
