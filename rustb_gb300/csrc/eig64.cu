@@ -734,6 +734,10 @@ __device__ void tri_solve64(int N, const double* d, const double* e, double lam,
     }
 }
 
+// Clusters that a warp takes at once, with 4 N doubles of scratch each.
+int cluster_lanes(int N) { return (int)std::max<size_t>(1, std::min<size_t>(32, (64 * 1024) / (32 * (size_t)N))); }
+size_t cluster_smem_bytes(int N) { return sizeof(double) * (size_t)N * (3 + 4 * cluster_lanes(N)); }
+
 // Vectors that tri64 left: clusters (runs of marked neighbours) and single
 // vectors that did not converge, one lane per cluster, inverse iteration with
 // modified Gram-Schmidt against the earlier members.  One warp per matrix, or per
@@ -1010,8 +1014,8 @@ int eig64(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* s
             tri64_kernel<true><<<(unsigned)ctas, thr, smem, st>>>(N, batch, mpc, parts, len, A, E, U, status_d);
             TBG_LAUNCHED("tri64_kernel");
             if (int r = order()) return r;
-            const int G = (int)std::max<size_t>(1, std::min<size_t>(32, (64 * 1024) / (32 * (size_t)N)));
-            const size_t csm = sizeof(double) * (size_t)N * (3 + 4 * G);
+            const int G = cluster_lanes(N);
+            const size_t csm = cluster_smem_bytes(N);
             if (int r = allow_smem(tri64_cluster_kernel, csm)) return r;
             tri64_cluster_kernel<<<(unsigned)std::min<int64_t>(batch * parts, (int64_t)nsm * 32), 32, csm, st>>>(
                 N, batch, G, parts, len, A, E, U);
@@ -1061,3 +1065,40 @@ int eig64(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* s
 }
 
 }  // namespace tbg
+
+// Internal test hooks (not part of the public header).
+// Dynamic shared memory of the solver's largest CTA for n bands (the panel kernel's with one
+// CTA per matrix), bytes.
+extern "C" int64_t tbg_internal_eig64_smem(int n) {
+    using namespace tbg;
+    size_t most = std::max(cluster_smem_bytes(n), (n <= 64 ? std::max(1, 128 / n) : 1) * ((tri_smem_bytes(n) + 15) & ~size_t(15)));
+    if (n <= kWarpMax)
+        most = std::max(most, sizeof(zc) * warp_smem_elems(n) * kWarpsPerCta);
+    else
+        most = std::max(most, eig64_fits(n) ? cta_smem_bytes(n, cta_threads(n)) : panel64_smem_bytes(n, 1));
+    return (int64_t)most;
+}
+namespace {
+__global__ void fast_math_kernel(int n, const double* x, double* rcp, double* rsq) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    rcp[i] = tbg::fast_rcp(x[i]);
+    rsq[i] = tbg::fast_rsqrt(fabs(x[i]));
+}
+}  // namespace
+// fast_rcp(x) and fast_rsqrt(|x|), host arrays.
+extern "C" int tbg_internal_fast_math(int n, const double* x, double* rcp, double* rsq) {
+    using namespace tbg;
+    if (n <= 0) return TBG_OK;
+    double* d = nullptr;
+    TBG_CUDA(cudaMalloc(&d, sizeof(double) * 3 * (size_t)n));
+    cudaError_t e = cudaMemcpy(d, x, sizeof(double) * n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        fast_math_kernel<<<(n + 255) / 256, 256>>>(n, d, d + n, d + 2 * (size_t)n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(rcp, d + n, sizeof(double) * n, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(rsq, d + 2 * (size_t)n, sizeof(double) * n, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? TBG_OK : cuda_error(e, "fast_math test");
+}

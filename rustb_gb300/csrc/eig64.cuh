@@ -69,6 +69,8 @@ __device__ __forceinline__ Reflector64 reflector64_of(zc alpha, double xn, F res
     return r;
 }
 
+// Dynamic shared memory of a CTA of that reduction, C of them per matrix.
+inline size_t panel64_smem_bytes(int N, int C) { return sizeof(zc) * ((size_t)N + 2 * (((size_t)N + C - 1) / C)); }
 // Reduction by a cluster of CTAs per matrix (eig64_big.cu); a column stays in
 // shared memory (models have at most 4096 bands).
 int hetrd64_big(cudaStream_t st, int N, int64_t batch, zc* A, int* status_d);

@@ -578,9 +578,8 @@ int hetrd64_big(cudaStream_t st, int N, int64_t batch, zc* A, int* status_d) {
     cfg.numAttrs = 1;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    auto smem_of = [&](int c) { return sizeof(zc) * ((size_t)N + 2 * ((N + c - 1) / c)); };
     for (;; --C) {
-        const size_t smem = smem_of(C);
+        const size_t smem = panel64_smem_bytes(N, C);
         if (int r = allow_smem(panel64_kernel, smem)) return r;
         cfg.dynamicSmemBytes = smem;
         cfg.gridDim = dim3((unsigned)(batch * C));
