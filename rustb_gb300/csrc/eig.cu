@@ -368,6 +368,8 @@ __global__ void __launch_bounds__(MINB == 3 ? 320 : 512, MINB) heev_kernel(int N
                                                    float* __restrict__ de_out) {
     static_assert(!HYB || A_SMEM, "the hybrid layout extends the shared-memory one");
     if (!HYB) r0 = 0;
+    // the tridiagonal stage alone, from (d, e): only the three-CTA form is launched so
+    const bool tri_only = MINB == 3 && !HYB && tri_de != nullptr;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     EigShared<T> sh;
     {
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(MINB == 3 ? 320 : 512, MINB) heev_kernel(int N
             if constexpr (HYB) return (r < r0) ? Ag + doff(r) : A + (doff(r) - e0s);
             return A + doff(r);
         };
-        if (tri_de) {
+        if (tri_only) {
             // tridiagonal form given (TMEM-resident reduction): d then e
             const float* src = tri_de + (size_t)b * 2 * N;
             for (int i = tid; i < N; i += nthr) {
@@ -629,7 +631,7 @@ __global__ void __launch_bounds__(MINB == 3 ? 320 : 512, MINB) heev_kernel(int N
         if constexpr (A_SMEM) {
             // reflectors (packed rows) and tau to the back-transformation pass;
             // the matrix's shared memory then serves the eigenvector scratch
-            if (Uout && !tri_de) {
+            if (Uout && !tri_only) {
                 const size_t pe = packed_elems<true>(N);
                 cx<T>* dst = Awork + (size_t)b * (pe + N);
                 for (size_t i = tid; i < pe; i += nthr) dst[i] = (HYB && i < e0) ? Ag[i] : A[i - e0s];
