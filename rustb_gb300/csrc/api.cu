@@ -45,8 +45,9 @@ int cuda_error(cudaError_t e, const char* where) {
 void count_launch(int n) { g_launches += n; }
 
 static std::atomic<int64_t> g_scratch_cap{INT64_MAX};
+size_t scratch_cap() { return (size_t)g_scratch_cap.load(std::memory_order_relaxed); }
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
-    if ((int64_t)bytes > g_scratch_cap.load(std::memory_order_relaxed)) return cudaErrorMemoryAllocation;
+    if (bytes > scratch_cap()) return cudaErrorMemoryAllocation;
     const cudaError_t e = cudaMallocAsync(p, bytes, st);
     if (e != cudaSuccess) cudaGetLastError();
     return e;

@@ -1009,13 +1009,22 @@ __global__ void __launch_bounds__(256) gauge64_kernel(int64_t nk, int N, int npr
 // The digit image of the paired table for the tensor-core form, built once per
 // model; the caller holds g_hop_mu.  R = 0 is left to gauge64_kernel: on-site energies are often
 // a thousand times the hoppings, and the velocities, which have no such term, would
-// carry errors relative to them.  Without memory for it m.oz_img stays null.
+// carry errors relative to them.  The image is 1.8 times the hopping table and stays while
+// the model does, so it is made only while it takes at most an eighth of the free memory
+// (sets of many models); without it m.oz_img stays null and the sums take the direct form.
 int ensure_table_image(ModelDev& m, cudaStream_t st) {
     if (m.oz_img || m.nonfinite || m.hop_np == 0) return TBG_OK;
     const int64_t NN = (int64_t)m.nsta * m.nsta;
+    const size_t bytes = oz64_table_image_bytes(m.hop_np, NN);
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+        cudaGetLastError();
+        return TBG_OK;
+    }
+    if (bytes > std::min(free_b / 8, scratch_cap())) return TBG_OK;
     void* img = nullptr;
     int* eb = nullptr;
-    if (cudaMalloc(&img, oz64_table_image_bytes(m.hop_np, NN)) != cudaSuccess ||
+    if (cudaMalloc(&img, bytes) != cudaSuccess ||
         cudaMalloc(&eb, sizeof(int) * NN) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(img);

@@ -251,6 +251,7 @@ int allow_smem(K kern, size_t need) {
 // Stream-ordered allocation of scratch whose failure has a smaller form to fall back to
 // (tests lower what it grants: tbg_internal_scratch_cap).
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st);
+size_t scratch_cap();
 
 // ---------------------------------------------------------- kernel drivers --
 // Fourier sum, direct form: for nk k-points (device k, (nk, dim)), outputs

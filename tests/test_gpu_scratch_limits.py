@@ -50,6 +50,16 @@ def test_fourier_sums_without_scratch():
     assert np.max(np.abs(got - H)) <= 1e-12 * np.max(np.abs(m.ham))
 
 
+def test_no_room_for_the_tables_image():
+    k = np.random.default_rng(9).uniform(0, 1, (200, 3))
+    H, names = limited(0, lambda: W.random_model(3, 24, False, 2, seed=9).gen_ham_batch(k))
+    assert "oz64_fourier_kernel" in names
+    # 62 pairs of 576 columns take 2.1 MB, H 1.8 MB
+    got, names = limited(2000000, lambda: W.random_model(3, 24, False, 2, seed=9).gen_ham_batch(k))
+    assert "oz64_fourier_kernel" not in names
+    assert np.max(np.abs(got - H)) <= 1e-12 * np.max(np.abs(H))
+
+
 def test_product_images_in_parts():
     m = W.random_model(2, 40, False, 1, seed=7)
     k = np.random.default_rng(7).uniform(0, 1, (70, 2))
