@@ -545,7 +545,7 @@ int berry_tail(Ctx& ctx, BerryJob& J, int64_t nkc, int64_t* clusters_d) {
         rc = spin_dress(ctx.st, N, m.norb, nkc, J.spin, J.V, 2 * NN, J.scratch);
         if (rc) return rc;
     }
-    rc = eig_batched(ctx.st, N, nkc, J.H, J.E, J.U, nullptr, 0, J.status_d);
+    rc = eig_batched(ctx.st, N, nkc, J.H, J.E, J.U, J.status_d);
     if (rc) return rc;
     return berry_rotate(ctx.st, N, nkc, J.U, J.V, J.V + NN, 2 * NN, J.E, J.eta, J.Om, J.scratch, J.Met,
                         J.status_d);
@@ -598,7 +598,7 @@ struct MeshEnergies {
         TBG_LAUNCHED("kmesh_kernel");
         int rc = fourier_direct(*M, ctx.st, nkc, k_d, TBG_GAUGE_ATOM, 0, nullptr, H, nullptr, NN, 0, status_d);
         if (rc) return rc;
-        return eig_batched(ctx.st, N, nkc, H, E, nullptr, nullptr, 0, status_d);
+        return eig_batched(ctx.st, N, nkc, H, E, nullptr, status_d);
     }
 };
 
@@ -846,7 +846,7 @@ static int solve_impl(const tbg_model* m, int64_t nk, const double* k, double* E
         TBG_CUDA(cudaMemcpyAsync(k_d, k + c0 * M.dim, sizeof(double) * nkc * M.dim, cudaMemcpyHostToDevice, ctx.st));
         rc = fourier_direct(M, ctx.st, nkc, k_d, TBG_GAUGE_ATOM, 0, nullptr, H, nullptr, NN, 0, status_d);
         if (rc) return rc;
-        rc = eig_batched(ctx.st, N, nkc, H, E, U, nullptr, 0, status_d);
+        rc = eig_batched(ctx.st, N, nkc, H, E, U, status_d);
         if (rc) return rc;
         ctx.fetch_status(status_d);
         TBG_CUDA(cudaMemcpyAsync(E_out + c0 * N, E, sizeof(double) * nkc * N, cudaMemcpyDeviceToHost, ctx.st));
@@ -1471,7 +1471,7 @@ int tbg_wilson_loops(const tbg_model* m, int64_t n_loops, int64_t n_k, const dou
                 if ((rc = mixed_berry(ctx.st, N, np, Hp, nullptr, nullptr, 0.0, E, nullptr, mwork, mwb, status_d,
                                       nullptr, nullptr, U)))
                     return rc;
-            } else if ((rc = eig_batched(ctx.st, N, np, H, E, U, nullptr, 0, status_d, occ_lo, occ_hi - occ_lo + 1))) {
+            } else if ((rc = eig_batched(ctx.st, N, np, H, E, U, status_d, occ_lo, occ_hi - occ_lo + 1))) {
                 return rc;
             }
         }

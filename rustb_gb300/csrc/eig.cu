@@ -91,15 +91,6 @@ __device__ __forceinline__ void block_sum2(T& a, T& b, T* red) {
     __syncthreads();
 }
 
-__device__ __forceinline__ unsigned hash32(unsigned x) {
-    x ^= x >> 16;
-    x *= 0x7feb352dU;
-    x ^= x >> 15;
-    x *= 0x846ca68bU;
-    x ^= x >> 16;
-    return x;
-}
-
 // Number of eigenvalues of the tridiagonal (d, e2 = e^2) strictly below x.
 template <typename T>
 __device__ __forceinline__ int sturm_count(int N, const T* __restrict__ d, const T* __restrict__ e2, T x,
@@ -1500,8 +1491,7 @@ std::atomic<int>& jacobi_max_n_ref() {
 int jacobi_max_n() { return jacobi_max_n_ref().load(std::memory_order_relaxed); }
 
 // FP64 driver (plain path): A destroyed, U complex<double>.
-int eig_batched(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, void* work,
-                size_t work_bytes, int* status_d, int first, int ncol) {
+int eig_batched(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* status_d, int first, int ncol) {
     if (batch <= 0) return TBG_OK;
     if (N <= kSmallMaxN) return eig_small(st, N, batch, A, E, U, status_d);  // one thread per matrix
     if (N <= jacobi_max_n()) return eig_jacobi(st, N, batch, A, E, U, status_d);  // one warp per matrix

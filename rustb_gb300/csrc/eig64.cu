@@ -683,15 +683,6 @@ __global__ void __launch_bounds__(256) tri64_order_kernel(int N, int64_t batch, 
     }
 }
 
-__device__ __forceinline__ unsigned hash32(unsigned x) {
-    x ^= x >> 16;
-    x *= 0x7feb352dU;
-    x ^= x >> 15;
-    x *= 0x846ca68bU;
-    x ^= x >> 16;
-    return x;
-}
-
 // One inverse-iteration solve (T - lam I) y = x in place (stride G), by
 // elimination with partial pivoting; u0 (reciprocals), u1, u2 hold the rows of U.
 __device__ void tri_solve64(int N, const double* d, const double* e, double lam, double pert, double* x, double* u0,

@@ -199,6 +199,16 @@ struct ModelDev {
     int* oz_EB = nullptr;          // its column exponents (nsta^2)
 };
 
+// Start vectors of the inverse iterations (a published integer mixer).
+__device__ __forceinline__ unsigned hash32(unsigned x) {
+    x ^= x >> 16;
+    x *= 0x7feb352dU;
+    x ^= x >> 15;
+    x *= 0x846ca68bU;
+    x ^= x >> 16;
+    return x;
+}
+
 // ------------------------------------------------------------------ errors --
 int set_error(int code, const std::string& msg);
 int cuda_error(cudaError_t e, const char* where);
@@ -304,8 +314,8 @@ int fourier_mixed_packed(ModelDev& m, cudaStream_t st, bool* packed);
 // columns are then undefined).  precision: 0 = FP64, 1 = FP32 solve (U32 out, FP32 values) used by
 // the mixed path.
 size_t eig_workspace_bytes(int N, int64_t batch, int precision);
-int eig_batched(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, void* work,
-                size_t work_bytes, int* status_d, int first = 0, int ncol = -1);
+int eig_batched(cudaStream_t st, int N, int64_t batch, zc* A, double* E, zc* U, int* status_d, int first = 0,
+                int ncol = -1);
 // The FP64 solver behind it (eig64.cu): A destroyed, U may be null, nothing
 // allocated; timed = false launches the kernels without event records.
 bool eig64_fits(int N);

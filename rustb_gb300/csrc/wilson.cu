@@ -434,7 +434,7 @@ int wilson_from_vectors(cudaStream_t st, const ModelDev& m, int64_t n_loops, int
     for (int q = 0; q < 2; ++q) {
         wl_hermitian_kernel<<<nblk(n_loops * nn), 256, 0, st>>>(n_loops, n_occ, phis[q], P, Hz);
         TBG_LAUNCHED("wl_hermitian_kernel");
-        if (int rc = eig_batched(st, n_occ, n_loops, Hz, Ez, Vs[q], nullptr, 0, status_d)) return rc;
+        if (int rc = eig_batched(st, n_occ, n_loops, Hz, Ez, Vs[q], status_d)) return rc;
     }
     wl_phases_kernel<<<(unsigned)std::min<int64_t>(n_loops, 152 * 16), 128, sizeof(double) * 2 * n_occ, st>>>(
         n_loops, n_occ, P, V1, V2, out);
