@@ -125,9 +125,11 @@ int wl_overlap_oz64(cudaStream_t st, int64_t n_loops, int T, int N, int n, int f
     cudaFreeAsync(buf, st);
     return rc;
 }
-// Fewest bands (of which n_occ wanted) for which that beats one output per thread
-// from L1: 4032 overlaps of 32 of 64 bands 0.64 against 3.9 ms
-constexpr int kOverlapMinN = 32, kOverlapMinOcc = 12;
+// Whether that beats one output per thread from L1 for n_occ of N bands.  1024 overlaps, this
+// form / the other: 12 of 32 bands 0.111 / 0.097 ms, 16 of 32 0.112 / 0.134, 14 of 40 0.140 /
+// 0.147, 12 of 48 0.145 / 0.141, 12 of 64 0.149 / 0.167, 32 of 64 0.15 / 1.0, 12 of 128 0.23 / 0.37,
+// 64 of 128 0.36 / 8.2.
+constexpr bool overlap_oz64_pays(int N, int n_occ) { return N >= 32 && n_occ >= 12 && N * n_occ >= 512; }
 
 // C = A B (n x n, shared memory), all threads of the block.
 __device__ void smem_mm(int n, const zc* A, const zc* B, zc* C) {
@@ -394,7 +396,7 @@ int wilson_from_vectors(cudaStream_t st, const ModelDev& m, int64_t n_loops, int
         wl_endphase_kernel<<<nblk(n_loops * N), 256, 0, st>>>(n_loops, n_k, m.dim, kv_d, N, m.tau_d, endph);
         TBG_LAUNCHED("wl_endphase_kernel");
         KTimer kt(st, "wl_overlap_kernel");
-        if (first_occ >= 0 && N >= kOverlapMinN && n_occ >= kOverlapMinOcc) {
+        if (first_occ >= 0 && overlap_oz64_pays(N, n_occ)) {
             if (int rc = wl_overlap_oz64(st, n_loops, T, N, n_occ, first_occ, U, endph, O, status_d)) return rc;
         } else {
             wl_overlap_kernel<<<(unsigned)(n_loops * T), 256, 0, st>>>(N, n_occ, T, U, occ_d, endph, O);
