@@ -747,7 +747,6 @@ int tbg_model_destroy(tbg_model* m) {
     cudaFree(M.hop_EB);
     cudaFree(M.hop_pair_d);
     cudaFree(M.pair_T);
-    cudaFree(M.hop_wexp_d);
     cudaFree(M.oz_img);
     cudaFree(M.oz_EB);
     M.ham = nullptr;

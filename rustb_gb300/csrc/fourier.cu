@@ -743,44 +743,44 @@ int ensure_pair_table(ModelDev& m, cudaStream_t st) {
     for (int p = 0; p < np; ++p)
         if (len[p] > 0.0 && std::isfinite(len[p]))
             wexp[p] = std::min(48, std::max(0, (int)std::lround(std::log2(len[p] / shortest))));
-    int *pair_d = nullptr, *pj_d = nullptr, *wexp_d = nullptr;
+    // one block for what the device needs beside the table: the pairs' R, their weights, their
+    // -R and the flags
+    const int n1 = std::max(np, 1);
+    std::vector<int> idx((size_t)3 * n1 + 1, 0);
+    std::copy(pi.begin(), pi.end(), idx.begin());
+    std::copy(wexp.begin(), wexp.end(), idx.begin() + n1);
+    std::copy(pj.begin(), pj.end(), idx.begin() + 2 * n1);
+    int* idx_d = nullptr;
     zc* T = nullptr;
     int rc = TBG_OK;
     if (cudaMalloc(&T, sizeof(zc) * 2 * (size_t)Kc * NN) != cudaSuccess ||
-        cudaMalloc(&pair_d, sizeof(int) * std::max(np, 1)) != cudaSuccess ||
-        cudaMalloc(&wexp_d, sizeof(int) * std::max(np, 1)) != cudaSuccess ||
-        cudaMalloc(&pj_d, sizeof(int) * (std::max(np, 1) + 1)) != cudaSuccess)
+        cudaMalloc(&idx_d, sizeof(int) * idx.size()) != cudaSuccess)
         rc = set_error(TBG_E_OOM, "paired hop table");
-    int* nonfinite_d = pj_d + std::max(np, 1);
-    if (!rc && cudaMemsetAsync(nonfinite_d, 0, sizeof(int), st) != cudaSuccess)
-        rc = set_error(TBG_E_CUDA, "paired hop table flag");
-    if (!rc && np > 0 &&
-        (cudaMemcpy(pair_d, pi.data(), sizeof(int) * np, cudaMemcpyHostToDevice) != cudaSuccess ||
-         cudaMemcpy(pj_d, pj.data(), sizeof(int) * np, cudaMemcpyHostToDevice) != cudaSuccess))
+    if (!rc && cudaMemcpyAsync(idx_d, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice, st) != cudaSuccess)
         rc = set_error(TBG_E_CUDA, "paired hop table indices");
     if (!rc) {
+        int* flags_d = idx_d + 3 * n1;
         pair_table_kernel<<<(unsigned)std::min<int64_t>(((int64_t)Kc * NN + 255) / 256, 152 * 64), 256, 0, st>>>(
-            np, pair_d, pj_d, z, NN, m.ham, T, nonfinite_d);
+            np, idx_d, idx_d + 2 * n1, z, NN, m.ham, T, flags_d);
         count_launch();
-        int nf = 0;  // flags of the table
-        cudaError_t e = cudaMemcpyAsync(&nf, nonfinite_d, sizeof(int), cudaMemcpyDeviceToHost, st);
+        int flags = 0;
+        cudaError_t e = cudaMemcpyAsync(&flags, flags_d, sizeof(int), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // other streams use the table next
+        if (e == cudaSuccess && (flags & 2)) {
+            e = cudaMemsetAsync(idx_d + n1, 0, sizeof(int) * n1, st);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        }
         if (e != cudaSuccess) rc = cuda_error(e, "paired hop table");
-        m.nonfinite = (nf & 1) != 0;
-        if (nf & 2) std::fill(wexp.begin(), wexp.end(), 0);
-        if (!rc && cudaMemcpy(wexp_d, wexp.data(), sizeof(int) * wexp.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-            rc = set_error(TBG_E_CUDA, "paired hop table weights");
+        m.nonfinite = (flags & 1) != 0;
     }
-    cudaFree(pj_d);
     if (rc) {
         cudaFree(T);
-        cudaFree(pair_d);
-        cudaFree(wexp_d);
+        cudaFree(idx_d);
         return rc;
     }
-    m.hop_wexp_d = wexp_d;
+    m.hop_pair_d = idx_d;
+    m.hop_wexp_d = idx_d + n1;
     m.pair_T = T;
-    m.hop_pair_d = pair_d;
     m.hop_np = np;
     m.hop_K = Kc;
     return TBG_OK;

@@ -194,7 +194,7 @@ struct ModelDev {
     int* hop_pair_d = nullptr;
     zc* pair_T = nullptr;          // the paired table (2 hop_K rows, nsta^2 columns)
     bool nonfinite = false;        // the table holds NaN or Inf (found when it is paired)
-    int* hop_wexp_d = nullptr;     // per pair: its weight in the FP64-accurate products, 2^w
+    int* hop_wexp_d = nullptr;     // per pair (in hop_pair_d's block): its weight in the FP64-accurate products, 2^w
     void* oz_img = nullptr;        // digit image of pair_T for the FP64-accurate products, R = 0 apart
     int* oz_EB = nullptr;          // its column exponents (nsta^2)
 };
