@@ -705,6 +705,9 @@ int tbg_model_create(int dim, int spin, int64_t norb, int64_t nR, const int64_t*
     if (e == cudaSuccess) e = cudaMemcpy(M.tau_d, tau.data(), sizeof(double) * tau.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMalloc(&M.taucart_d, sizeof(double) * tc.size());
     if (e == cudaSuccess) e = cudaMemcpy(M.taucart_d, tc.data(), sizeof(double) * tc.size(), cudaMemcpyHostToDevice);
+    // a copy from pageable memory returns once it is staged, and the calls' streams do not
+    // wait for this one
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
         const int code = cuda_error(e, "tbg_model_create upload");
         tbg_model_destroy(m);
@@ -728,6 +731,7 @@ int tbg_model_set_rmatrix(tbg_model* m, int64_t n_rmat, const double* rmatrix) {
     const size_t bytes = sizeof(zc) * (size_t)n_rmat * m->d.dim * m->d.nsta * m->d.nsta;
     cudaError_t e = cudaMalloc(&m->d.rmatrix, bytes);
     if (e == cudaSuccess) e = cudaMemcpy(m->d.rmatrix, rmatrix, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // as in tbg_model_create
     if (e != cudaSuccess) return cuda_error(e, "tbg_model_set_rmatrix");
     m->d.n_rmat = n_rmat;
     return TBG_OK;

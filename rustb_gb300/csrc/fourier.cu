@@ -809,7 +809,8 @@ int build_hop_table(ModelDev& m, cudaStream_t st) {
         std::vector<int> cm((size_t)NP);
         for (int a = 0; a < N; ++a)
             for (int b = a; b < N; ++b) cm[(size_t)upper_index(N, a, b)] = a * N + b;
-        if (cudaMemcpy(colmap, cm.data(), sizeof(int) * NP, cudaMemcpyHostToDevice) != cudaSuccess)
+        if (cudaMemcpyAsync(colmap, cm.data(), sizeof(int) * NP, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess)  // cm goes
             rc = set_error(TBG_E_CUDA, "hop table column map");
     }
     if (!rc)
