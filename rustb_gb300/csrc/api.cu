@@ -81,8 +81,8 @@ void configure_pool() {
 // one after the other, a call each: 866 us a model, 313 with).  A
 // lane serves one call at a time.  Creating and destroying the stream, some fifteen
 // stream-ordered allocations and a synchronous copy per small result took half of
-// the smallest calls (Hall conductivity of 961 k-points 235 -> 101 us, gen_v at one
-// k-point 122 -> 57 us).
+// the smallest calls (Hall conductivity of 961 k-points 235 -> 90 us, gen_v at one
+// k-point 122 -> 56 us).
 struct Lane {
     int device = 0;
     cudaStream_t st = nullptr;

@@ -32,10 +32,10 @@
 // diagonal, A(j, j) = (d_j, e_j), A(j + 1, j) = tau_j, and the cluster marks
 // sit in A(N - 1, 0 ..).  Nothing is allocated.
 //
-// Eigenpairs of 1024 matrices of 128 bands 82.9 -> 20.7 ms (reduction 13.7,
-// tridiagonal 2.6, back-transformation 17.5 by single reflectors and 4.3 in
+// Eigenpairs of 1024 matrices of 128 bands 82.9 -> 21.6 ms (reduction 13.7,
+// tridiagonal 2.7, back-transformation 17.3 by single reflectors and 5.2 in
 // blocks on the tensor cores; the first two at 0.8 to 1.0 of the 1.06 TFLOP/s
-// that the FP64 pipe does), 4032 of 64 bands 77 -> 14.7,
+// that the FP64 pipe does), 4032 of 64 bands 77 -> 15.7,
 // 2304 of 26 bands 7.5 -> 1.14, against one kernel with FP64 bisection, the
 // matrix in L2 and reflectors applied by eight lanes per column.
 
@@ -932,16 +932,18 @@ int launch_bt(cudaStream_t st, int N, int64_t batch, const zc* A, zc* U, int fir
 
 // Whether the back-transformation takes the blocked form.  Its FP64 work (T) is a
 // small part of the 4 N^3 FMA of bt64, which does not go beyond 256 bands; below
-// kWYWork the launches of a block cost more than that saves, and below kWYMinN
-// bands too little of a 128-row tile is used (1024 x 128 bands 4.6 against 17.5 ms,
-// 4032 x 64 5.7 against 7.9, 200 x 64 0.49 against 0.67, 50 x 97 0.55 against 0.53,
-// 460 x 48 0.61 against 0.50)
-constexpr int kWYMinN = 56;
-constexpr double kWYWork = 1.8e8;
+// kWYWork a block of reflectors the launches cost more than that saves, and below kWYMinN
+// bands too little of a 128-row tile is used.  Blocks / single reflectors: 1000 x 56 bands
+// 1.58 / 1.31 ms, 100 x 64 0.38 / 0.40, 1000 x 64 1.83 / 2.41, 50 x 97 0.62 / 0.53, 100 x 97
+// 0.72 / 0.97, 16 and 24 x 128 0.66 / 0.70 and 0.67 / 0.81, 1024 x 128 5.2 / 17.3, 12 and
+// 100 x 160 0.86 / 0.73 and 1.4 / 4.7, 10 x 200 1.16 / 1.14, 8 x 250 1.36 / 1.65.
+constexpr int kWYMinN = 64;
+constexpr double kWYWork = 1.0e8;
 static bool use_wy(int N, int64_t batch, int ncol) {
-    // (T's part is the same for fewer columns: 32 of 64, 4032 matrices, 5.2 against 4.5 ms)
+    // (T's part is the same for fewer columns: 32 of 64 bands, 4032 matrices, 5.2 ms before the
+    // leading ones were added apart, against 4.5)
     return N > 256 || (N >= kWYMinN && (2 * ncol > N || N >= 96) &&
-                       4.0 * N * N * (double)ncol * batch >= kWYWork);
+                       4.0 * N * N * (double)ncol * batch >= kWYWork * ((N + 62) / 64));
 }
 
 // Largest matrix whose packed triangle and vectors fit one CTA's shared memory.

@@ -45,7 +45,7 @@
 // (ozaki_tc.cu).
 //
 // 1024 products of 128 bands: one of the four of the rotation 13.8 ms on the FP64
-// pipe in 64 x 64 tiles, 0.55 here (0.93 with one MMA per pair and A cut by the
+// pipe in 64 x 64 tiles, 0.53 here (0.93 with one MMA per pair and A cut by the
 // tiles' own warps).
 
 #include <cuda_bf16.h>

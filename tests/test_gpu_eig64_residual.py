@@ -12,7 +12,7 @@ from test_gpu_eig64 import eig_f64, random_hermitian
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,nk", [(64, 200), (97, 60), (128, 30), (161, 14), (170, 12), (256, 4)])
+@pytest.mark.parametrize("n,nk", [(64, 200), (97, 60), (128, 30), (161, 14), (170, 12), (170, 24), (256, 4), (256, 8)])
 def test_residual_of_blocked_reflectors(n, nk):
     H = random_hermitian(np.random.default_rng(n), nk, n)
     E, U = eig_f64(H)
