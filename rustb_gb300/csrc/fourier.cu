@@ -685,7 +685,7 @@ __global__ void phases_real_kernel(int64_t nk, int dim, const double* __restrict
         double sn, cs;
         sincos(kTwoPi * s, &sn, &cs);
         if (wexp) {
-            const double w = scalbn(1.0, -wexp[c + skip - 1]);
+            const double w = __hiloint2double((1023 - wexp[c + skip - 1]) << 20, 0);  // 2^-wexp
             cs *= w;
             sn *= w;
         }
