@@ -11,7 +11,7 @@
 // 256.  So after every 96 terms at most the levels 4 .. 1 pass what exceeds a digit
 // on to the level before them, in tensor memory and exactly (carry), and after 256
 // the sums are drained and added in FP64.  (All 256 in one go lost the last bits of
-// levels 2 to 4 when the digits were large and their products did not cancel: 10^-9 of
+// levels 2 to 4 when the digits were large and their products did not cancel: 10^-8 of
 // the scale.)  Levels 5 and 6 may lose their last place, 2^-54 of the product's scale
 // 2^(EA + EB), but only where the sum itself is some 100 times the scale.  The level sums are put
 // together as 64-bit integers (an FP64 addition costs as much as dozens of integer
